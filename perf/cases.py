@@ -463,7 +463,7 @@ def _hash64(z):
     return z ^ shifted(z, 31)
 
 
-def _samples64(rows, seed, tilt=0.08):
+def _samples64(rows, seed, tilt=float(F(0.08))):
     """The lobes of a dielectric cylinder (Marschner et al. 2003, d'Eon et al. 2011) and the dual-scattering
     back lobe (Zinke et al. 2008), 64-point Gauss-Legendre over the entry angle."""
     index = torch.arange(rows, device="cuda", dtype=torch.int64)
