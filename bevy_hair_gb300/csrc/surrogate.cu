@@ -25,9 +25,13 @@ namespace {
 
 using namespace mlp;
 
-constexpr int kGl = 64;
-__constant__ double c_gl_x[kGl];
-__constant__ double c_gl_w[kGl];
+constexpr int kGl = 64;         // quadrature order
+constexpr int kPairs = kGl / 2;  // nodes with gamma_i > 0; the others mirror them
+// Per positive node: gamma_i, weight (Jacobian cos(gamma_i) included), sin and cos of gamma_i.
+__constant__ double c_gl_x[kPairs];
+__constant__ double c_gl_w[kPairs];
+__constant__ double c_gl_sin[kPairs];
+__constant__ double c_gl_cos[kPairs];
 constexpr double kPiD = 3.14159265358979323846;
 
 // ------------------------------------------------------------ FP64 lobes
@@ -40,46 +44,91 @@ constexpr double kPiD = 3.14159265358979323846;
 //   Phi_p = 2 p gamma_t - 2 gamma_i + p pi,  A_0 = F,  A_1 = (1-F)^2 T,  A_2 = (1-F)^2 F T^2,
 // and the local back-scattering of the dual-scattering model (Zinke et al.
 // 2008, Eqs. 13-17) from the same lobes' exact forward/backward azimuthal
-// masses (wrapped-Gaussian CDF).  Longitudinal shapes follow shade.wesl:124-128.
+// masses.  Longitudinal shapes follow shade.wesl:124-128.
+//
+// The kernel is bound by the FP64 pipe (a small fraction of the FP32 rate on
+// this GPU), so the work is arranged to issue as few FP64 instructions as the
+// same quadrature allows:
+//  - the nodes are symmetric and A_p is even in gamma_i, so F, T and gamma_t
+//    are formed for 32 nodes instead of 64, from tabulated sin / cos of the
+//    nodes;
+//  - the backward mass of the wrapped Gaussian, the part of it in [-pi/2,
+//    pi/2], is even in the exit azimuth c and has the Fourier series
+//      1/2 + (2/pi) sum over odd n of (-1)^((n-1)/2) exp(-n^2 beta_n^2 / 2) / n cos(n c),
+//    whose terms fall below 3e-17 after at most 22 (beta_n >= 0.2), 10 on
+//    average.  One Clenshaw recurrence in cos(2c) per node and lobe (cos c
+//    comes from gamma_t and gamma_i by angle sums) replaces 11 error functions;
+//    the forward mass is the rest of 1;
+//  - of the three images of the wrapped density, the far one is below 4e-14
+//    of the central one and is scaled from it in float.
+// 262,144 samples: 76.2 ms with 64 nodes and the 11 error functions a node
+// and lobe, 12.9 ms so (both on 152 SMs).
 
-__device__ double fresnel_d(double c, double eta) {
-    c = fmin(fmax(c, 0.0), 1.0);
-    const double st2 = (1.0 - c * c) / (eta * eta);
-    if (st2 >= 1.0) return 1.0;
-    const double ct = sqrt(1.0 - st2);
-    const double rs = (c - eta * ct) / (c + eta * ct);
-    const double rp = (eta * c - ct) / (eta * c + ct);
-    return 0.5 * (rs * rs + rp * rp);
-}
+constexpr int kBackTerms = 22;  // odd n up to 43: n^2 beta_n^2 / 2 > 38 beyond, for beta_n >= 0.2
+constexpr double kBackCut = 38.0;
 
-__device__ double gauss_d(double b, double x) {
+__device__ __forceinline__ double gauss_d(double b, double x) {
     const double bb = fmax(b, 1e-3);
     return exp(-0.5 * x * x / (bb * bb)) / (2.5066282746310002 * bb);
 }
 
 struct NodeTerms {
-    double f, gi, gt, tr[3];
+    double gt_sin, gt_cos;  // sine and cosine of gamma_t
+    double f, tr[3];
 };
 
-// One quadrature node at gamma_i = u (h = sin u).
-__device__ __forceinline__ NodeTerms node_terms(double u, double cos_td, double eta_p, double cos_tt, double eta,
-                                                const double sa[3]) {
+// The terms of the quadrature nodes +-gamma_i (sin su, cos cu) that do not
+// depend on the sign: gamma_t for +gamma_i, Fresnel and transmittance.
+__device__ __forceinline__ NodeTerms node_terms(double su, double cu, double cos_td, double inv_eta_p,
+                                                double inv_cos_tt2, double eta, double inv_eta2, const double sa[3]) {
     NodeTerms n;
-    n.gi = u;
-    n.gt = asin(sin(u) / eta_p);
-    n.f = fresnel_d(cos_td * cos(u), eta);
-    const double path = 2.0 * cos(n.gt) / cos_tt;
+    n.gt_sin = su * inv_eta_p;
+    n.gt_cos = sqrt(1.0 - n.gt_sin * n.gt_sin);
+    const double c = fmin(fmax(cos_td * cu, 0.0), 1.0);
+    const double st2 = (1.0 - c * c) * inv_eta2;
+    if (st2 >= 1.0) {
+        n.f = 1.0;
+    } else {
+        const double ct = sqrt(1.0 - st2);
+        // 1/2 (A^2 / B^2 + C^2 / D^2) over one denominator
+        const double a = c - eta * ct, b = c + eta * ct, cc = eta * c - ct, d = eta * c + ct;
+        const double ad = a * d, bc = b * cc, bd = b * d;
+        n.f = 0.5 * (ad * ad + bc * bc) / (bd * bd);
+    }
+    const double path = n.gt_cos * inv_cos_tt2;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) n.tr[c] = exp(-sa[c] * path);
+    for (int c2 = 0; c2 < 3; ++c2) n.tr[c2] = exp(-sa[c2] * path);
     return n;
 }
 
-__device__ __forceinline__ double attenuation(const NodeTerms& n, int p, int c) {
-    const double omf2 = (1.0 - n.f) * (1.0 - n.f);
-    return p == 0 ? n.f : (p == 1 ? omf2 * n.tr[c] : omf2 * n.f * n.tr[c] * n.tr[c]);
+// Unnormalised wrapped Gaussian exp(-d^2 i) over the images d, d +- 2 pi, at
+// the angle x (any real).
+__device__ __forceinline__ double wrapped_gauss(double x, double i) {
+    const double two_pi = 2.0 * kPiD;
+    const double h = fabs(x - two_pi * rint(x * (1.0 / two_pi)));
+    double e = exp(-h * h * i);
+    const double n = two_pi - h;  // the nearer image
+    const double fall = 4.0 * kPiD * i;
+    // below 4e-18 of the central term it does not change the sum
+    const double near_ = fall * (kPiD - h) < 40.0 ? exp(-n * n * i) : 0.0;
+    e += e * (double)__expf(-(float)(fall * (kPiD + h)));  // the farther image
+    return e + near_;
 }
 
-__device__ void lobes_fp64(const float* in, double tilt, double out[12]) {
+// Sums over the L lanes that share a sample (L a power of two).
+template <int L>
+__device__ __forceinline__ double lane_sum(double v) {
+#pragma unroll
+    for (int o = 1; o < L; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// The twelve lobes of one sample on L adjacent lanes (all of the warp's lanes
+// call it; every lane of a sample gets the result).  q: this thread's column
+// of kBackTerms shared doubles, `stride` apart.
+template <int L>
+__device__ void lobes_fp64(const float* in, double tilt, double* q, int stride, double out[12]) {
+    const int sub = (int)(threadIdx.x & (L - 1));
     const double sin_i = fmin(fmax((double)in[0], -1.0), 1.0), sin_o = fmin(fmax((double)in[1], -1.0), 1.0);
     const double phi = atan2((double)in[3], (double)in[2]);
     const double sa[3] = {in[4], in[5], in[6]};
@@ -87,74 +136,101 @@ __device__ void lobes_fp64(const float* in, double tilt, double out[12]) {
     const double th_i = asin(sin_i), th_o = asin(sin_o), th_h = th_i + th_o;
     const double alpha[3] = {tilt, -0.5 * tilt, -1.5 * tilt};
     const double beta[3] = {beta_m, 0.5 * beta_m, 2.0 * beta_m};
-    const double two_pi = 2.0 * kPiD;
+    const double inv_eta2 = 1.0 / (eta * eta);
 
     // single scattering at theta_d = (theta_o - theta_i) / 2
     {
         const double td = 0.5 * (th_o - th_i);
         const double cos_td = fmax(cos(td), 1e-3), sin_td = sin(td);
-        const double eta_p = sqrt(eta * eta - sin_td * sin_td) / cos_td;
-        const double sin_tt = sin_td / eta, cos_tt = sqrt(1.0 - sin_tt * sin_tt);
+        const double inv_eta_p = cos_td / sqrt(eta * eta - sin_td * sin_td);
+        const double sin_tt = sin_td / eta, inv_cos_tt2 = 2.0 / sqrt(1.0 - sin_tt * sin_tt);
         const double inv2s2 = 0.5 / (beta_n * beta_n), norm = 1.0 / (2.5066282746310002 * beta_n);
-        double n[3][3] = {};
-        for (int i = 0; i < kGl; ++i) {
-            const NodeTerms nt = node_terms(c_gl_x[i], cos_td, eta_p, cos_tt, eta, sa);
+        double n0 = 0.0, n1[3] = {}, n2[3] = {};
+        for (int i = sub; i < kPairs; i += L) {
+            const double u = c_gl_x[i];
+            const NodeTerms nt =
+                node_terms(c_gl_sin[i], c_gl_cos[i], cos_td, inv_eta_p, inv_cos_tt2, eta, inv_eta2, sa);
+            const double gt = asin(nt.gt_sin);
+            const double w = c_gl_w[i];
+            // exit azimuths p pi +- (2 p gamma_t - 2 gamma_i) of the two nodes
+            double d[3];
 #pragma unroll
             for (int p = 0; p < 3; ++p) {
-                const double d = remainder(phi - (2.0 * p * nt.gt - 2.0 * nt.gi + p * kPiD), two_pi);
-                const double dm = d - two_pi, dp = d + two_pi;
-                const double D = norm * (exp(-d * d * inv2s2) + exp(-dp * dp * inv2s2) + exp(-dm * dm * inv2s2));
-                const double wd = c_gl_w[i] * D;
+                const double a = 2.0 * p * gt - 2.0 * u, x = phi - p * kPiD;
+                d[p] = w * (wrapped_gauss(x - a, inv2s2) + wrapped_gauss(x + a, inv2s2));
+            }
+            const double omf2 = (1.0 - nt.f) * (1.0 - nt.f);
+            n0 += d[0] * nt.f;
+            const double d1 = d[1] * omf2, d2 = d[2] * omf2 * nt.f;
 #pragma unroll
-                for (int c = 0; c < 3; ++c) n[p][c] += wd * attenuation(nt, p, c);
+            for (int c = 0; c < 3; ++c) {
+                n1[c] += d1 * nt.tr[c];
+                n2[c] += d2 * (nt.tr[c] * nt.tr[c]);
             }
         }
+        n0 = lane_sum<L>(n0);
+        const double m0 = norm * gauss_d(beta[0], th_h - alpha[0]), m1 = norm * gauss_d(beta[1], th_h - alpha[1]),
+                     m2 = norm * gauss_d(beta[2], th_h - alpha[2]);
 #pragma unroll
-        for (int p = 0; p < 3; ++p) {
-            const double m = gauss_d(beta[p], th_h - alpha[p]);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) out[3 * p + c] = m * 0.5 * n[p][c];
+        for (int c = 0; c < 3; ++c) {
+            out[c] = m0 * 0.5 * n0;
+            out[3 + c] = m1 * 0.5 * lane_sum<L>(n1[c]);
+            out[6 + c] = m2 * 0.5 * lane_sum<L>(n2[c]);
         }
     }
 
     // dual scattering at the specular cone, theta_d = theta_o (shade.wesl:444)
     const double cos_to = fmax(sqrt(fmax(1.0 - sin_o * sin_o, 1e-6)), 1e-3);
     const double sin_to = sqrt(fmax(0.0, 1.0 - cos_to * cos_to));
-    const double eta_p = sqrt(eta * eta - sin_to * sin_to) / cos_to;
-    const double sin_tt = sin_to / eta, cos_tt = sqrt(1.0 - sin_tt * sin_tt);
-    const double r = 1.0 / (beta_n * 1.4142135623730951);
-    double fwd[3][3] = {}, back[3][3] = {};
-    for (int i = 0; i < kGl; ++i) {
-        const NodeTerms nt = node_terms(c_gl_x[i], cos_to, eta_p, cos_tt, eta, sa);
+    const double inv_eta_p = cos_to / sqrt(eta * eta - sin_to * sin_to);
+    const double sin_tt = sin_to / eta, inv_cos_tt2 = 2.0 / sqrt(1.0 - sin_tt * sin_tt);
+    // coefficients of the backward mass's odd cosine series
+    const double half_b2 = 0.5 * beta_n * beta_n;
+    int terms = 0;
+    for (; terms < kBackTerms; ++terms) {
+        const double n = 2 * terms + 1;
+        if (n * n * half_b2 > kBackCut) break;
+        q[terms * stride] = (terms & 1 ? -2.0 : 2.0) / (kPiD * n) * exp(-n * n * half_b2);
+    }
+    auto back_mass = [&](double cos_c) {
+        const double x = 4.0 * cos_c * cos_c - 2.0;  // 2 cos 2c
+        double b1 = 0.0, b2 = 0.0;
+        for (int k = terms - 1; k >= 0; --k) {
+            const double b0 = fma(x, b1, q[k * stride] - b2);
+            b2 = b1;
+            b1 = b0;
+        }
+        return fma(cos_c, b1 - b2, 0.5);
+    };
+    double all0 = 0.0, all1[3] = {}, all2[3] = {}, back0 = 0.0, back1[3] = {}, back2[3] = {};
+    for (int i = sub; i < kPairs; i += L) {
+        const double su = c_gl_sin[i], cu = c_gl_cos[i];
+        const NodeTerms nt = node_terms(su, cu, cos_to, inv_eta_p, inv_cos_tt2, eta, inv_eta2, sa);
+        // cosines of 2 gamma_t p - 2 gamma_i + p pi (the mirrored node's has the same)
+        const double c2u = 1.0 - 2.0 * su * su, s2u = 2.0 * su * cu;
+        const double c2t = 1.0 - 2.0 * nt.gt_sin * nt.gt_sin, s2t = 2.0 * nt.gt_sin * nt.gt_cos;
+        const double c4t = 1.0 - 2.0 * s2t * s2t, s4t = 2.0 * s2t * c2t;
+        const double mb0 = back_mass(c2u), mb1 = back_mass(-(c2t * c2u + s2t * s2u)), mb2 = back_mass(c4t * c2u + s4t * s2u);
+        const double w = 2.0 * c_gl_w[i];
+        const double omf2 = w * (1.0 - nt.f) * (1.0 - nt.f);
+        const double wa0 = w * nt.f;
+        all0 += wa0;
+        back0 += wa0 * mb0;
 #pragma unroll
-        for (int p = 0; p < 3; ++p) {
-            // Wrapped-Gaussian masses of [-pi/2, pi/2] (back) and [pi/2, 3pi/2]
-            // (forward) about the wrapped exit azimuth: shifts -2..2 of the
-            // points pi/2 + j pi, j = -5..5.
-            const double c0 = remainder(2.0 * p * nt.gt - 2.0 * nt.gi + p * kPiD, two_pi);
-            double e[11];
-#pragma unroll
-            for (int j = 0; j < 11; ++j) e[j] = erf((0.5 * kPiD + (j - 5) * kPiD - c0) * r);
-            const double mb = 0.5 * (((e[9] - e[8]) + (e[7] - e[6])) + ((e[5] - e[4]) + (e[3] - e[2])) + (e[1] - e[0]));
-            const double mf =
-                0.5 * (((e[10] - e[9]) + (e[8] - e[7])) + ((e[6] - e[5]) + (e[4] - e[3])) + (e[2] - e[1]));
-            const double w = c_gl_w[i];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const double wa = w * attenuation(nt, p, c);
-                back[p][c] += wa * mb;
-                fwd[p][c] += wa * mf;
-            }
+        for (int c = 0; c < 3; ++c) {
+            const double wa1 = omf2 * nt.tr[c], wa2 = omf2 * nt.f * (nt.tr[c] * nt.tr[c]);
+            all1[c] += wa1;
+            all2[c] += wa2;
+            back1[c] += wa1 * mb1;
+            back2[c] += wa2 * mb2;
         }
     }
+    all0 = lane_sum<L>(all0);
+    back0 = lane_sum<L>(back0);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        double f[3], b[3];
-#pragma unroll
-        for (int p = 0; p < 3; ++p) {
-            f[p] = 0.5 * fwd[p][c];
-            b[p] = 0.5 * back[p][c];
-        }
+        const double b[3] = {0.5 * back0, 0.5 * lane_sum<L>(back1[c]), 0.5 * lane_sum<L>(back2[c])};
+        const double f[3] = {0.5 * all0 - b[0], 0.5 * lane_sum<L>(all1[c]) - b[1], 0.5 * lane_sum<L>(all2[c]) - b[2]};
         const double a_f = fmin(f[0] + f[1] + f[2], 0.95);
         const double a_b = b[0] + b[1] + b[2];
         const double b2[3] = {beta[0] * beta[0], beta[1] * beta[1], beta[2] * beta[2]};
@@ -199,9 +275,14 @@ struct SampleArgs {
 // Training distribution: sin theta_i, sin theta_o uniform in [-1, 1); phi
 // uniform in [0, pi); sigma_a log-uniform in [0.02, 8]; beta_m uniform in
 // [0.03, 0.3]; beta_n uniform in [0.2, 0.8]; eta = 1.55.
-__global__ void __launch_bounds__(128) samples_kernel(const SampleArgs a) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.n) return;
+// L lanes share a sample's quadrature nodes; a warp whose last samples lie past
+// the count evaluates the last one again and stores nothing.
+constexpr int kSampleThreads = 128;
+template <int L>
+__global__ void __launch_bounds__(kSampleThreads) samples_kernel(const SampleArgs a) {
+    __shared__ double s_q[kBackTerms][kSampleThreads];
+    const uint32_t own = (blockIdx.x * kSampleThreads + threadIdx.x) / L;
+    const uint32_t k = min(own, a.n - 1u);
     const uint64_t idx = a.first + k;
     float x[10];
     x[0] = 2.0f * unit_float(a.seed, idx, 0) - 1.0f;
@@ -215,10 +296,11 @@ __global__ void __launch_bounds__(128) samples_kernel(const SampleArgs a) {
     x[7] = 0.03f + 0.27f * unit_float(a.seed, idx, 6);
     x[8] = 0.2f + 0.6f * unit_float(a.seed, idx, 7);
     x[9] = 1.55f;
+    double out[12];
+    lobes_fp64<L>(x, a.tilt, &s_q[0][threadIdx.x], kSampleThreads, out);
+    if (own >= a.n || threadIdx.x % L != 0) return;
 #pragma unroll
     for (int i = 0; i < 10; ++i) a.inputs[(size_t)k * 10 + i] = x[i];
-    double out[12];
-    lobes_fp64(x, a.tilt, out);
 #pragma unroll
     for (int i = 0; i < 12; ++i) {
         if (a.lobes) a.lobes[(size_t)k * 12 + i] = out[i];
@@ -936,10 +1018,16 @@ cudaError_t ensure_device_setup(int device) {
     if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
     cudaError_t e = cudaSuccess;
     if (!g_gl_ready[device]) {
-        double x[kGl], w[kGl];
-        gauss_legendre(x, w);
-        e = cudaMemcpyToSymbol(c_gl_x, x, sizeof(x));
-        if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_gl_w, w, sizeof(w));
+        double x[kGl], w[kGl], s[kPairs], c[kPairs];
+        gauss_legendre(x, w);  // descending: the first half are the positive nodes
+        for (int i = 0; i < kPairs; ++i) {
+            s[i] = std::sin(x[i]);
+            c[i] = std::cos(x[i]);
+        }
+        e = cudaMemcpyToSymbol(c_gl_x, x, sizeof(s));
+        if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_gl_w, w, sizeof(s));
+        if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_gl_sin, s, sizeof(s));
+        if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_gl_cos, c, sizeof(c));
         if (e != cudaSuccess) return e;
         g_gl_ready[device] = true;
     }
@@ -1211,7 +1299,17 @@ hg_status hg_mlp_samples(hg_ctx* ctx, uint64_t seed, uint64_t first, uint32_t co
     a.inputs = inputs;
     a.targets = targets;
     a.lobes = lobes;
-    hg::samples_kernel<<<(count + 127u) / 128u, 128, 0, ctx->stream>>>(a);
+    // A lane per sample while that gives every SM a block; below, eight lanes
+    // share a sample's 32 nodes (1,000 samples: SMALL_BEFORE ms with one lane,
+    // SMALL_AFTER ms with eight; at 262,144 the per-sample work that the eight
+    // lanes repeat makes them slower).
+    if (count >= (uint32_t)ctx->sm_count * hg::kSampleThreads) {
+        const uint32_t blocks = (count + hg::kSampleThreads - 1u) / hg::kSampleThreads;
+        hg::samples_kernel<1><<<blocks, hg::kSampleThreads, 0, ctx->stream>>>(a);
+    } else {
+        const uint32_t per = hg::kSampleThreads / 8u;
+        hg::samples_kernel<8><<<(count + per - 1u) / per, hg::kSampleThreads, 0, ctx->stream>>>(a);
+    }
     MLP_CUDA(ctx, cudaGetLastError());
     return HG_OK;
 }

@@ -226,6 +226,23 @@ def test_gpu_samples_match_the_fp64_integrator(renderer):
 
 
 @gpu
+@pytest.mark.parametrize("n", [1, 15, 17, 19_455, 19_456, 19_500])
+def test_samples_at_the_edges_of_the_lane_split(renderer, n):
+    """Eight lanes a sample below sm_count x 128 samples (19,456 on 152 SMs),
+    one from there on, ragged last blocks: the integrator's lobes either way,
+    with the bounds of the test above, and nothing written past the end."""
+    torch, dev = _torch()
+    x = torch.full((n + 1, 10), 7.0, dtype=torch.float32, device=dev)
+    lob = torch.full((n + 1, 12), 7.0, dtype=torch.float64, device=dev)
+    S.samples(renderer, 4321, 5, n, x, None, lob)
+    renderer.synchronize()
+    xs, ls = x.cpu().numpy(), lob.cpu().numpy()
+    assert (xs[n] == 7.0).all() and (ls[n] == 7.0).all()
+    pick = np.unique(np.concatenate([np.arange(min(n, 200)), np.arange(max(n - 200, 0), n)]))
+    np.testing.assert_allclose(ls[pick], oracle.lobes(xs[pick], tilt=TILT), rtol=1e-10, atol=1e-14)
+
+
+@gpu
 def test_karis_lobes_kernel_matches_the_fp64_karis_fit(renderer):
     torch, dev = _torch()
     xs = _inputs(4096, 11)
