@@ -75,8 +75,7 @@ struct hg_mlp {
     void* w16 = nullptr;       // __half[n_params], parameter layout
     void* wt16 = nullptr;      // __half[13312], W2^T W3^T W4^T W5^T (4 x 64 network only)
     float* loss = nullptr;     // device scalar
-    void* scratch = nullptr;   // transposed activations and gradients, (16 + 4*64 + 4*64 + 16) x ld halves
-    uint32_t ld_capacity = 0;
+    float* part = nullptr;     // training: a partial gradient (n_params floats) per block, then their losses
     uint64_t step = 0;
 };
 

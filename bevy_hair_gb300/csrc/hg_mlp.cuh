@@ -140,34 +140,6 @@ struct WarpIo {
     float y[32][kOut + 1];
 };
 
-// One layer: acc[mt][nt] = bias + A[mt] * W^T for N = 8*NT outputs, K = 16*KT
-// inputs; bias may be null (zero).
-template <int NT, int KT, int PAD>
-__device__ __forceinline__ void layer(float acc[2][NT][4], const uint32_t a[2][KT][4], const __half (*w)[PAD],
-                                      const float* bias, int g, int t) {
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-        const float bl = bias ? bias[nt * 8 + 2 * t] : 0.0f, bh = bias ? bias[nt * 8 + 2 * t + 1] : 0.0f;
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-            acc[mt][nt][0] = bl;
-            acc[mt][nt][1] = bh;
-            acc[mt][nt][2] = bl;
-            acc[mt][nt][3] = bh;
-        }
-    }
-#pragma unroll
-    for (int kt = 0; kt < KT; ++kt) {
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            const __half* row = w[nt * 8 + g] + kt * 16 + 2 * t;
-            const uint32_t b0 = ld32(row), b1 = ld32(row + 8);
-            mma(acc[0][nt], a[0][kt], b0, b1);
-            mma(acc[1][nt], a[1][kt], b0, b1);
-        }
-    }
-}
-
 // C fragments of a 64-wide layer -> A fragments of the next (C n-tiles 2kt
 // and 2kt+1 form k-tile kt).  RELU applies max(x, 0) first.
 template <bool RELU>
@@ -247,34 +219,6 @@ __device__ __forceinline__ void output_rows(WarpIo& io, const float out[2][2][4]
     __syncwarp();
 }
 
-// Forward pass of the 32 samples held by the warp's lanes: x[] are this
-// lane's normalised inputs, y[] receives this lane's 12 network outputs
-// (transformed space).  Every lane of the warp must call it.
-__device__ __forceinline__ void forward(const FwdWeights& w, WarpIo& io, const float x[kUsedIn],
-                                        float y[kUsedOut]) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    uint32_t a0[2][1][4];
-    input_frags(io, x, a0, lane, g, t);
-    float acc[2][8][4];
-    uint32_t a[2][4][4];
-    layer<8, 1, kPadIn>(acc, a0, w.w1, w.b1, g, t);
-    c_to_a<true>(acc, a);
-    layer<8, 4, kPadHid>(acc, a, w.w2, w.b2, g, t);
-    c_to_a<true>(acc, a);
-    layer<8, 4, kPadHid>(acc, a, w.w3, w.b3, g, t);
-    c_to_a<true>(acc, a);
-    layer<8, 4, kPadHid>(acc, a, w.w4, w.b4, g, t);
-    c_to_a<true>(acc, a);
-    float out[2][2][4];
-    layer<2, 4, kPadHid>(out, a, w.w5, w.b5, g, t);
-    output_rows(io, out, y, lane, g, t);
-}
-
-// ---------------------------------------------------------------- inference path
-// The same network with the weight fragments read by ldmatrix (four B
-// fragments per instruction) and ReLU fused into the FP16 conversion; the
-// values are identical to forward().
-
 __device__ __forceinline__ void ldsm_x4(uint32_t r[4], const void* p) {
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
@@ -289,13 +233,15 @@ __device__ __forceinline__ uint32_t pack_relu(float lo, float hi) {
     return d;
 }
 
+// One layer: acc[mt][nt] = bias + A[mt] * W^T for N = 8*NT outputs, K = 16*KT
+// inputs; bias may be null (zero).  Four B fragments per ldmatrix.
 template <int NT, int KT, int PAD>
 __device__ __forceinline__ void layer_ldsm(float acc[2][NT][4], const uint32_t a[2][KT][4], const __half (*w)[PAD],
                                            const float* bias, int lane) {
     const int t = lane & 3, mat = lane >> 3, r = lane & 7;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-        const float bl = bias[nt * 8 + 2 * t], bh = bias[nt * 8 + 2 * t + 1];
+        const float bl = bias ? bias[nt * 8 + 2 * t] : 0.0f, bh = bias ? bias[nt * 8 + 2 * t + 1] : 0.0f;
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt) {
             acc[mt][nt][0] = bl;
@@ -332,6 +278,10 @@ __device__ __forceinline__ void relu_to_a(const float acc[2][8][4], uint32_t a[2
         }
 }
 
+// Forward pass of the 32 samples held by the warp's lanes: x[] are this
+// lane's normalised inputs, y[] receives this lane's 12 network outputs
+// (transformed space).  Every lane of the warp must call it.  ReLU is fused
+// into the FP16 conversion.
 __device__ __forceinline__ void forward_fast(const FwdWeights& w, WarpIo& io, const float x[kUsedIn],
                                              float y[kUsedOut]) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;

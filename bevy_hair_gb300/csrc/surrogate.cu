@@ -1,9 +1,8 @@
 // Learned shading surrogate: FP64 training samples of the hair lobes, the
-// FP16 tensor-core networks' inference and training kernels (4 x 64: forward
-// + backward per warp, split-K weight gradients, Adam; compact 2 x 32:
-// forward, backward and weight gradients per warp on mma.sync, block-summed
-// gradients, Adam), and their C entry
-// points.  The reference has no counterpart; the shading it replaces is the
+// FP16 tensor-core networks' inference and training kernels (4 x 64 and compact
+// 2 x 32: forward, backward and weight gradients of a 128-sample tile per
+// block on mma.sync, partial gradients summed by the Adam kernel), and their
+// C entry points.  The reference has no counterpart; the shading it replaces is the
 // Karis fit of shade.wesl:94-190.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -376,261 +375,6 @@ __global__ void __launch_bounds__(kWarps * 32) infer_small_kernel(const InferArg
     }
 }
 
-// Training of the compact network on the tensor cores (mma.sync m16n8k16,
-// FP16 operands, FP32 accumulation).  A warp takes 32 samples at a time:
-//  forward   the inference network itself (mlps::forward's layers), keeping
-//            the FP16 activations and the ReLU masks;
-//  backward  dY = 2 (y - target) for the three BSDF channels, then
-//            dZ2 = (dY W3) . [Z2 > 0] and dZ1 = (dZ2 W2) . [Z1 > 0], each a
-//            product with a transposed weight matrix held in shared memory;
-//  gradients dW = dZ^T A over the warp's samples, with the activations and
-//            deltas transposed to [unit][sample] in shared memory so the
-//            sample dimension is the MMAs' K; bias gradients are the row sums
-//            of the transposed deltas.
-// The deltas enter the MMAs rounded to FP16 (the usual mixed-precision
-// backward); the block sums its warps' gradients in shared memory and adds
-// them to `grad` once.  The loss is the sum over samples and the three
-// channels of (y - target)^2; the targets are formed from the twelve lobes
-// of hg_mlp_samples (mlps::bsdf_target).
-struct SmallTrainArgs {
-    const float* inputs;   // [n][10] raw
-    const float* targets;  // [n][12] transformed lobes
-    uint32_t n;
-    const __half* w16;
-    const float* params;
-    float* grad;  // += d(sum of squared errors) / d(params)
-    float* loss;  // += sum of squared errors
-};
-
-constexpr int kSmallTrainWarps = 4;
-constexpr int kSampPad = 40;  // halves per transposed row: 32 samples + 8 (conflict-free ldmatrix)
-
-// Per-warp transposes: [unit][sample].
-struct SmallStage {
-    __half x[mlps::kIn][kSampPad];
-    __half a1[mlps::kHid][kSampPad];
-    __half a2[mlps::kHid][kSampPad];
-    __half dy[mlps::kOut][kSampPad];
-    __half dz2[mlps::kHid][kSampPad];
-    __half dz1[mlps::kHid][kSampPad];
-};
-
-// Every array that ldmatrix reads starts on a 16-byte boundary (its rows are
-// multiples of 16 bytes), which the static_asserts below check.
-struct SmallTrainSmem {
-    alignas(16) mlps::Weights w;                        // forward weights (padded rows) and biases
-    alignas(16) __half w3t[mlps::kHid][mlps::kPadIn];  // W3^T: [hidden][output]
-    alignas(16) __half w2t[mlps::kHid][mlps::kPadHid]; // W2^T: [hidden 1][hidden 2]
-    float zero[mlps::kHid];
-    float grad[mlps::kParams];
-    float loss;
-    alignas(16) mlp::WarpIo io[kSmallTrainWarps];
-    alignas(16) SmallStage st[kSmallTrainWarps];
-};
-static_assert(offsetof(SmallTrainSmem, w) % 16 == 0 && offsetof(SmallTrainSmem, w3t) % 16 == 0 &&
-                  offsetof(SmallTrainSmem, w2t) % 16 == 0 && offsetof(SmallTrainSmem, st) % 16 == 0 &&
-                  offsetof(SmallTrainSmem, io) % 16 == 0,
-              "ldmatrix operands on 16-byte boundaries");
-static_assert(offsetof(mlps::Weights, w2) % 16 == 0 && offsetof(mlps::Weights, w3) % 16 == 0, "weight rows");
-static_assert(sizeof(SmallStage) % 16 == 0 && offsetof(SmallStage, a1) % 16 == 0 && offsetof(SmallStage, a2) % 16 == 0 &&
-                  offsetof(SmallStage, dy) % 16 == 0 && offsetof(SmallStage, dz2) % 16 == 0 &&
-                  offsetof(SmallStage, dz1) % 16 == 0 && (kSampPad * 2) % 16 == 0,
-              "transposed rows on 16-byte boundaries");
-static_assert((mlps::kPadIn * 2) % 16 == 0 && (mlps::kPadHid * 2) % 16 == 0, "padded weight rows");
-constexpr size_t kSmallTrainSmem = sizeof(SmallTrainSmem);
-
-// A packed FP16 pair of A fragment a[mt][kt][r] (rows = samples) into the
-// transpose dst[unit][sample].
-template <int KT>
-__device__ __forceinline__ void stage_frags(__half (*dst)[kSampPad], const uint32_t a[2][KT][4], int g, int t) {
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int kt = 0; kt < KT; ++kt)
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int unit = kt * 16 + 2 * t + ((r >> 1) ? 8 : 0);
-                const int sample = mt * 16 + g + ((r & 1) ? 8 : 0);
-                const __half2 v = *reinterpret_cast<const __half2*>(&a[mt][kt][r]);
-                dst[unit][sample] = __low2half(v);
-                dst[unit + 1][sample] = __high2half(v);
-            }
-}
-
-// C fragments of a 32-wide layer times a 32-bit mask (bit (mt*4 + nt)*4 + e)
-// -> FP16 A fragments.
-__device__ __forceinline__ void masked_to_a(const float acc[2][4][4], uint32_t mask, uint32_t a[2][2][4]) {
-    auto m = [&](int mt, int nt, int e) { return (mask >> ((mt * 4 + nt) * 4 + e)) & 1u ? acc[mt][nt][e] : 0.0f; };
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int kt = 0; kt < 2; ++kt) {
-            a[mt][kt][0] = mlp::pack_h2(m(mt, 2 * kt, 0), m(mt, 2 * kt, 1));
-            a[mt][kt][1] = mlp::pack_h2(m(mt, 2 * kt, 2), m(mt, 2 * kt, 3));
-            a[mt][kt][2] = mlp::pack_h2(m(mt, 2 * kt + 1, 0), m(mt, 2 * kt + 1, 1));
-            a[mt][kt][3] = mlp::pack_h2(m(mt, 2 * kt + 1, 2), m(mt, 2 * kt + 1, 3));
-        }
-}
-
-__device__ __forceinline__ uint32_t positive_mask(const float acc[2][4][4]) {
-    uint32_t m = 0;
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) m |= (acc[mt][nt][e] > 0.0f ? 1u : 0u) << ((mt * 4 + nt) * 4 + e);
-    return m;
-}
-
-// dW[m][n] += sum over the 32 samples of A[m][s] B[n][s] for MT 16-row tiles
-// of A (rows m0..) and NT 8-row tiles of B, both [unit][sample], added to the
-// shared gradient at grad[(m) * ld + n].
-template <int MT, int NT>
-__device__ __forceinline__ void wgrad(const __half (*A)[kSampPad], const __half (*B)[kSampPad], float* grad, int ld,
-                                      int lane) {
-    const int g = lane >> 2, t = lane & 3, mat = lane >> 3, r = lane & 7;
-    float acc[MT][NT][4];
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) acc[mt][nt][0] = acc[mt][nt][1] = acc[mt][nt][2] = acc[mt][nt][3] = 0.0f;
-#pragma unroll
-    for (int kt = 0; kt < 2; ++kt) {
-        uint32_t af[MT][4];
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-            mlp::ldsm_x4(af[mt], &A[mt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8][kt * 16 + (lane >> 4) * 8]);
-#pragma unroll
-        for (int nt = 0; nt < NT; nt += 2) {
-            uint32_t b[4];
-            mlp::ldsm_x4(b, &B[(nt + (mat >> 1)) * 8 + r][kt * 16 + (mat & 1) * 8]);
-#pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-                mlp::mma(acc[mt][nt], af[mt], b[0], b[1]);
-                mlp::mma(acc[mt][nt + 1], af[mt], b[2], b[3]);
-            }
-        }
-    }
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            const int row = mt * 16 + g, col = nt * 8 + 2 * t;
-            atomicAdd(&grad[row * ld + col], acc[mt][nt][0]);
-            atomicAdd(&grad[row * ld + col + 1], acc[mt][nt][1]);
-            atomicAdd(&grad[(row + 8) * ld + col], acc[mt][nt][2]);
-            atomicAdd(&grad[(row + 8) * ld + col + 1], acc[mt][nt][3]);
-        }
-}
-
-__global__ void __launch_bounds__(kSmallTrainWarps * 32) small_train_kernel(const SmallTrainArgs a) {
-    extern __shared__ __align__(16) unsigned char smem_small[];
-    SmallTrainSmem& S = *reinterpret_cast<SmallTrainSmem*>(smem_small);
-    const int tid = threadIdx.x, nth = blockDim.x;
-    mlps::load(S.w, a.w16, a.params, tid, nth);
-    for (int i = tid; i < mlps::kHid * mlps::kOut; i += nth) {
-        const int j = i / mlps::kOut, o = i % mlps::kOut;  // W3^T[j][o] = W3[o][j]
-        S.w3t[j][o] = a.w16[mlps::kW3 + o * mlps::kHid + j];
-    }
-    for (int i = tid; i < mlps::kHid * mlps::kHid; i += nth) {
-        const int j1 = i / mlps::kHid, j2 = i % mlps::kHid;  // W2^T[j1][j2] = W2[j2][j1]
-        S.w2t[j1][j2] = a.w16[mlps::kW2 + j2 * mlps::kHid + j1];
-    }
-    for (int i = tid; i < mlps::kHid; i += nth) S.zero[i] = 0.0f;
-    for (int i = tid; i < mlps::kParams; i += nth) S.grad[i] = 0.0f;
-    if (tid == 0) S.loss = 0.0f;
-    __syncthreads();
-    const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    mlp::WarpIo& io = S.io[warp];
-    SmallStage& st = S.st[warp];
-    float loss = 0.0f;
-    bool any = false;
-    for (uint32_t base = (blockIdx.x * kSmallTrainWarps + warp) * 32u; base < a.n;
-         base += gridDim.x * kSmallTrainWarps * 32u) {
-        any = true;
-        const uint32_t k = base + lane;
-        const bool valid = k < a.n;
-        float raw[10], xn[10];
-        load_raw(a.inputs, k, valid, raw);
-        normalise(raw, xn);
-        // forward (the inference roundings: FP16 inputs, weights and activations)
-        uint32_t a0[2][1][4];
-        mlp::input_frags(io, xn, a0, lane, g, t);
-        float acc[2][4][4];
-        uint32_t a1[2][2][4], a2[2][2][4];
-        mlp::layer_ldsm<4, 1, mlps::kPadIn>(acc, a0, S.w.w1, S.w.b1, lane);
-        const uint32_t mask1 = positive_mask(acc);
-        mlps::relu_to_a(acc, a1);
-        mlp::layer_ldsm<4, 2, mlps::kPadHid>(acc, a1, S.w.w2, S.w.b2, lane);
-        const uint32_t mask2 = positive_mask(acc);
-        mlps::relu_to_a(acc, a2);
-        float out[2][2][4];
-        mlp::layer_ldsm<2, 2, mlps::kPadHid>(out, a2, S.w.w3, S.w.b3, lane);
-        float y[mlp::kUsedOut];  // output_rows fills 12 columns; the first mlps::kUsedOut are outputs
-        mlp::output_rows(io, out, y, lane, g, t);
-        // dY of this lane's sample, as the next product's A operand
-        float dy[mlps::kUsedOut];
-#pragma unroll
-        for (int o = 0; o < mlps::kUsedOut; ++o) {
-            float d = 0.0f;
-            if (valid) {
-                float t12[12];
-#pragma unroll
-                for (int c = 0; c < 12; ++c) t12[c] = __ldg(&a.targets[(size_t)k * 12 + c]);
-                d = y[o] - mlps::bsdf_target(t12, o);
-            }
-            loss += d * d;
-            dy[o] = 2.0f * d;
-        }
-        float dyx[mlp::kUsedIn];
-#pragma unroll
-        for (int c = 0; c < mlp::kUsedIn; ++c) dyx[c] = c < mlps::kUsedOut ? dy[c] : 0.0f;
-        uint32_t ady[2][1][4];
-        mlp::input_frags(io, dyx, ady, lane, g, t);
-        // backward through the layers
-        mlp::layer_ldsm<4, 1, mlps::kPadIn>(acc, ady, S.w3t, S.zero, lane);  // dY W3
-        uint32_t dz2[2][2][4], dz1[2][2][4];
-        masked_to_a(acc, mask2, dz2);
-        mlp::layer_ldsm<4, 2, mlps::kPadHid>(acc, dz2, S.w2t, S.zero, lane);  // dZ2 W2
-        masked_to_a(acc, mask1, dz1);
-        // transposes [unit][sample]
-        stage_frags<1>(st.x, a0, g, t);
-        stage_frags<2>(st.a1, a1, g, t);
-        stage_frags<2>(st.a2, a2, g, t);
-        stage_frags<1>(st.dy, ady, g, t);
-        stage_frags<2>(st.dz2, dz2, g, t);
-        stage_frags<2>(st.dz1, dz1, g, t);
-        __syncwarp();
-        // weight gradients over the warp's samples, then bias gradients
-        wgrad<1, 4>(st.dy, st.a2, S.grad + mlps::kW3, mlps::kHid, lane);
-        wgrad<2, 4>(st.dz2, st.a1, S.grad + mlps::kW2, mlps::kHid, lane);
-        wgrad<2, 2>(st.dz1, st.x, S.grad + mlps::kW1, mlps::kIn, lane);
-        {
-            float s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
-#pragma unroll 8
-            for (int q = 0; q < 32; ++q) {
-                s1 += __half2float(st.dz1[lane][q]);
-                s2 += __half2float(st.dz2[lane][q]);
-                if (lane < mlps::kOut) s3 += __half2float(st.dy[lane][q]);
-            }
-            atomicAdd(&S.grad[mlps::kB1 + lane], s1);
-            atomicAdd(&S.grad[mlps::kB2 + lane], s2);
-            if (lane < mlps::kOut) atomicAdd(&S.grad[mlps::kB3 + lane], s3);
-        }
-        __syncwarp();
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, off);
-    if (lane == 0 && any) atomicAdd(&S.loss, loss);
-    __syncthreads();
-    for (int i = tid; i < mlps::kParams; i += nth) {
-        const float gv = S.grad[i];
-        if (gv != 0.0f) atomicAdd(&a.grad[i], gv);
-    }
-    if (tid == 0 && S.loss != 0.0f) atomicAdd(a.loss, S.loss);
-}
-
 // The same evaluation on tcgen05: four chains of two 128-row evaluations per CTA.
 __global__ void __launch_bounds__(tc::kThreads, 1) infer_tc_kernel(const InferArgs a, uint32_t* err) {
     extern __shared__ __align__(128) uint8_t smem_tc[];
@@ -671,35 +415,36 @@ __global__ void __launch_bounds__(tc::kThreads, 1) infer_tc_kernel(const InferAr
 
 // ------------------------------------------------------------ training
 
-// Per-warp transpose stage: [unit][32 samples + 8 pad].
-struct Stage {
-    __half v[kHid][40];
-};
+// stmatrix of four 8x8 FP16 matrices, each stored transposed: lane l gives the
+// address of stored row l % 8 of matrix l / 8.
+__device__ __forceinline__ void stsm_x4_trans(void* p, const uint32_t r[4]) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};\n" ::"r"(a), "r"(r[0]),
+                 "r"(r[1]), "r"(r[2]), "r"(r[3])
+                 : "memory");
+}
 
-// Write packed fragments (KT k-tiles of 16 units, rows = the warp's 32
-// samples) to dst[unit][col0 + sample] through the stage.
+__device__ __forceinline__ void ldsm_x2(uint32_t r[2], const void* p) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n" : "=r"(r[0]), "=r"(r[1]) : "r"(a));
+}
+
+constexpr int kTrainWarps = 4;
+constexpr int kTrainTile = 32 * kTrainWarps;  // samples a block takes at a time, 32 per warp
+constexpr int kTilePad = kTrainTile + 8;      // halves per transposed row (conflict-free ldmatrix and stmatrix)
+
+// Packed A fragments (KT k-tiles of 16 units, rows = the warp's 32 samples)
+// into dst[unit][col0 + sample].  Fragment register r covers units
+// (r >> 1) * 8.. and samples (r & 1) * 8.., so one transposing stmatrix stores
+// a 16 x 16 block.
 template <int KT>
-__device__ __forceinline__ void store_t(Stage& st, const uint32_t a[2][KT][4], __half* __restrict__ dst, uint32_t ld,
-                                        uint32_t col0, int lane, int g, int t) {
+__device__ __forceinline__ void store_t(__half (*dst)[kTilePad], const uint32_t a[2][KT][4], int col0, int lane) {
+    const int r = lane >> 3, i = lane & 7;
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
         for (int kt = 0; kt < KT; ++kt)
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int unit = kt * 16 + 2 * t + ((r >> 1) ? 8 : 0);
-                const int sample = mt * 16 + g + ((r & 1) ? 8 : 0);
-                const __half2 v = *reinterpret_cast<const __half2*>(&a[mt][kt][r]);
-                st.v[unit][sample] = __low2half(v);
-                st.v[unit + 1][sample] = __high2half(v);
-            }
-    __syncwarp();
-#pragma unroll
-    for (int i = lane; i < KT * 16 * 4; i += 32) {
-        const int u = i >> 2, c = (i & 3) * 8;
-        *reinterpret_cast<uint4*>(dst + (size_t)u * ld + col0 + c) = *reinterpret_cast<const uint4*>(&st.v[u][c]);
-    }
-    __syncwarp();
+            stsm_x4_trans(&dst[kt * 16 + (r >> 1) * 8 + i][col0 + mt * 16 + (r & 1) * 8], a[mt][kt]);
 }
 
 __device__ __forceinline__ void apply_mask(float acc[2][8][4], uint64_t m) {
@@ -712,205 +457,361 @@ __device__ __forceinline__ void apply_mask(float acc[2][8][4], uint64_t m) {
                 if (!((m >> ((mt * 8 + nt) * 4 + e)) & 1ull)) acc[mt][nt][e] = 0.0f;
 }
 
-struct TrainArgs {
-    const float* inputs;   // [n][10]
-    const float* targets;  // [n][12] transformed
-    uint32_t n, ld;        // samples; row length of the transposed buffers (multiple of 32, >= n)
-    const __half* w16;
-    const __half* wt16;
-    const float* params;
-    __half* xt;    // [16][ld]   layer-1 inputs
-    __half* ht;    // [4][64][ld] hidden activations h1..h4
-    __half* dzt;   // [4][64][ld] pre-activation gradients of layers 1..4
-    __half* dz5t;  // [16][ld]   output gradients
-    float* loss;   // += sum of squared errors
-};
-
-// Forward and backward of 32 samples per warp.  The loss is the sum over
-// samples and the 12 outputs of (y - target)^2, so dL/dy = 2 (y - target);
-// the 1/(n*12) of the mean is applied by the optimiser.
-__global__ void __launch_bounds__(kWarps * 32, 1) train_kernel(const TrainArgs a) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    FwdWeights& fw = *reinterpret_cast<FwdWeights*>(smem);
-    BwdWeights& bw = *reinterpret_cast<BwdWeights*>(smem + sizeof(FwdWeights));
-    WarpIo* io = reinterpret_cast<WarpIo*>(smem + sizeof(FwdWeights) + sizeof(BwdWeights));
-    Stage* stage = reinterpret_cast<Stage*>(io + kWarps);
-    load_fwd(fw, a.w16, a.params, threadIdx.x, blockDim.x);
-    load_bwd(bw, a.wt16, threadIdx.x, blockDim.x);
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const uint32_t base = (blockIdx.x * kWarps + warp) * 32u;
-    if (base >= a.n) return;
-    const uint32_t i = base + lane;
-    const bool valid = i < a.n;
-    WarpIo& w_io = io[warp];
-    Stage& st = stage[warp];
-    const size_t plane = (size_t)kHid * a.ld;
-
-    float raw[10], x[10];
-    load_raw(a.inputs, i, valid, raw);
-    normalise(raw, x);
-    uint32_t a0[2][1][4];
-    input_frags(w_io, x, a0, lane, g, t);
-    store_t<1>(st, a0, a.xt, a.ld, base, lane, g, t);
-
-    float acc[2][8][4];
-    uint32_t h[2][4][4];
-    uint64_t m1, m2, m3, m4;
-    layer<8, 1, kPadIn>(acc, a0, fw.w1, fw.b1, g, t);
-    c_to_a<true>(acc, h);
-    m1 = relu_mask(h);
-    store_t<4>(st, h, a.ht, a.ld, base, lane, g, t);
-    layer<8, 4, kPadHid>(acc, h, fw.w2, fw.b2, g, t);
-    c_to_a<true>(acc, h);
-    m2 = relu_mask(h);
-    store_t<4>(st, h, a.ht + plane, a.ld, base, lane, g, t);
-    layer<8, 4, kPadHid>(acc, h, fw.w3, fw.b3, g, t);
-    c_to_a<true>(acc, h);
-    m3 = relu_mask(h);
-    store_t<4>(st, h, a.ht + 2 * plane, a.ld, base, lane, g, t);
-    layer<8, 4, kPadHid>(acc, h, fw.w4, fw.b4, g, t);
-    c_to_a<true>(acc, h);
-    m4 = relu_mask(h);
-    store_t<4>(st, h, a.ht + 3 * plane, a.ld, base, lane, g, t);
-    float out[2][2][4];
-    layer<2, 4, kPadHid>(out, h, fw.w5, fw.b5, g, t);
-
-    // Targets into the C layout through the warp's output stage; column 16
-    // flags a real sample.
-#pragma unroll
-    for (int c = 0; c < kUsedOut; ++c) w_io.y[lane][c] = valid ? __ldg(&a.targets[(size_t)i * 12 + c]) : 0.0f;
-    w_io.y[lane][16] = valid ? 1.0f : 0.0f;
-    __syncwarp();
-    float lsum = 0.0f;
-    uint32_t d5[2][1][4];
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt) {
-        float dy[2][4];
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int r = mt * 16 + g + ((e >> 1) ? 8 : 0), c = nt * 8 + 2 * t + (e & 1);
-                float d = 0.0f;
-                if (c < kUsedOut && w_io.y[r][16] != 0.0f) d = out[mt][nt][e] - w_io.y[r][c];
-                lsum += d * d;
-                dy[nt][e] = 2.0f * d;
-            }
-        d5[mt][0][0] = pack_h2(dy[0][0], dy[0][1]);
-        d5[mt][0][1] = pack_h2(dy[0][2], dy[0][3]);
-        d5[mt][0][2] = pack_h2(dy[1][0], dy[1][1]);
-        d5[mt][0][3] = pack_h2(dy[1][2], dy[1][3]);
+// Two adjacent partial gradients: stored by the block's first tile, added to
+// by its later ones (the same thread, so in a fixed order).
+__device__ __forceinline__ void put2(float* p, float x, float y, bool add) {
+    float2 v = make_float2(x, y);
+    if (add) {
+        const float2 o = *reinterpret_cast<const float2*>(p);
+        v.x += o.x;
+        v.y += o.y;
     }
-    __syncwarp();
-    store_t<1>(st, d5, a.dz5t, a.ld, base, lane, g, t);
-
-    layer<8, 1, kPadIn>(acc, d5, bw.w5t, nullptr, g, t);
-    apply_mask(acc, m4);
-    c_to_a<false>(acc, h);
-    store_t<4>(st, h, a.dzt + 3 * plane, a.ld, base, lane, g, t);
-    layer<8, 4, kPadHid>(acc, h, bw.w4t, nullptr, g, t);
-    apply_mask(acc, m3);
-    c_to_a<false>(acc, h);
-    store_t<4>(st, h, a.dzt + 2 * plane, a.ld, base, lane, g, t);
-    layer<8, 4, kPadHid>(acc, h, bw.w3t, nullptr, g, t);
-    apply_mask(acc, m2);
-    c_to_a<false>(acc, h);
-    store_t<4>(st, h, a.dzt + plane, a.ld, base, lane, g, t);
-    layer<8, 4, kPadHid>(acc, h, bw.w2t, nullptr, g, t);
-    apply_mask(acc, m1);
-    c_to_a<false>(acc, h);
-    store_t<4>(st, h, a.dzt, a.ld, base, lane, g, t);
-
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-    if (lane == 0) atomicAdd(a.loss, lsum);
+    *reinterpret_cast<float2*>(p) = v;
 }
 
-struct WgradArgs {
-    const __half* xt;
-    const __half* ht;
-    const __half* dzt;
-    const __half* dz5t;
-    uint32_t ld, n_pad, chunk;
-    float* grad;
-};
-
-__device__ __forceinline__ uint32_t ldg32(const __half* p) { return __ldg(reinterpret_cast<const unsigned int*>(p)); }
-
-__device__ __forceinline__ float h2sum(uint32_t v) {
-    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&v));
-    return f.x + f.y;
-}
-
-// dW[m0.., n0..] += A[m][k0:k1] * B[n][k0:k1]^T (A = dZ^T, B = H^T, both
-// [unit][sample]); optional row sums of A for the bias gradient.
+// Rows m0..m0+15, columns n0..n0+8*NT-1 of dW = A B^T over a tile's samples
+// (A = dZ^T, B = H^T, both [unit][sample] in shared memory) into the block's
+// partial gradient gw (row length n_cols); with gb, also the row sums of A
+// (the bias gradient), as a product with ones.  One warp.
 template <int NT>
-__device__ __forceinline__ void wgrad_tile(const __half* __restrict__ A, const __half* __restrict__ B, uint32_t ld,
-                                           int m0, int n0, uint32_t k0, uint32_t k1, float* gw, int n_cols, float* gb,
-                                           int g, int t) {
-    float acc[NT][4] = {};
-    float s0 = 0.0f, s1 = 0.0f;
-    const __half* r0 = A + (size_t)(m0 + g) * ld + 2 * t;
-    const __half* r1 = A + (size_t)(m0 + g + 8) * ld + 2 * t;
-#pragma unroll 2
-    for (uint32_t k = k0; k < k1; k += 16) {
-        const uint32_t af[4] = {ldg32(r0 + k), ldg32(r1 + k), ldg32(r0 + k + 8), ldg32(r1 + k + 8)};
-        if (gb) {
-            s0 += h2sum(af[0]) + h2sum(af[2]);
-            s1 += h2sum(af[1]) + h2sum(af[3]);
-        }
+__device__ __forceinline__ void wgrad_tile(const __half (*A)[kTilePad], const __half (*B)[kTilePad], int m0, int n0,
+                                           float* gw, int n_cols, float* gb, bool add, int lane) {
+    const int g = lane >> 2, t = lane & 3, mat = lane >> 3, r = lane & 7;
+    float acc[NT][4] = {}, sum[4] = {};
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            const __half* br = B + (size_t)(n0 + nt * 8 + g) * ld + k + 2 * t;
-            mma(acc[nt], af, ldg32(br), ldg32(br + 8));
+    for (int k = 0; k < kTrainTile; k += 16) {
+        uint32_t af[4];
+        ldsm_x4(af, &A[m0 + r + (mat & 1) * 8][k + (mat >> 1) * 8]);
+        if (gb) mma(sum, af, 0x3C003C00u, 0x3C003C00u);
+#pragma unroll
+        for (int nt = 0; nt + 1 < NT; nt += 2) {
+            uint32_t b[4];
+            ldsm_x4(b, &B[n0 + (nt + (mat >> 1)) * 8 + r][k + (mat & 1) * 8]);
+            mma(acc[nt], af, b[0], b[1]);
+            mma(acc[nt + 1], af, b[2], b[3]);
+        }
+        if (NT & 1) {
+            uint32_t b[2];
+            ldsm_x2(b, &B[n0 + (NT - 1) * 8 + r][k + (mat & 1) * 8]);
+            mma(acc[NT - 1], af, b[0], b[1]);
         }
     }
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-        const int c = n0 + nt * 8 + 2 * t;
-        atomicAdd(gw + (m0 + g) * n_cols + c, acc[nt][0]);
-        atomicAdd(gw + (m0 + g) * n_cols + c + 1, acc[nt][1]);
-        atomicAdd(gw + (m0 + g + 8) * n_cols + c, acc[nt][2]);
-        atomicAdd(gw + (m0 + g + 8) * n_cols + c + 1, acc[nt][3]);
+        float* p = gw + (m0 + g) * n_cols + n0 + nt * 8 + 2 * t;
+        put2(p, acc[nt][0], acc[nt][1], add);
+        put2(p + 8 * n_cols, acc[nt][2], acc[nt][3], add);
     }
-    if (gb) {
-        s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
-        s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
-        s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
-        s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
-        if (t == 0) {
-            atomicAdd(gb + m0 + g, s0);
-            atomicAdd(gb + m0 + g + 8, s1);
-        }
+    if (gb && t == 0) {
+        gb[m0 + g] = sum[0] + (add ? gb[m0 + g] : 0.0f);
+        gb[m0 + g + 8] = sum[2] + (add ? gb[m0 + g + 8] : 0.0f);
     }
 }
 
-// grid (chunks, 5 layers), 4 warps.
-__global__ void __launch_bounds__(128) wgrad_kernel(const WgradArgs a) {
-    const int layer = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const uint32_t k0 = blockIdx.x * a.chunk;
-    const uint32_t k1 = min(k0 + a.chunk, a.n_pad);
-    if (k0 >= k1) return;
-    const size_t plane = (size_t)kHid * a.ld;
-    switch (layer) {
-        case 0:
-            wgrad_tile<2>(a.dzt, a.xt, a.ld, 16 * warp, 0, k0, k1, a.grad + kW1, kIn, a.grad + kB1, g, t);
-            break;
-        case 1:
-        case 2:
-        case 3: {
-            const int wofs = layer == 1 ? kW2 : (layer == 2 ? kW3 : kW4);
-            const int bofs = layer == 1 ? kB2 : (layer == 2 ? kB3 : kB4);
-            wgrad_tile<8>(a.dzt + layer * plane, a.ht + (layer - 1) * plane, a.ld, 16 * warp, 0, k0, k1,
-                          a.grad + wofs, kHid, a.grad + bofs, g, t);
-            break;
+struct TrainArgs {
+    const float* inputs;   // [n][10]
+    const float* targets;  // [n][12] transformed
+    uint32_t n;
+    const __half* w16;
+    const __half* wt16;    // transposed copies (4 x 64 network only)
+    const float* params;
+    float* part;  // [blocks][parameters] partial gradients, written whole
+    float* loss_part;  // [blocks] partial sums of squared errors
+};
+
+struct TrainSmem {
+    FwdWeights fw;
+    BwdWeights bw;
+    __half x[kIn][kTilePad];          // layer-1 inputs, [unit][sample]
+    __half h[4][kHid][kTilePad];      // hidden activations h1..h4
+    __half dz[4][kHid][kTilePad];     // pre-activation gradients of layers 1..4
+    __half dz5[kOut][kTilePad];       // output gradients
+    WarpIo io[kTrainWarps];
+    float loss[kTrainWarps];
+};
+static_assert(sizeof(FwdWeights) % 16 == 0 && sizeof(BwdWeights) % 16 == 0 && (kTilePad * 2) % 16 == 0 &&
+                  offsetof(TrainSmem, x) % 16 == 0 && offsetof(TrainSmem, io) % 16 == 0,
+              "ldmatrix rows on 16-byte boundaries");
+static_assert(sizeof(TrainSmem) <= 227 * 1024, "train kernel shared memory");
+
+// One training batch: forward, backward and weight gradients of 128-sample
+// tiles, everything between the batch's rows and the block's partial gradient
+// in registers and shared memory.  Each warp runs 32 samples forward and
+// backward on mma.sync and leaves its activations and deltas transposed in
+// shared memory; then the block's warps share the weight-gradient products
+// over the tile's 128 samples (warp w takes 16 rows of each dW).  Partial
+// gradients go to the block's own slice with plain stores and the optimiser
+// sums the slices, so nothing is zeroed, no atomics contend and the result
+// does not depend on the blocks' order.  The loss is the sum over samples and
+// the 12 outputs of (y - target)^2, so dL/dy = 2 (y - target); the 1/(n*12)
+// of the mean is applied by the optimiser.
+//
+// Bound by latency and shared-memory traffic: at a batch of 16,384 an SM holds
+// one tile.  Before, the activations went through memory (17 MB) to a second
+// kernel whose 40 blocks summed dW serially: 157 us a step of 16,384 samples;
+// 23.4 us now (152 SMs).
+__global__ void __launch_bounds__(kTrainTile, 1) train_kernel(const TrainArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    load_fwd(S.fw, a.w16, a.params, threadIdx.x, blockDim.x);
+    load_bwd(S.bw, a.wt16, threadIdx.x, blockDim.x);
+    __syncthreads();
+    WarpIo& w_io = S.io[warp];
+    const int col0 = 32 * warp;
+    float* part = a.part + (size_t)blockIdx.x * kParams;
+    float lsum = 0.0f;
+    bool add = false;
+    for (uint32_t base = blockIdx.x * kTrainTile; base < a.n; base += gridDim.x * kTrainTile) {
+        const uint32_t i = base + threadIdx.x;
+        const bool valid = i < a.n;
+        // the targets are read up front: they are needed only after the forward pass
+        float tgt[kUsedOut];
+#pragma unroll
+        for (int c = 0; c < kUsedOut; ++c) tgt[c] = valid ? __ldg(&a.targets[(size_t)i * 12 + c]) : 0.0f;
+        float raw[10], x[10];
+        load_raw(a.inputs, i, valid, raw);
+        normalise(raw, x);
+        uint32_t a0[2][1][4];
+        input_frags(w_io, x, a0, lane, g, t);
+        store_t<1>(S.x, a0, col0, lane);
+
+        float acc[2][8][4];
+        uint32_t h[2][4][4];
+        uint64_t m1, m2, m3, m4;
+        layer_ldsm<8, 1, kPadIn>(acc, a0, S.fw.w1, S.fw.b1, lane);
+        c_to_a<true>(acc, h);
+        m1 = relu_mask(h);
+        store_t<4>(S.h[0], h, col0, lane);
+        layer_ldsm<8, 4, kPadHid>(acc, h, S.fw.w2, S.fw.b2, lane);
+        c_to_a<true>(acc, h);
+        m2 = relu_mask(h);
+        store_t<4>(S.h[1], h, col0, lane);
+        layer_ldsm<8, 4, kPadHid>(acc, h, S.fw.w3, S.fw.b3, lane);
+        c_to_a<true>(acc, h);
+        m3 = relu_mask(h);
+        store_t<4>(S.h[2], h, col0, lane);
+        layer_ldsm<8, 4, kPadHid>(acc, h, S.fw.w4, S.fw.b4, lane);
+        c_to_a<true>(acc, h);
+        m4 = relu_mask(h);
+        store_t<4>(S.h[3], h, col0, lane);
+        float out[2][2][4];
+        layer_ldsm<2, 4, kPadHid>(out, h, S.fw.w5, S.fw.b5, lane);
+
+        // Targets into the C layout through the warp's output stage; column 16
+        // flags a real sample.
+#pragma unroll
+        for (int c = 0; c < kUsedOut; ++c) w_io.y[lane][c] = tgt[c];
+        w_io.y[lane][16] = valid ? 1.0f : 0.0f;
+        __syncwarp();
+        uint32_t d5[2][1][4];
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+            float dy[2][4];
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int r = mt * 16 + g + ((e >> 1) ? 8 : 0), c = nt * 8 + 2 * t + (e & 1);
+                    float d = 0.0f;
+                    if (c < kUsedOut && w_io.y[r][16] != 0.0f) d = out[mt][nt][e] - w_io.y[r][c];
+                    lsum += d * d;
+                    dy[nt][e] = 2.0f * d;
+                }
+            d5[mt][0][0] = pack_h2(dy[0][0], dy[0][1]);
+            d5[mt][0][1] = pack_h2(dy[0][2], dy[0][3]);
+            d5[mt][0][2] = pack_h2(dy[1][0], dy[1][1]);
+            d5[mt][0][3] = pack_h2(dy[1][2], dy[1][3]);
         }
-        default:
-            wgrad_tile<2>(a.dz5t, a.ht + 3 * plane, a.ld, 0, 16 * warp, k0, k1, a.grad + kW5, kHid,
-                          warp == 0 ? a.grad + kB5 : nullptr, g, t);
-            break;
+        __syncwarp();
+        store_t<1>(S.dz5, d5, col0, lane);
+
+        layer_ldsm<8, 1, kPadIn>(acc, d5, S.bw.w5t, nullptr, lane);
+        apply_mask(acc, m4);
+        c_to_a<false>(acc, h);
+        store_t<4>(S.dz[3], h, col0, lane);
+        layer_ldsm<8, 4, kPadHid>(acc, h, S.bw.w4t, nullptr, lane);
+        apply_mask(acc, m3);
+        c_to_a<false>(acc, h);
+        store_t<4>(S.dz[2], h, col0, lane);
+        layer_ldsm<8, 4, kPadHid>(acc, h, S.bw.w3t, nullptr, lane);
+        apply_mask(acc, m2);
+        c_to_a<false>(acc, h);
+        store_t<4>(S.dz[1], h, col0, lane);
+        layer_ldsm<8, 4, kPadHid>(acc, h, S.bw.w2t, nullptr, lane);
+        apply_mask(acc, m1);
+        c_to_a<false>(acc, h);
+        store_t<4>(S.dz[0], h, col0, lane);
+        __syncthreads();
+
+        wgrad_tile<8>(S.dz[3], S.h[2], 16 * warp, 0, part + kW4, kHid, part + kB4, add, lane);
+        wgrad_tile<8>(S.dz[2], S.h[1], 16 * warp, 0, part + kW3, kHid, part + kB3, add, lane);
+        wgrad_tile<8>(S.dz[1], S.h[0], 16 * warp, 0, part + kW2, kHid, part + kB2, add, lane);
+        wgrad_tile<2>(S.dz[0], S.x, 16 * warp, 0, part + kW1, kIn, part + kB1, add, lane);
+        wgrad_tile<2>(S.dz5, S.h[3], 0, 16 * warp, part + kW5, kHid, warp == 0 ? part + kB5 : nullptr, add, lane);
+        add = true;
+        __syncthreads();  // the next tile overwrites what the products read
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+    if (lane == 0) S.loss[warp] = lsum;
+    __syncthreads();
+    if (threadIdx.x == 0) a.loss_part[blockIdx.x] = (S.loss[0] + S.loss[1]) + (S.loss[2] + S.loss[3]);
+}
+
+// Training of the compact network on the tensor cores (mma.sync m16n8k16,
+// FP16 operands, FP32 accumulation).  A warp takes 32 samples at a time:
+//  forward   the inference network itself (mlps::forward's layers), keeping
+//            the FP16 activations and the ReLU masks;
+//  backward  dY = 2 (y - target) for the three BSDF channels, then
+//            dZ2 = (dY W3) . [Z2 > 0] and dZ1 = (dZ2 W2) . [Z1 > 0], each a
+//            product with a transposed weight matrix held in shared memory;
+//  gradients dW = dZ^T A over the block's 128 samples, with the activations
+//            and deltas transposed to [unit][sample] in shared memory so the
+//            sample dimension is the MMAs' K and the warps share the output
+//            tiles; bias gradients are products with ones.
+// The deltas enter the MMAs rounded to FP16 (the usual mixed-precision
+// backward).  Partial gradients go to the block's own slice, as in
+// train_kernel.  The loss is the sum over samples and the three channels of
+// (y - target)^2; the targets are formed from the twelve lobes of
+// hg_mlp_samples (mlps::bsdf_target).
+//
+// Bound by latency (a batch of 16,384 is one tile per block, on 128 blocks).
+// Before, each warp added its 2,128 sums to shared memory and each block to
+// global memory by atomics, with a loss copy and a memset after every step:
+// 25.5 us a step of 16,384 samples; SMALL_23.4 us now.
+struct SmallTrainSmem {
+    alignas(16) mlps::Weights w;                       // forward weights (padded rows) and biases
+    alignas(16) __half w3t[mlps::kHid][mlps::kPadIn];  // W3^T: [hidden][output]
+    alignas(16) __half w2t[mlps::kHid][mlps::kPadHid]; // W2^T: [hidden 1][hidden 2]
+    // [unit][sample]
+    alignas(16) __half x[mlps::kIn][kTilePad];
+    __half a1[mlps::kHid][kTilePad];
+    __half a2[mlps::kHid][kTilePad];
+    __half dy[mlps::kOut][kTilePad];
+    __half dz2[mlps::kHid][kTilePad];
+    __half dz1[mlps::kHid][kTilePad];
+    alignas(16) mlp::WarpIo io[kTrainWarps];
+    float loss[kTrainWarps];
+};
+static_assert(offsetof(SmallTrainSmem, w) % 16 == 0 && offsetof(SmallTrainSmem, w3t) % 16 == 0 &&
+                  offsetof(SmallTrainSmem, w2t) % 16 == 0 && offsetof(SmallTrainSmem, x) % 16 == 0 &&
+                  offsetof(SmallTrainSmem, io) % 16 == 0,
+              "ldmatrix operands on 16-byte boundaries");
+static_assert(offsetof(mlps::Weights, w2) % 16 == 0 && offsetof(mlps::Weights, w3) % 16 == 0, "weight rows");
+static_assert((mlps::kPadIn * 2) % 16 == 0 && (mlps::kPadHid * 2) % 16 == 0, "padded weight rows");
+constexpr size_t kSmallTrainSmem = sizeof(SmallTrainSmem);
+
+// C fragments of a 32-wide layer times a 32-bit mask (bit (mt*4 + nt)*4 + e)
+// -> FP16 A fragments.
+__device__ __forceinline__ void masked_to_a(const float acc[2][4][4], uint32_t mask, uint32_t a[2][2][4]) {
+    auto m = [&](int mt, int nt, int e) { return (mask >> ((mt * 4 + nt) * 4 + e)) & 1u ? acc[mt][nt][e] : 0.0f; };
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int kt = 0; kt < 2; ++kt) {
+            a[mt][kt][0] = mlp::pack_h2(m(mt, 2 * kt, 0), m(mt, 2 * kt, 1));
+            a[mt][kt][1] = mlp::pack_h2(m(mt, 2 * kt, 2), m(mt, 2 * kt, 3));
+            a[mt][kt][2] = mlp::pack_h2(m(mt, 2 * kt + 1, 0), m(mt, 2 * kt + 1, 1));
+            a[mt][kt][3] = mlp::pack_h2(m(mt, 2 * kt + 1, 2), m(mt, 2 * kt + 1, 3));
+        }
+}
+
+__device__ __forceinline__ uint32_t positive_mask(const float acc[2][4][4]) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) m |= (acc[mt][nt][e] > 0.0f ? 1u : 0u) << ((mt * 4 + nt) * 4 + e);
+    return m;
+}
+
+__global__ void __launch_bounds__(kTrainTile) small_train_kernel(const TrainArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_small[];
+    SmallTrainSmem& S = *reinterpret_cast<SmallTrainSmem*>(smem_small);
+    const int tid = threadIdx.x, nth = blockDim.x;
+    mlps::load(S.w, a.w16, a.params, tid, nth);
+    for (int i = tid; i < mlps::kHid * mlps::kOut; i += nth) {
+        const int j = i / mlps::kOut, o = i % mlps::kOut;  // W3^T[j][o] = W3[o][j]
+        S.w3t[j][o] = a.w16[mlps::kW3 + o * mlps::kHid + j];
+    }
+    for (int i = tid; i < mlps::kHid * mlps::kHid; i += nth) {
+        const int j1 = i / mlps::kHid, j2 = i % mlps::kHid;  // W2^T[j1][j2] = W2[j2][j1]
+        S.w2t[j1][j2] = a.w16[mlps::kW2 + j2 * mlps::kHid + j1];
+    }
+    __syncthreads();
+    const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    mlp::WarpIo& io = S.io[warp];
+    const int col0 = 32 * warp;
+    float* part = a.part + (size_t)blockIdx.x * mlps::kParams;
+    float loss = 0.0f;
+    bool add = false;
+    for (uint32_t base = blockIdx.x * kTrainTile; base < a.n; base += gridDim.x * kTrainTile) {
+        const uint32_t k = base + tid;
+        const bool valid = k < a.n;
+        // the targets are read up front: they are needed only after the forward pass
+        float t12[12];
+#pragma unroll
+        for (int c = 0; c < 12; ++c) t12[c] = valid ? __ldg(&a.targets[(size_t)k * 12 + c]) : 0.0f;
+        float raw[10], xn[10];
+        load_raw(a.inputs, k, valid, raw);
+        normalise(raw, xn);
+        // forward (the inference roundings: FP16 inputs, weights and activations)
+        uint32_t a0[2][1][4];
+        mlp::input_frags(io, xn, a0, lane, g, t);
+        float acc[2][4][4];
+        uint32_t a1[2][2][4], a2[2][2][4];
+        mlp::layer_ldsm<4, 1, mlps::kPadIn>(acc, a0, S.w.w1, S.w.b1, lane);
+        const uint32_t mask1 = positive_mask(acc);
+        mlps::relu_to_a(acc, a1);
+        mlp::layer_ldsm<4, 2, mlps::kPadHid>(acc, a1, S.w.w2, S.w.b2, lane);
+        const uint32_t mask2 = positive_mask(acc);
+        mlps::relu_to_a(acc, a2);
+        float out[2][2][4];
+        mlp::layer_ldsm<2, 2, mlps::kPadHid>(out, a2, S.w.w3, S.w.b3, lane);
+        float y[mlp::kUsedOut];  // output_rows fills 12 columns; the first mlps::kUsedOut are outputs
+        mlp::output_rows(io, out, y, lane, g, t);
+        store_t<1>(S.x, a0, col0, lane);
+        store_t<2>(S.a1, a1, col0, lane);
+        store_t<2>(S.a2, a2, col0, lane);
+        // dY of this lane's sample, as the next product's A operand
+        float dyx[mlp::kUsedIn] = {};
+#pragma unroll
+        for (int o = 0; o < mlps::kUsedOut; ++o) {
+            const float d = valid ? y[o] - mlps::bsdf_target(t12, o) : 0.0f;
+            loss += d * d;
+            dyx[o] = 2.0f * d;
+        }
+        uint32_t ady[2][1][4];
+        mlp::input_frags(io, dyx, ady, lane, g, t);
+        // backward through the layers
+        mlp::layer_ldsm<4, 1, mlps::kPadIn>(acc, ady, S.w3t, nullptr, lane);  // dY W3
+        uint32_t dz2[2][2][4], dz1[2][2][4];
+        masked_to_a(acc, mask2, dz2);
+        mlp::layer_ldsm<4, 2, mlps::kPadHid>(acc, dz2, S.w2t, nullptr, lane);  // dZ2 W2
+        masked_to_a(acc, mask1, dz1);
+        store_t<1>(S.dy, ady, col0, lane);
+        store_t<2>(S.dz2, dz2, col0, lane);
+        store_t<2>(S.dz1, dz1, col0, lane);
+        __syncthreads();
+        // warp w: rows 16 (w / 2).. and half the columns of dW2, dW1; 8 columns of dW3
+        const int m0 = 16 * (warp >> 1), half = warp & 1;
+        wgrad_tile<2>(S.dz2, S.a1, m0, 16 * half, part + mlps::kW2, mlps::kHid, half ? nullptr : part + mlps::kB2, add,
+                      lane);
+        wgrad_tile<1>(S.dz1, S.x, m0, 8 * half, part + mlps::kW1, mlps::kIn, half ? part + mlps::kB1 : nullptr, add,
+                      lane);
+        wgrad_tile<1>(S.dy, S.a2, 0, 8 * warp, part + mlps::kW3, mlps::kHid, warp == 0 ? part + mlps::kB3 : nullptr,
+                      add, lane);
+        add = true;
+        __syncthreads();  // the next tile overwrites what the products read
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, off);
+    if (lane == 0) S.loss[warp] = loss;
+    __syncthreads();
+    if (tid == 0) a.loss_part[blockIdx.x] = (S.loss[0] + S.loss[1]) + (S.loss[2] + S.loss[3]);
 }
 
 struct AdamArgs {
@@ -920,28 +821,59 @@ struct AdamArgs {
     float* grad;
     __half* w16;
     __half* wt16;
+    const float* part;       // [blocks][parameters] partial gradients, or null (conversion only)
+    const float* loss_part;  // [blocks]
+    uint32_t blocks;
+    float* loss;             // the batch's sum of squared errors, nullable
     float lr_t, beta1, beta2, eps_t, gscale;
-    int update;
+    int update;              // 1: Adam step; 0: the summed gradient into grad, parameters as they are
 };
 
-// Adam (Kingma and Ba 2015) with the bias corrections folded into lr_t and
-// eps_t; then the FP16 forward and transposed copies.
-__global__ void adam_kernel(const AdamArgs a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kParams) return;
+constexpr int kAdamParams = 64, kAdamSplit = 4;  // parameters per block, threads that share one's slices
+
+// The sum over the blocks' partial gradients, then Adam (Kingma and Ba 2015)
+// with the bias corrections folded into lr_t and eps_t, then the FP16 forward
+// (and, for the 4 x 64 network, transposed) copies.  Four threads share a
+// parameter's slices (7.5 MB for 128 blocks of the 4 x 64 network, in L2) and
+// add up in a fixed order.
+template <int N, bool TRANSPOSED>
+__global__ void __launch_bounds__(kAdamParams* kAdamSplit) adam_kernel(const AdamArgs a) {
+    __shared__ float s_sum[kAdamSplit][kAdamParams];
+    const int q = threadIdx.x % kAdamParams, split = threadIdx.x / kAdamParams;
+    const int i = blockIdx.x * kAdamParams + q;
+    float gr = 0.0f;
+    if (a.part && i < N) {
+#pragma unroll 8
+        for (uint32_t b = split; b < a.blocks; b += kAdamSplit) gr += __ldcg(&a.part[(size_t)b * N + i]);
+    }
+    s_sum[split][q] = gr;
+    if (a.loss && blockIdx.x == 0 && threadIdx.x < 32) {
+        float l = 0.0f;
+        for (uint32_t b = threadIdx.x; b < a.blocks; b += 32) l += __ldcg(&a.loss_part[b]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+        if (threadIdx.x == 0) *a.loss = l;
+    }
+    __syncthreads();
+    if (split != 0 || i >= N) return;
+    gr = (s_sum[0][q] + s_sum[1][q]) + (s_sum[2][q] + s_sum[3][q]);
+    if (a.part && !a.update) {
+        a.grad[i] = gr;
+        return;
+    }
     float p = a.params[i];
     if (a.update) {
-        const float gr = a.grad[i] * a.gscale;
+        gr *= a.gscale;
         const float m = a.beta1 * a.m[i] + (1.0f - a.beta1) * gr;
         const float v = a.beta2 * a.v[i] + (1.0f - a.beta2) * gr * gr;
         a.m[i] = m;
         a.v[i] = v;
         p -= a.lr_t * m / (sqrtf(v) + a.eps_t);
         a.params[i] = p;
-        a.grad[i] = 0.0f;
     }
     const __half hp = __float2half_rn(p);
     a.w16[i] = hp;
+    if (!TRANSPOSED) return;
     int tofs = -1, rows = 0, cols = kHid, rel = 0;
     if (i >= kW2 && i < kB2) tofs = kT2, rows = kHid, rel = i - kW2;
     else if (i >= kW3 && i < kB3) tofs = kT3, rows = kHid, rel = i - kW3;
@@ -953,29 +885,10 @@ __global__ void adam_kernel(const AdamArgs a) {
     }
 }
 
-// Adam for the compact network (no transposed copies).
-__global__ void adam_small_kernel(const AdamArgs a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= mlps::kParams) return;
-    float p = a.params[i];
-    if (a.update) {
-        const float gr = a.grad[i] * a.gscale;
-        const float m = a.beta1 * a.m[i] + (1.0f - a.beta1) * gr;
-        const float v = a.beta2 * a.v[i] + (1.0f - a.beta2) * gr * gr;
-        a.m[i] = m;
-        a.v[i] = v;
-        p -= a.lr_t * m / (sqrtf(v) + a.eps_t);
-        a.params[i] = p;
-        a.grad[i] = 0.0f;
-    }
-    a.w16[i] = __float2half_rn(p);
-}
-
 // ------------------------------------------------------------ host side
 
 constexpr size_t kFwdSmem = sizeof(FwdWeights) + kWarps * sizeof(WarpIo);
-constexpr size_t kTrainSmem = sizeof(FwdWeights) + sizeof(BwdWeights) + kWarps * (sizeof(WarpIo) + sizeof(Stage));
-static_assert(kTrainSmem <= 227 * 1024, "train kernel shared memory");
+constexpr size_t kTrainSmem = sizeof(TrainSmem);
 
 std::mutex g_init_mutex;
 bool g_gl_ready[64] = {};
@@ -1063,7 +976,21 @@ hg_status cuda_fail(hg_ctx* ctx, cudaError_t e, const char* where) {
         if (e_ != cudaSuccess) return cuda_fail(ctx, e_, #expr); \
     } while (0)
 
-cudaError_t convert(hg_mlp* m, int update, float lr_t, float eps_t, float gscale) {
+// Most blocks a training launch uses: one (the 4 x 64 network, whose tile
+// fills an SM's shared memory) or two per SM; a block with several tiles adds
+// them up in its slice.
+uint32_t max_train_blocks(const hg_mlp* m) {
+    return (uint32_t)m->ctx->sm_count * (m->arch == HG_MLP_ARCH_COMPACT ? 2u : 1u);
+}
+
+uint32_t train_blocks(const hg_mlp* m, uint32_t n) {
+    return std::min(n / kTrainTile + (n % kTrainTile != 0u), max_train_blocks(m));
+}
+
+// The FP16 copies of the parameters; with `blocks` partial gradients (and
+// losses) in m->part, first their sum and either an Adam step (update) or
+// the summed gradient into m->grad.
+cudaError_t convert(hg_mlp* m, uint32_t blocks, int update, float lr_t, float eps_t, float gscale, float* loss) {
     AdamArgs a;
     a.params = m->params;
     a.m = m->adam_m;
@@ -1071,83 +998,42 @@ cudaError_t convert(hg_mlp* m, int update, float lr_t, float eps_t, float gscale
     a.grad = m->grad;
     a.w16 = reinterpret_cast<__half*>(m->w16);
     a.wt16 = reinterpret_cast<__half*>(m->wt16);
+    a.part = blocks ? m->part : nullptr;
+    a.loss_part = m->part + (size_t)max_train_blocks(m) * m->n_params;
+    a.blocks = blocks;
+    a.loss = blocks ? loss : nullptr;
     a.lr_t = lr_t;
     a.beta1 = 0.9f;
     a.beta2 = 0.999f;
     a.eps_t = eps_t;
     a.gscale = gscale;
     a.update = update;
+    const uint32_t grid = (m->n_params + kAdamParams - 1) / kAdamParams;
+    const int threads = kAdamParams * kAdamSplit;
     if (m->arch == HG_MLP_ARCH_COMPACT)
-        adam_small_kernel<<<(mlps::kParams + 255) / 256, 256, 0, m->ctx->stream>>>(a);
+        adam_kernel<mlps::kParams, false><<<grid, threads, 0, m->ctx->stream>>>(a);
     else
-        adam_kernel<<<(kParams + 255) / 256, 256, 0, m->ctx->stream>>>(a);
+        adam_kernel<kParams, true><<<grid, threads, 0, m->ctx->stream>>>(a);
     return cudaGetLastError();
 }
 
-// Grow the transposed activation buffers to hold n samples.
-cudaError_t ensure_scratch(hg_mlp* m, uint32_t n) {
-    const uint32_t ld = (n + 31u) & ~31u;
-    if (ld <= m->ld_capacity) return cudaSuccess;
-    cudaStreamSynchronize(m->ctx->stream);
-    if (m->scratch) cudaFree(m->scratch);
-    m->scratch = nullptr;
-    m->ld_capacity = 0;
-    const size_t halves = (size_t)(kIn + 4 * kHid + 4 * kHid + kOut) * ld;
-    cudaError_t e = cudaMalloc(&m->scratch, halves * sizeof(__half));
-    if (e != cudaSuccess) return e;
-    m->ld_capacity = ld;
-    return cudaSuccess;
-}
-
-// Forward + backward + weight gradients of n samples into m->grad (sum of
-// squared errors) and m->loss.
+// Forward, backward and weight gradients of n samples into m->part:
+// train_blocks(m, n) partial gradients and losses.
 cudaError_t run_gradients(hg_mlp* m, const float* inputs, const float* targets, uint32_t n) {
-    if (m->arch == HG_MLP_ARCH_COMPACT) {
-        SmallTrainArgs s;
-        s.inputs = inputs;
-        s.targets = targets;
-        s.n = n;
-        s.w16 = reinterpret_cast<const __half*>(m->w16);
-        s.params = m->params;
-        s.grad = m->grad;
-        s.loss = m->loss;
-        // persistent warps: each takes several 32-sample tiles, each block adds its sums once
-        const uint32_t tiles = (n + 31u) / 32u;
-        const uint32_t want = (tiles + kSmallTrainWarps - 1) / kSmallTrainWarps;
-        const uint32_t blocks = std::max(1u, std::min(want, (uint32_t)m->ctx->sm_count * 4u));
-        small_train_kernel<<<blocks, kSmallTrainWarps * 32, kSmallTrainSmem, m->ctx->stream>>>(s);
-        return cudaGetLastError();
-    }
-    const uint32_t ld = m->ld_capacity;
-    __half* s = reinterpret_cast<__half*>(m->scratch);
     TrainArgs a;
     a.inputs = inputs;
     a.targets = targets;
     a.n = n;
-    a.ld = ld;
     a.w16 = reinterpret_cast<const __half*>(m->w16);
     a.wt16 = reinterpret_cast<const __half*>(m->wt16);
     a.params = m->params;
-    a.xt = s;
-    a.ht = s + (size_t)kIn * ld;
-    a.dzt = a.ht + (size_t)4 * kHid * ld;
-    a.dz5t = a.dzt + (size_t)4 * kHid * ld;
-    a.loss = m->loss;
-    const uint32_t warps = (n + 31u) / 32u;
-    train_kernel<<<(warps + kWarps - 1) / kWarps, kWarps * 32, kTrainSmem, m->ctx->stream>>>(a);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    WgradArgs w;
-    w.xt = a.xt;
-    w.ht = a.ht;
-    w.dzt = a.dzt;
-    w.dz5t = a.dz5t;
-    w.ld = ld;
-    w.n_pad = warps * 32u;
-    w.chunk = 2048u;
-    w.grad = m->grad;
-    dim3 grid((w.n_pad + w.chunk - 1) / w.chunk, 5);
-    wgrad_kernel<<<grid, 128, 0, m->ctx->stream>>>(w);
+    a.part = m->part;
+    a.loss_part = m->part + (size_t)max_train_blocks(m) * m->n_params;
+    const uint32_t blocks = train_blocks(m, n);
+    if (m->arch == HG_MLP_ARCH_COMPACT)
+        small_train_kernel<<<blocks, kTrainTile, kSmallTrainSmem, m->ctx->stream>>>(a);
+    else
+        train_kernel<<<blocks, kTrainTile, kTrainSmem, m->ctx->stream>>>(a);
     return cudaGetLastError();
 }
 
@@ -1223,10 +1109,11 @@ hg_status hg_mlp_create_arch(hg_ctx* ctx, uint32_t arch, hg_mlp** out) {
     if (e == cudaSuccess && arch == HG_MLP_ARCH_DEEP)
         e = cudaMalloc(&m->wt16, sizeof(__half) * hg::mlp::kTransposed);
     if (e == cudaSuccess) e = cudaMalloc(&m->loss, sizeof(float));
-    for (void* p : {(void*)m->params, (void*)m->grad, (void*)m->adam_m, (void*)m->adam_v})
+    if (e == cudaSuccess)
+        e = cudaMalloc(&m->part, sizeof(float) * (size_t)hg::max_train_blocks(m) * (m->n_params + 1u));
+    for (void* p : {(void*)m->params, (void*)m->adam_m, (void*)m->adam_v})
         if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, pf, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(m->loss, 0, sizeof(float), ctx->stream);
-    if (e == cudaSuccess) e = hg::convert(m, 0, 0.0f, 0.0f, 0.0f);
+    if (e == cudaSuccess) e = hg::convert(m, 0, 0, 0.0f, 0.0f, 0.0f, nullptr);
     if (e != cudaSuccess) {
         hg_mlp_destroy(m);
         return cuda_fail(ctx, e, "creating the surrogate");
@@ -1244,7 +1131,7 @@ void hg_mlp_destroy(hg_mlp* m) {
         if (ctx->surrogate == m) ctx->surrogate = nullptr;
     }
     for (void* p : {(void*)m->params, (void*)m->grad, (void*)m->adam_m, (void*)m->adam_v, (void*)m->w16,
-                    (void*)m->wt16, (void*)m->loss, m->scratch})
+                    (void*)m->wt16, (void*)m->loss, (void*)m->part})
         if (p) cudaFree(p);
     delete m;
 }
@@ -1266,8 +1153,7 @@ hg_status hg_mlp_set_params(hg_mlp* m, const float* params, uint32_t count) {
     MLP_CUDA(ctx, cudaMemcpyAsync(m->params, params, pf, cudaMemcpyHostToDevice, ctx->stream));
     MLP_CUDA(ctx, cudaMemsetAsync(m->adam_m, 0, pf, ctx->stream));
     MLP_CUDA(ctx, cudaMemsetAsync(m->adam_v, 0, pf, ctx->stream));
-    MLP_CUDA(ctx, cudaMemsetAsync(m->grad, 0, pf, ctx->stream));
-    MLP_CUDA(ctx, hg::convert(m, 0, 0.0f, 0.0f, 0.0f));
+    MLP_CUDA(ctx, hg::convert(m, 0, 0, 0.0f, 0.0f, 0.0f, nullptr));
     MLP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     m->step = 0;
     return HG_OK;
@@ -1300,9 +1186,8 @@ hg_status hg_mlp_samples(hg_ctx* ctx, uint64_t seed, uint64_t first, uint32_t co
     a.targets = targets;
     a.lobes = lobes;
     // A lane per sample while that gives every SM a block; below, eight lanes
-    // share a sample's 32 nodes (1,000 samples: SMALL_BEFORE ms with one lane,
-    // SMALL_AFTER ms with eight; at 262,144 the per-sample work that the eight
-    // lanes repeat makes them slower).
+    // share a sample's 32 nodes (1,000 samples: 0.98 ms with one lane, 0.20 ms
+    // with eight).
     if (count >= (uint32_t)ctx->sm_count * hg::kSampleThreads) {
         const uint32_t blocks = (count + hg::kSampleThreads - 1u) / hg::kSampleThreads;
         hg::samples_kernel<1><<<blocks, hg::kSampleThreads, 0, ctx->stream>>>(a);
@@ -1339,15 +1224,12 @@ hg_status hg_mlp_gradients(hg_mlp* m, const float* inputs, const float* targets,
     hg_ctx* ctx = m->ctx;
     if (count == 0 || !inputs || !targets || !grad) return fail(ctx, HG_INVALID_ARG, "empty batch or null buffer");
     MLP_CUDA(ctx, cudaPeekAtLastError());
-    if (m->arch == HG_MLP_ARCH_DEEP) MLP_CUDA(ctx, hg::ensure_scratch(m, count));
     const size_t pf = sizeof(float) * m->n_params;
-    MLP_CUDA(ctx, cudaMemsetAsync(m->grad, 0, pf, ctx->stream));
-    MLP_CUDA(ctx, cudaMemsetAsync(m->loss, 0, sizeof(float), ctx->stream));
     MLP_CUDA(ctx, hg::run_gradients(m, inputs, targets, count));
+    MLP_CUDA(ctx, hg::convert(m, hg::train_blocks(m, count), 0, 0.0f, 0.0f, 0.0f, m->loss));
     MLP_CUDA(ctx, cudaMemcpyAsync(grad, m->grad, pf, cudaMemcpyDeviceToHost, ctx->stream));
     float l = 0.0f;
     MLP_CUDA(ctx, cudaMemcpyAsync(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-    MLP_CUDA(ctx, cudaMemsetAsync(m->grad, 0, pf, ctx->stream));
     MLP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     if (loss) *loss = l;
     return HG_OK;
@@ -1360,17 +1242,13 @@ hg_status hg_mlp_train_step(hg_mlp* m, const float* inputs, const float* targets
     if (count == 0 || !inputs || !targets) return fail(ctx, HG_INVALID_ARG, "empty batch or null buffer");
     if (!(lr >= 0.0f) || !std::isfinite(lr)) return fail(ctx, HG_INVALID_ARG, "learning rate must be finite, >= 0");
     MLP_CUDA(ctx, cudaPeekAtLastError());
-    if (m->arch == HG_MLP_ARCH_DEEP) MLP_CUDA(ctx, hg::ensure_scratch(m, count));
     MLP_CUDA(ctx, hg::run_gradients(m, inputs, targets, count));
     m->step += 1;
     const double b1t = 1.0 - std::pow(0.9, (double)m->step), b2t = 1.0 - std::pow(0.999, (double)m->step);
     const float lr_t = (float)(lr * std::sqrt(b2t) / b1t);
     const float eps_t = (float)(1e-8 * std::sqrt(b2t));
-    MLP_CUDA(ctx, hg::convert(m, 1, lr_t, eps_t, 1.0f / ((float)count * (float)hg_mlp_output_count(m))));
-    if (loss_sum) {
-        MLP_CUDA(ctx, cudaMemcpyAsync(loss_sum, m->loss, sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
-    }
-    MLP_CUDA(ctx, cudaMemsetAsync(m->loss, 0, sizeof(float), ctx->stream));
+    MLP_CUDA(ctx, hg::convert(m, hg::train_blocks(m, count), 1, lr_t, eps_t,
+                              1.0f / ((float)count * (float)hg_mlp_output_count(m)), loss_sum));
     return HG_OK;
 }
 
