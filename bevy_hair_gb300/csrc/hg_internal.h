@@ -68,6 +68,7 @@ struct hg_mlp {
     hg_ctx* ctx = nullptr;
     uint32_t arch = 0;         // HG_MLP_ARCH_*
     uint32_t n_params = 0;     // HG_MLP_PARAMS or HG_MLP_COMPACT_PARAMS
+    void* arena = nullptr;     // the one allocation every array below lies in
     float* params = nullptr;   // n_params floats
     float* grad = nullptr;
     float* adam_m = nullptr;
@@ -75,7 +76,10 @@ struct hg_mlp {
     void* w16 = nullptr;       // __half[n_params], parameter layout
     void* wt16 = nullptr;      // __half[13312], W2^T W3^T W4^T W5^T (4 x 64 network only)
     float* loss = nullptr;     // device scalar
-    float* part = nullptr;     // training: a partial gradient (n_params floats) per block, then their losses
+    float* loss_part = nullptr;  // training: the blocks' losses
+    float* part = nullptr;     // training: partial gradients (n_params floats each); 4 x 64: in the allocation of acts
+    void* acts = nullptr;      // 4 x 64 training: activations and deltas of tile_capacity tiles, then part
+    uint32_t tile_capacity = 0;
     uint64_t step = 0;
 };
 

@@ -96,13 +96,6 @@ __device__ __forceinline__ void load_fwd(FwdWeights& s, const __half* __restrict
     }
 }
 
-__device__ __forceinline__ void load_bwd(BwdWeights& s, const __half* __restrict__ wt16, int tid, int nthreads) {
-    copy_rows<kPadHid>(s.w2t, wt16 + kT2, kHid, kHid, tid, nthreads);
-    copy_rows<kPadHid>(s.w3t, wt16 + kT3, kHid, kHid, tid, nthreads);
-    copy_rows<kPadHid>(s.w4t, wt16 + kT4, kHid, kHid, tid, nthreads);
-    copy_rows<kPadIn>(s.w5t, wt16 + kT5, kHid, kOut, tid, nthreads);
-}
-
 __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
     __half2 v = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
@@ -139,47 +132,6 @@ struct WarpIo {
     __half x[32][kIn + 8];
     float y[32][kOut + 1];
 };
-
-// C fragments of a 64-wide layer -> A fragments of the next (C n-tiles 2kt
-// and 2kt+1 form k-tile kt).  RELU applies max(x, 0) first.
-template <bool RELU>
-__device__ __forceinline__ void c_to_a(const float acc[2][8][4], uint32_t a[2][4][4]) {
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int kt = 0; kt < 4; ++kt) {
-            const float* lo = acc[mt][2 * kt];
-            const float* hi = acc[mt][2 * kt + 1];
-            if (RELU) {
-                a[mt][kt][0] = pack_h2(fmaxf(lo[0], 0.0f), fmaxf(lo[1], 0.0f));
-                a[mt][kt][1] = pack_h2(fmaxf(lo[2], 0.0f), fmaxf(lo[3], 0.0f));
-                a[mt][kt][2] = pack_h2(fmaxf(hi[0], 0.0f), fmaxf(hi[1], 0.0f));
-                a[mt][kt][3] = pack_h2(fmaxf(hi[2], 0.0f), fmaxf(hi[3], 0.0f));
-            } else {
-                a[mt][kt][0] = pack_h2(lo[0], lo[1]);
-                a[mt][kt][1] = pack_h2(lo[2], lo[3]);
-                a[mt][kt][2] = pack_h2(hi[0], hi[1]);
-                a[mt][kt][3] = pack_h2(hi[2], hi[3]);
-            }
-        }
-}
-
-// Bit (mt*8 + nt)*4 + e of the mask is set when the FP16 activation at C
-// position (mt, nt, e) is positive, i.e. where the ReLU passes gradients.
-__device__ __forceinline__ uint64_t relu_mask(const uint32_t a[2][4][4]) {
-    uint64_t m = 0;
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const uint32_t word = a[mt][nt >> 1][(nt & 1) * 2 + (e >> 1)];
-                const uint32_t bits = (e & 1) ? (word >> 16) : (word & 0xffffu);
-                if (bits & 0x7fffu) m |= 1ull << ((mt * 8 + nt) * 4 + e);
-            }
-    return m;
-}
 
 // Stage this lane's 16 inputs as FP16 and build the first layer's A fragments.
 __device__ __forceinline__ void input_frags(WarpIo& io, const float x[kUsedIn], uint32_t a0[2][1][4], int lane,

@@ -429,32 +429,113 @@ __device__ __forceinline__ void ldsm_x2(uint32_t r[2], const void* p) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n" : "=r"(r[0]), "=r"(r[1]) : "r"(a));
 }
 
-constexpr int kTrainWarps = 4;
-constexpr int kTrainTile = 32 * kTrainWarps;  // samples a block takes at a time, 32 per warp
-constexpr int kTilePad = kTrainTile + 8;      // halves per transposed row (conflict-free ldmatrix and stmatrix)
-
-// Packed A fragments (KT k-tiles of 16 units, rows = the warp's 32 samples)
-// into dst[unit][col0 + sample].  Fragment register r covers units
-// (r >> 1) * 8.. and samples (r & 1) * 8.., so one transposing stmatrix stores
-// a 16 x 16 block.
-template <int KT>
-__device__ __forceinline__ void store_t(__half (*dst)[kTilePad], const uint32_t a[2][KT][4], int col0, int lane) {
-    const int r = lane >> 3, i = lane & 7;
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int kt = 0; kt < KT; ++kt)
-            stsm_x4_trans(&dst[kt * 16 + (r >> 1) * 8 + i][col0 + mt * 16 + (r & 1) * 8], a[mt][kt]);
+__device__ __forceinline__ void ldsm_x4_trans(uint32_t r[4], const void* p) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a));
 }
 
-__device__ __forceinline__ void apply_mask(float acc[2][8][4], uint64_t m) {
+// Asynchronous copy of a rows x cols block of halves (cols a multiple of 8)
+// into padded shared rows; wait_copies() before the block's barrier.
+template <int PAD>
+__device__ __forceinline__ void copy_rows_async(__half (*dst)[PAD], const __half* __restrict__ src, int rows, int cols,
+                                                int tid, int nthreads) {
+    const int per_row = cols / 8;
+    for (int i = tid; i < rows * per_row; i += nthreads) {
+        const int r = i / per_row, c = (i - r * per_row) * 8;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(&dst[r][c])),
+                     "l"(src + r * cols + c)
+                     : "memory");
+    }
+}
+__device__ __forceinline__ void wait_copies() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// The training kernels are programmatic dependents of one another (train,
+// Adam, train, ...): a kernel's blocks may be placed while the one before
+// finishes, and wait here, before they touch memory, until it has completed.
+__device__ __forceinline__ void wait_for_previous_kernel() {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
+constexpr int kTrainWarps = 8;
+constexpr int kTrainThreads = 32 * kTrainWarps;
+constexpr int kTrainTile = 16 * kTrainWarps;  // samples a block takes at a time, 16 (one MMA row tile) per warp
+constexpr int kTilePad = kTrainTile + 8;      // halves per transposed row (conflict-free ldmatrix and stmatrix)
+
+// acc[nt] = bias + A W^T for 16 samples, N = 8*NT outputs, K = 16*KT inputs;
+// bias may be null (zero).  The products are those of layer_ldsm.
+template <int NT, int KT, int PAD>
+__device__ __forceinline__ void layer16(float acc[NT][4], const uint32_t a[KT][4], const __half (*w)[PAD],
+                                        const float* bias, int lane) {
+    const int t = lane & 3, mat = lane >> 3, r = lane & 7;
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+    for (int nt = 0; nt < NT; ++nt) {
+        acc[nt][0] = acc[nt][2] = bias ? bias[nt * 8 + 2 * t] : 0.0f;
+        acc[nt][1] = acc[nt][3] = bias ? bias[nt * 8 + 2 * t + 1] : 0.0f;
+    }
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt)
+    for (int kt = 0; kt < KT; ++kt) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (!((m >> ((mt * 8 + nt) * 4 + e)) & 1ull)) acc[mt][nt][e] = 0.0f;
+        for (int nt = 0; nt < NT; nt += 2) {
+            uint32_t b[4];
+            ldsm_x4(b, &w[(nt + (mat >> 1)) * 8 + r][kt * 16 + (mat & 1) * 8]);
+            mma(acc[nt], a[kt], b[0], b[1]);
+            mma(acc[nt + 1], a[kt], b[2], b[3]);
+        }
+    }
+}
+
+// C fragments of a 16*KT-wide layer -> A fragments of the next; RELU applies
+// max(x, 0) first.
+template <bool RELU, int KT>
+__device__ __forceinline__ void c_to_a16(const float acc[2 * KT][4], uint32_t a[KT][4]) {
+    auto v = [](float x) { return RELU ? fmaxf(x, 0.0f) : x; };
+#pragma unroll
+    for (int kt = 0; kt < KT; ++kt)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float* c = acc[2 * kt + h];
+            a[kt][2 * h] = pack_h2(v(c[0]), v(c[1]));
+            a[kt][2 * h + 1] = pack_h2(v(c[2]), v(c[3]));
+        }
+}
+
+// The address of lane's row of the 16 x 16 block kt of [unit][sample] storage
+// that fragment registers r = lane / 8 transpose to and from: units
+// (r >> 1) * 8.., samples (r & 1) * 8...
+__device__ __forceinline__ __half* block_row(__half (*m)[kTilePad], int kt, int col0, int lane) {
+    const int r = lane >> 3, i = lane & 7;
+    return &m[kt * 16 + (r >> 1) * 8 + i][col0 + (r & 1) * 8];
+}
+
+// A fragments (rows = the warp's 16 samples) into dst[unit][col0 + sample].
+template <int KT>
+__device__ __forceinline__ void store_t(__half (*dst)[kTilePad], const uint32_t a[KT][4], int col0, int lane) {
+#pragma unroll
+    for (int kt = 0; kt < KT; ++kt) stsm_x4_trans(block_row(dst, kt, col0, lane), a[kt]);
+}
+
+// C fragments, zeroed where the ReLU output stored in h[unit][col0 + sample]
+// is zero -> A fragments.  The stored values are +0 or positive, so bit 15 of
+// value + 0x7fff says "not zero"; the byte permute spreads it over the half.
+template <int KT>
+__device__ __forceinline__ void masked_to_a16(const float acc[2 * KT][4], __half (*h)[kTilePad], uint32_t a[KT][4],
+                                              int col0, int lane) {
+    c_to_a16<false, KT>(acc, a);
+#pragma unroll
+    for (int kt = 0; kt < KT; ++kt) {
+        uint32_t v[4];
+        ldsm_x4_trans(v, block_row(h, kt, col0, lane));
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            uint32_t m;
+            asm("prmt.b32 %0, %1, 0, 0xBB99;\n" : "=r"(m) : "r"(v[r] + 0x7fff7fffu));
+            a[kt][r] &= m;
+        }
+    }
 }
 
 // Two adjacent partial gradients: stored by the block's first tile, added to
@@ -469,44 +550,32 @@ __device__ __forceinline__ void put2(float* p, float x, float y, bool add) {
     *reinterpret_cast<float2*>(p) = v;
 }
 
-// Rows m0..m0+15, columns n0..n0+8*NT-1 of dW = A B^T over a tile's samples
-// (A = dZ^T, B = H^T, both [unit][sample] in shared memory) into the block's
+// Rows m0..m0+15, columns n0..n0+7 of dW = A B^T over a tile's samples (A =
+// dZ^T, B = H^T, both [unit][sample] in shared memory) into the block's
 // partial gradient gw (row length n_cols); with gb, also the row sums of A
 // (the bias gradient), as a product with ones.  One warp.
-template <int NT>
 __device__ __forceinline__ void wgrad_tile(const __half (*A)[kTilePad], const __half (*B)[kTilePad], int m0, int n0,
                                            float* gw, int n_cols, float* gb, bool add, int lane) {
     const int g = lane >> 2, t = lane & 3, mat = lane >> 3, r = lane & 7;
-    float acc[NT][4] = {}, sum[4] = {};
+    float acc[4] = {}, sum[4] = {};
 #pragma unroll
     for (int k = 0; k < kTrainTile; k += 16) {
-        uint32_t af[4];
+        uint32_t af[4], b[2];
         ldsm_x4(af, &A[m0 + r + (mat & 1) * 8][k + (mat >> 1) * 8]);
+        ldsm_x2(b, &B[n0 + r][k + (mat & 1) * 8]);
         if (gb) mma(sum, af, 0x3C003C00u, 0x3C003C00u);
-#pragma unroll
-        for (int nt = 0; nt + 1 < NT; nt += 2) {
-            uint32_t b[4];
-            ldsm_x4(b, &B[n0 + (nt + (mat >> 1)) * 8 + r][k + (mat & 1) * 8]);
-            mma(acc[nt], af, b[0], b[1]);
-            mma(acc[nt + 1], af, b[2], b[3]);
-        }
-        if (NT & 1) {
-            uint32_t b[2];
-            ldsm_x2(b, &B[n0 + (NT - 1) * 8 + r][k + (mat & 1) * 8]);
-            mma(acc[NT - 1], af, b[0], b[1]);
-        }
+        mma(acc, af, b[0], b[1]);
     }
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-        float* p = gw + (m0 + g) * n_cols + n0 + nt * 8 + 2 * t;
-        put2(p, acc[nt][0], acc[nt][1], add);
-        put2(p + 8 * n_cols, acc[nt][2], acc[nt][3], add);
-    }
+    float* p = gw + (m0 + g) * n_cols + n0 + 2 * t;
+    put2(p, acc[0], acc[1], add);
+    put2(p + 8 * n_cols, acc[2], acc[3], add);
     if (gb && t == 0) {
         gb[m0 + g] = sum[0] + (add ? gb[m0 + g] : 0.0f);
         gb[m0 + g + 8] = sum[2] + (add ? gb[m0 + g + 8] : 0.0f);
     }
 }
+
+struct TileActs;
 
 struct TrainArgs {
     const float* inputs;   // [n][10]
@@ -515,154 +584,384 @@ struct TrainArgs {
     const __half* w16;
     const __half* wt16;    // transposed copies (4 x 64 network only)
     const float* params;
-    float* part;  // [blocks][parameters] partial gradients, written whole
+    TileActs* acts;    // 4 x 64: [tiles] activations and deltas for wgrad_kernel
+    float* part;       // compact: [blocks][parameters] partial gradients, written whole
     float* loss_part;  // [blocks] partial sums of squared errors
 };
+
+// A tile's network inputs and targets, one row per sample.
+struct TileRows {
+    __half x[kTrainTile][kIn + 8];     // normalised inputs
+    float y[kTrainTile][kUsedOut + 1]; // targets; column kUsedOut: 1 for a real sample
+};
+
+// The tile from sample `base`: the first half of the block's threads loads and
+// normalises the inputs, the second the targets.  Ends with a barrier.
+__device__ __forceinline__ void load_tile(TileRows& rows, const TrainArgs& a, uint32_t base) {
+    const int row = threadIdx.x % kTrainTile;
+    const uint32_t i = base + row;
+    const bool valid = i < a.n;
+    if (threadIdx.x < kTrainTile) {
+        float raw[10], x[10];
+        load_raw(a.inputs, i, valid, raw);
+        normalise(raw, x);
+#pragma unroll
+        for (int k = 0; k < kIn; k += 2)
+            *reinterpret_cast<uint32_t*>(&rows.x[row][k]) =
+                pack_h2(k < kUsedIn ? x[k] : 0.0f, k + 1 < kUsedIn ? x[k + 1] : 0.0f);
+    } else {
+#pragma unroll
+        for (int c = 0; c < kUsedOut; ++c) rows.y[row][c] = valid ? __ldg(&a.targets[(size_t)i * 12 + c]) : 0.0f;
+        rows.y[row][kUsedOut] = valid ? 1.0f : 0.0f;
+    }
+    __syncthreads();
+}
+static_assert(kTrainThreads == 2 * kTrainTile, "half of the threads load inputs, half targets");
+
+__device__ __forceinline__ void input_frags16(const TileRows& rows, uint32_t a0[1][4], int col0, int g, int t) {
+    a0[0][0] = ld32(&rows.x[col0 + g][2 * t]);
+    a0[0][1] = ld32(&rows.x[col0 + g + 8][2 * t]);
+    a0[0][2] = ld32(&rows.x[col0 + g][2 * t + 8]);
+    a0[0][3] = ld32(&rows.x[col0 + g + 8][2 * t + 8]);
+}
+
+// The block's sum of squared errors from its threads' shares.
+__device__ __forceinline__ void put_loss(float lsum, float* s_loss, float* out) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+    if ((threadIdx.x & 31) == 0) s_loss[threadIdx.x >> 5] = lsum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float l = 0.0f;
+        for (int w = 0; w < kTrainWarps; ++w) l += s_loss[w];
+        *out = l;
+    }
+}
+
+// What the 4 x 64 network's weight gradients need of a tile, [unit][sample]:
+// written to memory whole, padding and all, so that one bulk copy stores it
+// and a row range of it loads as one.
+struct TileActs {
+    __half x[kIn][kTilePad];       // layer-1 inputs
+    __half h[4][kHid][kTilePad];   // hidden activations h1..h4
+    __half dz[4][kHid][kTilePad];  // pre-activation gradients of layers 1..4
+    __half dz5[kOut][kTilePad];    // output gradients
+};
+constexpr uint32_t kActRowBytes = kTilePad * 2;
+constexpr uint32_t kActRowH = kIn, kActRowDz = kActRowH + 4 * kHid, kActRowDz5 = kActRowDz + 4 * kHid;
+static_assert(sizeof(TileActs) == (kActRowDz5 + kOut) * kActRowBytes && kActRowBytes % 16 == 0, "rows of 272 bytes");
 
 struct TrainSmem {
     FwdWeights fw;
     BwdWeights bw;
-    __half x[kIn][kTilePad];          // layer-1 inputs, [unit][sample]
-    __half h[4][kHid][kTilePad];      // hidden activations h1..h4
-    __half dz[4][kHid][kTilePad];     // pre-activation gradients of layers 1..4
-    __half dz5[kOut][kTilePad];       // output gradients
-    WarpIo io[kTrainWarps];
+    TileActs act;
+    TileRows rows;
     float loss[kTrainWarps];
 };
-static_assert(sizeof(FwdWeights) % 16 == 0 && sizeof(BwdWeights) % 16 == 0 && (kTilePad * 2) % 16 == 0 &&
-                  offsetof(TrainSmem, x) % 16 == 0 && offsetof(TrainSmem, io) % 16 == 0,
-              "ldmatrix rows on 16-byte boundaries");
+static_assert(sizeof(FwdWeights) % 16 == 0 && sizeof(BwdWeights) % 16 == 0 && offsetof(TrainSmem, act) % 16 == 0,
+              "ldmatrix rows and bulk copies on 16-byte boundaries");
 static_assert(sizeof(TrainSmem) <= 227 * 1024, "train kernel shared memory");
 
-// One training batch: forward, backward and weight gradients of 128-sample
-// tiles, everything between the batch's rows and the block's partial gradient
-// in registers and shared memory.  Each warp runs 32 samples forward and
-// backward on mma.sync and leaves its activations and deltas transposed in
-// shared memory; then the block's warps share the weight-gradient products
-// over the tile's 128 samples (warp w takes 16 rows of each dW).  Partial
-// gradients go to the block's own slice with plain stores and the optimiser
-// sums the slices, so nothing is zeroed, no atomics contend and the result
-// does not depend on the blocks' order.  The loss is the sum over samples and
-// the 12 outputs of (y - target)^2, so dL/dy = 2 (y - target); the 1/(n*12)
-// of the mean is applied by the optimiser.
+// Forward and backward of 128-sample tiles of a training batch, 16 samples a
+// warp on mma.sync; activations and deltas are transposed in shared memory
+// (stmatrix) and leave with one bulk copy per tile for wgrad_kernel.  The
+// loss is the sum over samples and the 12 outputs of (y - target)^2, so dL/dy
+// = 2 (y - target); the 1/(n*12) of the mean is applied by the optimiser.
 //
-// Bound by latency and shared-memory traffic: at a batch of 16,384 an SM holds
-// one tile.  Before, the activations went through memory (17 MB) to a second
-// kernel whose 40 blocks summed dW serially: 157 us a step of 16,384 samples;
-// 23.4 us now (152 SMs).
-__global__ void __launch_bounds__(kTrainTile, 1) train_kernel(const TrainArgs a) {
+// Bound by latency: at a batch of 16,384 an SM holds one tile, and a tile is
+// ten dependent layers.  Eight warps of 16 samples (two per scheduler) hide
+// more of it than four of 32, although each weight fragment then feeds half
+// the products.  A step of 16,384 samples (152 SMs): 157 us with a row-per-lane
+// transpose through memory and a weight-gradient kernel of 40 blocks, 22 us
+// now (by ncu, cold caches: this kernel 11 us, wgrad_kernel 9.4, Adam 3.8).
+__global__ void __launch_bounds__(kTrainThreads, 1) train_kernel(const TrainArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    load_fwd(S.fw, a.w16, a.params, threadIdx.x, blockDim.x);
-    load_bwd(S.bw, a.wt16, threadIdx.x, blockDim.x);
-    __syncthreads();
-    WarpIo& w_io = S.io[warp];
-    const int col0 = 32 * warp;
-    float* part = a.part + (size_t)blockIdx.x * kParams;
+    TileActs& A = S.act;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    wait_for_previous_kernel();
+    copy_rows_async<kPadIn>(S.fw.w1, a.w16 + kW1, kHid, kIn, tid, kTrainThreads);
+    copy_rows_async<kPadHid>(S.fw.w2, a.w16 + kW2, kHid, kHid, tid, kTrainThreads);
+    copy_rows_async<kPadHid>(S.fw.w3, a.w16 + kW3, kHid, kHid, tid, kTrainThreads);
+    copy_rows_async<kPadHid>(S.fw.w4, a.w16 + kW4, kHid, kHid, tid, kTrainThreads);
+    copy_rows_async<kPadHid>(S.fw.w5, a.w16 + kW5, kOut, kHid, tid, kTrainThreads);
+    copy_rows_async<kPadHid>(S.bw.w2t, a.wt16 + kT2, kHid, kHid, tid, kTrainThreads);
+    copy_rows_async<kPadHid>(S.bw.w3t, a.wt16 + kT3, kHid, kHid, tid, kTrainThreads);
+    copy_rows_async<kPadHid>(S.bw.w4t, a.wt16 + kT4, kHid, kHid, tid, kTrainThreads);
+    copy_rows_async<kPadIn>(S.bw.w5t, a.wt16 + kT5, kHid, kOut, tid, kTrainThreads);
+    for (int i = tid; i < kHid; i += kTrainThreads) {
+        S.fw.b1[i] = a.params[kB1 + i];
+        S.fw.b2[i] = a.params[kB2 + i];
+        S.fw.b3[i] = a.params[kB3 + i];
+        S.fw.b4[i] = a.params[kB4 + i];
+        if (i < kOut) S.fw.b5[i] = a.params[kB5 + i];
+    }
+    const int col0 = 16 * warp;
     float lsum = 0.0f;
-    bool add = false;
-    for (uint32_t base = blockIdx.x * kTrainTile; base < a.n; base += gridDim.x * kTrainTile) {
-        const uint32_t i = base + threadIdx.x;
-        const bool valid = i < a.n;
-        // the targets are read up front: they are needed only after the forward pass
-        float tgt[kUsedOut];
-#pragma unroll
-        for (int c = 0; c < kUsedOut; ++c) tgt[c] = valid ? __ldg(&a.targets[(size_t)i * 12 + c]) : 0.0f;
-        float raw[10], x[10];
-        load_raw(a.inputs, i, valid, raw);
-        normalise(raw, x);
-        uint32_t a0[2][1][4];
-        input_frags(w_io, x, a0, lane, g, t);
-        store_t<1>(S.x, a0, col0, lane);
+    const uint32_t tiles = a.n / kTrainTile + (a.n % kTrainTile != 0u);
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        wait_copies();  // the weights, before the first tile's barrier
+        // the previous tile's copy must have read the tile buffer (its issuer waits)
+        if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+        load_tile(S.rows, a, tile * kTrainTile);
+        uint32_t a0[1][4];
+        input_frags16(S.rows, a0, col0, g, t);
+        store_t<1>(A.x, a0, col0, lane);
 
-        float acc[2][8][4];
-        uint32_t h[2][4][4];
-        uint64_t m1, m2, m3, m4;
-        layer_ldsm<8, 1, kPadIn>(acc, a0, S.fw.w1, S.fw.b1, lane);
-        c_to_a<true>(acc, h);
-        m1 = relu_mask(h);
-        store_t<4>(S.h[0], h, col0, lane);
-        layer_ldsm<8, 4, kPadHid>(acc, h, S.fw.w2, S.fw.b2, lane);
-        c_to_a<true>(acc, h);
-        m2 = relu_mask(h);
-        store_t<4>(S.h[1], h, col0, lane);
-        layer_ldsm<8, 4, kPadHid>(acc, h, S.fw.w3, S.fw.b3, lane);
-        c_to_a<true>(acc, h);
-        m3 = relu_mask(h);
-        store_t<4>(S.h[2], h, col0, lane);
-        layer_ldsm<8, 4, kPadHid>(acc, h, S.fw.w4, S.fw.b4, lane);
-        c_to_a<true>(acc, h);
-        m4 = relu_mask(h);
-        store_t<4>(S.h[3], h, col0, lane);
-        float out[2][2][4];
-        layer_ldsm<2, 4, kPadHid>(out, h, S.fw.w5, S.fw.b5, lane);
+        float acc[8][4];
+        uint32_t h[4][4];
+        layer16<8, 1, kPadIn>(acc, a0, S.fw.w1, S.fw.b1, lane);
+        c_to_a16<true, 4>(acc, h);
+        store_t<4>(A.h[0], h, col0, lane);
+        layer16<8, 4, kPadHid>(acc, h, S.fw.w2, S.fw.b2, lane);
+        c_to_a16<true, 4>(acc, h);
+        store_t<4>(A.h[1], h, col0, lane);
+        layer16<8, 4, kPadHid>(acc, h, S.fw.w3, S.fw.b3, lane);
+        c_to_a16<true, 4>(acc, h);
+        store_t<4>(A.h[2], h, col0, lane);
+        layer16<8, 4, kPadHid>(acc, h, S.fw.w4, S.fw.b4, lane);
+        c_to_a16<true, 4>(acc, h);
+        store_t<4>(A.h[3], h, col0, lane);
+        float out[2][4];
+        layer16<2, 4, kPadHid>(out, h, S.fw.w5, S.fw.b5, lane);
 
-        // Targets into the C layout through the warp's output stage; column 16
-        // flags a real sample.
+        float dy[2][4];
 #pragma unroll
-        for (int c = 0; c < kUsedOut; ++c) w_io.y[lane][c] = tgt[c];
-        w_io.y[lane][16] = valid ? 1.0f : 0.0f;
-        __syncwarp();
-        uint32_t d5[2][1][4];
+        for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-            float dy[2][4];
+            for (int e = 0; e < 4; ++e) {
+                const int r = col0 + g + (e >> 1) * 8, c = nt * 8 + 2 * t + (e & 1);
+                float d = 0.0f;
+                if (c < kUsedOut && S.rows.y[r][kUsedOut] != 0.0f) d = out[nt][e] - S.rows.y[r][c];
+                lsum += d * d;
+                dy[nt][e] = 2.0f * d;
+            }
+        uint32_t d5[1][4];
+        c_to_a16<false, 1>(dy, d5);
+        store_t<1>(A.dz5, d5, col0, lane);
+        __syncwarp();  // the warp's stored activations, read back as masks
+
+        layer16<8, 1, kPadIn>(acc, d5, S.bw.w5t, nullptr, lane);
+        masked_to_a16<4>(acc, A.h[3], h, col0, lane);
+        store_t<4>(A.dz[3], h, col0, lane);
+        layer16<8, 4, kPadHid>(acc, h, S.bw.w4t, nullptr, lane);
+        masked_to_a16<4>(acc, A.h[2], h, col0, lane);
+        store_t<4>(A.dz[2], h, col0, lane);
+        layer16<8, 4, kPadHid>(acc, h, S.bw.w3t, nullptr, lane);
+        masked_to_a16<4>(acc, A.h[1], h, col0, lane);
+        store_t<4>(A.dz[1], h, col0, lane);
+        layer16<8, 4, kPadHid>(acc, h, S.bw.w2t, nullptr, lane);
+        masked_to_a16<4>(acc, A.h[0], h, col0, lane);
+        store_t<4>(A.dz[0], h, col0, lane);
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        __syncthreads();
+        if (tid == 0) {
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n"
+                         "cp.async.bulk.commit_group;\n" ::"l"(a.acts + tile),
+                         "r"((uint32_t)__cvta_generic_to_shared(&A)), "r"((uint32_t)sizeof(TileActs))
+                         : "memory");
+        }
+    }
+    put_loss(lsum, S.loss, a.loss_part + blockIdx.x);
+    if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
+}
+
+// Weight gradients of the 4 x 64 network, dW = dZ^T H over chunks of 2,048
+// samples (16 tiles): block (c, u) computes unit u of chunk c and stores it in
+// the chunk's partial gradient, which the optimiser sums.  Units: 64 rows x 32
+// columns of dW2, dW3, dW4 (two each), dW1, dW5.  Four warps take 16 rows each
+// (dW5: 16 columns each) and run the chunk's samples through their
+// accumulators in one chain of 128 products, 16 samples at a time, with the
+// next step's fragments loaded ahead; bias gradients are the row sums of the
+// same dZ fragments.  A fifth warp brings the tiles' rows by bulk copies,
+// kWgradStages tiles ahead.
+//
+// Bound by the latency of that chain: the chain's length is what rounds the
+// sums, so it is not split further, and finer units only shorten each step.
+// Six stages also keep a second block off the SM (two blocks of 104 KB shared
+// one while others stood idle).  By ncu, a batch of
+// 16,384: 192 us with 40 blocks reading global memory, 14.9 us with two
+// blocks an SM and no fragments loaded ahead, 9.4 us so.  (Products over
+// each 128-sample tile in train_kernel itself, summed by the optimiser, take
+// 16 us a step instead of 22, but round differently: 4e-6 of the gradient,
+// which a few steps at a high learning rate amplify.)
+constexpr uint32_t kChunkTiles = 16;
+constexpr int kWgradUnits = 8, kWgradStages = 6, kWgradWarps = 4, kWgradThreads = 32 * (kWgradWarps + 1);
+struct WgradStage {
+    __half rows[96][kTilePad];  // dZ rows, then H rows
+};
+struct WgradSmem {
+    alignas(128) WgradStage st[kWgradStages];
+    alignas(8) uint64_t full[kWgradStages];   // the stage's copies have arrived
+    alignas(8) uint64_t empty[kWgradStages];  // the warps are done with it
+};
+constexpr size_t kWgradSmem = sizeof(WgradSmem);
+static_assert(kWgradSmem <= 227 * 1024 && kWgradSmem > 114 * 1024 && sizeof(WgradStage) % 16 == 0,
+              "weight-gradient stages: one block per SM");
+
+struct WgradArgs {
+    const TileActs* acts;  // [tiles]
+    uint32_t tiles;
+    float* part;           // [chunks][parameters]
+    uint32_t* err;
+};
+
+// Rows of a tile's activations that a unit reads: dZ rows, then H rows.
+struct WgradRows {
+    uint32_t a, rows_a, b, rows_b;
+};
+
+__device__ __forceinline__ float h2sum(uint32_t v) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&v));
+    return f.x + f.y;
+}
+
+// The copying warp (one lane): the unit's rows of every tile of the chunk, a
+// stage each, as stages become free.  False when one did not in time.
+__device__ __forceinline__ bool wgrad_copy(WgradSmem& S, const TileActs* acts, uint32_t tiles, WgradRows u) {
+    const uint32_t full = (uint32_t)__cvta_generic_to_shared(S.full), empty = (uint32_t)__cvta_generic_to_shared(S.empty);
+    for (uint32_t k = 0; k < tiles; ++k) {
+        const uint32_t s = k % kWgradStages, round = k / kWgradStages;
+        if (round > 0 && !tc::mbar_wait(empty + 8u * s, (round - 1u) & 1u)) return false;
+        const char* tile = reinterpret_cast<const char*>(acts + k);
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&S.st[s]), mbar = full + 8u * s;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(mbar),
+                     "r"((u.rows_a + u.rows_b) * kActRowBytes)
+                     : "memory");
+        auto copy = [&](uint32_t to, uint32_t row, uint32_t rows) {
+            asm volatile(
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(to),
+                "l"(tile + (size_t)row * kActRowBytes), "r"(rows * kActRowBytes), "r"(mbar)
+                : "memory");
+        };
+        copy(dst, u.a, u.rows_a);
+        copy(dst + u.rows_a * kActRowBytes, u.b, u.rows_b);
+    }
+    // every copy has landed before the block may end, whatever the other warps did
+    bool ok = true;
+    for (uint32_t s = 0; s < kWgradStages && s < tiles; ++s) {
+        const uint32_t last = (tiles - 1u - s) / kWgradStages;
+        ok = tc::mbar_wait(full + 8u * s, last & 1u) && ok;
+    }
+    return ok;
+}
+
+// One warp's 16 x (8 NT) products over the chunk's tiles; a_row, b_row: its
+// first rows in a stage; BIAS: also the row sums of A.  False when a tile did
+// not arrive in time.
+template <int NT, bool BIAS>
+__device__ __forceinline__ bool wgrad_chain(WgradSmem& S, uint32_t tiles, int a_row, int b_row, float acc[4][4],
+                                            float& s0, float& s1, int lane) {
+    const int mat = lane >> 3, r = lane & 7;
+    const uint32_t full = (uint32_t)__cvta_generic_to_shared(S.full), empty = (uint32_t)__cvta_generic_to_shared(S.empty);
+    for (uint32_t k = 0; k < tiles; ++k) {
+        const uint32_t s = k % kWgradStages;
+        if (!__all_sync(0xffffffffu, tc::mbar_wait(full + 8u * s, (k / kWgradStages) & 1u))) return false;
+        const __half* pa = &S.st[s].rows[a_row + r + (mat & 1) * 8][(mat >> 1) * 8];
+        const __half* pb = &S.st[s].rows[b_row + (mat >> 1) * 8 + r][(mat & 1) * 8];
+        uint32_t af[2][4], b[2][NT / 2][4];
+        auto load = [&](int buf, int c) {
+            ldsm_x4(af[buf], pa + c);
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt)
+            for (int q = 0; q < NT / 2; ++q) ldsm_x4(b[buf][q], pb + q * 16 * kTilePad + c);
+        };
+        load(0, 0);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int r = mt * 16 + g + ((e >> 1) ? 8 : 0), c = nt * 8 + 2 * t + (e & 1);
-                    float d = 0.0f;
-                    if (c < kUsedOut && w_io.y[r][16] != 0.0f) d = out[mt][nt][e] - w_io.y[r][c];
-                    lsum += d * d;
-                    dy[nt][e] = 2.0f * d;
-                }
-            d5[mt][0][0] = pack_h2(dy[0][0], dy[0][1]);
-            d5[mt][0][1] = pack_h2(dy[0][2], dy[0][3]);
-            d5[mt][0][2] = pack_h2(dy[1][0], dy[1][1]);
-            d5[mt][0][3] = pack_h2(dy[1][2], dy[1][3]);
+        for (int i = 0; i < kTrainTile / 16; ++i) {
+            const int cur = i & 1;
+            if (i + 1 < kTrainTile / 16) load(cur ^ 1, 16 * (i + 1));
+#pragma unroll
+            for (int q = 0; q < NT / 2; ++q) {
+                mma(acc[2 * q], af[cur], b[cur][q][0], b[cur][q][1]);
+                mma(acc[2 * q + 1], af[cur], b[cur][q][2], b[cur][q][3]);
+            }
+            if (BIAS) {
+                s0 += h2sum(af[cur][0]) + h2sum(af[cur][2]);
+                s1 += h2sum(af[cur][1]) + h2sum(af[cur][3]);
+            }
         }
         __syncwarp();
-        store_t<1>(S.dz5, d5, col0, lane);
+        if (lane == 0)
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(empty + 8u * s) : "memory");
+    }
+    return true;
+}
 
-        layer_ldsm<8, 1, kPadIn>(acc, d5, S.bw.w5t, nullptr, lane);
-        apply_mask(acc, m4);
-        c_to_a<false>(acc, h);
-        store_t<4>(S.dz[3], h, col0, lane);
-        layer_ldsm<8, 4, kPadHid>(acc, h, S.bw.w4t, nullptr, lane);
-        apply_mask(acc, m3);
-        c_to_a<false>(acc, h);
-        store_t<4>(S.dz[2], h, col0, lane);
-        layer_ldsm<8, 4, kPadHid>(acc, h, S.bw.w3t, nullptr, lane);
-        apply_mask(acc, m2);
-        c_to_a<false>(acc, h);
-        store_t<4>(S.dz[1], h, col0, lane);
-        layer_ldsm<8, 4, kPadHid>(acc, h, S.bw.w2t, nullptr, lane);
-        apply_mask(acc, m1);
-        c_to_a<false>(acc, h);
-        store_t<4>(S.dz[0], h, col0, lane);
-        __syncthreads();
-
-        wgrad_tile<8>(S.dz[3], S.h[2], 16 * warp, 0, part + kW4, kHid, part + kB4, add, lane);
-        wgrad_tile<8>(S.dz[2], S.h[1], 16 * warp, 0, part + kW3, kHid, part + kB3, add, lane);
-        wgrad_tile<8>(S.dz[1], S.h[0], 16 * warp, 0, part + kW2, kHid, part + kB2, add, lane);
-        wgrad_tile<2>(S.dz[0], S.x, 16 * warp, 0, part + kW1, kIn, part + kB1, add, lane);
-        wgrad_tile<2>(S.dz5, S.h[3], 0, 16 * warp, part + kW5, kHid, warp == 0 ? part + kB5 : nullptr, add, lane);
-        add = true;
-        __syncthreads();  // the next tile overwrites what the products read
+__global__ void __launch_bounds__(kWgradThreads, 1) wgrad_kernel(const WgradArgs a) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    WgradSmem& S = *reinterpret_cast<WgradSmem*>(smem);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const uint32_t chunk = blockIdx.x, unit = blockIdx.y;
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < kWgradStages; ++k) {
+            tc::mbar_init((uint32_t)__cvta_generic_to_shared(&S.full[k]), 1);
+            tc::mbar_init((uint32_t)__cvta_generic_to_shared(&S.empty[k]), kWgradWarps);
+        }
+        tc::fence_mbar_init();
+    }
+    __syncthreads();
+    wait_for_previous_kernel();
+    const TileActs* acts = a.acts + (size_t)chunk * kChunkTiles;
+    const uint32_t tiles = min(kChunkTiles, a.tiles - chunk * kChunkTiles);
+    float* part = a.part + (size_t)chunk * kParams;
+    // units 0..5: dW4, dW3, dW2 = dz[l] h[l - 1]^T, 32 columns each; 6: dW1; 7: dW5
+    const int l = unit < 6u ? 3 - (int)(unit >> 1) : 0, half = (int)(unit & 1u);
+    const WgradRows rows = unit < 6u    ? WgradRows{kActRowDz + l * kHid, kHid, kActRowH + (l - 1) * kHid + 32 * half, 32}
+                           : unit == 6u ? WgradRows{kActRowDz, kHid, 0, kIn}
+                                        : WgradRows{kActRowDz5, kOut, kActRowH + 3 * kHid, kHid};
+    if (warp == kWgradWarps) {
+        if (lane == 0 && !wgrad_copy(S, acts, tiles, rows)) atomicOr(a.err, tc::kErrTimeout);
+        return;
+    }
+    float acc[4][4] = {}, s0 = 0.0f, s1 = 0.0f;
+    bool ok;
+    float *gw, *gb = nullptr;
+    int m0 = 16 * warp, n0 = 0, ncols = kHid, ntiles = 4;
+    if (unit < 6u) {
+        ok = half ? wgrad_chain<4, false>(S, tiles, m0, kHid, acc, s0, s1, lane)
+                  : wgrad_chain<4, true>(S, tiles, m0, kHid, acc, s0, s1, lane);
+        gw = part + (l == 3 ? kW4 : l == 2 ? kW3 : kW2);
+        if (!half) gb = part + (l == 3 ? kB4 : l == 2 ? kB3 : kB2);
+        n0 = 32 * half;
+    } else if (unit == 6u) {
+        ntiles = 2;
+        ok = wgrad_chain<2, true>(S, tiles, m0, kHid, acc, s0, s1, lane);
+        gw = part + kW1;
+        gb = part + kB1;
+        ncols = kIn;
+    } else {  // 16 columns a warp
+        ntiles = 2;
+        ok = wgrad_chain<2, true>(S, tiles, 0, kOut + 16 * warp, acc, s0, s1, lane);
+        gw = part + kW5;
+        if (warp == 0) gb = part + kB5;
+        m0 = 0;
+        n0 = 16 * warp;
+    }
+    if (!ok) {
+        if (lane == 0) atomicOr(a.err, tc::kErrTimeout);
+        return;
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-    if (lane == 0) S.loss[warp] = lsum;
-    __syncthreads();
-    if (threadIdx.x == 0) a.loss_part[blockIdx.x] = (S.loss[0] + S.loss[1]) + (S.loss[2] + S.loss[3]);
+    for (int nt = 0; nt < 4; ++nt) {
+        if (nt >= ntiles) break;
+        float* p = gw + (m0 + g) * ncols + n0 + nt * 8 + 2 * t;
+        *reinterpret_cast<float2*>(p) = make_float2(acc[nt][0], acc[nt][1]);
+        *reinterpret_cast<float2*>(p + 8 * ncols) = make_float2(acc[nt][2], acc[nt][3]);
+    }
+    s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+    s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
+    if (gb && t == 0) {
+        gb[m0 + g] = s0;
+        gb[m0 + g + 8] = s1;
+    }
 }
 
 // Training of the compact network on the tensor cores (mma.sync m16n8k16,
-// FP16 operands, FP32 accumulation).  A warp takes 32 samples at a time:
-//  forward   the inference network itself (mlps::forward's layers), keeping
-//            the FP16 activations and the ReLU masks;
+// FP16 operands, FP32 accumulation).  A warp takes 16 samples at a time:
+//  forward   the inference network's products, keeping the FP16 activations
+//            and the ReLU masks;
 //  backward  dY = 2 (y - target) for the three BSDF channels, then
 //            dZ2 = (dY W3) . [Z2 > 0] and dZ1 = (dZ2 W2) . [Z1 > 0], each a
 //            product with a transposed weight matrix held in shared memory;
@@ -671,15 +970,16 @@ __global__ void __launch_bounds__(kTrainTile, 1) train_kernel(const TrainArgs a)
 //            sample dimension is the MMAs' K and the warps share the output
 //            tiles; bias gradients are products with ones.
 // The deltas enter the MMAs rounded to FP16 (the usual mixed-precision
-// backward).  Partial gradients go to the block's own slice, as in
-// train_kernel.  The loss is the sum over samples and the three channels of
+// backward).  Partial gradients go to the block's own slice with plain stores
+// and the optimiser sums the slices, so nothing is zeroed, no atomics contend
+// and the result does not depend on the blocks' order.  The loss is the sum over samples and the three channels of
 // (y - target)^2; the targets are formed from the twelve lobes of
 // hg_mlp_samples (mlps::bsdf_target).
 //
 // Bound by latency (a batch of 16,384 is one tile per block, on 128 blocks).
-// Before, each warp added its 2,128 sums to shared memory and each block to
-// global memory by atomics, with a loss copy and a memset after every step:
-// 25.5 us a step of 16,384 samples; SMALL_23.4 us now.
+// A step of 16,384 samples: 25.5 us with shared and global atomics, a loss
+// copy and a memset; 16.6 us with partial gradients and four warps of 32
+// samples; 8.7 us so.
 struct SmallTrainSmem {
     alignas(16) mlps::Weights w;                       // forward weights (padded rows) and biases
     alignas(16) __half w3t[mlps::kHid][mlps::kPadIn];  // W3^T: [hidden][output]
@@ -691,48 +991,61 @@ struct SmallTrainSmem {
     __half dy[mlps::kOut][kTilePad];
     __half dz2[mlps::kHid][kTilePad];
     __half dz1[mlps::kHid][kTilePad];
-    alignas(16) mlp::WarpIo io[kTrainWarps];
+    TileRows rows;
     float loss[kTrainWarps];
 };
 static_assert(offsetof(SmallTrainSmem, w) % 16 == 0 && offsetof(SmallTrainSmem, w3t) % 16 == 0 &&
-                  offsetof(SmallTrainSmem, w2t) % 16 == 0 && offsetof(SmallTrainSmem, x) % 16 == 0 &&
-                  offsetof(SmallTrainSmem, io) % 16 == 0,
+                  offsetof(SmallTrainSmem, w2t) % 16 == 0 && offsetof(SmallTrainSmem, x) % 16 == 0,
               "ldmatrix operands on 16-byte boundaries");
 static_assert(offsetof(mlps::Weights, w2) % 16 == 0 && offsetof(mlps::Weights, w3) % 16 == 0, "weight rows");
 static_assert((mlps::kPadIn * 2) % 16 == 0 && (mlps::kPadHid * 2) % 16 == 0, "padded weight rows");
 constexpr size_t kSmallTrainSmem = sizeof(SmallTrainSmem);
 
-// C fragments of a 32-wide layer times a 32-bit mask (bit (mt*4 + nt)*4 + e)
-// -> FP16 A fragments.
-__device__ __forceinline__ void masked_to_a(const float acc[2][4][4], uint32_t mask, uint32_t a[2][2][4]) {
-    auto m = [&](int mt, int nt, int e) { return (mask >> ((mt * 4 + nt) * 4 + e)) & 1u ? acc[mt][nt][e] : 0.0f; };
+// C fragments of a 32-wide layer, zeroed where `mask` (bit nt*4 + e) is clear
+// -> A fragments.
+__device__ __forceinline__ void masked_to_a(const float acc[4][4], uint32_t mask, uint32_t a[2][4]) {
+    float v[4][4];
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+    for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-        for (int kt = 0; kt < 2; ++kt) {
-            a[mt][kt][0] = mlp::pack_h2(m(mt, 2 * kt, 0), m(mt, 2 * kt, 1));
-            a[mt][kt][1] = mlp::pack_h2(m(mt, 2 * kt, 2), m(mt, 2 * kt, 3));
-            a[mt][kt][2] = mlp::pack_h2(m(mt, 2 * kt + 1, 0), m(mt, 2 * kt + 1, 1));
-            a[mt][kt][3] = mlp::pack_h2(m(mt, 2 * kt + 1, 2), m(mt, 2 * kt + 1, 3));
-        }
+        for (int e = 0; e < 4; ++e) v[nt][e] = (mask >> (nt * 4 + e)) & 1u ? acc[nt][e] : 0.0f;
+    c_to_a16<false, 2>(v, a);
 }
 
-__device__ __forceinline__ uint32_t positive_mask(const float acc[2][4][4]) {
+__device__ __forceinline__ uint32_t positive_mask(const float acc[4][4]) {
     uint32_t m = 0;
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+    for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) m |= (acc[mt][nt][e] > 0.0f ? 1u : 0u) << ((mt * 4 + nt) * 4 + e);
+        for (int e = 0; e < 4; ++e) m |= (acc[nt][e] > 0.0f ? 1u : 0u) << (nt * 4 + e);
     return m;
 }
 
-__global__ void __launch_bounds__(kTrainTile) small_train_kernel(const TrainArgs a) {
+// max(x, 0) fused into the FP16 conversion, as the inference path does it.
+__device__ __forceinline__ void relu_to_a16(const float acc[4][4], uint32_t a[2][4]) {
+#pragma unroll
+    for (int kt = 0; kt < 2; ++kt)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float* c = acc[2 * kt + h];
+            a[kt][2 * h] = pack_relu(c[0], c[1]);
+            a[kt][2 * h + 1] = pack_relu(c[2], c[3]);
+        }
+}
+
+__global__ void __launch_bounds__(kTrainThreads) small_train_kernel(const TrainArgs a) {
     extern __shared__ __align__(16) unsigned char smem_small[];
     SmallTrainSmem& S = *reinterpret_cast<SmallTrainSmem*>(smem_small);
-    const int tid = threadIdx.x, nth = blockDim.x;
-    mlps::load(S.w, a.w16, a.params, tid, nth);
+    const int tid = threadIdx.x, nth = kTrainThreads;
+    wait_for_previous_kernel();
+    copy_rows_async<mlps::kPadIn>(S.w.w1, a.w16 + mlps::kW1, mlps::kHid, mlps::kIn, tid, nth);
+    copy_rows_async<mlps::kPadHid>(S.w.w2, a.w16 + mlps::kW2, mlps::kHid, mlps::kHid, tid, nth);
+    copy_rows_async<mlps::kPadHid>(S.w.w3, a.w16 + mlps::kW3, mlps::kOut, mlps::kHid, tid, nth);
+    for (int i = tid; i < mlps::kHid; i += nth) {
+        S.w.b1[i] = a.params[mlps::kB1 + i];
+        S.w.b2[i] = a.params[mlps::kB2 + i];
+        if (i < mlps::kOut) S.w.b3[i] = a.params[mlps::kB3 + i];
+    }
     for (int i = tid; i < mlps::kHid * mlps::kOut; i += nth) {
         const int j = i / mlps::kOut, o = i % mlps::kOut;  // W3^T[j][o] = W3[o][j]
         S.w3t[j][o] = a.w16[mlps::kW3 + o * mlps::kHid + j];
@@ -741,77 +1054,76 @@ __global__ void __launch_bounds__(kTrainTile) small_train_kernel(const TrainArgs
         const int j1 = i / mlps::kHid, j2 = i % mlps::kHid;  // W2^T[j1][j2] = W2[j2][j1]
         S.w2t[j1][j2] = a.w16[mlps::kW2 + j2 * mlps::kHid + j1];
     }
-    __syncthreads();
     const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    mlp::WarpIo& io = S.io[warp];
-    const int col0 = 32 * warp;
+    const int col0 = 16 * warp;
     float* part = a.part + (size_t)blockIdx.x * mlps::kParams;
-    float loss = 0.0f;
+    float lsum = 0.0f;
+    const uint32_t tiles = a.n / kTrainTile + (a.n % kTrainTile != 0u);
     bool add = false;
-    for (uint32_t base = blockIdx.x * kTrainTile; base < a.n; base += gridDim.x * kTrainTile) {
-        const uint32_t k = base + tid;
-        const bool valid = k < a.n;
-        // the targets are read up front: they are needed only after the forward pass
-        float t12[12];
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        wait_copies();  // the weights, before the first tile's barrier
+        load_tile(S.rows, a, tile * kTrainTile);
+        // the three BSDF targets, one row per thread of the first half (read
+        // behind the barrier after the forward pass)
+        if (tid < kTrainTile) {
+            float y[mlps::kUsedOut];
 #pragma unroll
-        for (int c = 0; c < 12; ++c) t12[c] = valid ? __ldg(&a.targets[(size_t)k * 12 + c]) : 0.0f;
-        float raw[10], xn[10];
-        load_raw(a.inputs, k, valid, raw);
-        normalise(raw, xn);
-        // forward (the inference roundings: FP16 inputs, weights and activations)
-        uint32_t a0[2][1][4];
-        mlp::input_frags(io, xn, a0, lane, g, t);
-        float acc[2][4][4];
-        uint32_t a1[2][2][4], a2[2][2][4];
-        mlp::layer_ldsm<4, 1, mlps::kPadIn>(acc, a0, S.w.w1, S.w.b1, lane);
-        const uint32_t mask1 = positive_mask(acc);
-        mlps::relu_to_a(acc, a1);
-        mlp::layer_ldsm<4, 2, mlps::kPadHid>(acc, a1, S.w.w2, S.w.b2, lane);
-        const uint32_t mask2 = positive_mask(acc);
-        mlps::relu_to_a(acc, a2);
-        float out[2][2][4];
-        mlp::layer_ldsm<2, 2, mlps::kPadHid>(out, a2, S.w.w3, S.w.b3, lane);
-        float y[mlp::kUsedOut];  // output_rows fills 12 columns; the first mlps::kUsedOut are outputs
-        mlp::output_rows(io, out, y, lane, g, t);
-        store_t<1>(S.x, a0, col0, lane);
-        store_t<2>(S.a1, a1, col0, lane);
-        store_t<2>(S.a2, a2, col0, lane);
-        // dY of this lane's sample, as the next product's A operand
-        float dyx[mlp::kUsedIn] = {};
+            for (int o = 0; o < mlps::kUsedOut; ++o) y[o] = mlps::bsdf_target(S.rows.y[tid], o);
 #pragma unroll
-        for (int o = 0; o < mlps::kUsedOut; ++o) {
-            const float d = valid ? y[o] - mlps::bsdf_target(t12, o) : 0.0f;
-            loss += d * d;
-            dyx[o] = 2.0f * d;
+            for (int o = 0; o < mlps::kUsedOut; ++o) S.rows.y[tid][o] = y[o];
         }
-        uint32_t ady[2][1][4];
-        mlp::input_frags(io, dyx, ady, lane, g, t);
-        // backward through the layers
-        mlp::layer_ldsm<4, 1, mlps::kPadIn>(acc, ady, S.w3t, nullptr, lane);  // dY W3
-        uint32_t dz2[2][2][4], dz1[2][2][4];
-        masked_to_a(acc, mask2, dz2);
-        mlp::layer_ldsm<4, 2, mlps::kPadHid>(acc, dz2, S.w2t, nullptr, lane);  // dZ2 W2
-        masked_to_a(acc, mask1, dz1);
+        // forward (the inference roundings: FP16 inputs, weights and activations)
+        uint32_t a0[1][4], a1[2][4], a2[2][4];
+        input_frags16(S.rows, a0, col0, g, t);
+        store_t<1>(S.x, a0, col0, lane);
+        float acc[4][4];
+        layer16<4, 1, mlps::kPadIn>(acc, a0, S.w.w1, S.w.b1, lane);
+        const uint32_t mask1 = positive_mask(acc);
+        relu_to_a16(acc, a1);
+        store_t<2>(S.a1, a1, col0, lane);
+        layer16<4, 2, mlps::kPadHid>(acc, a1, S.w.w2, S.w.b2, lane);
+        const uint32_t mask2 = positive_mask(acc);
+        relu_to_a16(acc, a2);
+        store_t<2>(S.a2, a2, col0, lane);
+        float out[2][4];
+        layer16<2, 2, mlps::kPadHid>(out, a2, S.w.w3, S.w.b3, lane);
+        __syncthreads();  // the targets
+        // dY as the next product's A operand
+        float dy[2][4];
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int r = col0 + g + (e >> 1) * 8, c = nt * 8 + 2 * t + (e & 1);
+                float d = 0.0f;
+                if (c < mlps::kUsedOut && S.rows.y[r][kUsedOut] != 0.0f) d = out[nt][e] - S.rows.y[r][c];
+                lsum += d * d;
+                dy[nt][e] = 2.0f * d;
+            }
+        uint32_t ady[1][4], dz2[2][4], dz1[2][4];
+        c_to_a16<false, 1>(dy, ady);
         store_t<1>(S.dy, ady, col0, lane);
+        // backward through the layers
+        layer16<4, 1, mlps::kPadIn>(acc, ady, S.w3t, nullptr, lane);  // dY W3
+        masked_to_a(acc, mask2, dz2);
         store_t<2>(S.dz2, dz2, col0, lane);
+        layer16<4, 2, mlps::kPadHid>(acc, dz2, S.w2t, nullptr, lane);  // dZ2 W2
+        masked_to_a(acc, mask1, dz1);
         store_t<2>(S.dz1, dz1, col0, lane);
         __syncthreads();
-        // warp w: rows 16 (w / 2).. and half the columns of dW2, dW1; 8 columns of dW3
-        const int m0 = 16 * (warp >> 1), half = warp & 1;
-        wgrad_tile<2>(S.dz2, S.a1, m0, 16 * half, part + mlps::kW2, mlps::kHid, half ? nullptr : part + mlps::kB2, add,
-                      lane);
-        wgrad_tile<1>(S.dz1, S.x, m0, 8 * half, part + mlps::kW1, mlps::kIn, half ? part + mlps::kB1 : nullptr, add,
-                      lane);
-        wgrad_tile<1>(S.dy, S.a2, 0, 8 * warp, part + mlps::kW3, mlps::kHid, warp == 0 ? part + mlps::kB3 : nullptr,
-                      add, lane);
+        // warp w: 8 columns of 16 rows of dW2; then dW1 (warps 0..3) and dW3 (warps 4..7)
+        wgrad_tile(S.dz2, S.a1, 16 * (warp >> 2), 8 * (warp & 3), part + mlps::kW2, mlps::kHid,
+                      (warp & 3) ? nullptr : part + mlps::kB2, add, lane);
+        if (warp < 4)
+            wgrad_tile(S.dz1, S.x, 16 * (warp >> 1), 8 * (warp & 1), part + mlps::kW1, mlps::kIn,
+                          (warp & 1) ? part + mlps::kB1 : nullptr, add, lane);
+        else
+            wgrad_tile(S.dy, S.a2, 0, 8 * (warp - 4), part + mlps::kW3, mlps::kHid,
+                          warp == 5 ? part + mlps::kB3 : nullptr, add, lane);
         add = true;
         __syncthreads();  // the next tile overwrites what the products read
     }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, off);
-    if (lane == 0) S.loss[warp] = loss;
-    __syncthreads();
-    if (tid == 0) a.loss_part[blockIdx.x] = (S.loss[0] + S.loss[1]) + (S.loss[2] + S.loss[3]);
+    put_loss(lsum, S.loss, a.loss_part + blockIdx.x);
 }
 
 struct AdamArgs {
@@ -821,51 +1133,61 @@ struct AdamArgs {
     float* grad;
     __half* w16;
     __half* wt16;
-    const float* part;       // [blocks][parameters] partial gradients, or null (conversion only)
+    const float* part;       // [parts][parameters] partial gradients, or null (conversion only)
     const float* loss_part;  // [blocks]
-    uint32_t blocks;
+    uint32_t parts, blocks;
     float* loss;             // the batch's sum of squared errors, nullable
     float lr_t, beta1, beta2, eps_t, gscale;
     int update;              // 1: Adam step; 0: the summed gradient into grad, parameters as they are
 };
 
-constexpr int kAdamParams = 64, kAdamSplit = 4;  // parameters per block, threads that share one's slices
+constexpr int kAdamParams = 32, kAdamSplit = 16;  // parameters per block, threads that share one's slices
 
-// The sum over the blocks' partial gradients, then Adam (Kingma and Ba 2015)
+// The sum of the partial gradients, then Adam (Kingma and Ba 2015)
 // with the bias corrections folded into lr_t and eps_t, then the FP16 forward
-// (and, for the 4 x 64 network, transposed) copies.  Four threads share a
-// parameter's slices (7.5 MB for 128 blocks of the 4 x 64 network, in L2) and
-// add up in a fixed order.
+// (and, for the 4 x 64 network, transposed) copies.  Sixteen threads share a
+// parameter's partials, so that each has its loads in flight at once, and add
+// up in a fixed order.
 template <int N, bool TRANSPOSED>
 __global__ void __launch_bounds__(kAdamParams* kAdamSplit) adam_kernel(const AdamArgs a) {
     __shared__ float s_sum[kAdamSplit][kAdamParams];
     const int q = threadIdx.x % kAdamParams, split = threadIdx.x / kAdamParams;
     const int i = blockIdx.x * kAdamParams + q;
-    float gr = 0.0f;
+    wait_for_previous_kernel();
+    const bool own = split == 0 && i < N;
+    float p = 0.0f, m = 0.0f, v = 0.0f, gr = 0.0f;
+    if (own) {
+        p = a.params[i];
+        if (a.update) {
+            m = a.m[i];
+            v = a.v[i];
+        }
+    }
     if (a.part && i < N) {
 #pragma unroll 8
-        for (uint32_t b = split; b < a.blocks; b += kAdamSplit) gr += __ldcg(&a.part[(size_t)b * N + i]);
+        for (uint32_t b = split; b < a.parts; b += kAdamSplit) gr += __ldcg(&a.part[(size_t)b * N + i]);
     }
     s_sum[split][q] = gr;
-    if (a.loss && blockIdx.x == 0 && threadIdx.x < 32) {
+    if (a.loss && blockIdx.x == 0 && split == 1) {
         float l = 0.0f;
-        for (uint32_t b = threadIdx.x; b < a.blocks; b += 32) l += __ldcg(&a.loss_part[b]);
+        for (uint32_t b = q; b < a.blocks; b += kAdamParams) l += __ldcg(&a.loss_part[b]);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-        if (threadIdx.x == 0) *a.loss = l;
+        if (q == 0) *a.loss = l;
     }
     __syncthreads();
-    if (split != 0 || i >= N) return;
-    gr = (s_sum[0][q] + s_sum[1][q]) + (s_sum[2][q] + s_sum[3][q]);
+    if (!own) return;
+    gr = 0.0f;
+#pragma unroll
+    for (int s = 0; s < kAdamSplit; ++s) gr += s_sum[s][q];
     if (a.part && !a.update) {
         a.grad[i] = gr;
         return;
     }
-    float p = a.params[i];
     if (a.update) {
         gr *= a.gscale;
-        const float m = a.beta1 * a.m[i] + (1.0f - a.beta1) * gr;
-        const float v = a.beta2 * a.v[i] + (1.0f - a.beta2) * gr * gr;
+        m = a.beta1 * m + (1.0f - a.beta1) * gr;
+        v = a.beta2 * v + (1.0f - a.beta2) * gr * gr;
         a.m[i] = m;
         a.v[i] = v;
         p -= a.lr_t * m / (sqrtf(v) + a.eps_t);
@@ -949,6 +1271,8 @@ cudaError_t ensure_device_setup(int device) {
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem);
         if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgradSmem);
+        if (e == cudaSuccess)
             e = cudaFuncSetAttribute(infer_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)tc::kSmemBytes);
         if (e == cudaSuccess)
@@ -977,20 +1301,61 @@ hg_status cuda_fail(hg_ctx* ctx, cudaError_t e, const char* where) {
     } while (0)
 
 // Most blocks a training launch uses: one (the 4 x 64 network, whose tile
-// fills an SM's shared memory) or two per SM; a block with several tiles adds
-// them up in its slice.
+// fills an SM's shared memory) or two per SM.
 uint32_t max_train_blocks(const hg_mlp* m) {
     return (uint32_t)m->ctx->sm_count * (m->arch == HG_MLP_ARCH_COMPACT ? 2u : 1u);
 }
 
-uint32_t train_blocks(const hg_mlp* m, uint32_t n) {
-    return std::min(n / kTrainTile + (n % kTrainTile != 0u), max_train_blocks(m));
+uint32_t train_tiles(uint32_t n) { return n / kTrainTile + (n % kTrainTile != 0u); }
+
+uint32_t train_blocks(const hg_mlp* m, uint32_t n) { return std::min(train_tiles(n), max_train_blocks(m)); }
+
+// Partial gradients of a batch of n: one per chunk of tiles (4 x 64) or per block.
+uint32_t train_parts(const hg_mlp* m, uint32_t n) {
+    if (m->arch == HG_MLP_ARCH_COMPACT) return train_blocks(m, n);
+    return (train_tiles(n) + kChunkTiles - 1) / kChunkTiles;
 }
 
-// The FP16 copies of the parameters; with `blocks` partial gradients (and
-// losses) in m->part, first their sum and either an Adam step (update) or
-// the summed gradient into m->grad.
-cudaError_t convert(hg_mlp* m, uint32_t blocks, int update, float lr_t, float eps_t, float gscale, float* loss) {
+// 4 x 64: the tiles' activations and the chunks' partial gradients, grown to n
+// samples (the compact network's partials are allocated with it).
+cudaError_t ensure_scratch(hg_mlp* m, uint32_t n) {
+    const uint32_t tiles = train_tiles(n);
+    if (m->arch == HG_MLP_ARCH_COMPACT || tiles <= m->tile_capacity) return cudaSuccess;
+    cudaStreamSynchronize(m->ctx->stream);
+    if (m->acts) cudaFree(m->acts);
+    m->acts = nullptr;
+    m->part = nullptr;
+    m->tile_capacity = 0;
+    const size_t acts = sizeof(TileActs) * (size_t)tiles;
+    cudaError_t e = cudaMalloc(&m->acts, acts + sizeof(float) * (size_t)m->n_params * train_parts(m, n));
+    if (e != cudaSuccess) return e;
+    m->part = reinterpret_cast<float*>(static_cast<char*>(m->acts) + acts);
+    m->tile_capacity = tiles;
+    return cudaSuccess;
+}
+
+// A launch that may be placed while the stream's previous kernel finishes
+// (see wait_for_previous_kernel).
+template <class Args>
+cudaError_t launch_dependent(void (*kernel)(const Args), dim3 grid, int threads, size_t smem, cudaStream_t stream,
+                             const Args& args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args);
+}
+
+// The FP16 copies of the parameters; after a training launch of n > 0 samples,
+// first the sum of its partial gradients and either an Adam step (update) or
+// the sum into m->grad.
+cudaError_t convert(hg_mlp* m, uint32_t n, int update, float lr_t, float eps_t, float gscale, float* loss) {
     AdamArgs a;
     a.params = m->params;
     a.m = m->adam_m;
@@ -998,10 +1363,11 @@ cudaError_t convert(hg_mlp* m, uint32_t blocks, int update, float lr_t, float ep
     a.grad = m->grad;
     a.w16 = reinterpret_cast<__half*>(m->w16);
     a.wt16 = reinterpret_cast<__half*>(m->wt16);
-    a.part = blocks ? m->part : nullptr;
-    a.loss_part = m->part + (size_t)max_train_blocks(m) * m->n_params;
-    a.blocks = blocks;
-    a.loss = blocks ? loss : nullptr;
+    a.part = n ? m->part : nullptr;
+    a.loss_part = m->loss_part;
+    a.parts = n ? train_parts(m, n) : 0u;
+    a.blocks = n ? train_blocks(m, n) : 0u;
+    a.loss = n ? loss : nullptr;
     a.lr_t = lr_t;
     a.beta1 = 0.9f;
     a.beta2 = 0.999f;
@@ -1010,15 +1376,14 @@ cudaError_t convert(hg_mlp* m, uint32_t blocks, int update, float lr_t, float ep
     a.update = update;
     const uint32_t grid = (m->n_params + kAdamParams - 1) / kAdamParams;
     const int threads = kAdamParams * kAdamSplit;
-    if (m->arch == HG_MLP_ARCH_COMPACT)
-        adam_kernel<mlps::kParams, false><<<grid, threads, 0, m->ctx->stream>>>(a);
-    else
-        adam_kernel<kParams, true><<<grid, threads, 0, m->ctx->stream>>>(a);
-    return cudaGetLastError();
+    return m->arch == HG_MLP_ARCH_COMPACT
+               ? launch_dependent(adam_kernel<mlps::kParams, false>, dim3(grid), threads, 0, m->ctx->stream, a)
+               : launch_dependent(adam_kernel<kParams, true>, dim3(grid), threads, 0, m->ctx->stream, a);
 }
 
-// Forward, backward and weight gradients of n samples into m->part:
-// train_blocks(m, n) partial gradients and losses.
+// Forward, backward and weight gradients of n samples into m->part (sized by
+// ensure_scratch): train_parts(m, n) partial gradients, train_blocks(m, n)
+// losses.
 cudaError_t run_gradients(hg_mlp* m, const float* inputs, const float* targets, uint32_t n) {
     TrainArgs a;
     a.inputs = inputs;
@@ -1027,14 +1392,21 @@ cudaError_t run_gradients(hg_mlp* m, const float* inputs, const float* targets, 
     a.w16 = reinterpret_cast<const __half*>(m->w16);
     a.wt16 = reinterpret_cast<const __half*>(m->wt16);
     a.params = m->params;
+    a.acts = static_cast<TileActs*>(m->acts);
     a.part = m->part;
-    a.loss_part = m->part + (size_t)max_train_blocks(m) * m->n_params;
+    a.loss_part = m->loss_part;
+    const cudaStream_t st = m->ctx->stream;
     const uint32_t blocks = train_blocks(m, n);
     if (m->arch == HG_MLP_ARCH_COMPACT)
-        small_train_kernel<<<blocks, kTrainTile, kSmallTrainSmem, m->ctx->stream>>>(a);
-    else
-        train_kernel<<<blocks, kTrainTile, kTrainSmem, m->ctx->stream>>>(a);
-    return cudaGetLastError();
+        return launch_dependent(small_train_kernel, dim3(blocks), kTrainThreads, kSmallTrainSmem, st, a);
+    cudaError_t e = launch_dependent(train_kernel, dim3(blocks), kTrainThreads, kTrainSmem, st, a);
+    if (e != cudaSuccess) return e;
+    WgradArgs w;
+    w.acts = a.acts;
+    w.tiles = train_tiles(n);
+    w.part = m->part;
+    w.err = m->ctx->err;
+    return launch_dependent(wgrad_kernel, dim3(train_parts(m, n), kWgradUnits), kWgradThreads, kWgradSmem, st, w);
 }
 
 }  // namespace
@@ -1100,19 +1472,34 @@ hg_status hg_mlp_create_arch(hg_ctx* ctx, uint32_t arch, hg_mlp** out) {
     m->ctx = ctx;
     m->arch = arch;
     m->n_params = arch == HG_MLP_ARCH_COMPACT ? (uint32_t)hg::mlps::kParams : (uint32_t)hg::mlp::kParams;
+    // one allocation, each array on a 256-byte boundary
+    size_t bytes = 0;
+    auto place = [&](size_t n) {
+        const size_t at = bytes;
+        bytes += (n + 255u) & ~(size_t)255u;
+        return at;
+    };
     const size_t pf = sizeof(float) * m->n_params;
-    cudaError_t e = cudaMalloc(&m->params, pf);
-    if (e == cudaSuccess) e = cudaMalloc(&m->grad, pf);
-    if (e == cudaSuccess) e = cudaMalloc(&m->adam_m, pf);
-    if (e == cudaSuccess) e = cudaMalloc(&m->adam_v, pf);
-    if (e == cudaSuccess) e = cudaMalloc(&m->w16, sizeof(__half) * m->n_params);
-    if (e == cudaSuccess && arch == HG_MLP_ARCH_DEEP)
-        e = cudaMalloc(&m->wt16, sizeof(__half) * hg::mlp::kTransposed);
-    if (e == cudaSuccess) e = cudaMalloc(&m->loss, sizeof(float));
-    if (e == cudaSuccess)
-        e = cudaMalloc(&m->part, sizeof(float) * (size_t)hg::max_train_blocks(m) * (m->n_params + 1u));
-    for (void* p : {(void*)m->params, (void*)m->adam_m, (void*)m->adam_v})
-        if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, pf, ctx->stream);
+    const size_t at_params = place(pf), at_m = place(pf), at_v = place(pf), zeroed = bytes, at_grad = place(pf),
+                 at_w16 = place(sizeof(__half) * m->n_params),
+                 at_wt16 = place(arch == HG_MLP_ARCH_DEEP ? sizeof(__half) * hg::mlp::kTransposed : 0),
+                 at_loss = place(sizeof(float)),
+                 at_loss_part = place(sizeof(float) * hg::max_train_blocks(m)),
+                 at_part = place(arch == HG_MLP_ARCH_COMPACT ? pf * hg::max_train_blocks(m) : 0);
+    cudaError_t e = cudaMalloc(&m->arena, bytes);
+    if (e == cudaSuccess) {
+        char* base = static_cast<char*>(m->arena);
+        m->params = reinterpret_cast<float*>(base + at_params);
+        m->adam_m = reinterpret_cast<float*>(base + at_m);
+        m->adam_v = reinterpret_cast<float*>(base + at_v);
+        m->grad = reinterpret_cast<float*>(base + at_grad);
+        m->w16 = base + at_w16;
+        m->wt16 = arch == HG_MLP_ARCH_DEEP ? base + at_wt16 : nullptr;
+        m->loss = reinterpret_cast<float*>(base + at_loss);
+        m->loss_part = reinterpret_cast<float*>(base + at_loss_part);
+        m->part = arch == HG_MLP_ARCH_COMPACT ? reinterpret_cast<float*>(base + at_part) : nullptr;
+        e = cudaMemsetAsync(m->arena, 0, zeroed, ctx->stream);
+    }
     if (e == cudaSuccess) e = hg::convert(m, 0, 0, 0.0f, 0.0f, 0.0f, nullptr);
     if (e != cudaSuccess) {
         hg_mlp_destroy(m);
@@ -1130,9 +1517,8 @@ void hg_mlp_destroy(hg_mlp* m) {
         cudaStreamSynchronize(ctx->stream);
         if (ctx->surrogate == m) ctx->surrogate = nullptr;
     }
-    for (void* p : {(void*)m->params, (void*)m->grad, (void*)m->adam_m, (void*)m->adam_v, (void*)m->w16,
-                    (void*)m->wt16, (void*)m->loss, (void*)m->part})
-        if (p) cudaFree(p);
+    if (m->arena) cudaFree(m->arena);
+    if (m->acts) cudaFree(m->acts);
     delete m;
 }
 
@@ -1185,16 +1571,20 @@ hg_status hg_mlp_samples(hg_ctx* ctx, uint64_t seed, uint64_t first, uint32_t co
     a.inputs = inputs;
     a.targets = targets;
     a.lobes = lobes;
-    // A lane per sample while that gives every SM a block; below, eight lanes
-    // share a sample's 32 nodes (1,000 samples: 0.98 ms with one lane, 0.20 ms
-    // with eight).
-    if (count >= (uint32_t)ctx->sm_count * hg::kSampleThreads) {
-        const uint32_t blocks = (count + hg::kSampleThreads - 1u) / hg::kSampleThreads;
-        hg::samples_kernel<1><<<blocks, hg::kSampleThreads, 0, ctx->stream>>>(a);
-    } else {
-        const uint32_t per = hg::kSampleThreads / 8u;
-        hg::samples_kernel<8><<<(count + per - 1u) / per, hg::kSampleThreads, 0, ctx->stream>>>(a);
-    }
+    // As many lanes share a sample's 32 nodes as leave at most one 128-thread
+    // block per SM: the FP64 pipe is then still one warp deep everywhere.  The
+    // lanes repeat the work outside the nodes, so more of them than that lose
+    // (19,000 samples on 152 SMs: 0.98 ms with one lane, 1.61 ms with eight;
+    // 1,000 samples: 0.98 and 0.20 ms).
+    const uint64_t room = (uint64_t)ctx->sm_count * hg::kSampleThreads;
+    const uint32_t lanes = (uint64_t)count * 8u <= room ? 8u : (uint64_t)count * 4u <= room ? 4u
+                           : (uint64_t)count * 2u <= room ? 2u : 1u;
+    const uint32_t per = hg::kSampleThreads / lanes;
+    const uint32_t blocks = count / per + (count % per != 0u);
+    if (lanes == 8u) hg::samples_kernel<8><<<blocks, hg::kSampleThreads, 0, ctx->stream>>>(a);
+    else if (lanes == 4u) hg::samples_kernel<4><<<blocks, hg::kSampleThreads, 0, ctx->stream>>>(a);
+    else if (lanes == 2u) hg::samples_kernel<2><<<blocks, hg::kSampleThreads, 0, ctx->stream>>>(a);
+    else hg::samples_kernel<1><<<blocks, hg::kSampleThreads, 0, ctx->stream>>>(a);
     MLP_CUDA(ctx, cudaGetLastError());
     return HG_OK;
 }
@@ -1225,8 +1615,9 @@ hg_status hg_mlp_gradients(hg_mlp* m, const float* inputs, const float* targets,
     if (count == 0 || !inputs || !targets || !grad) return fail(ctx, HG_INVALID_ARG, "empty batch or null buffer");
     MLP_CUDA(ctx, cudaPeekAtLastError());
     const size_t pf = sizeof(float) * m->n_params;
+    MLP_CUDA(ctx, hg::ensure_scratch(m, count));
     MLP_CUDA(ctx, hg::run_gradients(m, inputs, targets, count));
-    MLP_CUDA(ctx, hg::convert(m, hg::train_blocks(m, count), 0, 0.0f, 0.0f, 0.0f, m->loss));
+    MLP_CUDA(ctx, hg::convert(m, count, 0, 0.0f, 0.0f, 0.0f, m->loss));
     MLP_CUDA(ctx, cudaMemcpyAsync(grad, m->grad, pf, cudaMemcpyDeviceToHost, ctx->stream));
     float l = 0.0f;
     MLP_CUDA(ctx, cudaMemcpyAsync(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
@@ -1242,12 +1633,13 @@ hg_status hg_mlp_train_step(hg_mlp* m, const float* inputs, const float* targets
     if (count == 0 || !inputs || !targets) return fail(ctx, HG_INVALID_ARG, "empty batch or null buffer");
     if (!(lr >= 0.0f) || !std::isfinite(lr)) return fail(ctx, HG_INVALID_ARG, "learning rate must be finite, >= 0");
     MLP_CUDA(ctx, cudaPeekAtLastError());
+    MLP_CUDA(ctx, hg::ensure_scratch(m, count));
     MLP_CUDA(ctx, hg::run_gradients(m, inputs, targets, count));
     m->step += 1;
     const double b1t = 1.0 - std::pow(0.9, (double)m->step), b2t = 1.0 - std::pow(0.999, (double)m->step);
     const float lr_t = (float)(lr * std::sqrt(b2t) / b1t);
     const float eps_t = (float)(1e-8 * std::sqrt(b2t));
-    MLP_CUDA(ctx, hg::convert(m, hg::train_blocks(m, count), 1, lr_t, eps_t,
+    MLP_CUDA(ctx, hg::convert(m, count, 1, lr_t, eps_t,
                               1.0f / ((float)count * (float)hg_mlp_output_count(m)), loss_sum));
     return HG_OK;
 }

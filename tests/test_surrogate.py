@@ -226,11 +226,12 @@ def test_gpu_samples_match_the_fp64_integrator(renderer):
 
 
 @gpu
-@pytest.mark.parametrize("n", [1, 15, 17, 19_455, 19_456, 19_500])
+@pytest.mark.parametrize("n", [1, 17, 2432, 2433, 4864, 4865, 9728, 9729, 19_500])
 def test_samples_at_the_edges_of_the_lane_split(renderer, n):
-    """Eight lanes a sample below sm_count x 128 samples (19,456 on 152 SMs),
-    one from there on, ragged last blocks: the integrator's lobes either way,
-    with the bounds of the test above, and nothing written past the end."""
+    """Eight, four, two or one lanes share a sample (the lines lie at 1/8, 1/4
+    and 1/2 of sm_count x 128 samples, 19,456 on 152 SMs), ragged last blocks:
+    the integrator's lobes either way, with the bounds of the test above, and
+    nothing written past the end."""
     torch, dev = _torch()
     x = torch.full((n + 1, 10), 7.0, dtype=torch.float32, device=dev)
     lob = torch.full((n + 1, 12), 7.0, dtype=torch.float64, device=dev)
@@ -483,6 +484,42 @@ def test_compact_forward_matches_the_oracle_emulation(renderer, which):
         assert np.abs(got - want).mean() < 1e-3
         np.testing.assert_allclose(got, want, rtol=0, atol=3e-2)
         np.testing.assert_allclose(lob_all[:n], 1e-3 * np.expm1(np.maximum(got, 0)), rtol=1e-5, atol=1e-9)
+    s.close()
+
+
+@gpu
+@pytest.mark.parametrize("arch", [0, COMPACT])
+@pytest.mark.parametrize("n", [127, 128, 129, 2049, 19_457, 38_913])
+def test_gradients_at_the_edges_of_the_training_tiles(renderer, arch, n):
+    """Ragged and whole 128-sample tiles, and batches whose blocks take a second
+    tile (beyond 152 tiles, the compact network beyond 304), against the FP64
+    reference with the bounds of the two tests of 3,000 samples; the same batch
+    twice gives the same gradient, and training steps agree with Adam applied
+    to it."""
+    torch, dev = _torch()
+    xs = _inputs(n, 31)
+    ts = np.log1p(oracle.lobes(xs, tilt=TILT, model="karis") / 1e-3).astype(np.float32)
+    x, t = torch.from_numpy(xs).to(dev), torch.from_numpy(ts).to(dev)
+    p = S.init_params(23, arch)
+    s = S.Surrogate(renderer, p, arch)
+    g, loss = s.gradients(x, t, n)
+    want, want_loss = mlp_ref.gradients(p, xs, ts, arch=arch)
+    assert loss == pytest.approx(want_loss, rel=2e-3)
+    err = np.linalg.norm(g - want) / np.linalg.norm(want)
+    assert err < (5e-3 if arch == COMPACT else 2e-2), err
+    again, loss2 = s.gradients(x, t, n)
+    np.testing.assert_array_equal(again, g)
+    assert loss2 == loss
+    got_loss = torch.zeros(1, dtype=torch.float32, device=dev)
+    s.train_step(x, t, n, 1e-3, got_loss)
+    renderer.synchronize()
+    assert float(got_loss) == loss
+    # the first Adam step moves a parameter by lr g / (|g| + eps); the kernel's
+    # float32 1 - 0.999f is 1.3e-5 off 0.001, half of it under the root (6.4e-9
+    # of a step of 1e-3), and p itself rounds
+    gm = g.astype(np.float64) / (n * s.n_out)
+    step = 1e-3 * gm / (np.abs(gm) + 1e-8)
+    np.testing.assert_allclose(s.get_params(), p - step, rtol=2e-7, atol=2e-8)
     s.close()
 
 
