@@ -12,7 +12,12 @@ namespace hg {
 namespace {
 
 constexpr int kFilterRadius = 5;
-constexpr int kTileX = 32, kTileY = 8;
+
+// Images of at most this many pixels give a pair four threads, or two.
+// Measured (us): 96 x 64: 10.3 with four, 14.4 with two, 16.5 with one;
+// 640 x 360: 20.6, 26.2, 20.8; 512 x 512: 30.8, 28.7 (64 registers), 33.0;
+// 960 x 540: 33.4, 29.0, 32.7; 1280 x 720: 51.1, 45.1, 36.6.
+constexpr uint64_t kFilterSplit4 = 240u * 1024u, kFilterSplit2 = 512u * 1024u;
 
 struct FilterArgs {
     hg_hair_params p;
@@ -46,92 +51,186 @@ __device__ __forceinline__ float sqrt_bound(float r) {
     return x;
 }
 
+// Taps of row dy of a pixel's window whose distance from the strand's line
+// through the pixel is at most half a pixel (the strip of filter.wgsl:63), as
+// bits dx + 5.  The line distance is |dx ts.y - dy ts.x|, so the taps form an
+// interval of dx, found from its two ends; filter.wgsl's own float expression
+// (below) lies within 1.5e-6 of that distance, and a row with an end within
+// 1e-5 (in distance) of an integer dx, or one without finite ends (a
+// horizontal tangent), is decided tap by tap with that expression, rounding
+// for rounding.  strip2: the largest x with sqrt_rn(x) <= 1/2.
+__device__ __forceinline__ uint32_t strip_row(float2 ts, float inv_ty, int dy, float strip2) {
+    const float mid = (float)dy * ts.x * inv_ty, half = 0.5f * fabsf(inv_ty), slack = 1e-5f * fabsf(inv_ty);
+    const float lo = mid - half, hi = mid + half;
+    if (fabsf(lo - rintf(lo)) > slack && fabsf(hi - rintf(hi)) > slack) {
+        const int jl = max(f2i(ceilf(lo)), -kFilterRadius), jh = min(f2i(floorf(hi)), kFilterRadius);
+        return jl > jh ? 0u : (2u << (jh + kFilterRadius)) - (1u << (jl + kFilterRadius));
+    }
+    uint32_t m = 0;
+#pragma unroll
+    for (int dx = -kFilterRadius; dx <= kFilterRadius; ++dx) {
+        const float fdx = (float)dx, fdy = (float)dy;
+        const float d_par = fdx * ts.x + fdy * ts.y;
+        const float ex = fdx - ts.x * d_par, ey = fdy - ts.y * d_par;
+        // d_perp = sqrt_rn(e2); d_perp <= 0.5 exactly when e2 <= strip2
+        const float e2 = ex * ex + ey * ey;
+        if (e2 <= strip2) m |= 1u << (dx + kFilterRadius);
+    }
+    return m;
+}
+
+__device__ __forceinline__ float ex2(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// One pixel of a thread's pair: what its taps are weighed against, and its
+// sums.
+struct FilterPixel {
+    float2 ts;
+    float inv_ty;
+    float cx, cy, cz, p_norm;          // centre colour, normalised depth
+    float a, b, c;                     // dx^2, dx dy and dy^2 factors of a tap's exponent
+    float ax, ay, az, weight;          // weighted colour and weight
+    int h_center, h_cons;              // strip taps with a centre hit, with a conservative hit only
+    bool use_color;
+};
+
+// P's sums over tap's colour with weight w, where `keep`.
+__device__ __forceinline__ void accumulate(bool keep, float4 tap, float w, FilterPixel& P) {
+    asm("{\n.reg .pred p;\nsetp.ne.u32 p, %8, 0;\n"
+        "@p fma.rn.f32 %0, %4, %7, %0;\n@p fma.rn.f32 %1, %5, %7, %1;\n@p fma.rn.f32 %2, %6, %7, %2;\n"
+        "@p add.rn.f32 %3, %3, %7;\n}\n"
+        : "+f"(P.ax), "+f"(P.ay), "+f"(P.az), "+f"(P.weight)
+        : "f"(tap.x), "f"(tap.y), "f"(tap.z), "f"(w), "r"((uint32_t)keep));
+}
+
 // One TX x TY tile per CTA (tile (bx, by) of view a: fields p, center, cons,
-// shaded, filtered, filtered_depth).  The (TX+10) x (TY+10) neighbourhood is
-// staged in shared memory once: per texel the centre word's normalised depth
-// f32(depth)/16777214 (the exact value filter.wgsl:94 computes per tap; -1
-// marks an empty centre with a conservative hit, -2 both empty) and the shaded
-// colour.  Pixels without hair are written at once; the tile's hair pixels
-// are then listed and handed to the first threads, one each, so the 121-tap
-// loop runs in full warps instead of the lanes of the hair pixels of every
-// row.  Coverage decisions use exact arithmetic; the colour weights only
-// scale colour, so they use the fast exponential.
-template <int TX, int TY, class V>
+// shaded, filtered, filtered_depth), TX TY S / 2 threads.  The (TX+10) x (TY+10)
+// neighbourhood is staged in shared memory once: per texel the shaded colour
+// and the centre word's normalised depth f32(depth)/16777214 (the exact value
+// filter.wgsl:94 computes per tap; -1 marks an empty centre with a
+// conservative hit, -2 both empty or off screen), and per row two bit masks of
+// the texels with either kind of hit.  Pixels without hair are written at
+// once; pairs of vertically adjacent pixels with hair in either are then
+// listed and handed to the first threads, so the tap loop runs in full warps.
+//
+// The tap loop is bound by instruction issue and shared-memory bandwidth.  A
+// pair shares its taps' loads (12 rows for 2 x 11); the strip counts come from
+// bit masks (strip_row), row by row, instead of a distance and two tests per
+// tap; the spatial exponent is a quadratic form in (dx, dy) with one add and
+// one FMA per tap; and the depth test alone also rejects the texels without a
+// centre hit.  S threads (1, 2 or 4) share a pair, 12 / S rows each, and add
+// up by shuffles: small images leave the chip idle otherwise.  Coverage
+// decisions use exact arithmetic; the colour weights only scale colour, so
+// they use fused operations and the fast exponential.  Against a thread per pixel with 121 tests and a
+// distance each (us): 1920 x 1080 113 -> 79, 3840 x 2160 200 -> 141, 512 x 512
+// 42 -> 29, 96 x 64 22 -> 10.
+template <int TX, int TY, int S, class V>
 __device__ __forceinline__ void filter_tile(const V& a, int32_t bx, int32_t by) {
     constexpr int kHaloX = TX + 2 * kFilterRadius, kHaloY = TY + 2 * kFilterRadius;
-    constexpr int kWarps = TX * TY / 32;
-    static_assert(TX * TY % 32 == 0, "whole warps per tile");
-    __shared__ float s_norm[kHaloY][kHaloX];
-    __shared__ float4 s_col[kHaloY][kHaloX];
-    __shared__ uint16_t s_list[TX * TY];
-    __shared__ int s_warp_hair[kWarps];
+    constexpr int kPairs = TX * TY / 2, kThreads = kPairs * S, kWarps = kThreads / 32, kPairWarps = kPairs / 32;
+    constexpr int kRows = 2 * kFilterRadius + 2;  // rows a pair's two windows cover
+    static_assert(kPairs % 32 == 0 && kRows % S == 0 && kHaloX <= 64 && TX <= 32, "tile shape");
+    __shared__ float4 s_tap[kHaloY][kHaloX];  // colour, normalised depth or mark
+    __shared__ uint4 s_hits[kHaloY];          // bit per texel: centre hit (x, y), conservative hit only (z, w)
+    __shared__ uint16_t s_list[kPairs];       // pair | hair in its upper / lower pixel << 14, 15
+    __shared__ int s_warp_hair[kPairWarps];
     const hg_hair_params& p = a.p;
     const int32_t width = f2i(p.screen[0]), height = f2i(p.screen[1]);
     const int32_t x0 = bx * TX - kFilterRadius, y0 = by * TY - kFilterRadius;
-    const int tid = threadIdx.y * TX + threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int total = 0;
     {
-        const int32_t ox = bx * TX + threadIdx.x, oy = by * TY + threadIdx.y;
-        const bool own_inside = ox < width && oy < height;
-        const uint32_t own = (uint32_t)oy * (uint32_t)width + (uint32_t)ox;
-        const bool own_hair = own_inside && (!is_empty(__ldg(&a.center[own])) || !is_empty(__ldg(&a.cons[own])));
-        // pixels without hair (and every pixel of a tile without hair, which
-        // needs no halo) are written now
-        if (own_inside && !own_hair) {
-            a.filtered[own] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            a.filtered_depth[own] = 0.0f;
-        }
-        const uint32_t ballot = __ballot_sync(0xffffffffu, own_hair);
-        if ((tid & 31) == 0) s_warp_hair[tid >> 5] = __popc(ballot);
-        __syncthreads();
-        int base = 0, total = 0;
+        uint32_t entry = 0;
+        if (tid < kPairs) {
+            const int32_t ox = bx * TX + tid % TX;
+            unsigned long long c[2] = {}, k[2] = {};
+            bool inside[2];
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            const int c = s_warp_hair[w];
-            base += w < (tid >> 5) ? c : 0;
-            total += c;
-        }
-        if (total == 0) return;
-        if (own_hair) s_list[base + __popc(ballot & ((1u << (tid & 31)) - 1u))] = (uint16_t)tid;
-        // the halo: per texel the normalised centre depth (or -1 / -2) and
-        // the shaded colour, as the tap loop reads them
-        for (int i = tid; i < kHaloX * kHaloY; i += TX * TY) {
-            const int hx = i % kHaloX, hy = i / kHaloX;
-            const int32_t gx = x0 + hx, gy = y0 + hy;
-            float nrm = -2.0f;
-            float4 col = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (gx >= 0 && gy >= 0 && gx < width && gy < height) {
-                const size_t q = (size_t)gy * width + gx;
-                const unsigned long long c = __ldg(&a.center[q]);
-                if (!is_empty(c)) {
-                    nrm = __fdiv_rn(__uint2float_rn((uint32_t)(c >> 40)), 16777214.0f);
-                    col = __ldg(&a.shaded[q]);
-                } else if (!is_empty(__ldg(&a.cons[q]))) {
-                    nrm = -1.0f;
+            for (int q = 0; q < 2; ++q) {
+                const int32_t oy = by * TY + 2 * (tid / TX) + q;
+                inside[q] = ox < width && oy < height;
+                const uint32_t own = (uint32_t)oy * (uint32_t)width + (uint32_t)ox;
+                if (inside[q]) {
+                    c[q] = __ldg(&a.center[own]);
+                    k[q] = __ldg(&a.cons[own]);
                 }
             }
-            s_norm[hy][hx] = nrm;
-            s_col[hy][hx] = col;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                if (!inside[q]) continue;
+                if (!is_empty(c[q]) || !is_empty(k[q])) {
+                    entry |= 1u << (14 + q);
+                } else {
+                    const uint32_t own = (uint32_t)(by * TY + 2 * (tid / TX) + q) * (uint32_t)width + (uint32_t)ox;
+                    a.filtered[own] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    a.filtered_depth[own] = 0.0f;
+                }
+            }
+        }
+        const uint32_t ballot = __ballot_sync(0xffffffffu, entry != 0u);
+        if (lane == 0 && warp < kPairWarps) s_warp_hair[warp] = __popc(ballot);
+        __syncthreads();
+        int base = 0;
+#pragma unroll
+        for (int w = 0; w < kPairWarps; ++w) {
+            const int n = s_warp_hair[w];
+            base += w < warp ? n : 0;
+            total += n;
+        }
+        if (total == 0) return;  // a tile without hair needs no neighbourhood
+        if (entry) s_list[base + __popc(ballot & ((1u << lane) - 1u))] = (uint16_t)(entry | (uint32_t)tid);
+        // the neighbourhood, a warp per row; a warp's loads are all issued
+        // before any is looked at
+        constexpr int kWarpRows = (kHaloY + kWarps - 1) / kWarps, kHalves = (kHaloX + 31) / 32;
+        unsigned long long word[kWarpRows][kHalves];
+        float4 tap[kWarpRows][kHalves];
+#pragma unroll
+        for (int i = 0; i < kWarpRows; ++i)
+#pragma unroll
+            for (int h = 0; h < kHalves; ++h) {
+                const int hy = warp + i * kWarps, hx = 32 * h + lane;
+                const int32_t gx = x0 + hx, gy = y0 + hy;
+                word[i][h] = kEmptyU64;
+                tap[i][h] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (hy < kHaloY && hx < kHaloX && gx >= 0 && gy >= 0 && gx < width && gy < height) {
+                    const size_t q = (size_t)gy * width + gx;
+                    word[i][h] = __ldg(&a.center[q]);
+                    tap[i][h] = __ldg(&a.shaded[q]);
+                }
+            }
+#pragma unroll
+        for (int i = 0; i < kWarpRows; ++i) {
+            const int hy = warp + i * kWarps;
+            if (hy >= kHaloY) break;
+            uint32_t hit[2] = {0u, 0u}, only[2] = {0u, 0u};
+#pragma unroll
+            for (int h = 0; h < kHalves; ++h) {
+                const int hx = 32 * h + lane;
+                const int32_t gx = x0 + hx, gy = y0 + hy;
+                float4 v = tap[i][h];
+                v.w = -2.0f;
+                if (!is_empty(word[i][h])) {
+                    v.w = __fdiv_rn(__uint2float_rn((uint32_t)(word[i][h] >> 40)), 16777214.0f);
+                } else if (hx < kHaloX && gx >= 0 && gy >= 0 && gx < width && gy < height &&
+                           !is_empty(__ldg(&a.cons[(size_t)gy * width + gx]))) {
+                    v.w = -1.0f;
+                }
+                if (hx < kHaloX) s_tap[hy][hx] = v;
+                hit[h] = __ballot_sync(0xffffffffu, v.w >= 0.0f);
+                only[h] = __ballot_sync(0xffffffffu, v.w == -1.0f);
+            }
+            if (lane == 0) s_hits[hy] = make_uint4(hit[0], hit[1], only[0], only[1]);
         }
         __syncthreads();
-        if (tid >= total) return;  // no hair pixel left for this thread
     }
-    // this thread's hair pixel
-    const int src = s_list[tid];
-    const int sx = src % TX, sy = src / TX;
-    const int32_t px = bx * TX + sx, py = by * TY + sy;
-    const uint32_t pix = (uint32_t)py * (uint32_t)width + (uint32_t)px;
-    const unsigned long long center_word = __ldg(&a.center[pix]);
-    const unsigned long long cons_word = __ldg(&a.cons[pix]);
-    const bool center_hit = !is_empty(center_word), cons_hit = !is_empty(cons_word);
-    const int lx = sx + kFilterRadius, ly = sy + kFilterRadius;
-    const unsigned long long w = center_hit ? center_word : cons_word;
-    const uint32_t high = (uint32_t)(w >> 32), low = (uint32_t)w;
-    const f3 tangent = oct_decode(high & 0xffu, low >> 24u);
-    const uint32_t depth_q = high >> 8u;
-    const float view_dist = dequantize_depth(depth_q, p.screen[2], p.screen[3]);
-    const f3 world = reconstruct_world(p, px, py, view_dist);
-    const float2 ts = screen_tangent(p, world, tangent);
-    const float4 cc = __ldg(&a.shaded[pix]);
+    const int slot = tid / S, sub = tid % S;
+    if (S == 1 && slot >= total) return;  // no pair left for this thread
+    const uint32_t entry = s_list[min(slot, total - 1)];
+    const int pair = (int)(entry & 0x3fffu), sx = pair % TX, sy = 2 * (pair / TX);
+    const int32_t px = bx * TX + sx;
 
     const float s_par = fmaxf(p.filter_params[0], 0.05f);
     const float s_perp = fmaxf(p.filter_params[1], 0.02f);
@@ -142,73 +241,128 @@ __device__ __forceinline__ void filter_tile(const V& a, int32_t bx, int32_t by) 
     const float k_perp = 1.4426950408889634f / (sigma_perp * sigma_perp);
     const float k_col = 1.4426950408889634f / (0.9f * 0.9f);
     const float depth_reject = 1.45e-3f, closer_eps = 5e-4f;
-    const float strip2 = sqrt_bound(0.5f);  // the strip half-width of filter.wgsl:63
-    const float p_norm = __fdiv_rn(__uint2float_rn(depth_q), 16777214.0f);
-    const bool promote = !center_hit;
-    const bool use_color = !promote && cc.w > 0.0f;
+    const float strip2 = sqrt_bound(0.5f);
 
-    float ax = 0.0f, ay = 0.0f, az = 0.0f, weight = 0.0f, h_center = 0.0f, h_cons = 0.0f;
+    FilterPixel P[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        FilterPixel& P_ = P[q];
+        const bool hair = (entry >> (14 + q)) & 1u;
+        const int32_t py = by * TY + sy + q;
+        const uint32_t pix = (uint32_t)py * (uint32_t)width + (uint32_t)px;
+        P_.ax = P_.ay = P_.az = P_.weight = 0.0f;
+        P_.h_center = P_.h_cons = 0;
+        P_.use_color = false;
+        P_.cx = P_.cy = P_.cz = 0.0f;
+        P_.ts = make_float2(1.0f, 0.0f);
+        P_.p_norm = 1e9f;  // no tap is near it
+        if (hair) {
+            const unsigned long long center_word = __ldg(&a.center[pix]);
+            const bool center_hit = !is_empty(center_word);
+            const unsigned long long w = center_hit ? center_word : __ldg(&a.cons[pix]);
+            const uint32_t high = (uint32_t)(w >> 32), low = (uint32_t)w, depth_q = high >> 8u;
+            const f3 tangent = oct_decode(high & 0xffu, low >> 24u);
+            const float view_dist = dequantize_depth(depth_q, p.screen[2], p.screen[3]);
+            P_.ts = screen_tangent(p, reconstruct_world(p, px, py, view_dist), tangent);
+            const float4 cc = __ldg(&a.shaded[pix]);
+            P_.cx = cc.x;
+            P_.cy = cc.y;
+            P_.cz = cc.z;
+            P_.p_norm = __fdiv_rn(__uint2float_rn(depth_q), 16777214.0f);
+            P_.use_color = center_hit && cc.w > 0.0f;
+        }
+        P_.inv_ty = 1.0f / P_.ts.y;
+        const float xx = P_.ts.x * P_.ts.x, yy = P_.ts.y * P_.ts.y;
+        P_.a = __fmaf_rn(xx, k_par, yy * k_perp);
+        P_.b = 2.0f * P_.ts.x * P_.ts.y * (k_par - k_perp);
+        P_.c = __fmaf_rn(yy, k_par, xx * k_perp);
+    }
+
 #pragma unroll 1
-    for (int dy = -kFilterRadius; dy <= kFilterRadius; ++dy) {
-        const int32_t qy = py + dy;
-        if (qy < 0 || qy >= height) continue;
+    for (int r = sub * (kRows / S); r < (sub + 1) * (kRows / S); ++r) {
+        const uint4 hits = s_hits[sy + r];
+        const float4* row = &s_tap[sy + r][sx + kFilterRadius];
+        // window rows: dy = r - 5 of the upper pixel, r - 6 of the lower
+        float base[2][kFilterRadius + 1], slope[2], reject[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int dy = r - kFilterRadius - q;
+            const bool in = dy >= -kFilterRadius && dy <= kFilterRadius;
+            reject[q] = in ? depth_reject : -1.0f;
+            slope[q] = P[q].b * (float)dy;
+            const float c = P[q].c * (float)(dy * dy);
+#pragma unroll
+            for (int k = 0; k <= kFilterRadius; ++k) base[q][k] = __fmaf_rn(P[q].a, (float)(k * k), c);
+            if (in) {
+                const uint32_t strip = strip_row(P[q].ts, P[q].inv_ty, dy, strip2);
+                P[q].h_center += __popc(__funnelshift_r(hits.x, hits.y, sx) & strip);
+                P[q].h_cons += __popc(__funnelshift_r(hits.z, hits.w, sx) & strip);
+            }
+        }
 #pragma unroll
         for (int dx = -kFilterRadius; dx <= kFilterRadius; ++dx) {
-            const int32_t qx = px + dx;
-            if (qx < 0 || qx >= width) continue;
-            const float fdx = (float)dx, fdy = (float)dy;
-            const float d_par = fdx * ts.x + fdy * ts.y;
-            const float ex = fdx - ts.x * d_par, ey = fdy - ts.y * d_par;
-            // d_perp = sqrt_rn(e2); d_perp <= 0.5 exactly when e2 <= strip2
-            const float e2 = ex * ex + ey * ey;
-            const float nrm = s_norm[ly + dy][lx + dx];
-            if (e2 <= strip2) {
-                if (nrm >= 0.0f) {
-                    h_center += 1.0f;
-                } else if (nrm == -1.0f) {
-                    h_cons += 1.0f;
-                }
+            const float4 tap = row[dx];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                FilterPixel& P_ = P[q];
+                // evaluated for every tap, kept for those near in depth: predicated
+                // sums cost less than the branches around them
+                float e = __fmaf_rn(slope[q], (float)dx, base[q][dx < 0 ? -dx : dx]);
+                const float cx = P_.cx - tap.x, cy = P_.cy - tap.y, cz = P_.cz - tap.z;
+                const float ec = __fmaf_rn(__fmaf_rn(cz, cz, __fmaf_rn(cy, cy, cx * cx)), k_col, e);
+                e = P_.use_color ? ec : e;
+                accumulate(fabsf(tap.w - P_.p_norm) <= reject[q], tap, ex2(-e), P_);
             }
-            if (nrm < 0.0f) continue;
-            if (fabsf(nrm - p_norm) > depth_reject) continue;
-            const float4 qcol = s_col[ly + dy][lx + dx];
-            // The colour weights are compared within a tolerance, so they use
-            // fused multiply-adds (this file is otherwise built without
-            // contraction for the exact strip and coverage tests above).
-            float e = __fmaf_rn(d_par * d_par, k_par, e2 * k_perp);
-            if (use_color) {
-                const float cx = cc.x - qcol.x, cy = cc.y - qcol.y, cz = cc.z - qcol.z;
-                e = __fmaf_rn(__fmaf_rn(cz, cz, __fmaf_rn(cy, cy, cx * cx)), k_col, e);
-            }
-            const float wgt = exp2f(-e);
-            ax = __fmaf_rn(qcol.x, wgt, ax);
-            ay = __fmaf_rn(qcol.y, wgt, ay);
-            az = __fmaf_rn(qcol.z, wgt, az);
-            weight += wgt;
         }
     }
-    float cx = cc.x, cy = cc.y, cz = cc.z;
-    if (weight > 1e-5f) {
-        const float inv = 1.0f / weight;
-        cx = ax * inv;
-        cy = ay * inv;
-        cz = az * inv;
+    if (S > 1) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int o = 1; o < S; o <<= 1) {
+                P[q].ax += __shfl_xor_sync(0xffffffffu, P[q].ax, o);
+                P[q].ay += __shfl_xor_sync(0xffffffffu, P[q].ay, o);
+                P[q].az += __shfl_xor_sync(0xffffffffu, P[q].az, o);
+                P[q].weight += __shfl_xor_sync(0xffffffffu, P[q].weight, o);
+                P[q].h_center += __shfl_xor_sync(0xffffffffu, P[q].h_center, o);
+                P[q].h_cons += __shfl_xor_sync(0xffffffffu, P[q].h_cons, o);
+            }
+        if (slot >= total) return;
     }
-    const float coverage = __fdiv_rn(h_center, fmaxf(h_center + h_cons, 1.0f));
-    const float cons_depth = cons_hit ? __fdiv_rn(__uint2float_rn((uint32_t)(cons_word >> 40)), 16777214.0f) : 1.0f;
-    const float center_depth = p_norm;
-    const bool closer = cons_hit && center_hit && (center_depth - cons_depth) >= closer_eps;
-    float alpha = closer ? 1.0f : clampf(coverage, 0.0f, 1.0f);
-    if (promote && weight <= 1e-5f) {
-        alpha = 0.0f;
-        cx = cy = cz = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        // with several threads a pair, the first writes the upper pixel, the second the lower
+        if (!((entry >> (14 + q)) & 1u) || (S > 1 && sub != q)) continue;
+        const FilterPixel& P_ = P[q];
+        const uint32_t pix = (uint32_t)(by * TY + sy + q) * (uint32_t)width + (uint32_t)px;
+        const unsigned long long center_word = __ldg(&a.center[pix]), cons_word = __ldg(&a.cons[pix]);
+        const bool center_hit = !is_empty(center_word), cons_hit = !is_empty(cons_word);
+        const unsigned long long w = center_hit ? center_word : cons_word;
+        const float view_dist = dequantize_depth((uint32_t)(w >> 40), p.screen[2], p.screen[3]);
+        float cx = P_.cx, cy = P_.cy, cz = P_.cz;
+        if (P_.weight > 1e-5f) {
+            const float inv = 1.0f / P_.weight;
+            cx = P_.ax * inv;
+            cy = P_.ay * inv;
+            cz = P_.az * inv;
+        }
+        const float h_center = (float)P_.h_center, h_cons = (float)P_.h_cons;
+        const float coverage = __fdiv_rn(h_center, fmaxf(h_center + h_cons, 1.0f));
+        const float cons_depth = cons_hit ? __fdiv_rn(__uint2float_rn((uint32_t)(cons_word >> 40)), 16777214.0f) : 1.0f;
+        const bool closer = cons_hit && center_hit && (P_.p_norm - cons_depth) >= closer_eps;
+        float alpha = closer ? 1.0f : clampf(coverage, 0.0f, 1.0f);
+        if (!center_hit && P_.weight <= 1e-5f) {
+            alpha = 0.0f;
+            cx = cy = cz = 0.0f;
+        }
+        a.filtered[pix] = make_float4(cx, cy, cz, alpha);
+        a.filtered_depth[pix] = view_dist;
     }
-    a.filtered[pix] = make_float4(cx, cy, cz, alpha);
-    a.filtered_depth[pix] = view_dist;
 }
 
-__global__ void __launch_bounds__(kTileX* kTileY) filter_kernel(const FilterArgs a) {
-    filter_tile<kTileX, kTileY>(a, blockIdx.x, blockIdx.y);
+template <int TX, int TY, int S, int MIN_BLOCKS>
+__global__ void __launch_bounds__(TX* TY* S / 2, MIN_BLOCKS) filter_kernel(const FilterArgs a) {
+    filter_tile<TX, TY, S>(a, blockIdx.x, blockIdx.y);
 }
 
 // Tile t of the camera views' concatenated tile space -> (view, bx, by).
@@ -223,13 +377,13 @@ __device__ __forceinline__ uint32_t tile_view(const uint32_t* __restrict__ prefi
 }
 
 template <int TX, int TY>
-__global__ void __launch_bounds__(TX* TY) batch_filter_kernel(const BatchView* __restrict__ views,
+__global__ void __launch_bounds__(TX* TY / 2, 6) batch_filter_kernel(const BatchView* __restrict__ views,
                                                              const uint32_t* __restrict__ prefix, uint32_t n_cam) {
     const uint32_t v = tile_view(prefix, n_cam, blockIdx.x);
     const BatchView& a = views[v];
     const uint32_t t = blockIdx.x - prefix[v];
     const uint32_t tiles_x = (a.width + TX - 1) / TX;
-    filter_tile<TX, TY>(a, (int32_t)(t % tiles_x), (int32_t)(t / tiles_x));
+    filter_tile<TX, TY, 1>(a, (int32_t)(t % tiles_x), (int32_t)(t / tiles_x));
 }
 
 struct CompositeArgs {
@@ -303,9 +457,13 @@ cudaError_t launch_filter(hg_ctx* ctx, const hg_hair_params& p) {
     a.shaded = ctx->shaded;
     a.filtered = ctx->filtered;
     a.filtered_depth = ctx->filtered_depth;
-    dim3 block(kTileX, kTileY);
-    dim3 grid((ctx->width + kTileX - 1) / kTileX, (ctx->height + kTileY - 1) / kTileY);
-    filter_kernel<<<grid, block, 0, ctx->stream>>>(a);
+    const auto tiles = [&](uint32_t tx, uint32_t ty) {
+        return dim3((ctx->width + tx - 1) / tx, (ctx->height + ty - 1) / ty);
+    };
+    const uint64_t px = (uint64_t)ctx->width * ctx->height;
+    if (px <= kFilterSplit4) filter_kernel<16, 8, 4, 3><<<tiles(16, 8), 256, 0, ctx->stream>>>(a);
+    else if (px <= kFilterSplit2) filter_kernel<32, 8, 2, 4><<<tiles(32, 8), 256, 0, ctx->stream>>>(a);
+    else filter_kernel<16, 16, 1, 6><<<tiles(16, 16), 128, 0, ctx->stream>>>(a);
     return cudaGetLastError();
 }
 
@@ -325,10 +483,9 @@ cudaError_t launch_composite(hg_ctx* ctx, const hg_hair_params& p, uint32_t sour
 cudaError_t launch_batch_filter_composite(hg_ctx* ctx, const BatchDev& b) {
     cudaError_t e;
     if (b.filter && b.total_ftiles) {
-        if (b.filter_tile == 1) batch_filter_kernel<16, 16><<<b.total_ftiles, dim3(16, 16), 0, ctx->stream>>>(
+        if (b.filter_tile == 1) batch_filter_kernel<16, 16><<<b.total_ftiles, 128, 0, ctx->stream>>>(
             b.views, b.ftile_prefix, b.n_cam);
-        else batch_filter_kernel<kTileX, kTileY><<<b.total_ftiles, dim3(kTileX, kTileY), 0, ctx->stream>>>(
-            b.views, b.ftile_prefix, b.n_cam);
+        else batch_filter_kernel<32, 8><<<b.total_ftiles, 128, 0, ctx->stream>>>(b.views, b.ftile_prefix, b.n_cam);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     if (!b.composite || !b.total_px) return cudaSuccess;

@@ -344,6 +344,47 @@ def test_shade_filter_composite_within_tolerance(renderer, name):
     np.testing.assert_allclose(color, o_color, rtol=1e-6, atol=1e-7)
 
 
+@pytest.mark.parametrize("size", [(31, 9), (33, 17), (640, 384), (641, 384), (1024, 512), (1031, 517)])
+def test_filter_at_the_edges_of_its_thread_split(renderer, size):
+    """Four, two or one threads per pixel pair (up to 245,760 and 524,288 pixels),
+    ragged tiles, every kind of texel and tangents that lie along the rows or
+    toward the viewer: coverage and view distance exact, colour within the
+    filter's tolerance."""
+    w, h = size
+    sc = configs.config1(scale=0.02)
+    cam, _ = host.groom_params(configs._camera(w, h, 1000.0), sc.groom, sc.mesh.bounds_min, sc.mesh.bounds_max,
+                               sc.mesh.bundle_count, sc.directionals, sc.dom_size)
+    rng = np.random.default_rng(w * 4096 + h)
+    n = w * h
+    x, y = np.meshgrid(np.arange(w), np.arange(h))
+    base = 0.4 + 0.1 * np.sin(0.05 * x) * np.cos(0.07 * y)
+    depth = ((base.ravel() + rng.normal(0.0, 1e-3, n)) * 16777214.0).astype(np.uint64)
+    oct_x, oct_y = rng.integers(0, 256, n, dtype=np.uint64), rng.integers(0, 256, n, dtype=np.uint64)
+    axis = rng.random(n)
+    oct_x[axis < 0.1], oct_y[axis < 0.1] = 255, 128     # nearly along +X
+    oct_x[axis > 0.9], oct_y[axis > 0.9] = 128, 128     # nearly along +Z
+    words = (depth << np.uint64(40)) | (oct_x << np.uint64(32)) | (oct_y << np.uint64(24)) | np.uint64(0xFFF)
+    kind = rng.random(n)
+    center = np.where(kind < 0.6, words, EMPTY)
+    near = words - (rng.integers(0, 20_000, n, dtype=np.uint64) << np.uint64(40))
+    cons = np.where(kind < 0.8, np.where(kind < 0.3, near, words), EMPTY)
+    shaded = rng.random((n, 4)).astype(np.float32)
+    shaded[:, 3] = (rng.random(n) < 0.9).astype(np.float32)
+    renderer.ensure_targets(w, h, 0, 0)
+    renderer.write(abi.BUF_CENTER, center)
+    renderer.write(abi.BUF_CONSERVATIVE, cons)
+    renderer.write(abi.BUF_SHADED, shaded)
+    renderer.filter(cam)
+    assert renderer.synchronize() == 0
+    filt = renderer.read(abi.BUF_FILTERED).reshape(-1, 4)
+    fdepth = renderer.read(abi.BUF_FILTERED_DEPTH)
+    want, want_depth = oracle.filter_(cam, center, cons, shaded, np.zeros(n, dtype=np.float32))
+    want = np.asarray(want).reshape(-1, 4)
+    _assert_equal("filter alpha", filt[:, 3], want[:, 3])
+    _assert_equal("filter depth", fdepth, np.asarray(want_depth))
+    np.testing.assert_allclose(filt[:, :3], want[:, :3], rtol=FILTER_RTOL, atol=FILTER_ATOL)
+
+
 @pytest.mark.parametrize("scale", [0.02, 1.0])
 def test_full_frame_against_the_oracle_frame(renderer, scale):
     """hg_groom_frame against the oracle's whole hair_pass sequence; at scale 1
