@@ -742,10 +742,10 @@ def run_ours(args, rank, world, local):
     r.copy_wait()
     e2e_total = time.perf_counter() - t_s
     e2e_value, e2e_ms, _ = aggregate(dist, e2e_total * 1e3, float(seg_c) * args.steps)
-    # per frame: clear, 2 x lod, 2 x (scan offsets + expand), clear_dom, generate,
-    # camera raster (direct, the default: 2 stages + tile depths between them),
-    # 2 x DOM raster, shade, filter, clear_color, composite
-    launches = 18 * args.steps
+    # per frame: generate, lod, scan offsets and expand of both views, clear of both
+    # targets, camera raster (direct, the default: 2 stages + tile depths between
+    # them), 2 x DOM raster, shade, filter with colour clear and composite
+    launches = 11 * args.steps
 
     cpu = None
     if rank == 0 and not args.no_cpu_baseline:

@@ -247,7 +247,6 @@ void build_tables(hg_batch* b) {
     d.counters = b->d_counters;
     d.lights = b->d_lights;
     d.filter = b->cam[0].flags[1] != 0u;
-    d.composite = 1;
     d.depth_clear = b->cam[0].pass_mode[2] == 1u ? 0.0f : 1.0f;
     d.gen_blocks = (uint32_t)ctx->sm_count * b->gen_per_sm;
     d.raster_chunk = b->tuning.raster_chunk;
@@ -275,8 +274,8 @@ cudaError_t upload_tables(hg_batch* b) {
     return e;
 }
 
-// Part 0 of a frame: setup, raster, shade.  Part 1: filter, colour clear,
-// composite (the only writers of the colour/depth arenas).
+// Part 0 of a frame: setup, raster, shade.  Part 1: filter with colour clear
+// and composite (the only writer of the colour/depth arenas).
 cudaError_t enqueue_part(hg_batch* b, int part) {
     hg_ctx* ctx = b->ctx;
     if (part == 1) return hg::launch_batch_filter_composite(ctx, b->dev);
@@ -428,7 +427,7 @@ hg_status run_separate(hg_batch* b, const hg_shade_desc* d) {
         f.shade = *d;
         f.composite = 1;
         f.clear_color = 1;
-        hg_status s = hg_groom_frame(&view, b->grooms[i], &f);
+        hg_status s = hg::groom_frame_by_pass(&view, b->grooms[i], &f);
         ctx->light_slot = view.light_slot;
         if (s != HG_OK) {
             ctx->last_error = view.last_error;
@@ -645,7 +644,7 @@ hg_status hg_batch_launches(hg_batch* b, hg_batch_mode mode, uint32_t* launches)
     BATCH_CUDA(b->ctx, cudaEventSynchronize(b->uploaded));
     refresh_tables(b);
     if (mode == HG_BATCH_SEPARATE) {
-        // hg_groom_frame: clear, lod, scan (2 kernels), [generate, clear_dom, lod, scan (2), raster x2],
+        // the single passes: clear, lod, scan (2 kernels), [generate, clear_dom, lod, scan (2), raster x2],
         // clear colour, camera raster (2 stages + tile depths), shade, [filter], composite
         uint32_t total = 0;
         for (uint32_t i = 0; i < b->n; ++i)
@@ -662,8 +661,7 @@ hg_status hg_batch_launches(hg_batch* b, hg_batch_mode mode, uint32_t* launches)
     k += 2 + (d.total_tdepth ? 1 : 0);              // raster stages 1 and 2 (+ tile depths between them)
     k += d.n_views > d.n_cam ? 1 : 0;               // DOM layers
     k += d.total_tiles ? 1 : 0;                     // shade
-    k += d.filter ? 1 : 0;                          // filter
-    k += 2;                                         // clear colour, composite
+    k += d.total_tiles ? 1 : 0;                     // filter, colour clear and composite
     *launches = k;
     return HG_OK;
 }

@@ -26,6 +26,16 @@ struct FilterArgs {
     const float4* shaded;
     float4* filtered;
     float* filtered_depth;
+    float4* color;       // composite target (CompositeKind not kNone)
+    float* depth;
+    float depth_clear;   // kClear: the depth a pixel without hair gets
+};
+
+// What a pass that produces a pixel's final colour does with it.
+enum CompositeKind {
+    kNone,   // nothing: the composite pass follows
+    kBlend,  // composite onto the target
+    kClear   // composite onto a cleared target, written whole
 };
 
 // screen_tangent (filter.wgsl:9-18)
@@ -49,6 +59,39 @@ __device__ __forceinline__ float sqrt_bound(float r) {
         x = up;
     }
     return x;
+}
+
+// composite.wgsl:162-181 of one pixel with colour c (c.w its coverage) and
+// view distance view_dist; blend src*a + dst*(1-a) (alpha: a + dst_a*(1-a)),
+// depth test GreaterEqual when reverse-Z else LessEqual, depth write on.
+// With KIND kClear the target holds colour 0 and depth_clear.
+template <CompositeKind KIND>
+__device__ __forceinline__ void composite_one(const hg_hair_params& p, float4 c, float view_dist, float4* color,
+                                              float* depth_buf, float depth_clear, int32_t px, int32_t py,
+                                              uint32_t pix) {
+    float4 d = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float out_depth = depth_clear;
+    bool pass = false;
+    if (!(c.w < 0.001f)) {
+        const f3 world = reconstruct_world(p, px, py, view_dist);
+        const float4 clip = mat_mul(p.clip_from_world, world.x, world.y, world.z, 1.0f);
+        const float depth = clampf(__fdiv_rn(clip.z, fmaxf(clip.w, 1e-5f)), 0.0f, 1.0f);
+        const float dst_depth = KIND == kClear ? depth_clear : depth_buf[pix];
+        pass = p.pass_mode[2] == 1u ? depth >= dst_depth : depth <= dst_depth;
+        if (pass) {
+            if (KIND != kClear) d = color[pix];
+            const float ia = 1.0f - c.w;
+            d.x = c.x * c.w + d.x * ia;
+            d.y = c.y * c.w + d.y * ia;
+            d.z = c.z * c.w + d.z * ia;
+            d.w = c.w * 1.0f + d.w * ia;
+            out_depth = depth;
+        }
+    }
+    if (KIND == kClear || pass) {
+        color[pix] = d;
+        depth_buf[pix] = out_depth;
+    }
 }
 
 // Taps of row dy of a pixel's window whose distance from the strand's line
@@ -127,8 +170,8 @@ __device__ __forceinline__ void accumulate(bool keep, float4 tap, float w, Filte
 // they use fused operations and the fast exponential.  Against a thread per pixel with 121 tests and a
 // distance each (us): 1920 x 1080 113 -> 79, 3840 x 2160 200 -> 141, 512 x 512
 // 42 -> 29, 96 x 64 22 -> 10.
-template <int TX, int TY, int S, class V>
-__device__ __forceinline__ void filter_tile(const V& a, int32_t bx, int32_t by) {
+template <int TX, int TY, int S, CompositeKind KIND, class V>
+__device__ __forceinline__ void filter_tile(const V& a, int32_t bx, int32_t by, float depth_clear) {
     constexpr int kHaloX = TX + 2 * kFilterRadius, kHaloY = TY + 2 * kFilterRadius;
     constexpr int kPairs = TX * TY / 2, kThreads = kPairs * S, kWarps = kThreads / 32, kPairWarps = kPairs / 32;
     constexpr int kRows = 2 * kFilterRadius + 2;  // rows a pair's two windows cover
@@ -167,6 +210,10 @@ __device__ __forceinline__ void filter_tile(const V& a, int32_t bx, int32_t by) 
                     const uint32_t own = (uint32_t)(by * TY + 2 * (tid / TX) + q) * (uint32_t)width + (uint32_t)ox;
                     a.filtered[own] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     a.filtered_depth[own] = 0.0f;
+                    if (KIND == kClear) {
+                        a.color[own] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        a.depth[own] = depth_clear;
+                    }
                 }
             }
         }
@@ -355,14 +402,17 @@ __device__ __forceinline__ void filter_tile(const V& a, int32_t bx, int32_t by) 
             alpha = 0.0f;
             cx = cy = cz = 0.0f;
         }
-        a.filtered[pix] = make_float4(cx, cy, cz, alpha);
+        const float4 out = make_float4(cx, cy, cz, alpha);
+        a.filtered[pix] = out;
         a.filtered_depth[pix] = view_dist;
+        if (KIND != kNone)
+            composite_one<KIND>(p, out, view_dist, a.color, a.depth, depth_clear, px, by * TY + sy + q, pix);
     }
 }
 
-template <int TX, int TY, int S, int MIN_BLOCKS>
+template <int TX, int TY, int S, int MIN_BLOCKS, CompositeKind KIND>
 __global__ void __launch_bounds__(TX* TY* S / 2, MIN_BLOCKS) filter_kernel(const FilterArgs a) {
-    filter_tile<TX, TY, S>(a, blockIdx.x, blockIdx.y);
+    filter_tile<TX, TY, S, KIND>(a, blockIdx.x, blockIdx.y, a.depth_clear);
 }
 
 // Tile t of the camera views' concatenated tile space -> (view, bx, by).
@@ -378,12 +428,13 @@ __device__ __forceinline__ uint32_t tile_view(const uint32_t* __restrict__ prefi
 
 template <int TX, int TY>
 __global__ void __launch_bounds__(TX* TY / 2, 6) batch_filter_kernel(const BatchView* __restrict__ views,
-                                                             const uint32_t* __restrict__ prefix, uint32_t n_cam) {
+                                                             const uint32_t* __restrict__ prefix, uint32_t n_cam,
+                                                             float depth_clear) {
     const uint32_t v = tile_view(prefix, n_cam, blockIdx.x);
     const BatchView& a = views[v];
     const uint32_t t = blockIdx.x - prefix[v];
     const uint32_t tiles_x = (a.width + TX - 1) / TX;
-    filter_tile<TX, TY, 1>(a, (int32_t)(t % tiles_x), (int32_t)(t / tiles_x));
+    filter_tile<TX, TY, 1, kClear>(a, (int32_t)(t % tiles_x), (int32_t)(t / tiles_x), depth_clear);
 }
 
 struct CompositeArgs {
@@ -392,50 +443,36 @@ struct CompositeArgs {
     const float* depth_src;
     float4* color;
     float* depth;
+    float depth_clear;
 };
 
-// composite.wgsl:162-181; blend src*a + dst*(1-a) (alpha: a + dst_a*(1-a)),
-// depth test GreaterEqual when reverse-Z else LessEqual, depth write on.
-template <class V>
+template <CompositeKind KIND, class V>
 __device__ __forceinline__ void composite_pixel(const V& a, const float4* __restrict__ color_src,
-                                                const float* __restrict__ depth_src, int32_t px, int32_t py) {
+                                                const float* __restrict__ depth_src, float depth_clear, int32_t px,
+                                                int32_t py) {
     const hg_hair_params& p = a.p;
     const int32_t width = f2i(p.screen[0]), height = f2i(p.screen[1]);
     if (px >= width || py >= height) return;
     const uint32_t pix = (uint32_t)py * (uint32_t)width + (uint32_t)px;
-    const float4 c = __ldg(&color_src[pix]);
-    if (c.w < 0.001f) return;
-    const float view_dist = __ldg(&depth_src[pix]);
-    const f3 world = reconstruct_world(p, px, py, view_dist);
-    const float4 clip = mat_mul(p.clip_from_world, world.x, world.y, world.z, 1.0f);
-    const float depth = clampf(__fdiv_rn(clip.z, fmaxf(clip.w, 1e-5f)), 0.0f, 1.0f);
-    const float dst_depth = a.depth[pix];
-    const bool pass = p.pass_mode[2] == 1u ? depth >= dst_depth : depth <= dst_depth;
-    if (!pass) return;
-    a.depth[pix] = depth;
-    float4 d = a.color[pix];
-    const float ia = 1.0f - c.w;
-    d.x = c.x * c.w + d.x * ia;
-    d.y = c.y * c.w + d.y * ia;
-    d.z = c.z * c.w + d.z * ia;
-    d.w = c.w * 1.0f + d.w * ia;
-    a.color[pix] = d;
+    composite_one<KIND>(p, __ldg(&color_src[pix]), __ldg(&depth_src[pix]), a.color, a.depth, depth_clear, px, py, pix);
 }
 
+template <CompositeKind KIND>
 __global__ void composite_kernel(const CompositeArgs a) {
-    composite_pixel(a, a.color_src, a.depth_src, blockIdx.x * blockDim.x + threadIdx.x,
-                    blockIdx.y * blockDim.y + threadIdx.y);
+    composite_pixel<KIND>(a, a.color_src, a.depth_src, a.depth_clear, blockIdx.x * blockDim.x + threadIdx.x,
+                          blockIdx.y * blockDim.y + threadIdx.y);
 }
 
+// The shaded colour straight to the target (filter off).
 __global__ void batch_composite_kernel(const BatchView* __restrict__ views, const uint32_t* __restrict__ prefix,
-                                       uint32_t n_cam, uint32_t source_filtered) {
+                                       uint32_t n_cam, float depth_clear) {
     const uint32_t v = tile_view(prefix, n_cam, blockIdx.x);
     const BatchView& a = views[v];
     const uint32_t t = blockIdx.x - prefix[v];
     const uint32_t tiles_x = (a.width + blockDim.x - 1) / blockDim.x;
-    composite_pixel(a, source_filtered ? a.filtered : a.shaded, source_filtered ? a.filtered_depth : a.shaded_depth,
-                    (int32_t)((t % tiles_x) * blockDim.x + threadIdx.x),
-                    (int32_t)((t / tiles_x) * blockDim.y + threadIdx.y));
+    composite_pixel<kClear>(a, a.shaded, a.shaded_depth, depth_clear,
+                            (int32_t)((t % tiles_x) * blockDim.x + threadIdx.x),
+                            (int32_t)((t / tiles_x) * blockDim.y + threadIdx.y));
 }
 
 __global__ void clear_color_kernel(float4* __restrict__ color, float* __restrict__ depth, size_t pixels,
@@ -449,7 +486,21 @@ __global__ void clear_color_kernel(float4* __restrict__ color, float* __restrict
 
 }  // namespace
 
-cudaError_t launch_filter(hg_ctx* ctx, const hg_hair_params& p) {
+namespace {
+
+template <CompositeKind KIND>
+cudaError_t launch_filter_kind(hg_ctx* ctx, const FilterArgs& a) {
+    const auto tiles = [&](uint32_t tx, uint32_t ty) {
+        return dim3((ctx->width + tx - 1) / tx, (ctx->height + ty - 1) / ty);
+    };
+    const uint64_t px = (uint64_t)ctx->width * ctx->height;
+    if (px <= kFilterSplit4) filter_kernel<16, 8, 4, 3, KIND><<<tiles(16, 8), 256, 0, ctx->stream>>>(a);
+    else if (px <= kFilterSplit2) filter_kernel<32, 8, 2, 4, KIND><<<tiles(32, 8), 256, 0, ctx->stream>>>(a);
+    else filter_kernel<16, 16, 1, 6, KIND><<<tiles(16, 16), 128, 0, ctx->stream>>>(a);
+    return cudaGetLastError();
+}
+
+FilterArgs filter_args(hg_ctx* ctx, const hg_hair_params& p) {
     FilterArgs a;
     a.p = p;
     a.center = ctx->center;
@@ -457,44 +508,60 @@ cudaError_t launch_filter(hg_ctx* ctx, const hg_hair_params& p) {
     a.shaded = ctx->shaded;
     a.filtered = ctx->filtered;
     a.filtered_depth = ctx->filtered_depth;
-    const auto tiles = [&](uint32_t tx, uint32_t ty) {
-        return dim3((ctx->width + tx - 1) / tx, (ctx->height + ty - 1) / ty);
-    };
-    const uint64_t px = (uint64_t)ctx->width * ctx->height;
-    if (px <= kFilterSplit4) filter_kernel<16, 8, 4, 3><<<tiles(16, 8), 256, 0, ctx->stream>>>(a);
-    else if (px <= kFilterSplit2) filter_kernel<32, 8, 2, 4><<<tiles(32, 8), 256, 0, ctx->stream>>>(a);
-    else filter_kernel<16, 16, 1, 6><<<tiles(16, 16), 128, 0, ctx->stream>>>(a);
-    return cudaGetLastError();
+    a.color = ctx->color;
+    a.depth = ctx->depth;
+    a.depth_clear = 0.0f;
+    return a;
 }
 
-cudaError_t launch_composite(hg_ctx* ctx, const hg_hair_params& p, uint32_t source_filtered) {
+template <CompositeKind KIND>
+cudaError_t launch_composite_kind(hg_ctx* ctx, const hg_hair_params& p, uint32_t source_filtered, float depth_clear) {
     CompositeArgs a;
     a.p = p;
     a.color_src = source_filtered ? ctx->filtered : ctx->shaded;
     a.depth_src = source_filtered ? ctx->filtered_depth : ctx->shaded_depth;
     a.color = ctx->color;
     a.depth = ctx->depth;
+    a.depth_clear = depth_clear;
     dim3 block(32, 8);
     dim3 grid((ctx->width + 31) / 32, (ctx->height + 7) / 8);
-    composite_kernel<<<grid, block, 0, ctx->stream>>>(a);
+    composite_kernel<KIND><<<grid, block, 0, ctx->stream>>>(a);
     return cudaGetLastError();
 }
 
+}  // namespace
+
+cudaError_t launch_filter(hg_ctx* ctx, const hg_hair_params& p) {
+    return launch_filter_kind<kNone>(ctx, filter_args(ctx, p));
+}
+
+cudaError_t launch_composite(hg_ctx* ctx, const hg_hair_params& p, uint32_t source_filtered) {
+    return launch_composite_kind<kBlend>(ctx, p, source_filtered, 0.0f);
+}
+
+// The end of a frame in one launch: filter (when on) and composite, and with
+// `clear` the colour target's clear, which then is written once instead of
+// cleared, read and written (20 bytes a pixel for 60 and two launches).
+cudaError_t launch_filter_composite(hg_ctx* ctx, const hg_hair_params& p, bool filter, bool clear, float depth_clear) {
+    if (!filter)
+        return clear ? launch_composite_kind<kClear>(ctx, p, 0u, depth_clear)
+                     : launch_composite_kind<kBlend>(ctx, p, 0u, depth_clear);
+    FilterArgs a = filter_args(ctx, p);
+    a.depth_clear = depth_clear;
+    return clear ? launch_filter_kind<kClear>(ctx, a) : launch_filter_kind<kBlend>(ctx, a);
+}
+
+// Every item's filter (when on), colour clear and composite in one launch.
 cudaError_t launch_batch_filter_composite(hg_ctx* ctx, const BatchDev& b) {
-    cudaError_t e;
     if (b.filter && b.total_ftiles) {
         if (b.filter_tile == 1) batch_filter_kernel<16, 16><<<b.total_ftiles, 128, 0, ctx->stream>>>(
-            b.views, b.ftile_prefix, b.n_cam);
-        else batch_filter_kernel<32, 8><<<b.total_ftiles, 128, 0, ctx->stream>>>(b.views, b.ftile_prefix, b.n_cam);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            b.views, b.ftile_prefix, b.n_cam, b.depth_clear);
+        else batch_filter_kernel<32, 8><<<b.total_ftiles, 128, 0, ctx->stream>>>(b.views, b.ftile_prefix, b.n_cam,
+                                                                                b.depth_clear);
+    } else if (!b.filter && b.total_tiles) {
+        batch_composite_kernel<<<b.total_tiles, dim3(b.tile_w, b.tile_h), 0, ctx->stream>>>(b.views, b.tile_prefix,
+                                                                                           b.n_cam, b.depth_clear);
     }
-    if (!b.composite || !b.total_px) return cudaSuccess;
-    const int threads = 256;
-    const int blocks = (int)std::min<uint64_t>((b.total_px + threads - 1) / threads, (uint64_t)ctx->sm_count * 8);
-    clear_color_kernel<<<blocks, threads, 0, ctx->stream>>>(b.color, b.depth, b.total_px, b.depth_clear);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    batch_composite_kernel<<<b.total_tiles, dim3(b.tile_w, b.tile_h), 0, ctx->stream>>>(b.views, b.tile_prefix,
-                                                                                       b.n_cam, b.filter);
     return cudaGetLastError();
 }
 

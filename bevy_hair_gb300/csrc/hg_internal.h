@@ -132,7 +132,7 @@ struct hg_ctx {
     int light_slot = 0;
     // Side stream and events for the frame's independent DOM half.
     cudaStream_t side = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_gen = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_gen = nullptr, ev_setup = nullptr, ev_join = nullptr;
     int sm_count = 0;
     hg_mlp* surrogate = nullptr;   // bound by hg_mlp_bind, used by shade_model 1
     // light probe (hg_env_set): RGB9E5 mip chains, six faces per level
@@ -149,6 +149,10 @@ struct hg_ctx {
 };
 
 namespace hg {
+
+// hg_groom_frame as a sequence of the single passes (api.cu): one launch per
+// pass and view, for batch.cu's comparison mode.
+hg_status groom_frame_by_pass(hg_ctx* ctx, hg_groom* g, const hg_frame_desc* d);
 
 // Dual-scattering table of shade model 3 (shade.cu): 64 uvw.z levels x 129
 // view angles x 6 float4.
@@ -224,7 +228,7 @@ struct BatchDev {
     const hg_light* lights = nullptr;
     uint32_t n_lights = 0, ortho = 0;
     float exposure = 1.0f, depth_clear = 0.0f;
-    uint32_t filter = 1, composite = 1;
+    uint32_t filter = 1;
     uint32_t gen_blocks = 1;                  // grid of the generate pass (occupancy x SMs)
     // tuning
     uint32_t raster_chunk = 4, raster_blocks_per_sm = 1, tile_w = 32, tile_h = 8, filter_tile = 0;
@@ -237,6 +241,9 @@ cudaError_t launch_clear(hg_ctx* ctx);
 cudaError_t launch_clear_dom(hg_ctx* ctx);
 cudaError_t launch_lod(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p, int slot);
 cudaError_t launch_scan(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p, int slot);
+// A whole frame's setup: both targets' clears; lod and scan of both views (dom may be null).
+cudaError_t launch_frame_clear(hg_ctx* ctx, bool with_dom);
+cudaError_t launch_frame_setup(hg_ctx* ctx, hg_groom* g, const hg_hair_params& cam, const hg_hair_params* dom);
 cudaError_t launch_raster(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p, int slot, const float* scene);
 cudaError_t launch_generate(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p);
 void release_bins(hg_groom* g);  // frees the binned camera raster's scratch
@@ -268,6 +275,7 @@ cudaError_t launch_mlp_infer_tc(hg_mlp* m, const float* inputs, uint32_t n, floa
 cudaError_t launch_filter(hg_ctx* ctx, const hg_hair_params& p);
 cudaError_t launch_composite(hg_ctx* ctx, const hg_hair_params& p, uint32_t source_filtered);
 cudaError_t launch_clear_color(hg_ctx* ctx, float depth_clear);
+cudaError_t launch_filter_composite(hg_ctx* ctx, const hg_hair_params& p, bool filter, bool clear, float depth_clear);
 
 // receiver.cu
 cudaError_t launch_visibility(hg_ctx* ctx, const hg_shadow_light& L, const float* points, uint32_t n, float* out);

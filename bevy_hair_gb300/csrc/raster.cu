@@ -57,6 +57,41 @@ __global__ void clear_dom_kernel(uint32_t* __restrict__ dom, size_t texels, size
     if (tail < words) dom[tail] = tail < texels ? kDomEmpty : 0u;
 }
 
+// Both of the above in one launch, for a whole frame: the G-buffer's quads,
+// then the map's.
+__global__ void frame_clear_kernel(unsigned long long* __restrict__ center, unsigned long long* __restrict__ cons,
+                                   uint32_t* __restrict__ beta, size_t pixels, uint32_t* __restrict__ dom,
+                                   size_t texels, size_t words) {
+    const size_t px_quads = pixels / 4, quads = px_quads + words / 4;
+    const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+    const ulonglong2 e2 = make_ulonglong2(kEmptyU64, kEmptyU64);
+    const uint4 e4 = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
+    for (size_t q = first; q < quads; q += stride) {
+        if (q < px_quads) {
+            reinterpret_cast<ulonglong2*>(center)[2 * q] = e2;
+            reinterpret_cast<ulonglong2*>(center)[2 * q + 1] = e2;
+            reinterpret_cast<ulonglong2*>(cons)[2 * q] = e2;
+            reinterpret_cast<ulonglong2*>(cons)[2 * q + 1] = e2;
+            reinterpret_cast<uint4*>(beta)[q] = e4;
+        } else {
+            const size_t w = (q - px_quads) * 4;
+            uint4 v;
+            v.x = w + 0 < texels ? kDomEmpty : 0u;
+            v.y = w + 1 < texels ? kDomEmpty : 0u;
+            v.z = w + 2 < texels ? kDomEmpty : 0u;
+            v.w = w + 3 < texels ? kDomEmpty : 0u;
+            reinterpret_cast<uint4*>(dom)[q - px_quads] = v;
+        }
+    }
+    const size_t px_tail = px_quads * 4 + first, dom_tail = words / 4 * 4 + first;
+    if (px_tail < pixels) {
+        center[px_tail] = kEmptyU64;
+        cons[px_tail] = kEmptyU64;
+        beta[px_tail] = 0xffffffffu;
+    }
+    if (dom_tail < words) dom[dom_tail] = dom_tail < texels ? kDomEmpty : 0u;
+}
+
 // ------------------------------------------------------------------ lod
 
 __device__ __forceinline__ f3 to_world(const hg_hair_params& p, f3 q) {
@@ -343,6 +378,65 @@ __global__ void scan_expand_sorted_kernel(const hg_lod_record* __restrict__ lod,
             if (i >= capacity) break;
             reinterpret_cast<uint4*>(refs)[i] = make_uint4(b, s, rec.n_lod, rec.control_points);
             if (valid) draw_order[dpos + s] = i;
+        }
+    }
+}
+
+// ------------------------------------------------------------------ frame setup
+// lod and scan of a frame's camera view (with its draw order) and deep-opacity
+// view, one launch per step for both.
+
+struct SetupView {
+    hg_lod_record* lod;
+    uint32_t* depth_key;
+    uint32_t* offsets;
+    uint32_t* indirect;
+    hg_strand_ref* refs;
+    uint32_t* sorted;  // null: no draw order
+    uint32_t* sorted_off;
+    uint32_t* draw_order;
+    uint32_t* order_meta;
+    uint32_t count;  // bundles the view covers
+};
+
+struct SetupArgs {
+    hg_hair_params p[2];
+    SetupView v[2];
+    const hg_gpu_bundle* bundles;
+    const float4* layers;
+    uint32_t capacity;
+};
+
+__global__ void __launch_bounds__(256) frame_lod_kernel(const SetupArgs a) {
+    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    const uint32_t k = w < a.v[0].count ? 0u : 1u, b = w - (k ? a.v[0].count : 0u);
+    if (b >= a.v[k].count) return;
+    lod_bundle(a.p[k], a.bundles, a.layers, a.v[k].lod, a.v[k].depth_key, b, lane);
+}
+
+__global__ void __launch_bounds__(kScanThreads) frame_scan_offsets_kernel(const SetupArgs a) {
+    const SetupView& v = a.v[blockIdx.x];
+    scan_offsets_block(v.lod, v.count, a.capacity, v.offsets, v.indirect, v.depth_key, v.sorted, v.sorted_off,
+                       v.order_meta);
+}
+
+__global__ void __launch_bounds__(256) frame_scan_expand_kernel(const SetupArgs a) {
+    const uint32_t lane = threadIdx.x & 31u, warps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t total = a.v[0].count + a.v[1].count;
+    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < total; w += warps) {
+        const SetupView& v = a.v[w < a.v[0].count ? 0 : 1];
+        const uint32_t k = w < a.v[0].count ? w : w - a.v[0].count;
+        // with a draw order warp k takes the k-th live bundle in it, else bundle k
+        if (v.sorted && k >= v.order_meta[0]) continue;
+        const uint32_t b = v.sorted ? v.sorted[k] : k;
+        const bool order = v.sorted && v.order_meta[1] != 0u;
+        const hg_lod_record rec = v.lod[b];
+        const uint32_t off = v.offsets[b], dpos = order ? v.sorted_off[k] : 0u;
+        for (uint32_t s = lane; s < rec.n_lod; s += 32u) {
+            const uint32_t i = off + s;
+            if (i >= a.capacity) break;
+            reinterpret_cast<uint4*>(v.refs)[i] = make_uint4(b, s, rec.n_lod, rec.control_points);
+            if (order) v.draw_order[dpos + s] = i;
         }
     }
 }
@@ -2194,6 +2288,51 @@ cudaError_t launch_scan(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p, int s
         scan_expand_kernel<<<blocks, threads, 0, ctx->stream>>>(g->lod[slot], g->offsets[slot], count,
                                                                 g->ref_capacity, g->refs[slot]);
     }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_frame_clear(hg_ctx* ctx, bool with_dom) {
+    const size_t pixels = (size_t)ctx->width * ctx->height;
+    const size_t texels = with_dom ? (size_t)ctx->dom_w * ctx->dom_h : 0, words = texels * (1 + kDomLayers);
+    const int threads = 256;
+    const size_t quads = pixels / 4 + words / 4;
+    const int blocks = (int)std::min<size_t>((quads + threads - 1) / threads + 1, (size_t)ctx->sm_count * 8);
+    frame_clear_kernel<<<blocks, threads, 0, ctx->stream>>>(ctx->center, ctx->cons, ctx->beta, pixels, ctx->dom, texels,
+                                                            words);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_frame_setup(hg_ctx* ctx, hg_groom* g, const hg_hair_params& cam, const hg_hair_params* dom) {
+    SetupArgs a = {};
+    a.bundles = g->bundles;
+    a.layers = g->layers;
+    a.capacity = g->ref_capacity;
+    for (int s = 0; s < (dom ? 2 : 1); ++s) {
+        const hg_hair_params& p = s == 0 ? cam : *dom;
+        a.p[s] = p;
+        SetupView& v = a.v[s];
+        v.lod = g->lod[s];
+        v.depth_key = g->depth_key[s];
+        v.offsets = g->offsets[s];
+        v.indirect = g->indirect[s];
+        v.refs = g->refs[s];
+        v.sorted = s == 0 ? g->sorted[s] : nullptr;  // as launch_scan: the camera view's draw order only
+        v.sorted_off = g->sorted_off[s];
+        v.draw_order = g->draw_order[s];
+        v.order_meta = g->order_meta[s];
+        v.count = std::min(p.pass_mode[1], g->bundle_count);
+    }
+    const uint32_t total = a.v[0].count + a.v[1].count;
+    const int threads = 256;
+    cudaError_t e = cudaSuccess;
+    if (total) {
+        frame_lod_kernel<<<(total * 32u + threads - 1) / threads, threads, 0, ctx->stream>>>(a);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    frame_scan_offsets_kernel<<<dom ? 2 : 1, kScanThreads, 0, ctx->stream>>>(a);
+    if ((e = cudaGetLastError()) != cudaSuccess || !total) return e;
+    const int blocks = (int)std::min<uint32_t>((total * 32u + threads - 1) / threads, (uint32_t)ctx->sm_count * 8u);
+    frame_scan_expand_kernel<<<blocks, threads, 0, ctx->stream>>>(a);
     return cudaGetLastError();
 }
 

@@ -476,7 +476,7 @@ typedef struct hg_batch_tuning {
 typedef enum hg_batch_mode {
     HG_BATCH_GRAPH = 0,     /* replay the captured graph (recaptured when shapes or shade settings change) */
     HG_BATCH_LAUNCHES = 1,  /* the same batched launches issued directly */
-    HG_BATCH_SEPARATE = 2   /* hg_groom_frame per item (the unbatched path, for comparison) */
+    HG_BATCH_SEPARATE = 2   /* the single passes item by item (the unbatched path, for comparison) */
 } hg_batch_mode;
 
 hg_status hg_batch_create(hg_ctx* ctx, const hg_batch_item* items, uint32_t count, hg_batch** out);

@@ -415,6 +415,68 @@ def test_full_frame_against_the_oracle_frame(renderer, scale):
     g.close()
 
 
+@pytest.mark.parametrize("composite,clear_color", [(True, True), (True, False), (False, True)])
+@pytest.mark.parametrize("use_filter", [True, False])
+@pytest.mark.parametrize("deep_opacity", [True, False])
+def test_frame_equals_its_passes(renderer, deep_opacity, use_filter, composite, clear_color):
+    """hg_groom_frame's merged launches (setup of both views, both clears, filter
+    with colour clear and composite) against the single passes, every target
+    bit for bit, on a screen and map whose sizes leave vector tails."""
+    sc = configs.config1(scale=0.02)
+    sc.groom.deep_opacity, sc.groom.filter = deep_opacity, use_filter
+    w, h = 197, 131
+    sc.view = configs._camera(w, h, 1000.0)
+    sc.dom_size = (37, 37)
+    cam, dom = sc.params()
+    lights = sc.light_array()
+    r = renderer
+    r.ensure_targets(w, h, *sc.dom_size)
+    g = r.upload(sc.mesh)
+    rng = np.random.default_rng(5)
+    old_color = rng.random(w * h * 4).astype(np.float32)
+    old_depth = (rng.random(w * h) * 2e-4).astype(np.float32)
+    names = ["CENTER", "CONSERVATIVE", "BETA", "SHADED", "SHADED_DEPTH", "COLOR", "DEPTH"]
+    names += ["DOM"] if deep_opacity else []
+    names += ["FILTERED", "FILTERED_DEPTH"] if use_filter else []
+
+    def outputs(draw):
+        for n in names:  # nothing may be left over from the other way
+            ptr_bytes = r.buffer(getattr(abi, "BUF_" + n))[1]
+            r.write(getattr(abi, "BUF_" + n), np.full(ptr_bytes, 0x5A, dtype=np.uint8))
+        r.write(abi.BUF_COLOR, old_color)
+        r.write(abi.BUF_DEPTH, old_depth)
+        draw()
+        assert r.synchronize() == 0
+        return {n: r.read(getattr(abi, "BUF_" + n)).copy() for n in names}
+
+    def passes():
+        r.clear()
+        r.lod(g, cam, abi.SLOT_CAMERA)
+        r.scan(g, cam, abi.SLOT_CAMERA)
+        if deep_opacity:
+            r.generate(g, cam)
+            r.clear_dom()
+            r.lod(g, dom, abi.SLOT_DOM)
+            r.scan(g, dom, abi.SLOT_DOM)
+            r.raster(g, dom, abi.SLOT_DOM)
+            r.raster(g, host.dom_layers_params(dom), abi.SLOT_DOM)
+        r.raster(g, cam, abi.SLOT_CAMERA)
+        r.shade(cam, lights)
+        if use_filter:
+            r.filter(cam)
+        if composite and clear_color:
+            r.clear_color(0.0 if cam["pass_mode"][2] == 1 else 1.0)
+        if composite:
+            r.composite(cam, use_filter)
+
+    want = outputs(passes)
+    got = outputs(lambda: r.render_groom(g, cam, dom if deep_opacity else None, lights, composite=composite,
+                                         clear_color=clear_color))
+    for n in names:
+        _assert_equal(n, got[n].view(np.uint32), want[n].view(np.uint32))
+    g.close()
+
+
 def test_light_kinds(renderer):
     """Point, spot, directional (DOM) and rect lights, given out of kind order."""
     sc = configs.config1(scale=0.05)
