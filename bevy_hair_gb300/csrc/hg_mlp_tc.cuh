@@ -7,19 +7,31 @@
 // to ~2^-22 relative.
 //
 // A "chain" is one warpgroup (4 warps, 128 threads; thread r owns row r) that
-// runs two evaluations at once, each with its own input tile X (128 x 16),
-// hidden tile H (128 x 80), 64 TMEM columns and mbarrier.  Per layer one
-// thread issues an evaluation's MMAs and commits them to its mbarrier; all
-// 128 threads wait (bounded), read their row of the accumulator with
-// tcgen05.ld, apply ReLU + FP16 conversion and write it as the next layer's
-// input row.  While the warps work on one evaluation's accumulator the
-// tensor core runs the other's layer.  A CTA holds four chains (512
-// threads), all of the SM's 512 TMEM columns and 227 KB of shared memory.
+// runs one evaluation at a time in 104 TMEM columns: the accumulator (64), the
+// hidden activations (32 columns of FP16 pairs) and the inputs (8).  Per layer
+// one thread issues the MMAs and commits them to the chain's mbarrier; the 128
+// threads wait (bounded), read their row of the accumulator with tcgen05.ld,
+// apply ReLU + FP16 conversion and store it as the next layer's A operand
+// with tcgen05.st.  A CTA holds four chains (512 threads) and all of the SM's
+// 512 TMEM columns; while one chain converts, the tensor core runs another's
+// layer.
+//
+// The A operand lives in tensor memory because shared-memory bandwidth bounds
+// the alternative: with N = 64, an MMA that reads A (128 x 80) from shared
+// memory moves 30 KB per layer for 1.3 MFLOP, and every activation is stored
+// there first.  Only the weights (10 KB a layer) and the constant bias columns
+// stay in shared memory.  The elected lane takes the MMAs' operands from values
+// that are the same in the whole warp by construction (broadcast from lane 0):
+// from per-thread registers each MMA took ~100 cycles to issue.  Against two
+// evaluations a chain with A in shared memory (same outputs, bit for bit):
+// 1,000,003 rows 112 -> 48 us (with row-wise stores), shade model 1 at
+// 1920 x 1080 with 9 lights 391 -> 263 us.
 //
 // Shared-memory operand layout (K-major, no swizzle): 8 x 16-byte core
 // matrices; element (row, k) at (row/8)*SBO + (k/8)*LBO + (row%8)*16 + (k%8)*2
 // with LBO = 128 (core matrices adjacent along K are contiguous) and
-// SBO = (K/8)*128.
+// SBO = (K/8)*128.  A operands in TMEM: row r in lane r, elements 2j and 2j+1
+// in column j.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -38,25 +50,28 @@ constexpr uint32_t kKin = 16;   // 10 inputs, 2 bias columns, 4 zeros
 constexpr uint32_t kKhid = 80;  // 64 activations, 2 bias columns, 14 zeros
 constexpr uint32_t kLbo = 128;
 constexpr uint32_t kSboIn = (kKin / 8) * 128, kSboHid = (kKhid / 8) * 128;
-// Shared-memory byte offsets of one CTA (two chains).
+// Shared-memory byte offsets of one CTA.
 constexpr uint32_t kOffW1 = 0;
 constexpr uint32_t kOffW2 = kOffW1 + kHid * kKin * 2;
 constexpr uint32_t kOffW3 = kOffW2 + kHid * kKhid * 2;
 constexpr uint32_t kOffW4 = kOffW3 + kHid * kKhid * 2;
 constexpr uint32_t kOffW5 = kOffW4 + kHid * kKhid * 2;
 constexpr uint32_t kWeightBytes = kOffW5 + kOut * kKhid * 2;  // 35,328
-constexpr uint32_t kXBytes = kM * kKin * 2, kHBytes = kM * kKhid * 2;
-constexpr uint32_t kEvals = 2;    // evaluations in flight per chain
-constexpr uint32_t kChains = 4;   // warpgroups per CTA
-constexpr uint32_t kEvalBytes = kXBytes + kHBytes;
-constexpr uint32_t kGroupBytes = kEvals * kEvalBytes;
-constexpr uint32_t kOffBar = kWeightBytes + kChains * kGroupBytes;  // kChains * kEvals mbarriers, then the TMEM address
-constexpr uint32_t kOffSlot = kOffBar + 8 * kChains * kEvals;
+constexpr uint32_t kOffOnes = kWeightBytes;                   // 128 x 16: two columns of ones, the bias input
+constexpr uint32_t kChains = 4;                               // warpgroups per CTA
+constexpr uint32_t kOffStage = kOffOnes + kM * kKin * 2;      // per warp 32 x 13 floats: output rows (infer)
+constexpr uint32_t kStageFloats = 32 * (kUsedOut + 1);
+constexpr uint32_t kOffBar = kOffStage + 4 * kChains * kStageFloats * 4;  // kChains mbarriers, then the TMEM address
+constexpr uint32_t kOffSlot = kOffBar + 8 * kChains;
 constexpr uint32_t kSmemBytes = kOffSlot + 16;
-constexpr uint32_t kTmemCols = 512;  // per chain 128: per evaluation 64 (hidden accumulator; the output reuses 0..15)
+constexpr uint32_t kTmemCols = 512;
+// TMEM columns of a chain.
+constexpr uint32_t kChainCols = 128, kColAcc = 0, kColHid = 64, kColIn = 96;
 constexpr uint32_t kThreads = 128 * kChains;
 static_assert(kSmemBytes <= 232448, "shared memory per CTA");
-static_assert(kWeightBytes % 128 == 0 && kGroupBytes % 128 == 0, "tile alignment");
+static_assert(kWeightBytes % 128 == 0 && kOffStage % 128 == 0 && kOffBar % 8 == 0, "tile alignment");
+static_assert(kChains * kChainCols <= kTmemCols && kColHid + kHid / 2 <= kColIn && kColIn + kKin / 2 <= kChainCols,
+              "tensor memory columns");
 // Instruction descriptors (kind::f16): D F32, A and B F16, both K-major, M = 128.
 constexpr uint32_t kIdescHid = (1u << 4) | ((64u >> 3) << 17) | ((kM >> 4) << 24);
 constexpr uint32_t kIdescOut = (1u << 4) | ((16u >> 3) << 17) | ((kM >> 4) << 24);
@@ -96,6 +111,15 @@ __device__ __forceinline__ void mma(uint32_t d_tmem, uint64_t a, uint64_t b, uin
         "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
         "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// The same with the A operand (128 x 16 FP16, 8 columns) in tensor memory.
+__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t idesc,
+                                       uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 __device__ __forceinline__ void commit(uint32_t mbar_saddr) {
@@ -154,184 +178,170 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t v[16]) {
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 
-__device__ __forceinline__ void st_shared_v4(uint32_t saddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(saddr), "r"(a), "r"(b), "r"(c), "r"(d)
+// The value, unknown to the optimiser: keeps it from making a copy of the
+// caller's loop for either outcome of a test on it.
+__device__ __forceinline__ uint32_t opaque(uint32_t v) {
+    asm volatile("" : "+r"(v));
+    return v;
+}
+
+// One lane of the (converged) warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
+    return r != 0;
+}
+
+// This thread's row (lane) of 32 or 8 adjacent columns.
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t v[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+        "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};\n" ::"r"(taddr),
+        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]),
+        "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]),
+        "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t v[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"r"(taddr), "r"(v[0]),
+                 "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                  : "memory");
 }
-
-__device__ __forceinline__ void store_half(uint8_t* smem, uint32_t off, __half v) {
-    *reinterpret_cast<__half*>(smem + off) = v;
-}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 
 // The weight tiles of the CTA (every thread takes part): W[n][k] in the
-// canonical layout, the two bias columns after the real inputs.
+// canonical layout, the two bias columns (FP16 high and low parts) after the
+// real inputs.  A unit of 8 columns of a row is 16 contiguous bytes on both
+// sides; element by element this took 6 us more of every launch.
 __device__ __forceinline__ void load_weights(uint8_t* smem, const __half* __restrict__ w16,
                                              const float* __restrict__ params, int tid, int nthreads) {
-    auto bias_parts = [](float b, __half& hi, __half& lo) {
-        hi = __float2half_rn(b);
-        lo = __float2half_rn(b - __half2float(hi));
+    auto bias = [](float b) {
+        const __half hi = __float2half_rn(b), lo = __float2half_rn(b - __half2float(hi));
+        return (uint32_t)__half_as_ushort(hi) | (uint32_t)__half_as_ushort(lo) << 16;
     };
-    for (int i = tid; i < (int)(kHid * kKin); i += nthreads) {
-        const uint32_t n = i / kKin, k = i % kKin;
-        __half v = __float2half_rn(0.0f);
-        if (k < (uint32_t)kUsedIn) {
-            v = w16[kW1 + n * kIn + k];
-        } else if (k == (uint32_t)kUsedIn || k == (uint32_t)kUsedIn + 1) {
-            __half hi, lo;
-            bias_parts(params[kB1 + n], hi, lo);
-            v = k == (uint32_t)kUsedIn ? hi : lo;
+    for (int i = tid; i < (int)(kHid * kKin / 8); i += nthreads) {
+        const uint32_t n = i / (kKin / 8), k = i % (kKin / 8) * 8;
+        uint4 v = *reinterpret_cast<const uint4*>(w16 + kW1 + n * kIn + k);
+        if (k == 8u) {  // inputs 8, 9, then the bias columns 10, 11
+            v.y = bias(params[kB1 + n]);
+            v.z = v.w = 0u;
         }
-        store_half(smem, kOffW1 + canon(n, k, kSboIn), v);
+        *reinterpret_cast<uint4*>(smem + kOffW1 + canon(n, k, kSboIn)) = v;
     }
-    const int woff[3] = {kW2, kW3, kW4}, boff[3] = {kB2, kB3, kB4};
-    const uint32_t soff[3] = {kOffW2, kOffW3, kOffW4};
-    for (int l = 0; l < 3; ++l)
-        for (int i = tid; i < (int)(kHid * kKhid); i += nthreads) {
-            const uint32_t n = i / kKhid, k = i % kKhid;
-            __half v = __float2half_rn(0.0f);
-            if (k < (uint32_t)kHid) {
-                v = w16[woff[l] + n * kHid + k];
-            } else if (k == (uint32_t)kHid || k == (uint32_t)kHid + 1) {
-                __half hi, lo;
-                bias_parts(params[boff[l] + n], hi, lo);
-                v = k == (uint32_t)kHid ? hi : lo;
-            }
-            store_half(smem, soff[l] + canon(n, k, kSboHid), v);
+    const int woff[4] = {kW2, kW3, kW4, kW5}, boff[4] = {kB2, kB3, kB4, kB5};
+    const uint32_t soff[4] = {kOffW2, kOffW3, kOffW4, kOffW5};
+    for (int l = 0; l < 4; ++l)
+        for (int i = tid; i < (int)((l < 3 ? kHid : kOut) * kKhid / 8); i += nthreads) {
+            const uint32_t n = i / (kKhid / 8), k = i % (kKhid / 8) * 8;
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            if (k < (uint32_t)kHid) v = *reinterpret_cast<const uint4*>(w16 + woff[l] + n * kHid + k);
+            else if (k == (uint32_t)kHid) v.x = bias(params[boff[l] + n]);
+            *reinterpret_cast<uint4*>(smem + soff[l] + canon(n, k, kSboHid)) = v;
         }
-    for (int i = tid; i < (int)(kOut * kKhid); i += nthreads) {
-        const uint32_t n = i / kKhid, k = i % kKhid;
-        __half v = __float2half_rn(0.0f);
-        if (k < (uint32_t)kHid) {
-            v = w16[kW5 + n * kHid + k];
-        } else if (k == (uint32_t)kHid || k == (uint32_t)kHid + 1) {
-            __half hi, lo;
-            bias_parts(params[kB5 + n], hi, lo);
-            v = k == (uint32_t)kHid ? hi : lo;
-        }
-        store_half(smem, kOffW5 + canon(n, k, kSboHid), v);
-    }
 }
+static_assert(kW1 % 8 == 0 && kW2 % 8 == 0 && kW3 % 8 == 0 && kW4 % 8 == 0 && kW5 % 8 == 0 && kUsedIn == 10 &&
+                  kIn % 8 == 0,
+              "16-byte weight rows; inputs 8 and 9 share their block with the bias columns");
 
 struct Chain {
-    uint32_t w;              // shared address of the weights
-    uint32_t x[kEvals];      // shared addresses of the input tiles
-    uint32_t h[kEvals];      // and of the hidden tiles
-    uint32_t mbar[kEvals];   // shared addresses of the mbarriers
-    uint32_t tmem[kEvals];   // TMEM addresses of the accumulators (lane 0)
-    uint32_t phase[kEvals];  // parity of each mbarrier's next phase
-    uint32_t bar_id;         // named barrier of the warpgroup
-    uint32_t row;            // this thread's row, 0..127
+    uint32_t w;       // shared address of the weights
+    uint32_t mbar;    // shared address of the mbarrier
+    uint32_t tmem;    // TMEM address of the chain's columns, at this warp's lanes
+    uint32_t cols;    // the same at lane 0
+    uint32_t lead;    // 1 in the warpgroup's first warp, one lane of which issues the MMAs
+    uint32_t phase;   // parity of the mbarrier's next phase
+    uint32_t bar_id;  // named barrier of the warpgroup
+    uint32_t row;     // this thread's row, 0..127
 };
 
-// Row r of an H tile: the constant columns 64..79 (1, 1, then zeros), written once.
-__device__ __forceinline__ void init_hidden_row(uint32_t h, uint32_t row) {
-    const uint32_t one2 = 0x3C003C00u;  // two FP16 ones
-    st_shared_v4(h + canon(row, 64, kSboHid), one2, 0u, 0u, 0u);
-    st_shared_v4(h + canon(row, 72, kSboHid), 0u, 0u, 0u, 0u);
+// One layer's MMAs (the chain's first thread): KSTEPS products of 16 columns of
+// the A operand at TMEM column `a`, then, for hidden inputs, the bias columns.
+template <uint32_t KSTEPS, bool BIAS>
+__device__ __forceinline__ void issue(const Chain& c, uint32_t a, uint32_t w_off, uint32_t w_sbo, uint32_t idesc) {
+#pragma unroll
+    for (uint32_t ks = 0; ks < KSTEPS; ++ks)
+        mma_ts(c.cols + kColAcc, c.cols + a + 8u * ks, desc(c.w + w_off + ks * 2u * kLbo, w_sbo), idesc, ks);
+    if (BIAS)
+        mma(c.cols + kColAcc, desc(c.w + kOffOnes, kSboIn), desc(c.w + w_off + KSTEPS * 2u * kLbo, w_sbo), idesc, 1u);
+    commit(c.mbar);
 }
 
-// Row r of evaluation e's X from the normalised inputs (columns 10, 11 are the bias ones).
-__device__ __forceinline__ void write_input_row(const Chain& c, uint32_t e, const float x[kUsedIn]) {
-    st_shared_v4(c.x[e] + canon(c.row, 0, kSboIn), pack_h2(x[0], x[1]), pack_h2(x[2], x[3]), pack_h2(x[4], x[5]),
-                 pack_h2(x[6], x[7]));
-    st_shared_v4(c.x[e] + canon(c.row, 8, kSboIn), pack_h2(x[8], x[9]), 0x3C003C00u, 0u, 0u);
-}
-
-__device__ __forceinline__ void issue(uint32_t d, uint32_t a, uint32_t a_sbo, uint32_t b, uint32_t b_sbo,
-                                      uint32_t ksteps, uint32_t idesc) {
-    for (uint32_t ks = 0; ks < ksteps; ++ks)
-        mma(d, desc(a + ks * 2u * kLbo, a_sbo), desc(b + ks * 2u * kLbo, b_sbo), idesc, ks);
-}
-
-// Epilogue of one hidden layer of evaluation e: accumulator -> ReLU -> FP16 -> H row.
-__device__ __forceinline__ void hidden_epilogue(const Chain& c, uint32_t e) {
-    const uint32_t lane_base = (c.row & ~31u) << 16;
-    uint32_t v[64];
-    tmem_ld32(c.tmem[e] + lane_base, v);
-    tmem_ld32(c.tmem[e] + lane_base + 32u, v + 32);
+// The network on the row's normalised inputs: y receives this thread's 12
+// outputs.  Every thread of the warpgroup calls it.  Returns false (for the
+// whole warpgroup) when an MMA did not complete in time; the chain is then
+// unusable.
+__device__ __forceinline__ bool forward(Chain& c, const float x[kUsedIn], float y[kUsedOut]) {
+    {
+        const uint32_t in[8] = {pack_h2(x[0], x[1]), pack_h2(x[2], x[3]), pack_h2(x[4], x[5]), pack_h2(x[6], x[7]),
+                                pack_h2(x[8], x[9]), 0x3C003C00u,         0u,                  0u};
+        tmem_st8(c.tmem + kColIn, in);
+    }
+    tmem_wait_st();
+    fence_before();
+    if (group_sync_or(c.bar_id, false)) return false;
+    if (opaque(c.lead)) {
+        fence_after();
+        if (elect_one()) issue<1, false>(c, kColIn, kOffW1, kSboIn, kIdescHid);
+    }
+#pragma unroll
+    for (int layer = 0; layer < 4; ++layer) {
+        const bool ok = mbar_wait(c.mbar, c.phase);
+        if (ok) c.phase ^= 1u;  // after a timeout the phase stays the outstanding one
+        fence_after();
+        uint32_t h[kHid / 2];
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            uint32_t v[32];
+            tmem_ld32(c.tmem + kColAcc + 32u * half, v);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                h[16 * half + j] = pack_relu(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+        }
+        tmem_st32(c.tmem + kColHid, h);
+        tmem_wait_st();
+        fence_before();
+        if (group_sync_or(c.bar_id, !ok)) return false;
+        if (opaque(c.lead)) {
+            fence_after();
+            const uint32_t w = layer == 0 ? kOffW2 : layer == 1 ? kOffW3 : layer == 2 ? kOffW4 : kOffW5;
+            if (elect_one()) issue<4, true>(c, kColHid, w, kSboHid, layer < 3 ? kIdescHid : kIdescOut);
+        }
+    }
+    const bool ok = mbar_wait(c.mbar, c.phase);
+    if (ok) c.phase ^= 1u;
+    fence_after();
+    uint32_t o[16];
+    tmem_ld16(c.tmem + kColAcc, o);
     tmem_wait_ld();
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-        st_shared_v4(c.h[e] + canon(c.row, 8u * j, kSboHid),
-                     pack_relu(__uint_as_float(v[8 * j]), __uint_as_float(v[8 * j + 1])),
-                     pack_relu(__uint_as_float(v[8 * j + 2]), __uint_as_float(v[8 * j + 3])),
-                     pack_relu(__uint_as_float(v[8 * j + 4]), __uint_as_float(v[8 * j + 5])),
-                     pack_relu(__uint_as_float(v[8 * j + 6]), __uint_as_float(v[8 * j + 7])));
-}
-
-// The evaluations whose inputs are in X[0] (and X[1] when `two`): y0 / y1
-// receive this thread's 12 network outputs of each.  Every thread of the
-// warpgroup calls it with the same `two`.  Returns false (for the whole
-// warpgroup) when an MMA did not complete in time; the chain is then
-// unusable.
-__device__ __forceinline__ bool forward2(Chain& c, bool two, float y0[kUsedOut], float y1[kUsedOut]) {
-    const uint32_t ne = two ? 2u : 1u;
-    fence_proxy_async();
-    if (group_sync_or(c.bar_id, false)) return false;
-    if (c.row == 0) {
-        fence_after();
-        for (uint32_t e = 0; e < ne; ++e) {
-            issue(c.tmem[e], c.x[e], kSboIn, c.w + kOffW1, kSboIn, kKin / 16, kIdescHid);
-            commit(c.mbar[e]);
-        }
-    }
-    const uint32_t next_w[4] = {kOffW2, kOffW3, kOffW4, kOffW5};
-    for (int layer = 0; layer < 4; ++layer) {
-        for (uint32_t e = 0; e < ne; ++e) {
-            const bool ok = mbar_wait(c.mbar[e], c.phase[e]);
-            if (ok) c.phase[e] ^= 1u;  // after a timeout the phase stays the outstanding one
-            fence_after();
-            hidden_epilogue(c, e);
-            fence_proxy_async();
-            fence_before();
-            if (group_sync_or(c.bar_id, !ok)) return false;
-            if (c.row == 0) {
-                fence_after();
-                if (layer < 3)
-                    issue(c.tmem[e], c.h[e], kSboHid, c.w + next_w[layer], kSboHid, kKhid / 16, kIdescHid);
-                else
-                    issue(c.tmem[e], c.h[e], kSboHid, c.w + next_w[layer], kSboHid, kKhid / 16, kIdescOut);
-                commit(c.mbar[e]);
-            }
-        }
-    }
-    const uint32_t lane_base = (c.row & ~31u) << 16;
-    bool ok_all = true;
-    for (uint32_t e = 0; e < ne; ++e) {
-        const bool ok = mbar_wait(c.mbar[e], c.phase[e]);
-        if (ok) c.phase[e] ^= 1u;
-        ok_all = ok_all && ok;
-        fence_after();
-        uint32_t o[16];
-        tmem_ld16(c.tmem[e] + lane_base, o);
-        tmem_wait_ld();
-        float* y = e == 0 ? y0 : y1;
-#pragma unroll
-        for (int i = 0; i < kUsedOut; ++i) y[i] = __uint_as_float(o[i]);
-    }
+    for (int i = 0; i < kUsedOut; ++i) y[i] = __uint_as_float(o[i]);
     fence_before();
-    return !group_sync_or(c.bar_id, !ok_all);
+    return !group_sync_or(c.bar_id, !ok);
 }
 
-// CTA set-up: weights, the constant columns of every H tile, mbarriers, TMEM.
-// Every thread calls it; returns this thread's chain.
+// CTA set-up: weights, the constant bias input, mbarriers, TMEM.  Every thread
+// calls it; returns this thread's chain.
 __device__ __forceinline__ Chain setup(uint8_t* smem, const __half* w16, const float* params) {
-    const uint32_t tid = threadIdx.x, g = tid >> 7;
+    const uint32_t tid = threadIdx.x;
+    // broadcast from lane 0, so that the compiler knows it to be the same in
+    // the whole warp: the MMAs take their operands from uniform registers
+    const uint32_t warp = __shfl_sync(0xffffffffu, tid >> 5, 0), g = warp >> 2;
     const uint32_t base = smem_addr(smem);
     Chain c;
+    c.lead = (warp & 3u) == 0u ? 1u : 0u;
     c.w = base;
     c.bar_id = 1u + g;
     c.row = tid & 127u;
-    for (uint32_t e = 0; e < kEvals; ++e) {
-        c.x[e] = base + kWeightBytes + g * kGroupBytes + e * kEvalBytes;
-        c.h[e] = c.x[e] + kXBytes;
-        c.mbar[e] = base + kOffBar + 8u * (g * kEvals + e);
-        c.phase[e] = 0;
-        init_hidden_row(c.h[e], c.row);
-    }
+    c.mbar = base + kOffBar + 8u * g;
+    c.phase = 0;
     load_weights(smem, w16, params, (int)tid, (int)blockDim.x);
+    for (uint32_t i = tid; i < kM * kKin / 8u; i += blockDim.x)  // columns 0, 1 of every row are 1
+        *reinterpret_cast<uint4*>(smem + kOffOnes + canon(i >> 1, (i & 1u) * 8u, kSboIn)) =
+            make_uint4((i & 1u) ? 0u : 0x3C003C00u, 0u, 0u, 0u);
     if (tid == 0) {
-        for (uint32_t k = 0; k < kChains * kEvals; ++k) mbar_init(base + kOffBar + 8u * k, 1);
+        for (uint32_t k = 0; k < kChains; ++k) mbar_init(base + kOffBar + 8u * k, 1);
         fence_mbar_init();
     }
     if (tid < 32) {
@@ -342,16 +352,17 @@ __device__ __forceinline__ Chain setup(uint8_t* smem, const __half* w16, const f
     fence_before();
     __syncthreads();
     fence_after();
-    const uint32_t tbase = *reinterpret_cast<volatile uint32_t*>(smem + kOffSlot);
-    for (uint32_t e = 0; e < kEvals; ++e) c.tmem[e] = tbase + g * 128u + e * 64u;
+    const uint32_t tbase =
+        __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(smem + kOffSlot), 0);
+    c.cols = tbase + g * kChainCols;
+    c.tmem = c.cols + ((c.row & ~31u) << 16);
     return c;
 }
 
 // CTA tear-down after every chain has finished (or given up): bounded waits
 // for a failed chain's outstanding commits, then the TMEM is freed.
 __device__ __forceinline__ void teardown(uint8_t* smem, Chain& c, bool failed) {
-    if (failed)
-        for (uint32_t e = 0; e < kEvals; ++e) (void)mbar_wait(c.mbar[e], c.phase[e]);
+    if (failed) (void)mbar_wait(c.mbar, c.phase);
     fence_before();
     __syncthreads();
     if (threadIdx.x < 32) {

@@ -774,8 +774,6 @@ __global__ void karis_lobes_kernel(const float* __restrict__ in, uint32_t n, flo
 // own chunks, one network evaluation per light.  The light loop, the DOM
 // spread and the probe are those of shade_surrogate_kernel.
 
-constexpr uint32_t kLightsPerStep = 1;
-
 // Pixels whose centre word is not empty, appended in block order (one
 // atomic per block of kHairListThreads x kHairListPer pixels; each thread
 // loads its kHairListPer centre words before it looks at any); the others
@@ -958,43 +956,33 @@ __global__ void __launch_bounds__(mlp::tc::kThreads, 1)
                 color = vmul(spread_term(shape, ds, gm.theta_h, depth, dom_direct), ld3(L.color));
             }
         }
-        // lights two at a time: the chain's two evaluations
-        for (uint32_t i = 0; i < a.n_lights; i += kLightsPerStep) {
-            const bool two = kLightsPerStep == 2 && i + 1 < a.n_lights;
-            float weight[2] = {0.0f, 0.0f};
-            for (uint32_t e = 0; e < (two ? 2u : 1u); ++e) {
-                const hg_light& L = a.lights[i + e];
-                f3 incident;
-                float w = light_weight(L, world, incident);
-                if ((int)(i + e) == dom_light) w = dom_direct;
-                const bool use = active && w > 0.0f;
-                weight[e] = use ? w : 0.0f;
-                const f3 l = safe_normalize(incident);
-                const float sin_i = clampf(dot3(t_n, l), -1.0f, 1.0f);
-                const f3 t_i = sub3(l, mul3s(t_n, sin_i));
-                const float proj = sqrtf(fmaxf(dot3(t_i, t_i) * to2, 1e-8f));
-                const float cos_phi = clampf(dot3(t_i, t_o) / proj, -1.0f, 1.0f);
-                xin[0] = use ? sin_i : 0.0f;
-                xin[1] = use ? sin_o : 0.0f;
-                xin[2] = use ? cos_phi : 1.0f;
-                xin[3] = use ? sqrtf(fmaxf(1.0f - cos_phi * cos_phi, 0.0f)) : 0.0f;
-                mlp::tc::write_input_row(c, e, xin);
-            }
-            float yv[2][12];
-            if (!mlp::tc::forward2(c, two, yv[0], yv[1])) {
+        for (uint32_t i = 0; i < a.n_lights; ++i) {
+            const hg_light& L = a.lights[i];
+            f3 incident;
+            float w = light_weight(L, world, incident);
+            if ((int)i == dom_light) w = dom_direct;
+            const bool use = active && w > 0.0f;
+            const f3 l = safe_normalize(incident);
+            const float sin_i = clampf(dot3(t_n, l), -1.0f, 1.0f);
+            const f3 t_i = sub3(l, mul3s(t_n, sin_i));
+            const float proj = sqrtf(fmaxf(dot3(t_i, t_i) * to2, 1e-8f));
+            const float cos_phi = clampf(dot3(t_i, t_o) / proj, -1.0f, 1.0f);
+            xin[0] = use ? sin_i : 0.0f;
+            xin[1] = use ? sin_o : 0.0f;
+            xin[2] = use ? cos_phi : 1.0f;
+            xin[3] = use ? sqrtf(fmaxf(1.0f - cos_phi * cos_phi, 0.0f)) : 0.0f;
+            float q[12];
+            if (!mlp::tc::forward(c, xin, q)) {
                 failed = true;
                 break;
             }
-            for (uint32_t e = 0; e < (two ? 2u : 1u); ++e) {
-                if (!(weight[e] > 0.0f)) continue;
-                const float* q = yv[e];
-                f3 lobe = {mlp::decode_fast(q[0]) + mlp::decode_fast(q[3]) + mlp::decode_fast(q[6]),
-                           mlp::decode_fast(q[1]) + mlp::decode_fast(q[4]) + mlp::decode_fast(q[7]),
-                           mlp::decode_fast(q[2]) + mlp::decode_fast(q[5]) + mlp::decode_fast(q[8])};
-                lobe = add3(lobe, mul3s(mk3(mlp::decode_fast(q[9]), mlp::decode_fast(q[10]), mlp::decode_fast(q[11])),
-                                        kDensityBack));
-                color = add3(color, mul3s(vmul(lobe, ld3(a.lights[i + e].color)), weight[e]));
-            }
+            if (!use) continue;
+            f3 lobe = {mlp::decode_fast(q[0]) + mlp::decode_fast(q[3]) + mlp::decode_fast(q[6]),
+                       mlp::decode_fast(q[1]) + mlp::decode_fast(q[4]) + mlp::decode_fast(q[7]),
+                       mlp::decode_fast(q[2]) + mlp::decode_fast(q[5]) + mlp::decode_fast(q[8])};
+            lobe = add3(lobe, mul3s(mk3(mlp::decode_fast(q[9]), mlp::decode_fast(q[10]), mlp::decode_fast(q[11])),
+                                    kDensityBack));
+            color = add3(color, mul3s(vmul(lobe, ld3(L.color)), w));
         }
         if (failed) break;
         if (active) {

@@ -326,6 +326,23 @@ struct InferArgs {
     float* net;    // [n][12] network outputs, nullable
 };
 
+// A warp's rows of K outputs, one row per lane, to `rows` (at most 32)
+// consecutive rows of `out`, 32 consecutive words at a time.  stage: 32 (K + 1)
+// floats of the warp's own.
+template <int K>
+__device__ __forceinline__ void store_rows(float* stage, const float y[K], float* __restrict__ out, uint32_t rows,
+                                           uint32_t lane) {
+#pragma unroll
+    for (int c = 0; c < K; ++c) stage[lane * (K + 1) + c] = y[c];
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+        const uint32_t i = 32u * c + lane;
+        if (i < rows * K) out[i] = stage[i / K * (K + 1) + i % K];
+    }
+    __syncwarp();
+}
+
 __global__ void __launch_bounds__(kWarps * 32) infer_kernel(const InferArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     FwdWeights& w = *reinterpret_cast<FwdWeights*>(smem);
@@ -340,12 +357,12 @@ __global__ void __launch_bounds__(kWarps * 32) infer_kernel(const InferArgs a) {
         load_raw(a.inputs, i, valid, raw);
         normalise(raw, x);
         forward_fast(w, io[warp], x, y);
-        if (valid) {
+        const uint32_t rows = min(a.n - base, 32u);
+        if (a.net) store_rows<12>(&io[warp].y[0][0], y, a.net + (size_t)base * 12, rows, lane);
+        if (a.lobes) {
 #pragma unroll
-            for (int c = 0; c < 12; ++c) {
-                if (a.lobes) a.lobes[(size_t)i * 12 + c] = decode(y[c]);
-                if (a.net) a.net[(size_t)i * 12 + c] = y[c];
-            }
+            for (int c = 0; c < 12; ++c) y[c] = decode(y[c]);
+            store_rows<12>(&io[warp].y[0][0], y, a.lobes + (size_t)base * 12, rows, lane);
         }
     }
 }
@@ -365,48 +382,47 @@ __global__ void __launch_bounds__(kWarps * 32) infer_small_kernel(const InferArg
         load_raw(a.inputs, i, valid, raw);
         normalise(raw, x);
         mlps::forward(w, io[warp], x, y);
-        if (valid) {
+        constexpr int k = mlps::kUsedOut;
+        const uint32_t rows = min(a.n - base, 32u);
+        if (a.net) store_rows<k>(&io[warp].y[0][0], y, a.net + (size_t)base * k, rows, lane);
+        if (a.lobes) {
 #pragma unroll
-            for (int c = 0; c < mlps::kUsedOut; ++c) {
-                if (a.lobes) a.lobes[(size_t)i * mlps::kUsedOut + c] = decode(y[c]);
-                if (a.net) a.net[(size_t)i * mlps::kUsedOut + c] = y[c];
-            }
+            for (int c = 0; c < k; ++c) y[c] = decode(y[c]);
+            store_rows<k>(&io[warp].y[0][0], y, a.lobes + (size_t)base * k, rows, lane);
         }
     }
 }
 
-// The same evaluation on tcgen05: four chains of two 128-row evaluations per CTA.
+// The same evaluation on tcgen05: four chains of 128 rows per CTA.  A chunk's
+// inputs are read while the chunk before is evaluated; its outputs leave in
+// rows of 32 consecutive words (store_rows): a row per thread touched 12 times
+// the sectors.
 __global__ void __launch_bounds__(tc::kThreads, 1) infer_tc_kernel(const InferArgs a, uint32_t* err) {
     extern __shared__ __align__(128) uint8_t smem_tc[];
     tc::Chain c = tc::setup(smem_tc, a.w16, a.params);
-    const uint32_t g = threadIdx.x >> 7;
-    const uint32_t chunks = (a.n + tc::kM - 1) / tc::kM;
-    const uint32_t pairs = (chunks + 1) / 2;
+    const uint32_t g = threadIdx.x >> 7, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    float* stage = reinterpret_cast<float*>(smem_tc + tc::kOffStage) + warp * tc::kStageFloats;
+    const uint32_t chunks = a.n / tc::kM + (a.n % tc::kM != 0u);
+    const uint32_t step = gridDim.x * tc::kChains;
+    uint32_t ch = blockIdx.x * tc::kChains + g;
     bool failed = false;
-    for (uint32_t pc = blockIdx.x * tc::kChains + g; pc < pairs; pc += gridDim.x * tc::kChains) {
-        const bool two = 2 * pc + 1 < chunks;
-        uint32_t idx[2];
-        bool valid[2];
-        for (uint32_t e = 0; e < 2; ++e) {
-            idx[e] = (2 * pc + e) * tc::kM + c.row;
-            valid[e] = idx[e] < a.n && (e == 0 || two);
-            float raw[10], x[10];
-            load_raw(a.inputs, idx[e], valid[e], raw);
-            normalise(raw, x);
-            tc::write_input_row(c, e, x);
-        }
-        float y[2][12];
-        if (!tc::forward2(c, two, y[0], y[1])) {
+    float raw[10];
+    if (ch < chunks) load_raw(a.inputs, ch * tc::kM + c.row, ch * tc::kM + c.row < a.n, raw);
+    for (; ch < chunks; ch += step) {
+        float x[10], y[12];
+        normalise(raw, x);
+        if (ch + step < chunks) load_raw(a.inputs, (ch + step) * tc::kM + c.row, (ch + step) * tc::kM + c.row < a.n, raw);
+        if (!tc::forward(c, x, y)) {
             failed = true;
             break;
         }
-        for (uint32_t e = 0; e < 2; ++e) {
-            if (!valid[e]) continue;
+        const uint32_t first = ch * tc::kM + (c.row & ~31u);
+        const uint32_t rows = first < a.n ? min(a.n - first, 32u) : 0u;
+        if (a.net) store_rows<12>(stage, y, a.net + (size_t)first * 12, rows, lane);
+        if (a.lobes) {
 #pragma unroll
-            for (int k = 0; k < 12; ++k) {
-                if (a.lobes) a.lobes[(size_t)idx[e] * 12 + k] = decode(y[e][k]);
-                if (a.net) a.net[(size_t)idx[e] * 12 + k] = y[e][k];
-            }
+            for (int k = 0; k < 12; ++k) y[k] = decode(y[k]);
+            store_rows<12>(stage, y, a.lobes + (size_t)first * 12, rows, lane);
         }
     }
     if (failed && c.row == 0) atomicOr(err, tc::kErrTimeout);
@@ -1419,9 +1435,9 @@ cudaError_t launch_mlp_infer_tc(hg_mlp* m, const float* inputs, uint32_t n, floa
     a.params = m->params;
     a.lobes = lobes;
     a.net = net;
-    const uint32_t pairs = ((n + tc::kM - 1) / tc::kM + 1) / 2;
-    uint32_t blocks = (pairs + tc::kChains - 1) / tc::kChains;
-    // one CTA per SM: it holds all 512 TMEM columns and most of the shared memory
+    const uint32_t chunks = n / tc::kM + (n % tc::kM != 0u);
+    uint32_t blocks = (chunks + tc::kChains - 1) / tc::kChains;
+    // one CTA per SM: it holds all 512 TMEM columns
     const uint32_t cap = (uint32_t)m->ctx->sm_count;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
