@@ -72,6 +72,7 @@ void free_targets(hg_ctx* ctx) {
     free_dev(ctx->cons);
     free_dev(ctx->beta);
     free_dev(ctx->dom);
+    free_dev(ctx->dom_front);
     free_dev(ctx->shaded);
     free_dev(ctx->shaded_depth);
     free_dev(ctx->filtered);
@@ -366,6 +367,7 @@ hg_status hg_ensure_targets(hg_ctx* ctx, uint32_t width, uint32_t height, uint32
     alloc(ctx->cons, px * 8);
     alloc(ctx->beta, px * 4);
     alloc(ctx->dom, texels * (1 + HG_DOM_LAYERS) * 4);
+    alloc(ctx->dom_front, hg::front_words(dom_w, dom_h) * 4);
     alloc(ctx->shaded, px * 16);
     alloc(ctx->shaded_depth, px * 4);
     alloc(ctx->filtered, px * 16);

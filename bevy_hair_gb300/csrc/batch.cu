@@ -20,6 +20,7 @@ struct hg_batch {
     std::vector<hg_groom*> grooms;
     std::vector<uint32_t> w, h, dw, dh;
     std::vector<uint64_t> px_off, dom_off;   // per item, in pixels / words
+    std::vector<uint64_t> front_off;         // per item, in words of the tiled front planes
     std::vector<hg_hair_params> cam, dom;    // host copies of the uniforms
     std::vector<uint8_t> have;
     // arenas
@@ -27,6 +28,7 @@ struct hg_batch {
     unsigned long long* cons = nullptr;
     uint32_t* beta = nullptr;
     uint32_t* dommap = nullptr;
+    uint32_t* front = nullptr;
     float4* shaded = nullptr;
     float* shaded_depth = nullptr;
     float4* filtered = nullptr;
@@ -130,6 +132,7 @@ void free_batch(hg_batch* b) {
     free_dev(b->cons);
     free_dev(b->beta);
     free_dev(b->dommap);
+    free_dev(b->front);
     free_dev(b->shaded);
     free_dev(b->shaded_depth);
     free_dev(b->filtered);
@@ -188,6 +191,7 @@ void build_tables(hg_batch* b) {
             v.cons = b->cons + po;
             v.beta = b->beta + po;
             v.dom = b->dw[i] ? b->dommap + b->dom_off[i] : nullptr;
+            v.front = b->dw[i] ? b->front + b->front_off[i] : nullptr;
             v.shaded = b->shaded + po;
             v.shaded_depth = b->shaded_depth + po;
             v.filtered = b->filtered + po;
@@ -409,6 +413,7 @@ hg_status run_separate(hg_batch* b, const hg_shade_desc* d) {
         view.cons = b->cons + po;
         view.beta = b->beta + po;
         view.dom = b->dw[i] ? b->dommap + b->dom_off[i] : nullptr;
+        view.dom_front = b->dw[i] ? b->front + b->front_off[i] : nullptr;
         view.shaded = b->shaded + po;
         view.shaded_depth = b->shaded_depth + po;
         view.filtered = b->filtered + po;
@@ -489,7 +494,7 @@ hg_status hg_batch_create(hg_ctx* ctx, const hg_batch_item* items, uint32_t coun
     if (!b) return fail(ctx, HG_OUT_OF_MEMORY, "allocating the batch");
     b->ctx = ctx;
     b->n = count;
-    uint64_t px = 0, words = 0;
+    uint64_t px = 0, words = 0, front = 0;
     for (uint32_t i = 0; i < count; ++i) {
         b->grooms.push_back(items[i].groom);
         b->w.push_back(items[i].width);
@@ -498,6 +503,8 @@ hg_status hg_batch_create(hg_ctx* ctx, const hg_batch_item* items, uint32_t coun
         b->dh.push_back(items[i].dom_h);
         b->px_off.push_back(px);
         b->dom_off.push_back(words);
+        b->front_off.push_back(front);
+        front += hg::front_words(items[i].dom_w, items[i].dom_h);  // whole 128-byte lines
         // Slices start on 64-element boundaries: the single-view kernels that
         // the per-groom path runs on them use 16-byte vector stores.
         px += round_up64((uint64_t)items[i].width * items[i].height);
@@ -524,6 +531,7 @@ hg_status hg_batch_create(hg_ctx* ctx, const hg_batch_item* items, uint32_t coun
     alloc(b->cons, px * 8);
     alloc(b->beta, px * 4);
     alloc(b->dommap, words * 4);
+    alloc(b->front, front * 4);
     alloc(b->shaded, px * 16);
     alloc(b->shaded_depth, px * 4);
     alloc(b->filtered, px * 16);
@@ -644,11 +652,14 @@ hg_status hg_batch_launches(hg_batch* b, hg_batch_mode mode, uint32_t* launches)
     BATCH_CUDA(b->ctx, cudaEventSynchronize(b->uploaded));
     refresh_tables(b);
     if (mode == HG_BATCH_SEPARATE) {
-        // the single passes: clear, lod, scan (2 kernels), [generate, clear_dom, lod, scan (2), raster x2],
-        // clear colour, camera raster (2 stages + tile depths), shade, [filter], composite
+        // the single passes: clear, lod, scan (2 kernels), [generate, clear_dom, lod, scan (2), raster x2
+        // and a large groom's front plane], clear colour, camera raster (2 stages + tile depths), shade, [filter],
+        // composite
         uint32_t total = 0;
-        for (uint32_t i = 0; i < b->n; ++i)
+        for (uint32_t i = 0; i < b->n; ++i) {
             total += 1 + 1 + 2 + (b->dw[i] ? 7u : 0u) + 1 + 3 + 1 + (b->cam[i].flags[1] ? 1u : 0u) + 1;
+            if (b->dw[i] && hg::layers_use_plane(b->grooms[i]->strand_total, b->dw[i], b->dh[i])) total += 1;
+        }
         *launches = total;
         return HG_OK;
     }
@@ -659,7 +670,7 @@ hg_status hg_batch_launches(hg_batch* b, hg_batch_mode mode, uint32_t* launches)
     k += 1;                                         // scan offsets
     k += d.total_strands ? 1 : 0;                   // generate
     k += 2 + (d.total_tdepth ? 1 : 0);              // raster stages 1 and 2 (+ tile depths between them)
-    k += d.n_views > d.n_cam ? 1 : 0;               // DOM layers
+    k += d.n_views > d.n_cam ? 2 : 0;               // DOM front planes, DOM layers
     k += d.total_tiles ? 1 : 0;                     // shade
     k += d.total_tiles ? 1 : 0;                     // filter, colour clear and composite
     *launches = k;

@@ -465,9 +465,9 @@ constexpr int kDomGridRounds = 8;
 // control points are generated, so they share storage with the run list.
 struct alignas(16) StrandSmem {
     float4 cp[128];  // control point: model position, then world position + in_front flag
-    float4 ct[128];  // camera: world tangent xyz + w (uvw.z)
+    float4 ct[128];  // camera: world tangent xyz + w (uvw.z); DOM layers: the segment's walk
     float4 cs[128];  // screen xy, ao; camera: RN(1/n) for the segment's DDA step count n
-    float vd[128];   // camera: view distance of the control point (project_world)
+    float vd[128];   // camera: view distance of the control point (project_world); DOM layers: RN(1/len2)
     hg_strand_ref next_ref;  // the warp's next ref, copied ahead (cp.async)
     uint32_t next_idx;       // the draw-order entry after it
     uint32_t pad_[3];
@@ -487,6 +487,8 @@ struct alignas(16) StrandSmem {
 
 // Segments are cut into at most this many DDA steps.
 constexpr int kMaxSteps = 96;
+// And a DOM segment's walk visits at most this many texels.
+constexpr int kDomMaxSteps = 1024;
 
 // t = i / n, correctly rounded, for integers 0 <= i <= n <= kMaxSteps, from
 // rcp = RN(1/n): q0 = RN(i * rcp), the exact remainder i - q0 * n by FMA, and
@@ -517,6 +519,7 @@ struct RasterArgs {
     unsigned long long* cons;
     uint32_t* beta;
     uint32_t* dom;
+    const uint32_t* front;       // DOM layers: the tiled front depths, or nullptr (dom is read, a segment per lane)
     const float* scene;
     uint32_t* err;
     uint32_t bundle_count;
@@ -835,11 +838,12 @@ __device__ __forceinline__ bool on_screen(int32_t x, int32_t y, int32_t w, int32
 // (sm.u.run.off) and tag[k] (sm.u.run.seg).  The four
 // rounds' exclusive offsets come from two warp prefix sums, two rounds
 // sharing a 32-bit word 16 bits each (a round's total is at most
-// 32 (kMaxSteps + 1) < 2^16).  Leaves the strand's sample total and run
+// 32 (kMaxSteps + 1), or 32 kDomMaxSteps, < 2^16).  Leaves the strand's sample total and run
 // count.  Every lane of the warp calls it.
 __device__ __forceinline__ void append_runs4(StrandSmem& sm, const int32_t (&cnt)[4], const int32_t (&tag)[4],
                                              uint32_t lane, int32_t& total, int32_t& runs) {
-    static_assert(32 * (kMaxSteps + 1) < 65536, "a round's sample count must fit 16 bits");
+    static_assert(32 * (kMaxSteps + 1) < 65536 && 32 * kDomMaxSteps < 65536,
+                  "a round's sample count must fit 16 bits");
     uint32_t w01 = (uint32_t)cnt[0] | (uint32_t)cnt[1] << 16u, w23 = (uint32_t)cnt[2] | (uint32_t)cnt[3] << 16u;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -1230,43 +1234,194 @@ __device__ __forceinline__ void dom_write(const Args& a, int32_t px, int32_t py,
 // in one pixel.  (A flattened variant that spreads the walks' pixels evenly
 // over the lanes, each pixel found in closed form, measured slower on config
 // 2: segments average 3.3 pixels, and recomputing each pixel's segment state
-// costs more than the idle lanes of the per-lane walk.)
+// costs more than the idle lanes of the per-lane walk; the layers pass has its
+// own variant, raster_dom_layers.)
+template <int MODE, class Args>
+__device__ __forceinline__ void dom_walk(const Args& a, const StrandSmem& sm, uint32_t j, int32_t width, int32_t height,
+                                         float thickness) {
+    const float4 c0 = sm.cp[j], c1 = sm.cp[j + 1u];
+    if (c0.w == 0.0f && c1.w == 0.0f) return;
+    const float4 A4 = sm.cs[j], B4 = sm.cs[j + 1u];
+    const float2 A = make_float2(A4.x, A4.y), B = make_float2(B4.x, B4.y);
+    int32_t x0 = f2i(floorf(A.x)), y0 = f2i(floorf(A.y));
+    const int32_t x1 = f2i(floorf(B.x)), y1 = f2i(floorf(B.y));
+    const int32_t dx = iabs(isub(x1, x0)), dy = iabs(isub(y1, y0));
+    const int32_t sx = x0 < x1 ? 1 : -1, sy = y0 < y1 ? 1 : -1;
+    int32_t err = isub(dx, dy);
+    const float2 seg = sub2(B, A);
+    const float seg_len2 = fmaxf(dot2(seg, seg), 1e-6f);
+    bool skip = j != 0u && (x0 != x1 || y0 != y1);
+    const f3 p0 = xyz(c0), p1 = xyz(c1);
+    const int32_t ndy = (int32_t)(0u - (uint32_t)dy);
+    for (int step = 0; step < kDomMaxSteps; ++step) {
+        if (!skip) dom_write<MODE>(a, x0, y0, width, height, A, seg, seg_len2, p0, p1, thickness);
+        skip = false;
+        if (x0 == x1 && y0 == y1) break;
+        const int32_t e2 = iadd(err, err);
+        if (e2 > ndy) {
+            err = isub(err, dy);
+            x0 = iadd(x0, sx);
+        }
+        if (e2 < dx) {
+            err = iadd(err, dx);
+            y0 = iadd(y0, sy);
+        }
+    }
+}
+
 template <int MODE, class Args>
 __device__ __forceinline__ void raster_dom(const Args& a, StrandSmem& sm, uint32_t ncp, uint32_t lane) {
     const hg_hair_params& p = a.p;
     const int32_t width = f2i(p.screen[0]), height = f2i(p.screen[1]);
     // slice thickness of the layers pass (write_dom_pixel), the same for every texel
     const float thickness = __fdiv_rn(fmaxf(p.screen[3] - p.screen[2], 1e-3f), (float)kDomLayers);
-    for (uint32_t j = lane; j + 1u < ncp; j += 32u) {
-        float4 c0 = sm.cp[j], c1 = sm.cp[j + 1u];
-        if (c0.w == 0.0f && c1.w == 0.0f) continue;
-        float4 A4 = sm.cs[j], B4 = sm.cs[j + 1u];
-        float2 A = make_float2(A4.x, A4.y), B = make_float2(B4.x, B4.y);
-        int32_t x0 = f2i(floorf(A.x)), y0 = f2i(floorf(A.y));
-        int32_t x1 = f2i(floorf(B.x)), y1 = f2i(floorf(B.y));
-        int32_t dx = iabs(isub(x1, x0)), dy = iabs(isub(y1, y0));
-        int32_t sx = x0 < x1 ? 1 : -1, sy = y0 < y1 ? 1 : -1;
-        int32_t err = isub(dx, dy);
-        float2 seg = sub2(B, A);
-        float seg_len2 = fmaxf(dot2(seg, seg), 1e-6f);
-        bool skip = j != 0u && (x0 != x1 || y0 != y1);
-        f3 p0 = xyz(c0), p1 = xyz(c1);
-        const int32_t ndy = (int32_t)(0u - (uint32_t)dy);
-        for (int step = 0; step < 1024; ++step) {
-            if (!skip) dom_write<MODE>(a, x0, y0, width, height, A, seg, seg_len2, p0, p1, thickness);
-            skip = false;
-            if (x0 == x1 && y0 == y1) break;
-            int32_t e2 = iadd(err, err);
-            if (e2 > ndy) {
-                err = isub(err, dy);
-                x0 = iadd(x0, sx);
-            }
-            if (e2 < dx) {
-                err = iadd(err, dx);
-                y0 = iadd(y0, sy);
-            }
-        }
+    for (uint32_t j = lane; j + 1u < ncp; j += 32u) dom_walk<MODE>(a, sm, j, width, height, thickness);
+}
+
+// The map's front depths as the flattened layers pass reads them: dequantised
+// (as float bits; empty texels keep kDomEmpty, a NaN no depth has) and tiled, a
+// 32-byte sector holding 4 x 2 texels, a 128-byte line 8 x 4, so that the
+// texels of a short stretch of a strand share lines.
+__device__ __forceinline__ uint32_t front_index(uint32_t x, uint32_t y, uint32_t lines_x) {
+    return ((y >> 2) * lines_x + (x >> 3)) * 32u + ((y & 2u) << 3 | (x & 4u) << 1 | (y & 1u) << 2 | (x & 3u));
+}
+
+// Four texels of a row (half a sector) per thread, in plane order.
+__device__ __forceinline__ void front_quad(const hg_hair_params& p, const uint32_t* __restrict__ dom,
+                                           uint32_t* __restrict__ front, uint32_t w, uint32_t h, uint32_t lines_x,
+                                           uint32_t q) {
+    const uint32_t line = q >> 3, in = q & 7u;  // in: y1 x2 y0, the index bits above x's lowest two
+    const uint32_t x = line % lines_x * 8u + (in & 2u) * 2u;
+    const uint32_t y = line / lines_x * 4u + (in >> 2 & 1u) * 2u + (in & 1u);
+    uint32_t z[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4u; ++k) {
+        const uint32_t v = x + k < w && y < h ? __ldg(&dom[(size_t)y * w + x + k]) : kDomEmpty;
+        z[k] = v != kDomEmpty ? __float_as_uint(dequantize_depth(v, p.screen[2], p.screen[3])) : kDomEmpty;
     }
+    reinterpret_cast<uint4*>(front)[q] = make_uint4(z[0], z[1], z[2], z[3]);
+}
+
+__global__ void __launch_bounds__(256) dom_front_kernel(const hg_hair_params p, const uint32_t* __restrict__ dom,
+                                                        uint32_t* __restrict__ front, uint32_t w, uint32_t h,
+                                                        uint32_t quads) {
+    const uint32_t lines_x = (w + 7u) >> 3, q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < quads) front_quad(p, dom, front, w, h, lines_x, q);
+}
+
+// a / b, correctly rounded, from y = RN(1/b): a product, a residual and a
+// correction make a faithful quotient, and one more residual and correction
+// round it correctly (Markstein 1990; Cornea, Harrison and Tang 2002), as long
+// as nothing overflows and the residuals do not underflow.  For divisors that
+// several dividends share; five instructions.
+__device__ __forceinline__ float div_shared(float a, float b, float y) {
+    float q = __fmul_rn(a, y);
+    q = __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+    return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+}
+
+// The walk of raster_dom in closed form, for segments of fewer than 1,024
+// steps and coordinates below 2^20: it visits major + 1 texels (major, minor:
+// the larger and smaller of dx, dy), one step along the major axis each, and
+// after n of them the minor axis has made
+//   floor((2 n minor + major - 1) / (2 major)) = floor(n minor / major + (major - 1/2) / (2 major))
+// steps (its error term err = dx (1 + ny) - dy (1 + nx) makes one exactly when
+// 2 n minor > major (2 k + 1)).  The half keeps the argument at least
+// 1 / (4 major) > 2.4e-4 away from an integer, more than the 1.9e-4 that the
+// rounded quotients and the FMA can be off.
+constexpr float kDomWalkCoord = 1048576.0f;
+// Segment tags (beside the segment's index in bits 0..6).
+constexpr int32_t kTagSkip = 1 << 7, kTagXMajor = 1 << 8, kTagXNeg = 1 << 9, kTagYNeg = 1 << 10, kTagExactDiv = 1 << 11;
+
+// The layers pass of one generated strand (raster_dom<2>'s writes).  The
+// texels of every segment's walk are flattened into one list (append_runs4, as
+// the camera raster's samples are) that the 32 lanes walk 32 at a time, so a
+// warp's front-depth load covers 32 consecutive texels of the strand's path, 4
+// to 12 lines of the tiled plane.  With a segment per lane every lane's texel
+// was in a line of its own, and the pass, which issues a load and a reduction
+// per texel, was bound by the L1's one line a cycle (1920 x 1080 benchmark
+// frame: 63 M lines, about 0.41 M cycles an SM, all of its 212 us).  Now bound
+// by issue (74 % of the slots) and by the reductions' lines (L1 73 %); the
+// divisions have divisors that their samples share.  1920 x 1080 benchmark
+// frame (1024^2 map): 212 -> 202 us; 3840 x 2160 (2048^2): 775 -> 636.
+// (The depth pass, one reduction a texel, is faster with a segment per lane:
+// 146 against 180 us.)
+template <class Args>
+__device__ __forceinline__ void raster_dom_layers(const Args& a, StrandSmem& sm, uint32_t ncp, uint32_t lane) {
+    const hg_hair_params& p = a.p;
+    const int32_t width = f2i(p.screen[0]), height = f2i(p.screen[1]);
+    const float fw = __int2float_rn(width), fh = __int2float_rn(height);
+    const uint32_t lines_x = ((uint32_t)width + 7u) >> 3;
+    const float near_ = p.screen[2], far_ = p.screen[3];
+    const f3 cam = mk3(p.camera_pos[0], p.camera_pos[1], p.camera_pos[2]);
+    const f3 fwd = mk3(p.camera_forward[0], p.camera_forward[1], p.camera_forward[2]);
+    uint32_t* counters = a.dom + (size_t)((uint32_t)width * (uint32_t)height);
+    // slice thickness, the same for every texel
+    const float thickness = __fdiv_rn(fmaxf(far_ - near_, 1e-3f), (float)kDomLayers);
+    const float inv_thickness = __frcp_rn(thickness);
+    const bool range_ok = thickness < 1e30f && fabsf(near_) < 1e30f && fabsf(far_) < 1e30f;
+    int32_t cnt[4], tag[4];
+    uint32_t slow = 0;  // bit k: segment lane + 32 k is walked by its lane alone
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const uint32_t j = lane + 32u * k;
+        cnt[k] = tag[k] = 0;
+        if (j + 1u >= ncp) continue;
+        if (sm.cp[j].w == 0.0f && sm.cp[j + 1u].w == 0.0f) continue;
+        const float4 A = sm.cs[j], B = sm.cs[j + 1u];
+        const float fx0 = floorf(A.x), fy0 = floorf(A.y);
+        const float dx = floorf(B.x) - fx0, dy = floorf(B.y) - fy0;  // exact below 2^20
+        const float major = fmaxf(fabsf(dx), fabsf(dy)), minor = fminf(fabsf(dx), fabsf(dy));
+        if (!(fabsf(A.x) < kDomWalkCoord && fabsf(A.y) < kDomWalkCoord && fabsf(B.x) < kDomWalkCoord &&
+              fabsf(B.y) < kDomWalkCoord && major < (float)kDomMaxSteps && range_ok)) {
+            slow |= 1u << k;
+            continue;
+        }
+        const int32_t skip = j != 0u && major > 0.0f ? 1 : 0;
+        const float2 seg = make_float2(B.x - A.x, B.y - A.y);
+        // every dividend of t is RN(RN(cx sx) + RN(cy sy)) with offsets c of 0 or
+        // 2^-25..2^22: seg components of 0 or at least 2^-40 keep it 0 or a
+        // multiple of 2^-89, and the quotient below 2^64
+        const bool exact_div = (seg.x != 0.0f && fabsf(seg.x) < 0x1p-40f) || (seg.y != 0.0f && fabsf(seg.y) < 0x1p-40f);
+        cnt[k] = (int32_t)major + 1 - skip;
+        tag[k] = (int32_t)j | (skip ? kTagSkip : 0) | (fabsf(dx) >= fabsf(dy) ? kTagXMajor : 0) |
+                 (dx < 0.0f ? kTagXNeg : 0) | (dy < 0.0f ? kTagYNeg : 0) | (exact_div ? kTagExactDiv : 0);
+        // start texel's centre, the minor axis's steps per step and their offset
+        const float inv = major > 0.0f ? __frcp_rn(major) : 0.0f;
+        sm.ct[j] = make_float4(fx0 + 0.5f, fy0 + 0.5f, minor * inv, (major - 0.5f) * 0.5f * inv);
+        sm.vd[j] = __frcp_rn(fmaxf(dot2(seg, seg), 1e-6f));
+    }
+    int32_t total, runs;
+    append_runs4(sm, cnt, tag, lane, total, runs);
+    __syncwarp();
+    int32_t rw = 0;  // the run holding sample `base`
+    for (int32_t base = 0; base < total; base += 32) {
+        const int32_t s = min(base + (int32_t)lane, total - 1);
+        const int32_t r = run_of_lane(sm, runs, rw, base, lane);
+        if (base + (int32_t)lane >= total) continue;
+        const int32_t jn = sm.u.run.seg[r];
+        const int32_t j = jn & 0x7f;
+        const float n = __int2float_rn(s - sm.u.run.off[r] + (jn >> 7 & 1));
+        const float4 w = sm.ct[j];
+        const float m = floorf(__fmaf_rn(n, w.z, w.w));
+        const bool x_major = (jn & kTagXMajor) != 0;
+        const float ax = x_major ? n : m, ay = x_major ? m : n;
+        const float cx = w.x + ((jn & kTagXNeg) ? -ax : ax), cy = w.y + ((jn & kTagYNeg) ? -ay : ay);
+        if (!(cx >= 0.0f && cy >= 0.0f && cx < fw && cy < fh)) continue;
+        const uint32_t px = f2u(cx), py = f2u(cy);
+        const uint32_t cur = __ldg(&a.front[front_index(px, py, lines_x)]);
+        const float2 A = *reinterpret_cast<const float2*>(&sm.cs[j]), B = *reinterpret_cast<const float2*>(&sm.cs[j + 1]);
+        const float2 seg = sub2(B, A);
+        const float len2 = fmaxf(dot2(seg, seg), 1e-6f);
+        const float num = dot2(sub2(make_float2(cx, cy), A), seg);
+        const float t = clampf((jn & kTagExactDiv) ? __fdiv_rn(num, len2) : div_shared(num, len2, sm.vd[j]), 0.0f, 1.0f);
+        const float dist = dot3(sub3(mix3(xyz(sm.cp[j]), xyz(sm.cp[j + 1]), t), cam), fwd);
+        if (cur == kDomEmpty || dist <= near_ || dist >= far_) continue;
+        const float tt = div_shared(fmaxf(dist - __uint_as_float(cur), 0.0f), thickness, inv_thickness);
+        const uint32_t slice = min(f2u(tt), kDomLayers - 1u);
+        atomicAdd(&counters[(py * (uint32_t)width + px) * kDomLayers + slice], 1u);
+    }
+    for (; slow; slow &= slow - 1u) dom_walk<2>(a, sm, lane + 32u * (uint32_t)(__ffs(slow) - 1), width, height, thickness);
 }
 
 // Strand cache: every strand of the groom at kCacheCps control points, world
@@ -1456,6 +1611,8 @@ __global__ void __launch_bounds__(kRasterThreads, raster_min_blocks<MODE>()) ras
         if (MODE == 0) {
             float beta = __fdiv_rn(__uint2float_rn(ref.n_lod), __uint2float_rn(max(bundle.strand_count, 1u)));
             raster_camera(a, sm, ncp, uv, beta, lane, r2_max, a.tile_depth, a.tiles_x, deferred);
+        } else if (MODE == 2 && a.front) {
+            raster_dom_layers(a, sm, ncp, lane);
         } else {
             raster_dom<MODE>(a, sm, ncp, lane);
         }
@@ -1494,6 +1651,14 @@ __global__ void batch_clear_dom_kernel(const BatchView* __restrict__ views, cons
     uint32_t* map = dom + dom_prefix[blockIdx.y];
     for (size_t w = (size_t)blockIdx.x * blockDim.x + threadIdx.x; w < words; w += (size_t)gridDim.x * blockDim.x)
         map[w] = w < texels ? kDomEmpty : 0u;
+}
+
+// grid (X, DOM views): dom_front_kernel of every deep-opacity view.
+__global__ void __launch_bounds__(256) batch_dom_front_kernel(const BatchView* __restrict__ dom_views) {
+    const BatchView& v = dom_views[blockIdx.y];
+    const uint32_t lines_x = (v.dom_w + 7u) >> 3, quads = lines_x * ((v.dom_h + 3u) >> 2) * 8u;
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < quads; q += gridDim.x * blockDim.x)
+        front_quad(v.p, v.dom, v.front, v.dom_w, v.dom_h, lines_x, q);
 }
 
 __global__ void batch_lod_kernel(const BatchView* __restrict__ views, const uint32_t* __restrict__ prefix,
@@ -1647,7 +1812,7 @@ __global__ void __launch_bounds__(kRasterThreads, 6) batch_raster_kernel(const B
             const float2 uv = pcg_uv(ref.strand ^ (ref.bundle * 0x85ebca6bu));
             if (PHASE == 1) {
                 const uint32_t ncp = generate_strand<2>(a, sm, ref, bundle, uv, lane);
-                raster_dom<2>(a, sm, ncp, lane);
+                raster_dom_layers(a, sm, ncp, lane);
             } else if (cam) {
                 const float4* deferred = nullptr;
                 const uint32_t ncp = generate_strand<0>(a, sm, ref, bundle, uv, lane, PHASE == 2 ? &deferred : nullptr);
@@ -2373,6 +2538,7 @@ cudaError_t launch_raster(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p, int
     a.cons = ctx->cons;
     a.beta = ctx->beta;
     a.dom = ctx->dom;
+    a.front = nullptr;
     a.scene = scene;
     a.err = ctx->err;
     a.bundle_count = g->bundle_count;
@@ -2420,6 +2586,14 @@ cudaError_t launch_raster(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p, int
         raster_kernel<1><<<std::min(blocks, ctx->sm_count * raster_min_blocks<1>() * kDomGridRounds), kRasterThreads, 0,
                            ctx->stream>>>(a);
     } else {
+        if (layers_use_plane(g->strand_total, ctx->dom_w, ctx->dom_h)) {
+            const uint32_t quads = (uint32_t)(front_words(ctx->dom_w, ctx->dom_h) / 4u);
+            dom_front_kernel<<<(quads + 255u) / 256u, 256, 0, ctx->stream>>>(p, ctx->dom, ctx->dom_front, ctx->dom_w,
+                                                                          ctx->dom_h, quads);
+            const cudaError_t e = cudaGetLastError();
+            if (e != cudaSuccess) return e;
+            a.front = ctx->dom_front;
+        }
         raster_kernel<2><<<std::min(blocks, ctx->sm_count * raster_min_blocks<2>() * kDomGridRounds), kRasterThreads, 0,
                            ctx->stream>>>(a);
     }
@@ -2483,6 +2657,8 @@ cudaError_t launch_batch_raster(hg_ctx* ctx, const BatchDev& b) {
     batch_raster_kernel<2><<<blocks, kRasterThreads, 0, ctx->stream>>>(b.views, 0u, b.n_cam, b.counters + 2, chunk);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (b.n_views > b.n_cam) {
+        batch_dom_front_kernel<<<dim3(64, b.n_views - b.n_cam), 256, 0, ctx->stream>>>(b.views + b.n_cam);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
         batch_raster_kernel<1><<<blocks, kRasterThreads, 0, ctx->stream>>>(b.views, b.n_cam, b.n_views - b.n_cam,
                                                                            b.counters + 1, chunk);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;

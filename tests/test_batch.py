@@ -306,3 +306,66 @@ def test_batched_frame_keeps_the_strand_cache_honest(renderer):
     np.testing.assert_array_equal(renderer.read(abi.BUF_CENTER), center)
     np.testing.assert_array_equal(renderer.read(abi.BUF_CONSERVATIVE), cons)
     _close(b, grooms)
+
+
+def _zoom_on_strand(mesh, cam, dom, lights, magnify):
+    """The light's view magnified in x and y about a texel that a strand covers
+    (found in steps of at most 8, so that the strand stays in sight)."""
+    dom = dom.copy()
+    clip = dom["clip_from_world"].reshape(4, 4)  # column vectors; orthographic: w is 1
+    while magnify > 1.0:
+        step = min(magnify, 8.0)
+        w, h = int(dom["screen"][0]), int(dom["screen"][1])
+        depth = oracle.frame(mesh, cam, dom, lights)["dom"][: w * h].reshape(h, w)
+        ys, xs = np.nonzero(depth != np.uint32(0xFFFFFFFF))
+        mid = len(ys) // 2  # a walk of more than 1,024 texels ends before the map: stay where it is
+        centre = ((2 * xs[mid] + 1) / w - 1, 1 - (2 * ys[mid] + 1) / h) if len(ys) else (0.0, 0.0)
+        clip[3, :2] -= np.array(centre, dtype=np.float32)
+        clip[:, :2] *= np.float32(step)
+        magnify /= step
+    return dom
+
+
+@pytest.mark.parametrize("size, magnify", [
+    ((13, 7), 1.0),         # partial lines of the tiled front plane, segments within one texel
+    ((33, 101), 3.0),       # partial lines, starts off the map
+    ((512, 512), 40.0),     # segments of hundreds of texels
+    ((1000, 700), 100.0),   # segments on both sides of the 1,024-texel walk limit
+    ((64, 64), 1.0e5),      # screen coordinates beyond 2^20
+])
+def test_layers_walk_matches_the_oracle_at_its_edges(renderer, size, magnify):
+    """The layers pass's flattened walk (the batch always takes it) against the
+    oracle's texel by texel one, with the light's view magnified in x and y."""
+    bs = configs.config4(scale=0.01, items=3)
+    for s in bs.scenes:
+        s.dom_size = size
+    b, grooms, params = _make(renderer, bs)
+    lights = bs.light_array()
+    doms = [_zoom_on_strand(s.mesh, cam, dom, lights, magnify) for s, (cam, dom) in zip(bs.scenes, params)]
+    for k, (cam, _) in enumerate(params):
+        b.set_params(k, cam, doms[k])
+    b.frame(lights)
+    assert renderer.synchronize() == 0
+    for k, (cam, _) in enumerate(params):
+        want = oracle.frame(bs.scenes[k].mesh, cam, doms[k], lights)
+        np.testing.assert_array_equal(b.read(k, abi.BUF_DOM), want["dom"])
+    _close(b, grooms)
+
+
+def test_large_groom_layers_walk_equals_the_batched_one(renderer):
+    """A single groom from 32,768 strands up forms the front plane for its
+    layers pass; a smaller one walks a segment per lane.  Both draw the maps of
+    the batch, and the launch counts follow."""
+    scenes = [configs.config2(scale=n / 100_000) for n in (32_767, 32_768)]
+    bs = configs.BatchScene("layers", scenes, scenes[0].lights)
+    assert [s.mesh.strand_count() for s in scenes] == [32_767, 32_768]
+    b, grooms, _ = _make(renderer, bs)
+    lights = bs.light_array()
+    b.frame(lights, abi.BATCH_GRAPH)
+    assert renderer.synchronize() == 0
+    graph = _read_all(b, 2)
+    b.frame(lights, abi.BATCH_SEPARATE)
+    assert renderer.synchronize() == 0
+    _compare(graph, _read_all(b, 2))
+    assert b.launches(abi.BATCH_SEPARATE) == 18 + 19
+    _close(b, grooms)

@@ -9,6 +9,8 @@ without FMA contraction; a fused multiply-add is emulated exactly).
 * approx_depth (the division-free depth pre-test) stays within 5 units of
   quantize_depth.
 * sqrt_bound: sqrt_rn(x) <= r exactly when x <= sqrt_bound(r).
+* raster_dom_layers' closed form visits the texels of the Bresenham walk.
+* div_shared: a / b from RN(1/b) with two corrections is correctly rounded.
 """
 from fractions import Fraction
 
@@ -115,3 +117,50 @@ def test_sqrt_bound_decides_like_the_square_root():
         assert np.sqrt(np.nextafter(x, F(np.inf))) > r
         d = (x * (1 + rng.uniform(-1e-5, 1e-5, 20000))).astype(F)
         assert np.array_equal(np.sqrt(d) <= r, d <= x)
+
+
+def _walk_minor_steps(major, minor):
+    """Minor-axis steps made before each visited texel: the walk of raster_dom."""
+    err, k, out = major - minor, 0, []
+    for n in range(major + 1):
+        out.append(k)
+        if n == major and k == minor:
+            break
+        e2 = 2 * err
+        assert e2 > -minor or major == 0  # the major axis steps every time
+        err -= minor
+        if e2 < major:
+            err += major
+            k += 1
+    return np.array(out)
+
+
+def test_closed_form_walk_equals_the_bresenham_walk():
+    majors = list(range(0, 41)) + [63, 64, 65, 127, 251, 509, 510, 1021, 1022, 1023]
+    rng = np.random.default_rng(11)
+    for major in majors:
+        minors = range(major + 1) if major <= 40 else np.unique(np.r_[0, 1, major // 2, major - 1, major,
+                                                                     rng.integers(0, major + 1, 40)])
+        inv = _rn32(Fraction(1, major)) if major else F(0)
+        n = np.arange(major + 1)
+        offset = F(F(F(F(major) - F(0.5)) * F(0.5)) * inv)
+        for minor in minors:
+            minor = int(minor)
+            slope = F(F(minor) * inv)
+            # the product and sum are exact in double: one rounding, the FMA's
+            got = np.floor((n * float(slope) + float(offset)).astype(F)).astype(np.int64)
+            np.testing.assert_array_equal(got, _walk_minor_steps(major, minor), err_msg=f"{major} {minor}")
+
+
+def test_div_shared_is_correctly_rounded():
+    rng = np.random.default_rng(12)
+    a = F(rng.uniform(-2, 2, 3000) * 2.0 ** rng.integers(-40, 40, 3000))
+    b = F(rng.uniform(1, 2, 3000) * 2.0 ** rng.integers(-19, 30, 3000))
+    a[:6] = (0.0, 1e-6, 1.0, 3.0, 2.0 ** 24 - 1, 2.0 ** -89)
+    b[:6] = (1e-6, 1e-6, 1.0 + 2.0 ** -23, 1.0 - 2.0 ** -24, 2.0 - 2.0 ** -23, 2.0 ** 41)
+    for x, y in zip(a, b):
+        r = _rn32(Fraction(1) / Fraction(float(y)))
+        q = F(x * r)
+        for _ in range(2):
+            q = _fma32(_fma32(-q, y, x), r, q)
+        assert q == F(x / y), (x, y)
