@@ -460,6 +460,10 @@ constexpr int raster_min_blocks() { return MODE == 0 ? 6 : 7; }
 // config 2, 0.473 -> 0.426 ms on config 3).  The camera stages keep one
 // round (two measured 0.356 -> 0.364 ms).
 constexpr int kDomGridRounds = 8;
+// Resident blocks per SM of the cache's generation: the batched kernel needs 88
+// registers without a bound (5 blocks, 119 us on 24 grooms of the batch
+// benchmark's sizes; 6 blocks 113, 8 blocks and a few spills 110).
+constexpr int kGenBlocks = 8;
 
 // Per-warp shared memory, 7 KB.  The layer samples are needed only while
 // control points are generated, so they share storage with the run list.
@@ -1439,87 +1443,207 @@ struct GenArgs {
     uint32_t strands;
 };
 
-// The last control point (index 64) of up to 32 strands, finished together
-// one per lane: the model-space point and its neighbour 63, w and ao, from
-// generate_one, and the strand (and batch view) it belongs to.
-struct CacheTails {
-    float4 a[32];  // model point 64 xyz, ao
-    float4 b[32];  // model point 63 xyz, w
-    uint32_t strand[32];
-    uint32_t view[32];
+// Per-warp shared memory of the cache's generation.  `tails`: the last
+// control point (index 64) of up to 32 strands, finished together one per
+// lane; the strand and the batch view it belongs to.
+struct GenSmem {
+    float4 lp[2][16];  // layer sample: position, ao (of each strand of the pair)
+    float4 lt[2][16];  // layer tangent
+    float4 ls[2][16];  // style residual of each w layer at the strand's (u, v)
+    struct {
+        float4 a[32];  // model point 64 xyz, ao
+        float4 b[32];  // model point 63 xyz, w
+        uint32_t strand[32];
+        uint32_t view[32];
+    } tails;
 };
+static_assert(kLayerCount == 16 && kStyleW == 16, "two lanes a layer");
+static_assert(kCacheCps == 65, "two full rounds of 32 control points and one tail point");
 
-// Strand g of a groom into its cache slot (one warp): control points 0..63
-// on the 32 lanes in two rounds.  Point 64 alone would take a third round at
-// one lane in 32, so its inputs go to tails slot `slot` instead, and
-// finish_tails completes 32 strands' last points in one round.
-template <class Args>
-__device__ __forceinline__ void generate_one(const Args& a, uint32_t g, float4* lp, float4* lt, float4* ls,
-                                             uint32_t lane, CacheTails& tails, uint32_t slot, uint32_t view) {
-    static_assert(kCacheCps == 65, "two full rounds of 32 control points and one tail point");
-    const uint32_t b = a.strand_bundle[g];
-    const uint32_t s = g - a.strand_base[b];
-    const hg_gpu_bundle bundle = a.bundles[b];
-    const float2 uv = pcg_uv(s ^ (b * 0x85ebca6bu));
-    f3 mp[4];
-    float wk[4], aok[4];
-    model_cps(a.layers, a.style, lp, lt, ls, bundle, uv, kCacheCps, lane, mp, wk, aok);
-    float4* pos = a.cache + (size_t)g * (2u * kCacheCps);
-    float4* tan = pos + kCacheCps;
+// The corners of a bilinear lookup along u, of the pair's two strands at once:
+// xa and xb are the lane's corners of strands 0 and 1 (u0 in the strand's own
+// lane, u1 in the other), already weighted.  Returns the own strand's
+// u0 corner and gives its u1 corner in `other`.
+__device__ __forceinline__ float own_corner(float xa, float xb, bool second, float& other) {
+    other = __shfl_xor_sync(0xffffffffu, second ? xa : xb, 1);
+    return second ? xb : xa;
+}
+
+// The control points of a pair of strands at kCacheCps, into their cache slots
+// (one warp).  `mine`: the arguments of the lane's own strand g (even lanes the
+// first, odd lanes the second), of(v) those of view v.  Lanes without a strand
+// (valid false) repeat the last one and write nothing.  The operations are
+// model_cps' and generate_slot's, in their order; what differs is who does
+// them:
+//  - lanes 2 l and 2 l + 1 sample layer l of both strands' cages and style
+//    blocks, the two corners along u of one strand in one load: they share a
+//    128-byte line (the four corners of a layer are one line, a row of the
+//    style block is one), and a load costs the L1 a cycle a line;
+//  - lane 2 l + h then holds layer l of strand h: tangents of both at once;
+//  - the last point, w = 1, is the last layer's with t = 0 and is formed for
+//    both strands at once; its world position and tangent wait in a tails slot
+//    until finish_tail does 32 of them;
+//  - w = idx / 64 is a product, exactly.
+// Bound by the L1's wavefronts (74 % at 100,000 strands: 64 lines of samples a
+// strand, 48 of shared memory, 33 of shuffles, 18 of stores) and issue (68 %);
+// a strand per warp with a corner per load had 128 lines and a third round of
+// one lane: 115 -> 91 us on 100,000 strands.
+template <class Args, class Of>
+__device__ __forceinline__ void generate_pair(const Args& mine, Of of, uint32_t g, bool valid, uint32_t view,
+                                              GenSmem& sm, uint32_t slot, uint32_t lane) {
+    const uint32_t half = lane & 1u, layer = lane >> 1;
+    const bool second = half != 0u;
+    const uint32_t b = mine.strand_bundle[g];
+    const float2 uv = pcg_uv((g - mine.strand_base[b]) ^ (b * 0x85ebca6bu));
+    const float4* cage = mine.layers + 2u * (mine.bundles[b].layer_offset + layer * 4u);
+    const float4* block = mine.style + (mine.bundles[b].style_offset + layer * (kStyleU * kStyleV));
+    // the cage's weights and the style lookup of the own strand
+    const float4 wgt = make_float4((1.0f - uv.x) * (1.0f - uv.y), uv.x * (1.0f - uv.y), (1.0f - uv.x) * uv.y,
+                                   uv.x * uv.y);
+    const float su = clampf(uv.x, 0.0f, 1.0f) * (float)(kStyleU - 1u);
+    const float sv = clampf(uv.y, 0.0f, 1.0f) * (float)(kStyleV - 1u);
+    const uint32_t u0 = f2u(floorf(su)), v0 = f2u(floorf(sv));
+    const float tu = su - __uint2float_rn(u0), tv = sv - __uint2float_rn(v0);
+    const uint32_t row0 = v0 * kStyleU, row1 = min(v0 + 1u, kStyleV - 1u) * kStyleU;
+    // strand h: its layer's address and the lane's corner of it
+    float4 c0[2], c1[2];  // weighted cage corners: v0 row, v1 row
+    f3 s0[2], s1[2];      // weighted style corners
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        f3 prev, next;
-        if (k == 0) cp_neighbours<0>(mp, lane, prev, next);
-        if (k == 1) cp_neighbours<1>(mp, lane, prev, next);
-        const uint32_t idx = lane + 32u * k;
-        const f3 wp = to_world(a.p, mp[k]);
-        const f3 wt = cp_world_tangent(a.p, idx, kCacheCps, prev, mp[k], next);
-        pos[idx] = make_float4(wp.x, wp.y, wp.z, aok[k]);
-        tan[idx] = make_float4(wt.x, wt.y, wt.z, wk[k]);
+    for (int h = 0; h < 2; ++h) {
+        const int src = (int)((lane & ~1u) | (uint32_t)h);
+        const bool own = half == (uint32_t)h;
+        const float4* c = reinterpret_cast<const float4*>(
+            __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(cage), src)) + (own ? 0 : 2);
+        const float wx = __shfl_sync(0xffffffffu, wgt.x, src), wy = __shfl_sync(0xffffffffu, wgt.y, src);
+        const float wz = __shfl_sync(0xffffffffu, wgt.z, src), ww = __shfl_sync(0xffffffffu, wgt.w, src);
+        const uint32_t hu0 = __shfl_sync(0xffffffffu, u0, src);
+        const float htu = __shfl_sync(0xffffffffu, tu, src);
+        const float4* s = reinterpret_cast<const float4*>(
+            __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(block), src)) +
+                          (own ? hu0 : min(hu0 + 1u, kStyleU - 1u));
+        const uint32_t r0 = __shfl_sync(0xffffffffu, row0, src), r1 = __shfl_sync(0xffffffffu, row1, src);
+        const float4 a0 = __ldg(c), a1 = __ldg(c + 4);
+        const f3 b0 = xyz(__ldg(s + r0)), b1 = xyz(__ldg(s + r1));
+        const float w0 = own ? wx : wy, w1 = own ? wz : ww, ws = own ? 1.0f - htu : htu;
+        c0[h] = make_float4(a0.x * w0, a0.y * w0, a0.z * w0, a0.w * w0);
+        c1[h] = make_float4(a1.x * w1, a1.y * w1, a1.z * w1, a1.w * w1);
+        s0[h] = mul3s(b0, ws);
+        s1[h] = mul3s(b1, ws);
     }
-    // point 64 is slot 2 of lane 0; its neighbour 63 is slot 1 of lane 31
-    const f3 p63 = shfl_idx3(mp[1], 31);
-    if (lane == 0) {
-        tails.a[slot] = make_float4(mp[2].x, mp[2].y, mp[2].z, aok[2]);
-        tails.b[slot] = make_float4(p63.x, p63.y, p63.z, wk[2]);
-        tails.strand[slot] = g;
-        tails.view[slot] = view;
+    // bilinear4 and the style layer's lookup: the same products and sums
+    auto cage_sum = [&](float a0, float b0, float a1, float b1) {
+        float u1v0, u1v1;
+        const float u0v0 = own_corner(a0, b0, second, u1v0), u0v1 = own_corner(a1, b1, second, u1v1);
+        return ((u0v0 + u1v0) + u0v1) + u1v1;
+    };
+    const float4 loaded =
+        make_float4(cage_sum(c0[0].x, c0[1].x, c1[0].x, c1[1].x), cage_sum(c0[0].y, c0[1].y, c1[0].y, c1[1].y),
+                    cage_sum(c0[0].z, c0[1].z, c1[0].z, c1[1].z), cage_sum(c0[0].w, c0[1].w, c1[0].w, c1[1].w));
+    auto style_mix = [&](float a0, float b0, float a1, float b1) {
+        float o0, o1;
+        const float m0 = own_corner(a0, b0, second, o0), m1 = own_corner(a1, b1, second, o1);
+        return mixf(m0 + o0, m1 + o1, tv);
+    };
+    const f3 s = mk3(style_mix(s0[0].x, s0[1].x, s1[0].x, s1[1].x), style_mix(s0[0].y, s0[1].y, s1[0].y, s1[1].y),
+                     style_mix(s0[0].z, s0[1].z, s1[0].z, s1[1].z));
+    const float4 prev_l = shfl_up4(loaded, 2), next_l = shfl_down4(loaded, 2);
+    const f3 curr = xyz(loaded);
+    const f3 tl = calc_tangent(layer, kLayerCount, xyz(prev_l), curr, xyz(next_l));
+    sm.lp[half][layer] = loaded;
+    sm.lt[half][layer] = make_float4(tl.x, tl.y, tl.z, 0.0f);
+    sm.ls[half][layer] = make_float4(s.x, s.y, s.z, 0.0f);
+    const f3 last = add3(hermite(curr, curr, tl, tl, 0.0f), mix3(s, s, 0.0f));  // of lanes 30 and 31
+    const float last_ao = mixf(loaded.w, loaded.w, 0.0f);
+    if (layer == kLayerCount - 1u && valid) {
+        sm.tails.a[slot + half] = make_float4(last.x, last.y, last.z, last_ao);
+        sm.tails.strand[slot + half] = g;
+        sm.tails.view[slot + half] = view;
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (uint32_t h = 0; h < 2u; ++h) {
+        if (!__shfl_sync(0xffffffffu, valid ? 1 : 0, (int)h)) break;
+        const Args& a = of(__shfl_sync(0xffffffffu, view, (int)h));
+        float4* pos = a.cache + (size_t)__shfl_sync(0xffffffffu, g, (int)h) * (2u * kCacheCps);
+        float4* tan = pos + kCacheCps;
+        f3 mp[2];
+        float wk[2], aok[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const float w = __uint2float_rn(lane + 32u * k) * (1.0f / (float)(kCacheCps - 1u));
+            const float layers_f = w * (float)(kLayerCount - 1u);
+            const uint32_t i0 = f2u(floorf(layers_f)), i1 = i0 + 1u;  // w < 1
+            const float t = layers_f - __uint2float_rn(i0);
+            const float4 la = sm.lp[h][i0], lb = sm.lp[h][i1];
+            const f3 base = hermite(xyz(la), xyz(lb), xyz(sm.lt[h][i0]), xyz(sm.lt[h][i1]), t);
+            mp[k] = add3(base, mix3(xyz(sm.ls[h][i0]), xyz(sm.ls[h][i1]), t));
+            wk[k] = w;
+            aok[k] = mixf(la.w, lb.w, t);
+        }
+        // neighbours by rotation: point 32 to lane 31 through lane 0, point 31
+        // to lane 0 through lane 31, and point 64 to lane 31
+        const f3 prev0 = shfl_up3(mp[0]), next0 = shfl_idx3(lane == 0 ? mp[1] : mp[0], (int)((lane + 1u) & 31u));
+        const f3 prev1 = shfl_idx3(lane == 31 ? mp[0] : mp[1], (int)((lane + 31u) & 31u));
+        f3 next1 = shfl_down3(mp[1]);
+        const float4 p64 = sm.tails.a[slot + h];
+        if (lane == 31) {
+            next1 = xyz(p64);
+            sm.tails.b[slot + h] = make_float4(mp[1].x, mp[1].y, mp[1].z, 1.0f);
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const uint32_t idx = lane + 32u * k;
+            const f3 wp = to_world(a.p, mp[k]);
+            const f3 wt = cp_world_tangent(a.p, idx, kCacheCps, k == 0 ? prev0 : prev1, mp[k], k == 0 ? next0 : next1);
+            pos[idx] = make_float4(wp.x, wp.y, wp.z, aok[k]);
+            tan[idx] = make_float4(wt.x, wt.y, wt.z, wk[k]);
+        }
     }
     __syncwarp();
 }
 
 // Control point 64 of the strand in tails slot `slot` (a: that strand's
-// arguments), written as generate_one's third round would (cp_world_tangent
-// of the last point uses its previous neighbour and itself).  The lanes of a
-// warp finish up to 32 slots at once.
+// arguments): to_world and cp_world_tangent of the last point, which uses its
+// previous neighbour and itself.  The lanes of a warp finish up to 32 slots
+// at once.
 template <class Args>
-__device__ __forceinline__ void finish_tail(const Args& a, const CacheTails& tails, uint32_t slot) {
-    const float4 ta = tails.a[slot], tb = tails.b[slot];
+__device__ __forceinline__ void finish_tail(const Args& a, const GenSmem& sm, uint32_t slot) {
+    const float4 ta = sm.tails.a[slot], tb = sm.tails.b[slot];
     const f3 curr = mk3(ta.x, ta.y, ta.z), prev = mk3(tb.x, tb.y, tb.z);
     const uint32_t idx = kCacheCps - 1u;
     const f3 wp = to_world(a.p, curr);
     const f3 wt = cp_world_tangent(a.p, idx, kCacheCps, prev, curr, curr);
-    float4* pos = a.cache + (size_t)tails.strand[slot] * (2u * kCacheCps);
+    float4* pos = a.cache + (size_t)sm.tails.strand[slot] * (2u * kCacheCps);
     pos[idx] = make_float4(wp.x, wp.y, wp.z, ta.w);
     pos[kCacheCps + idx] = make_float4(wt.x, wt.y, wt.z, tb.w);
 }
 
-__global__ void __launch_bounds__(kRasterThreads) generate_kernel(const GenArgs a) {
-    __shared__ float4 lp[kRasterWarps][16];
-    __shared__ float4 lt[kRasterWarps][16];
-    __shared__ float4 ls[kRasterWarps][16];
-    __shared__ CacheTails tails[kRasterWarps];
+// Strands 0 .. total - 1 over the grid's warps, a pair at a time.
+// locate(g): g's view and its index in that view; of(v): view v's arguments.
+template <class Locate, class Of>
+__device__ __forceinline__ void generate_strands(GenSmem& sm, uint32_t total, Locate locate, Of of) {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t nwarps = gridDim.x * kRasterWarps;
+    const uint32_t step = 2u * gridDim.x * kRasterWarps;
     uint32_t n = 0;
-    for (uint32_t g = blockIdx.x * kRasterWarps + warp; g < a.strands; g += nwarps) {
-        generate_one(a, g, lp[warp], lt[warp], ls[warp], lane, tails[warp], n, 0u);
-        if (++n == 32u || g + nwarps >= a.strands) {
-            if (lane < n) finish_tail(a, tails[warp], lane);
+    for (uint32_t g0 = 2u * (blockIdx.x * kRasterWarps + warp); g0 < total; g0 += step) {
+        const uint32_t g = min(g0 + (lane & 1u), total - 1u);
+        const bool valid = g0 + (lane & 1u) < total;
+        uint32_t v = 0, s = g;
+        locate(g, v, s);
+        generate_pair(of(v), of, s, valid, v, sm, n, lane);
+        n += g0 + 1u < total ? 2u : 1u;
+        if (n == 32u || total - g0 <= step) {
+            if (lane < n) finish_tail(of(sm.tails.view[lane]), sm, lane);
             __syncwarp();
             n = 0;
         }
     }
+}
+
+__global__ void __launch_bounds__(kRasterThreads, kGenBlocks) generate_kernel(const GenArgs a) {
+    __shared__ GenSmem sm[kRasterWarps];
+    generate_strands(sm[threadIdx.x >> 5], a.strands, [](uint32_t, uint32_t&, uint32_t&) {},
+                     [&](uint32_t) -> const GenArgs& { return a; });
 }
 
 // Asynchronous global -> shared copies (cp.async) of the ref loop's next
@@ -1716,25 +1840,17 @@ __global__ void __launch_bounds__(256) batch_tile_depth_kernel(const BatchView* 
     if (lane == 0) a.tile_depth[tile] = held;
 }
 
-__global__ void __launch_bounds__(kRasterThreads) batch_generate_kernel(const BatchView* __restrict__ views,
+__global__ void __launch_bounds__(kRasterThreads, kGenBlocks) batch_generate_kernel(const BatchView* __restrict__ views,
                                                                         const uint32_t* __restrict__ prefix,
                                                                         uint32_t n_cam, uint32_t total) {
-    __shared__ float4 lp[kRasterWarps][16];
-    __shared__ float4 lt[kRasterWarps][16];
-    __shared__ float4 ls[kRasterWarps][16];
-    __shared__ CacheTails tails[kRasterWarps];
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t nwarps = gridDim.x * kRasterWarps;
-    uint32_t n = 0;
-    for (uint32_t g = blockIdx.x * kRasterWarps + warp; g < total; g += nwarps) {
-        const uint32_t v = find_view(prefix, n_cam, g);
-        generate_one(views[v], g - prefix[v], lp[warp], lt[warp], ls[warp], lane, tails[warp], n, v);
-        if (++n == 32u || g + nwarps >= total) {
-            if (lane < n) finish_tail(views[tails[warp].view[lane]], tails[warp], lane);
-            __syncwarp();
-            n = 0;
-        }
-    }
+    __shared__ GenSmem sm[kRasterWarps];
+    generate_strands(
+        sm[threadIdx.x >> 5], total,
+        [&](uint32_t g, uint32_t& v, uint32_t& s) {
+            v = find_view(prefix, n_cam, g);
+            s = g - prefix[v];
+        },
+        [&](uint32_t v) -> const BatchView& { return views[v]; });
 }
 
 // Persistent raster over the refs of views [first, first + n): warps take
@@ -2512,7 +2628,7 @@ cudaError_t launch_generate(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p) {
     a.strand_base = g->strand_base;
     a.cache = g->cache;
     a.strands = g->strand_total;
-    int blocks = blocks_for(ctx, (const void*)generate_kernel, kRasterThreads, g->strand_total, kRasterWarps);
+    int blocks = blocks_for(ctx, (const void*)generate_kernel, kRasterThreads, g->strand_total, 2 * kRasterWarps);
     generate_kernel<<<blocks, kRasterThreads, 0, ctx->stream>>>(a);
     return cudaGetLastError();
 }
@@ -2618,7 +2734,7 @@ cudaError_t launch_batch_setup(hg_ctx* ctx, const BatchDev& b) {
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     if (b.total_strands) {
-        const uint32_t need = (b.total_strands + kRasterWarps - 1) / kRasterWarps;
+        const uint32_t need = (b.total_strands + 2 * kRasterWarps - 1) / (2 * kRasterWarps);
         const uint32_t blocks = std::max(1u, std::min(need, b.gen_blocks));
         batch_generate_kernel<<<blocks, kRasterThreads, 0, ctx->stream>>>(b.views, b.strand_prefix, b.n_cam,
                                                                           b.total_strands);

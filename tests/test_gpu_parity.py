@@ -166,6 +166,35 @@ def test_strand_cache_gives_the_same_visibility(renderer, name):
     g.close()
 
 
+@pytest.mark.parametrize("n", [1, 2, 33, 160_001])
+def test_strand_cache_equals_strands_generated_in_the_raster(renderer, n):
+    """The cache's generation takes strands in pairs and their last points 32 at
+    a time (160,001: more than 16 pairs a warp, and an odd one); the rasters
+    without a cache generate a strand per warp."""
+    sc = configs.config1(scale=0.01)
+    sc.mesh = configs._mesh(n, 8, "curly", 77)
+    cam, dom = sc.params()
+    renderer.ensure_targets(sc.view.width, sc.view.height, *sc.dom_size)
+    g = renderer.upload(sc.mesh)
+    got = []
+    for cached in (False, True):
+        if cached:
+            renderer.generate(g, cam)
+        renderer.clear()
+        renderer.clear_dom()
+        for p, slot in ((cam, abi.SLOT_CAMERA), (dom, abi.SLOT_DOM)):
+            renderer.lod(g, p, slot)
+            renderer.scan(g, p, slot)
+            renderer.raster(g, p, slot)
+        renderer.raster(g, host.dom_layers_params(dom), abi.SLOT_DOM)
+        assert renderer.synchronize() == 0
+        got.append([renderer.read(b) for b in (abi.BUF_CENTER, abi.BUF_CONSERVATIVE, abi.BUF_BETA, abi.BUF_DOM)])
+    g.close()
+    for name, want, have in zip(("center", "conservative", "beta", "dom"), *got):
+        _assert_equal(name, have, want)
+    assert (got[0][1] != EMPTY).any()
+
+
 def test_dense_groom_with_tile_depth_rejection(renderer):
     """A dense groom at low resolution (deep overdraw) with a small deep
     opacity map: the later stages of the camera and DOM depth passes skip most
