@@ -107,15 +107,108 @@ __device__ __forceinline__ f3 lobe_mean(const Lobes& l, f3 total, f3 q) {
     return vdiv(num, vmaxs(total, 1e-5f));
 }
 
-// The azimuthal angles dual_scatter integrates over are fixed: per step i,
-// cos phi at u = (i + 0.5) / kScatterSteps for the back half (phi = u pi/2)
-// and the front half (phi = (1 + u) pi/2), with the factors of azimuthal()
-// that depend on phi alone: cos(phi/2), exp(-3.65 cos phi - 3.98) and
-// exp(17 cos phi - 16.78).  Filled from double precision on the host.
+// dual_scatter integrates azimuthal() over fixed angles: per step i,
+// u = (i + 0.5) / kScatterSteps, phi = u pi/2 for the back half and
+// (1 + u) pi/2 for the front half, each with weight w = pi / kScatterSteps.
+// What depends on phi alone is in this table, filled from double precision on
+// the host (index 0: back, 1: front), w folded in:
+//  - R, 0.25 c (f0 + (1 - f0) (1 - c cos theta_d)^5) with c = cos(phi/2), is a
+//    polynomial in s = 1 - cos theta_d, because 1 - c cos theta_d is
+//    (1 - c) + c s: the sum over the angles is one too, and its coefficients
+//    are positive, so nothing cancels;
+//  - TT: c, c (0.6 - 0.8 cos phi), and exp(-3.65 cos phi - 3.98) (1 - f0)^2;
+//  - TRT: the sum of exp(17 cos phi - 16.78).
+struct ScatterTable {
+    float r[2][6];
+    float4 tt[2][kScatterSteps];
+    float trt[2];
+};
+__constant__ ScatterTable c_scatter;
+
+// The statistics of dual_scatter (shade.wesl:166-190) from the lobes' integrals.
+__device__ __forceinline__ Dual dual_statistics(const Lobes& fwd, const Lobes& back, const Shape& shape) {
+    Dual d;
+    d.fwd = fwd;
+    f3 a_f = vmins(add3(add3(fwd.r, fwd.tt), fwd.trt), 0.95f);
+    f3 a_b = add3(add3(back.r, back.tt), back.trt);
+    f3 beta2 = vmul(shape.beta, shape.beta);
+    f3 beta_f2 = lobe_mean(fwd, a_f, beta2);
+    f3 alpha_b = lobe_mean(back, a_b, shape.alpha);
+    f3 beta_b2 = lobe_mean(back, a_b, beta2);
+    f3 af2 = vmul(a_f, a_f);
+    f3 rest = {1.0f - af2.x, 1.0f - af2.y, 1.0f - af2.z};
+    f3 ab2 = vmul(a_b, a_b);
+    f3 ab3 = vmul(ab2, a_b);
+    f3 rr = vmul(rest, rest);
+    f3 rest3 = vmul(rr, rest);
+    f3 a_back = add3(vdiv(vmul(a_b, af2), rest), vdiv(vmul(ab3, af2), rest3));
+    f3 t1 = {1.0f - 2.0f * ab2.x / rr.x, 1.0f - 2.0f * ab2.y / rr.y, 1.0f - 2.0f * ab2.z / rr.z};
+    f3 num2 = add3(mul3s(rr, 2.0f), vmul(mul3s(af2, 4.0f), ab2));
+    f3 delta_b = add3(vmul(alpha_b, t1), vdiv(vmul(alpha_b, num2), rest3));
+    f3 beta_f = vsqrt(beta_f2), beta_b = vsqrt(beta_b2);
+    f3 lead = add3(spl(1.0f), mul3s(af2, kDensityBack));
+    f3 s1 = vsqrt(add3(mul3s(beta_f2, 2.0f), beta_b2));
+    f3 s2 = vsqrt(add3(mul3s(beta_f2, 2.0f), mul3s(beta_b2, 3.0f)));
+    f3 numer = vmul(lead, add3(vmul(a_b, s1), vmul(ab3, s2)));
+    f3 den = vmaxs(add3(a_b, vmul(ab3, add3(mul3s(beta_f, 2.0f), mul3s(beta_b, 3.0f)))), 1e-5f);
+    f3 sigma_b = vdiv(numer, den);
+    d.a_f = a_f;
+    d.beta_f2 = beta_f2;
+    d.a_back = a_back;
+    d.delta_b = delta_b;
+    d.sigma_b2 = vmul(sigma_b, sigma_b);
+    return d;
+}
+
+// dual_scatter (shade.wesl:153-190); 0 < cos_theta_d <= 1.
+__device__ Dual dual_scatter(float cos_theta_d, f3 sigma_a, const Shape& shape) {
+    const float inv_ctd = 1.0f / cos_theta_d;
+    const float a = 1.0f / (1.19f * inv_ctd + 0.36f * cos_theta_d);
+    const float s = 1.0f - cos_theta_d;
+    const f3 ntau = mul3s(sigma_a, -2.0f * inv_ctd);
+    f3 tt[2] = {spl(0.0f), spl(0.0f)};
+#pragma unroll 2
+    for (int i = 0; i < kScatterSteps; ++i) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const float4 g = c_scatter.tt[half][i];
+            const float h = g.x + a * g.y, ha = h * a;
+            // (1 - F)^2 of the entry, its (1 - f0)^2 in the table
+            const float m = 1.0f - cos_theta_d * sqrtf(fmaxf(1.0f - h * h, 0.0f));
+            const float m2 = m * m, e = 1.0f - m2 * m2 * m, k = g.z * (e * e);
+            const float path = sqrtf(fmaxf(1.0f - ha * ha, 0.0f));
+            tt[half].x += expf(ntau.x * path) * k;
+            tt[half].y += expf(ntau.y * path) * k;
+            tt[half].z += expf(ntau.z * path) * k;
+        }
+    }
+    const float f_trt = fresnel(cos_theta_d * 0.5f);
+    const float k_trt = (1.0f - f_trt) * (1.0f - f_trt) * f_trt;
+    const f3 trt = mul3s(vexp(mul3s(ntau, 1.6f)), k_trt);  // path 3.2 / cos theta_d
+    const float s_low = (1.0f - s) - cos_theta_d;  // what the rounding of s left
+    auto sum_r = [&](const float (&c)[6]) {
+        float v = c[5], slope = 0.0f;
+#pragma unroll
+        for (int k = 4; k >= 0; --k) {
+            slope = slope * s + v;
+            v = v * s + c[k];
+        }
+        return v + slope * s_low;
+    };
+    const Lobes back = {spl(sum_r(c_scatter.r[0])), tt[0], mul3s(trt, c_scatter.trt[0])};
+    const Lobes fwd = {spl(sum_r(c_scatter.r[1])), tt[1], mul3s(trt, c_scatter.trt[1])};
+    return dual_statistics(fwd, back, shape);
+}
+
+// The same angle by angle, R and TRT included, which shade models 1 and 2 keep:
+// their network amplifies the last bit of its inputs, so that a change of the
+// code around them (another contraction of the same expressions) moves single
+// pixels by 1e-3, and their results stay what they were.  Only pixels in the
+// shadowed light's hair evaluate it.
 struct ScatterAngle {
     float cos_phi, cos_half_phi, k_tt, k_trt;
 };
-__constant__ ScatterAngle c_scatter[2 * kScatterSteps];  // [0, steps): back, [steps, 2 steps): front
+__constant__ ScatterAngle c_scatter_angle[2 * kScatterSteps];  // [0, steps): back, [steps, 2 steps): front
 
 // azimuthal() at one of those angles, with the terms that depend only on the
 // pixel (cos theta_d, sigma_a) computed once by the caller.
@@ -152,14 +245,13 @@ __device__ __forceinline__ Lobes azimuthal_at(const AzimuthPixel& q, const Scatt
     return r;
 }
 
-// dual_scatter (shade.wesl:153-190)
-__device__ Dual dual_scatter(float cos_theta_d, f3 sigma_a, const Shape& shape) {
+__device__ Dual dual_scatter_by_angle(float cos_theta_d, f3 sigma_a, const Shape& shape) {
     Lobes fwd = {spl(0.0f), spl(0.0f), spl(0.0f)}, back = fwd;
     const AzimuthPixel q = azimuth_pixel(cos_theta_d, sigma_a);
 #pragma unroll 2
     for (int i = 0; i < kScatterSteps; ++i) {
-        Lobes b = azimuthal_at(q, c_scatter[i]);
-        Lobes f = azimuthal_at(q, c_scatter[kScatterSteps + i]);
+        Lobes b = azimuthal_at(q, c_scatter_angle[i]);
+        Lobes f = azimuthal_at(q, c_scatter_angle[kScatterSteps + i]);
         back.r = add3(back.r, b.r);
         back.tt = add3(back.tt, b.tt);
         back.trt = add3(back.trt, b.trt);
@@ -170,37 +262,7 @@ __device__ Dual dual_scatter(float cos_theta_d, f3 sigma_a, const Shape& shape) 
     const float w = kPi / (float)kScatterSteps;
     fwd = {mul3s(fwd.r, w), mul3s(fwd.tt, w), mul3s(fwd.trt, w)};
     back = {mul3s(back.r, w), mul3s(back.tt, w), mul3s(back.trt, w)};
-    Dual d;
-    d.fwd = fwd;
-    f3 a_f = vmins(add3(add3(fwd.r, fwd.tt), fwd.trt), 0.95f);
-    f3 a_b = add3(add3(back.r, back.tt), back.trt);
-    f3 beta2 = vmul(shape.beta, shape.beta);
-    f3 beta_f2 = lobe_mean(fwd, a_f, beta2);
-    f3 alpha_b = lobe_mean(back, a_b, shape.alpha);
-    f3 beta_b2 = lobe_mean(back, a_b, beta2);
-    f3 af2 = vmul(a_f, a_f);
-    f3 rest = {1.0f - af2.x, 1.0f - af2.y, 1.0f - af2.z};
-    f3 ab2 = vmul(a_b, a_b);
-    f3 ab3 = vmul(ab2, a_b);
-    f3 rr = vmul(rest, rest);
-    f3 rest3 = vmul(rr, rest);
-    f3 a_back = add3(vdiv(vmul(a_b, af2), rest), vdiv(vmul(ab3, af2), rest3));
-    f3 t1 = {1.0f - 2.0f * ab2.x / rr.x, 1.0f - 2.0f * ab2.y / rr.y, 1.0f - 2.0f * ab2.z / rr.z};
-    f3 num2 = add3(mul3s(rr, 2.0f), vmul(mul3s(af2, 4.0f), ab2));
-    f3 delta_b = add3(vmul(alpha_b, t1), vdiv(vmul(alpha_b, num2), rest3));
-    f3 beta_f = vsqrt(beta_f2), beta_b = vsqrt(beta_b2);
-    f3 lead = add3(spl(1.0f), mul3s(af2, kDensityBack));
-    f3 s1 = vsqrt(add3(mul3s(beta_f2, 2.0f), beta_b2));
-    f3 s2 = vsqrt(add3(mul3s(beta_f2, 2.0f), mul3s(beta_b2, 3.0f)));
-    f3 numer = vmul(lead, add3(vmul(a_b, s1), vmul(ab3, s2)));
-    f3 den = vmaxs(add3(a_b, vmul(ab3, add3(mul3s(beta_f, 2.0f), mul3s(beta_b, 3.0f)))), 1e-5f);
-    f3 sigma_b = vdiv(numer, den);
-    d.a_f = a_f;
-    d.beta_f2 = beta_f2;
-    d.a_back = a_back;
-    d.delta_b = delta_b;
-    d.sigma_b2 = vmul(sigma_b, sigma_b);
-    return d;
+    return dual_statistics(fwd, back, shape);
 }
 
 // Angles of one light at a fibre (shade.wesl:196-206).
@@ -242,20 +304,60 @@ __device__ f3 spread_term(const Shape& shape, const Dual& ds, float theta_h, flo
     return vmul(mul3s(transmit, (1.0f - direct) * kDensityFront), inner);
 }
 
-// hair_bsdf (shade.wesl:193-244); t_n and v_n are the normalized tangent and view.
-__device__ __forceinline__ f3 hair_bsdf(f3 t_n, f3 v_n, f3 light, f3 sigma_a, const Shape& shape, const Dual& ds,
-                                        float depth) {
-    const Geometry gm = light_geometry(t_n, v_n, light);
-    Lobes n = azimuthal(gm.cos_theta_d, gm.cos_phi, sigma_a);
-    f3 x = spl(gm.theta_h);
-    f3 m = gaussian3(shape.beta, sub3(x, shape.alpha));
-    f3 single = add3(add3(mul3s(n.r, m.x), mul3s(n.tt, m.y)), mul3s(n.trt, m.z));
-    f3 g = gaussian3(vsqrt(ds.sigma_b2), sub3(x, ds.delta_b));
-    f3 back = mul3s(vmul(ds.a_back, g), 2.0f / kPi);
-    float direct = expf(-depth);
-    f3 color = mul3s(add3(single, mul3s(back, kDensityBack)), direct);
-    if (depth > 1e-3f) color = add3(color, spread_term(shape, ds, gm.theta_h, depth, direct));
-    return color;
+// The terms of hair_bsdf that every light of a pixel shares.  The three
+// longitudinal Gaussians have widths b, b/2 and 2 b (lobe_shape, b at least
+// 0.02), so exponent scale and norm of the first serve all, times powers of
+// two; the back lobe's a_back 2 / pi kDensityBack is in its norm.
+struct Fibre {
+    f3 t, v, t_o, sigma_a;
+    float theta_o, to2, tilt;
+    float g_k, g_k_low, g_n;  // -1 / (2 b^2) and what its rounding left, 1 / (b sqrt(2 pi))
+    f3 back_k, back_n, delta_b;
+};
+
+__device__ __forceinline__ Fibre make_fibre(f3 t_n, f3 v_n, f3 sigma_a, const Shape& shape, const Dual& ds) {
+    const float norm = 0.398942280f;  // 1 / sqrt(2 pi)
+    Fibre f;
+    f.t = t_n;
+    f.v = v_n;
+    f.sigma_a = sigma_a;
+    const float sin_o = clampf(dot3(t_n, v_n), -1.0f, 1.0f);
+    f.theta_o = asinf(sin_o);
+    f.t_o = sub3(v_n, mul3s(t_n, sin_o));
+    f.to2 = dot3(f.t_o, f.t_o);
+    f.tilt = shape.alpha.x;
+    const float b = shape.beta.x;
+    const float b2 = b * b, b2_low = __fmaf_rn(b, b, -b2);
+    f.g_k = -0.5f / b2;
+    f.g_k_low = __fmaf_rn(-f.g_k, b2_low, __fmaf_rn(-f.g_k, b2, -0.5f)) * (-2.0f * f.g_k);
+    f.g_n = norm / b;
+    const f3 sb2 = vmaxs(ds.sigma_b2, 1e-6f);
+    f.back_k = vdiv(spl(-0.5f), sb2);
+    f.back_n = vdiv(mul3s(ds.a_back, 2.0f / kPi * kDensityBack * norm), vsqrt(sb2));
+    f.delta_b = ds.delta_b;
+    return f;
+}
+
+// hair_bsdf (shade.wesl:193-244) toward the normalized direction l, without
+// the shadowed light's attenuation and forward spread.
+__device__ __forceinline__ f3 hair_bsdf(const Fibre& f, f3 l) {
+    const float sin_i = clampf(dot3(f.t, l), -1.0f, 1.0f);
+    const float theta_i = asinf(sin_i), theta_h = theta_i + f.theta_o;
+    const float cos_theta_d = fmaxf(cosf(0.5f * fabsf(theta_i - f.theta_o)), 1e-3f);
+    const f3 t_i = sub3(l, mul3s(f.t, sin_i));
+    const float proj = sqrtf(fmaxf(dot3(t_i, t_i) * f.to2, 1e-8f));
+    const float cos_phi = clampf(dot3(t_i, f.t_o) / proj, -1.0f, 1.0f);
+    const Lobes n = azimuthal(cos_theta_d, cos_phi, f.sigma_a);
+    const float x0 = theta_h - f.tilt, x1 = theta_h + 0.5f * f.tilt, x2 = theta_h + 1.5f * f.tilt;
+    auto gauss = [&](float x) {
+        const float q = x * x;
+        return expf(q * f.g_k + q * f.g_k_low) * f.g_n;
+    };
+    // a width of b / 2 is the argument doubled, one of 2 b the argument halved
+    const float m0 = gauss(x0), m1 = 2.0f * gauss(2.0f * x1), m2 = 0.5f * gauss(0.5f * x2);
+    const f3 xb = sub3(spl(theta_h), f.delta_b);
+    const f3 back = vmul(vexp(vmul(vmul(xb, xb), f.back_k)), f.back_n);
+    return add3(add3(add3(mul3s(n.r, m0), mul3s(n.tt, m1)), mul3s(n.trt, m2)), back);
 }
 
 // ---------------------------------------------------------------- light probe
@@ -451,138 +553,6 @@ struct ShadeArgs {
     float exposure;
 };
 
-// fs (shade.wesl:523-593) for pixel (x, y) of view v (fields p, center,
-// beta, dom, shaded, shaded_depth).  Lights arrive sorted by kind (point,
-// spot, directional, rect), the order the reference's loops visit them.
-template <class V>
-__device__ __forceinline__ void shade_pixel(const V& a, const hg_light* __restrict__ lights, uint32_t n_lights,
-                                            uint32_t ortho, float exposure, const EnvArgs& env, uint32_t x,
-                                            uint32_t y) {
-    const hg_hair_params& p = a.p;
-    const uint32_t width = f2u(p.screen[0]), height = f2u(p.screen[1]);
-    if (x >= width || y >= height) return;
-    const uint32_t pix = y * width + x;
-    const unsigned long long word = __ldg(&a.center[pix]);
-    if (is_empty(word)) {
-        a.shaded[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        a.shaded_depth[pix] = 0.0f;
-        return;
-    }
-    const uint32_t low = (uint32_t)word, high = (uint32_t)(word >> 32);
-    const uint32_t depth_q = high >> 8u;
-    const float view_dist = dequantize_depth(depth_q, p.screen[2], p.screen[3]);
-    const f3 world = reconstruct_world(p, (int32_t)x, (int32_t)y, view_dist);
-    const f3 tangent = oct_decode(high & 0xffu, low >> 24u);
-    const float uvw_z = (float)((low >> 6u) & 0x3fu) / 63.0f;
-    const float beta = (float)(__ldg(&a.beta[pix]) & 0xffu) / 255.0f;
-    const float roughness = fmaxf(p.appearance[0] * (0.65f + 0.7f * uvw_z), 0.04f);
-    const float tilt = p.appearance[1];
-    const float ascale = 0.65f + 0.35f * uvw_z;
-    const f3 albedo = {p.albedo[0] * ascale, p.albedo[1] * ascale, p.albedo[2] * ascale};
-    f3 view;
-    if (ortho) {
-        view = safe_normalize(mk3(p.clip_from_world[2], p.clip_from_world[6], p.clip_from_world[10]));
-    } else {
-        view = safe_normalize(sub3(ld3(p.camera_pos), world));
-    }
-
-    // direct_light (shade.wesl:429-521)
-    const Shape shape = lobe_shape(roughness, tilt);
-    const float tv = dot3(tangent, view);
-    const float cos_theta_o = sqrtf(fmaxf(1.0f - tv * tv, 1e-6f));
-    const f3 sigma_a = absorption_from_color(albedo, roughness);
-    const Dual ds = dual_scatter(cos_theta_o, sigma_a, shape);
-    f3 color = spl(0.0f);
-    bool dom_left = true;
-    const f3 t_n = safe_normalize(tangent), v_n = safe_normalize(view);
-    for (uint32_t i = 0; i < n_lights; ++i) {
-        const hg_light& L = lights[i];
-        const uint32_t kind = L.kind;
-        // each kind gives the incident direction, a weight and the DOM depth;
-        // one BSDF evaluation serves them all
-        f3 incident = spl(0.0f);
-        float weight = 0.0f, depth = 0.0f;
-        if (kind == HG_LIGHT_POINT || kind == HG_LIGHT_SPOT) {
-            f3 to_l = sub3(ld3(L.position), world);
-            float dist2 = dot3(to_l, to_l);
-            incident = safe_normalize(to_l);
-            float inv_r2 = 1.0f / fmaxf(L.range * L.range, 1e-8f);
-            weight = range_window(dist2, inv_r2) / fmaxf(dist2, 1e-4f);
-            if (kind == HG_LIGHT_SPOT) {
-                float cd = dot3(mul3s(ld3(L.direction), -1.0f), incident);
-                float sm = clampf(cd * L.spot[0] + L.spot[1], 0.0f, 1.0f);
-                weight *= sm * sm;
-            }
-        } else if (kind == HG_LIGHT_DIRECTIONAL) {
-            if (dom_left && (L.flags & HG_LIGHT_CASTS_SHADOWS)) {
-                depth = -logf(fmaxf(dom_visibility(p, a.dom, world, beta), 1e-6f));
-                dom_left = false;
-            }
-            incident = ld3(L.direction);
-            weight = 1.0f;
-        } else if (kind == HG_LIGHT_RECT) {
-            f3 to_c = sub3(ld3(L.position), world);
-            float dist2 = fmaxf(dot3(to_c, to_c), 1e-4f);
-            incident = mul3s(to_c, rsqrtf(dist2));
-            f3 normal = safe_normalize(cross3(ld3(L.up), ld3(L.right)));
-            float facing = fmaxf(dot3(normal, incident), 0.0f);
-            float solid = L.spot[0] * L.spot[1] * facing / dist2;
-            float range2 = fmaxf(L.range * L.range, 1e-4f);
-            weight = solid * range_window(dist2, 1.0f / range2);
-        }
-        if (weight > 0.0f) {
-            f3 lobe = hair_bsdf(t_n, v_n, incident, sigma_a, shape, ds, depth);
-            color = add3(color, mul3s(vmul(lobe, ld3(L.color)), weight));
-        }
-    }
-    if (env.spec) {
-        const f3 fiber_n = safe_normalize(sub3(view, mul3s(tangent, dot3(view, tangent))));
-        const f3 pr = probe_radiance(env, tangent, fiber_n, view, albedo, roughness, tilt);
-        color = add3(color, mul3s(pr, pixel_ao(p, low)));
-    }
-    color = mul3s(color, exposure);
-    a.shaded[pix] = make_float4(color.x, color.y, color.z, 1.0f);
-    a.shaded_depth[pix] = view_dist;
-}
-
-// Four blocks per SM (64 registers, some spilled) measured faster than three
-// (80 registers): the probe's and the DOM taps' loads want the extra warps.
-__global__ void __launch_bounds__(256, 4) shade_kernel(const ShadeArgs a, const EnvArgs env) {
-    shade_pixel(a, a.lights, a.n_lights, a.ortho, a.exposure, env, blockIdx.x * blockDim.x + threadIdx.x,
-                blockIdx.y * blockDim.y + threadIdx.y);
-}
-
-// Batched: one tile (blockDim.x x blockDim.y pixels) of one camera view per block.
-__global__ void __launch_bounds__(256, 4) batch_shade_kernel(const BatchView* __restrict__ views,
-                                                             const uint32_t* __restrict__ tile_prefix, uint32_t n_cam,
-                                                             const hg_light* __restrict__ lights, uint32_t n_lights,
-                                                             uint32_t ortho, float exposure, const EnvArgs env) {
-    uint32_t lo = 0, hi = n_cam;
-    while (hi - lo > 1u) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (tile_prefix[mid] <= blockIdx.x) lo = mid;
-        else hi = mid;
-    }
-    const BatchView& v = views[lo];
-    const uint32_t t = blockIdx.x - tile_prefix[lo];
-    const uint32_t tiles_x = (v.width + blockDim.x - 1) / blockDim.x;
-    shade_pixel(v, lights, n_lights, ortho, exposure, env, (t % tiles_x) * blockDim.x + threadIdx.x,
-                (t / tiles_x) * blockDim.y + threadIdx.y);
-}
-
-// The learned-surrogate variant of fs: the network gives R, TT, TRT and the
-// local back-scattering per pixel and light (hg_mlp.cuh); the DOM-shadowed
-// light's forward spread keeps the dual-scattering statistics of
-// dual_scatter.  A warp shades 32 pixels of one row and evaluates the
-// network for all of them per light, so every lane takes part in each
-// evaluation; pixels without hair run it on placeholder inputs.  Azimuthal
-// roughness beta_n, which the Karis fit does not have, is the fibre
-// roughness clamped to the trained range [0.2, 0.8].  Per-pixel work (view
-// and tangent, the shadowed light's DOM depth and spread) happens before the
-// light loop, so the loop holds little besides the network's fragments.
-constexpr int kSurrogateWarps = 8;
-constexpr size_t kSurrogateSmem = sizeof(mlp::FwdWeights) + kSurrogateWarps * sizeof(mlp::WarpIo);
-
 // Incident direction and weight (scalar factor on the light colour) of a
 // point, spot or rect light; directional lights have weight 1.
 __device__ __forceinline__ float light_weight(const hg_light& L, f3 world, f3& incident) {
@@ -617,6 +587,170 @@ __device__ __forceinline__ float light_weight(const hg_light& L, f3 world, f3& i
     incident = spl(0.0f);
     return 0.0f;
 }
+
+// fs (shade.wesl:523-593) for the hair pixel (x, y), centre word `word`, of
+// view v (fields p, center, beta, dom, shaded, shaded_depth).  Lights arrive
+// sorted by kind (point, spot, directional, rect), the order the reference's
+// loops visit them.  The light that receives the deep-opacity depth (the first
+// shadow-casting directional one) gives its forward spread before the light
+// loop, so that the loop holds the pixel's Fibre alone.
+//
+// Bound by instruction issue (0.77 a cycle): the pixel's dual_scatter and, per
+// light, two arcsines, a cosine and 13 exponentials.  With every light's
+// Gaussians divided out anew and all of azimuthal() summed angle by angle the
+// 1920 x 1080 benchmark frame took 123 us (111 M warp instructions; now 107 and
+// 95 M), 24 grooms of the batch benchmark 548 (513 M; now 426 and 385 M, a
+// third of it the pixel lists of shade_block).
+template <class V>
+__device__ __forceinline__ void shade_hair(const V& a, const hg_light* __restrict__ lights, uint32_t n_lights,
+                                           uint32_t ortho, float exposure, const EnvArgs& env, uint32_t x, uint32_t y,
+                                           unsigned long long word) {
+    const hg_hair_params& p = a.p;
+    const uint32_t pix = y * f2u(p.screen[0]) + x;
+    const uint32_t low = (uint32_t)word, high = (uint32_t)(word >> 32);
+    const uint32_t depth_q = high >> 8u;
+    const float view_dist = dequantize_depth(depth_q, p.screen[2], p.screen[3]);
+    const f3 world = reconstruct_world(p, (int32_t)x, (int32_t)y, view_dist);
+    const f3 tangent = oct_decode(high & 0xffu, low >> 24u);
+    const float uvw_z = (float)((low >> 6u) & 0x3fu) / 63.0f;
+    const float beta = (float)(__ldg(&a.beta[pix]) & 0xffu) / 255.0f;
+    const float roughness = fmaxf(p.appearance[0] * (0.65f + 0.7f * uvw_z), 0.04f);
+    const float tilt = p.appearance[1];
+    const float ascale = 0.65f + 0.35f * uvw_z;
+    const f3 albedo = {p.albedo[0] * ascale, p.albedo[1] * ascale, p.albedo[2] * ascale};
+    f3 view;
+    if (ortho) {
+        view = safe_normalize(mk3(p.clip_from_world[2], p.clip_from_world[6], p.clip_from_world[10]));
+    } else {
+        view = safe_normalize(sub3(ld3(p.camera_pos), world));
+    }
+
+    // direct_light (shade.wesl:429-521)
+    const f3 t_n = safe_normalize(tangent), v_n = safe_normalize(view);
+    uint32_t dom_light = 0;
+    while (dom_light < n_lights && !(lights[dom_light].kind == HG_LIGHT_DIRECTIONAL &&
+                                     (lights[dom_light].flags & HG_LIGHT_CASTS_SHADOWS)))
+        ++dom_light;
+    f3 color = spl(0.0f);
+    float dom_direct = 1.0f;
+    Fibre fibre;
+    {
+        const Shape shape = lobe_shape(roughness, tilt);
+        const float tv = dot3(tangent, view);
+        const f3 sigma_a = absorption_from_color(albedo, roughness);
+        const Dual ds = dual_scatter(sqrtf(fmaxf(1.0f - tv * tv, 1e-6f)), sigma_a, shape);
+        fibre = make_fibre(t_n, v_n, sigma_a, shape, ds);
+        if (dom_light < n_lights) {
+            const float depth = -logf(fmaxf(dom_visibility(p, a.dom, world, beta), 1e-6f));
+            dom_direct = expf(-depth);
+            if (depth > 1e-3f) {
+                const hg_light& L = lights[dom_light];
+                const float theta_h = asinf(clampf(dot3(t_n, safe_normalize(ld3(L.direction))), -1.0f, 1.0f)) +
+                                      fibre.theta_o;
+                color = vmul(spread_term(shape, ds, theta_h, depth, dom_direct), ld3(L.color));
+            }
+        }
+    }
+    for (uint32_t i = 0; i < n_lights; ++i) {
+        const hg_light& L = lights[i];
+        f3 incident;
+        float weight = light_weight(L, world, incident);
+        if (i == dom_light) weight = dom_direct;
+        if (weight > 0.0f) {
+            // point and spot directions are normalized already
+            const f3 l = L.kind == HG_LIGHT_POINT || L.kind == HG_LIGHT_SPOT ? incident : safe_normalize(incident);
+            color = add3(color, mul3s(vmul(hair_bsdf(fibre, l), ld3(L.color)), weight));
+        }
+    }
+    if (env.spec) {
+        const f3 fiber_n = safe_normalize(sub3(view, mul3s(tangent, dot3(view, tangent))));
+        const f3 pr = probe_radiance(env, tangent, fiber_n, view, albedo, roughness, tilt);
+        color = add3(color, mul3s(pr, pixel_ao(p, low)));
+    }
+    color = mul3s(color, exposure);
+    a.shaded[pix] = make_float4(color.x, color.y, color.z, 1.0f);
+    a.shaded_depth[pix] = view_dist;
+}
+
+// One block of at most kShadeThreads pixels of a view: empty pixels are written
+// at once, hair pixels are listed and shaded by the first threads, so that
+// only the list's last warp has idle lanes (sparse hair at a silhouette leaves
+// a third of a warp's own pixels empty).
+constexpr uint32_t kShadeThreads = 256;
+template <class V>
+__device__ __forceinline__ void shade_block(const V& a, const hg_light* __restrict__ lights, uint32_t n_lights,
+                                            uint32_t ortho, float exposure, const EnvArgs& env, uint32_t x0,
+                                            uint32_t y0) {
+    __shared__ unsigned long long s_word[kShadeThreads];
+    __shared__ uint16_t s_pixel[kShadeThreads];
+    __shared__ uint32_t s_warp[kShadeThreads / 32];
+    const uint32_t tid = threadIdx.y * blockDim.x + threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t width = f2u(a.p.screen[0]), height = f2u(a.p.screen[1]);
+    const uint32_t x = x0 + threadIdx.x, y = y0 + threadIdx.y, pix = y * width + x;
+    const bool inside = x < width && y < height;
+    const unsigned long long word = inside ? __ldg(&a.center[pix]) : kEmptyU64;
+    const bool hair = !is_empty(word);
+    if (inside && !hair) {
+        a.shaded[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        a.shaded_depth[pix] = 0.0f;
+    }
+    const uint32_t mask = __ballot_sync(0xffffffffu, hair);
+    if (lane == 0) s_warp[warp] = __popc(mask);
+    __syncthreads();
+    uint32_t at = __popc(mask & ((1u << lane) - 1u)), n = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kShadeThreads / 32; ++w) {
+        const uint32_t c = s_warp[w];
+        if (w < warp) at += c;
+        n += c;
+    }
+    if (hair) {
+        s_word[at] = word;
+        s_pixel[at] = (uint16_t)tid;
+    }
+    __syncthreads();
+    if (tid >= n) return;
+    const uint32_t q = s_pixel[tid];
+    shade_hair(a, lights, n_lights, ortho, exposure, env, x0 + q % blockDim.x, y0 + q / blockDim.x, s_word[tid]);
+}
+
+// Four blocks per SM (64 registers, some spilled): 107 us on the 1920 x 1080
+// benchmark frame; three (80 registers) 112, five (48) 108.  The batch's small
+// views wait more for their blocks' first loads: 24 grooms 448 us at four, 510
+// at three, 426 at five.
+__global__ void __launch_bounds__(kShadeThreads, 4) shade_kernel(const ShadeArgs a, const EnvArgs env) {
+    shade_block(a, a.lights, a.n_lights, a.ortho, a.exposure, env, blockIdx.x * blockDim.x, blockIdx.y * blockDim.y);
+}
+
+// Batched: one tile (blockDim.x x blockDim.y pixels) of one camera view per block.
+__global__ void __launch_bounds__(kShadeThreads, 5) batch_shade_kernel(const BatchView* __restrict__ views,
+                                                             const uint32_t* __restrict__ tile_prefix, uint32_t n_cam,
+                                                             const hg_light* __restrict__ lights, uint32_t n_lights,
+                                                             uint32_t ortho, float exposure, const EnvArgs env) {
+    uint32_t lo = 0, hi = n_cam;
+    while (hi - lo > 1u) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (tile_prefix[mid] <= blockIdx.x) lo = mid;
+        else hi = mid;
+    }
+    const BatchView& v = views[lo];
+    const uint32_t t = blockIdx.x - tile_prefix[lo];
+    const uint32_t tiles_x = (v.width + blockDim.x - 1) / blockDim.x;
+    shade_block(v, lights, n_lights, ortho, exposure, env, (t % tiles_x) * blockDim.x, (t / tiles_x) * blockDim.y);
+}
+
+// The learned-surrogate variant of fs: the network gives R, TT, TRT and the
+// local back-scattering per pixel and light (hg_mlp.cuh); the DOM-shadowed
+// light's forward spread keeps the dual-scattering statistics of
+// dual_scatter.  A warp shades 32 pixels of one row and evaluates the
+// network for all of them per light, so every lane takes part in each
+// evaluation; pixels without hair run it on placeholder inputs.  Azimuthal
+// roughness beta_n, which the Karis fit does not have, is the fibre
+// roughness clamped to the trained range [0.2, 0.8].  Per-pixel work (view
+// and tangent, the shadowed light's DOM depth and spread) happens before the
+// light loop, so the loop holds little besides the network's fragments.
+constexpr int kSurrogateWarps = 8;
+constexpr size_t kSurrogateSmem = sizeof(mlp::FwdWeights) + kSurrogateWarps * sizeof(mlp::WarpIo);
 
 __global__ void __launch_bounds__(kSurrogateWarps * 32, 2)
     shade_surrogate_kernel(const ShadeArgs a, const __half* __restrict__ w16, const float* __restrict__ mparams,
@@ -683,7 +817,7 @@ __global__ void __launch_bounds__(kSurrogateWarps * 32, 2)
             dom_direct = expf(-depth);
             if (depth > 1e-3f) {
                 const float tv = dot3(tangent, view);
-                const Dual ds = dual_scatter(sqrtf(fmaxf(1.0f - tv * tv, 1e-6f)), sigma_a, shape);
+                const Dual ds = dual_scatter_by_angle(sqrtf(fmaxf(1.0f - tv * tv, 1e-6f)), sigma_a, shape);
                 const Geometry gm = light_geometry(t_n, v_n, ld3(L.direction));
                 color = vmul(spread_term(shape, ds, gm.theta_h, depth, dom_direct), ld3(L.color));
             }
@@ -951,7 +1085,7 @@ __global__ void __launch_bounds__(mlp::tc::kThreads, 1)
             dom_direct = expf(-depth);
             if (depth > 1e-3f) {
                 const float tv = dot3(tangent, view);
-                const Dual ds = dual_scatter(sqrtf(fmaxf(1.0f - tv * tv, 1e-6f)), sigma_a, shape);
+                const Dual ds = dual_scatter_by_angle(sqrtf(fmaxf(1.0f - tv * tv, 1e-6f)), sigma_a, shape);
                 const Geometry gm = light_geometry(t_n, v_n, ld3(L.direction));
                 color = vmul(spread_term(shape, ds, gm.theta_h, depth, dom_direct), ld3(L.color));
             }
@@ -1405,19 +1539,34 @@ cudaError_t ensure_shade_setup(int device) {
     std::lock_guard<std::mutex> lock(mutex);
     if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
     if (ready[device]) return cudaSuccess;
-    ScatterAngle t[2 * kScatterSteps];
+    ScatterTable t = {};
+    ScatterAngle angles[2 * kScatterSteps];
     const double pi = 3.14159265358979323846;
-    for (int half = 0; half < 2; ++half)
+    const double r0 = (1.0 - kIor) / (1.0 + kIor), f0 = r0 * r0, weight = pi / kScatterSteps;
+    for (int half = 0; half < 2; ++half) {
+        double r[6] = {}, trt = 0.0;
         for (int i = 0; i < kScatterSteps; ++i) {
             const double u = (i + 0.5) / kScatterSteps;
-            const double c = std::cos((half + u) * 0.5 * pi);
-            ScatterAngle& g = t[half * kScatterSteps + i];
-            g.cos_phi = (float)c;
-            g.cos_half_phi = (float)std::sqrt(std::min(std::max(0.5 + 0.5 * c, 0.0), 1.0));
-            g.k_tt = (float)std::exp(-3.65 * c - 3.98);
-            g.k_trt = (float)std::exp(17.0 * c - 16.78);
+            const double cos_phi = std::cos((half + u) * 0.5 * pi);
+            const double c = std::sqrt(std::min(std::max(0.5 + 0.5 * cos_phi, 0.0), 1.0));
+            double binomial = 1.0;
+            r[0] += weight * 0.25 * c * f0;
+            for (int k = 0; k < 6; ++k) {
+                r[k] += weight * 0.25 * c * (1.0 - f0) * binomial * std::pow(1.0 - c, 5 - k) * std::pow(c, k);
+                binomial = binomial * (5 - k) / (k + 1);
+            }
+            t.tt[half][i] = make_float4((float)c, (float)(c * (0.6 - 0.8 * cos_phi)),
+                                        (float)(weight * std::exp(-3.65 * cos_phi - 3.98) * (1.0 - f0) * (1.0 - f0)),
+                                        0.0f);
+            trt += weight * std::exp(17.0 * cos_phi - 16.78);
+            angles[half * kScatterSteps + i] = {(float)cos_phi, (float)c, (float)std::exp(-3.65 * cos_phi - 3.98),
+                                                (float)std::exp(17.0 * cos_phi - 16.78)};
         }
-    cudaError_t e = cudaMemcpyToSymbol(c_scatter, t, sizeof(t));
+        for (int k = 0; k < 6; ++k) t.r[half][k] = (float)r[k];
+        t.trt[half] = (float)trt;
+    }
+    cudaError_t e = cudaMemcpyToSymbol(c_scatter, &t, sizeof(t));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_scatter_angle, angles, sizeof(angles));
     if (e == cudaSuccess) ready[device] = true;
     return e;
 }

@@ -532,6 +532,30 @@ def test_light_kinds(renderer):
     g.close()
 
 
+@pytest.mark.parametrize("size, keep", [((1, 1), 1.0), ((33, 9), 1.0), ((97, 61), 0.02), ((64, 24), 0.5), ((31, 40), 0.0)])
+def test_shade_lists_hair_pixels_of_partial_blocks(renderer, size, keep):
+    """The shade pass lists a block's hair pixels: blocks cut by the image's
+    edges, with all, some, one in fifty or none of their pixels covered, against
+    the oracle's pixel by pixel shading."""
+    sc = configs.config1(scale=0.02)
+    sc.view = configs._camera(*size, 160.0)
+    cam, dom = sc.params()
+    lights = sc.light_array()
+    renderer.ensure_targets(*size, *sc.dom_size)
+    g = renderer.upload(sc.mesh)
+    renderer.render_groom(g, cam, dom, lights)
+    assert renderer.synchronize() == 0
+    center, beta, dmap = renderer.read(abi.BUF_CENTER), renderer.read(abi.BUF_BETA), renderer.read(abi.BUF_DOM)
+    center[np.random.default_rng(5).random(center.shape) >= keep] = EMPTY
+    renderer.write(abi.BUF_CENTER, center)
+    renderer.shade(cam, lights)
+    assert renderer.synchronize() == 0
+    o_shaded, o_sdepth = oracle.shade(cam, center, beta, dmap, lights)
+    np.testing.assert_array_equal(renderer.read(abi.BUF_SHADED_DEPTH), o_sdepth)
+    np.testing.assert_allclose(renderer.read(abi.BUF_SHADED), o_shaded, rtol=SHADE_RTOL, atol=SHADE_ATOL)
+    g.close()
+
+
 def test_invalid_arguments_are_rejected(renderer):
     import ctypes as C
 
