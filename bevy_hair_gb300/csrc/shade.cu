@@ -304,6 +304,23 @@ __device__ f3 spread_term(const Shape& shape, const Dual& ds, float theta_h, flo
     return vmul(mul3s(transmit, (1.0f - direct) * kDensityFront), inner);
 }
 
+// A light's angles with the contraction written out.  Where a light lies along
+// the fibre the lobes turn a last bit of these into 1e-3 of the pixel, and the
+// compiler's choice of the product that a sum of products rounds changes with
+// the code around it; these are the ones it took when every light evaluated
+// light_geometry, so results do not move with the loop's shape.
+__device__ __forceinline__ float dot_fixed(f3 a, f3 b) {
+    return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+}
+__device__ __forceinline__ f3 normalize_fixed(f3 v) {
+    const float l2 = dot_fixed(v, v);
+    if (l2 < 1e-10f) return {0.0f, 1.0f, 0.0f};
+    return mul3s(v, inv_sqrt(l2));
+}
+__device__ __forceinline__ f3 reject_fixed(f3 v, f3 t, float s) {
+    return {__fmaf_rn(-t.x, s, v.x), __fmaf_rn(-t.y, s, v.y), __fmaf_rn(-t.z, s, v.z)};
+}
+
 // The terms of hair_bsdf that every light of a pixel shares.  The three
 // longitudinal Gaussians have widths b, b/2 and 2 b (lobe_shape, b at least
 // 0.02), so exponent scale and norm of the first serve all, times powers of
@@ -321,10 +338,10 @@ __device__ __forceinline__ Fibre make_fibre(f3 t_n, f3 v_n, f3 sigma_a, const Sh
     f.t = t_n;
     f.v = v_n;
     f.sigma_a = sigma_a;
-    const float sin_o = clampf(dot3(t_n, v_n), -1.0f, 1.0f);
+    const float sin_o = clampf(dot_fixed(t_n, v_n), -1.0f, 1.0f);
     f.theta_o = asinf(sin_o);
-    f.t_o = sub3(v_n, mul3s(t_n, sin_o));
-    f.to2 = dot3(f.t_o, f.t_o);
+    f.t_o = reject_fixed(v_n, t_n, sin_o);
+    f.to2 = dot_fixed(f.t_o, f.t_o);
     f.tilt = shape.alpha.x;
     const float b = shape.beta.x;
     const float b2 = b * b, b2_low = __fmaf_rn(b, b, -b2);
@@ -341,12 +358,12 @@ __device__ __forceinline__ Fibre make_fibre(f3 t_n, f3 v_n, f3 sigma_a, const Sh
 // hair_bsdf (shade.wesl:193-244) toward the normalized direction l, without
 // the shadowed light's attenuation and forward spread.
 __device__ __forceinline__ f3 hair_bsdf(const Fibre& f, f3 l) {
-    const float sin_i = clampf(dot3(f.t, l), -1.0f, 1.0f);
+    const float sin_i = clampf(dot_fixed(f.t, l), -1.0f, 1.0f);
     const float theta_i = asinf(sin_i), theta_h = theta_i + f.theta_o;
     const float cos_theta_d = fmaxf(cosf(0.5f * fabsf(theta_i - f.theta_o)), 1e-3f);
-    const f3 t_i = sub3(l, mul3s(f.t, sin_i));
-    const float proj = sqrtf(fmaxf(dot3(t_i, t_i) * f.to2, 1e-8f));
-    const float cos_phi = clampf(dot3(t_i, f.t_o) / proj, -1.0f, 1.0f);
+    const f3 t_i = reject_fixed(l, f.t, sin_i);
+    const float proj = sqrtf(fmaxf(dot_fixed(t_i, t_i) * f.to2, 1e-8f));
+    const float cos_phi = clampf(dot_fixed(t_i, f.t_o) / proj, -1.0f, 1.0f);
     const Lobes n = azimuthal(cos_theta_d, cos_phi, f.sigma_a);
     const float x0 = theta_h - f.tilt, x1 = theta_h + 0.5f * f.tilt, x2 = theta_h + 1.5f * f.tilt;
     auto gauss = [&](float x) {
@@ -598,8 +615,8 @@ __device__ __forceinline__ float light_weight(const hg_light& L, f3 world, f3& i
 // Bound by instruction issue (0.77 a cycle): the pixel's dual_scatter and, per
 // light, two arcsines, a cosine and 13 exponentials.  With every light's
 // Gaussians divided out anew and all of azimuthal() summed angle by angle the
-// 1920 x 1080 benchmark frame took 123 us (111 M warp instructions; now 107 and
-// 95 M), 24 grooms of the batch benchmark 548 (513 M; now 426 and 385 M, a
+// 1920 x 1080 benchmark frame took 123 us (111 M warp instructions; now 110 and
+// 97 M), 24 grooms of the batch benchmark 548 (513 M; now 433 and 393 M, a
 // third of it the pixel lists of shade_block).
 template <class V>
 __device__ __forceinline__ void shade_hair(const V& a, const hg_light* __restrict__ lights, uint32_t n_lights,
@@ -645,8 +662,8 @@ __device__ __forceinline__ void shade_hair(const V& a, const hg_light* __restric
             dom_direct = expf(-depth);
             if (depth > 1e-3f) {
                 const hg_light& L = lights[dom_light];
-                const float theta_h = asinf(clampf(dot3(t_n, safe_normalize(ld3(L.direction))), -1.0f, 1.0f)) +
-                                      fibre.theta_o;
+                const float sin_i = clampf(dot_fixed(t_n, normalize_fixed(ld3(L.direction))), -1.0f, 1.0f);
+                const float theta_h = asinf(sin_i) + fibre.theta_o;
                 color = vmul(spread_term(shape, ds, theta_h, depth, dom_direct), ld3(L.color));
             }
         }
@@ -656,11 +673,8 @@ __device__ __forceinline__ void shade_hair(const V& a, const hg_light* __restric
         f3 incident;
         float weight = light_weight(L, world, incident);
         if (i == dom_light) weight = dom_direct;
-        if (weight > 0.0f) {
-            // point and spot directions are normalized already
-            const f3 l = L.kind == HG_LIGHT_POINT || L.kind == HG_LIGHT_SPOT ? incident : safe_normalize(incident);
-            color = add3(color, mul3s(vmul(hair_bsdf(fibre, l), ld3(L.color)), weight));
-        }
+        if (weight > 0.0f)
+            color = add3(color, mul3s(vmul(hair_bsdf(fibre, normalize_fixed(incident)), ld3(L.color)), weight));
     }
     if (env.spec) {
         const f3 fiber_n = safe_normalize(sub3(view, mul3s(tangent, dot3(view, tangent))));
@@ -714,10 +728,10 @@ __device__ __forceinline__ void shade_block(const V& a, const hg_light* __restri
     shade_hair(a, lights, n_lights, ortho, exposure, env, x0 + q % blockDim.x, y0 + q / blockDim.x, s_word[tid]);
 }
 
-// Four blocks per SM (64 registers, some spilled): 107 us on the 1920 x 1080
-// benchmark frame; three (80 registers) 112, five (48) 108.  The batch's small
-// views wait more for their blocks' first loads: 24 grooms 448 us at four, 510
-// at three, 426 at five.
+// Four blocks per SM (64 registers, some spilled): 110 us on the 1920 x 1080
+// benchmark frame; three (80 registers) 4 % more, five (48) 1 %.  The batch's
+// small views wait more for their blocks' first loads: 24 grooms 433 us at
+// five, 5 % more at four, 19 % at three.
 __global__ void __launch_bounds__(kShadeThreads, 4) shade_kernel(const ShadeArgs a, const EnvArgs env) {
     shade_block(a, a.lights, a.n_lights, a.ortho, a.exposure, env, blockIdx.x * blockDim.x, blockIdx.y * blockDim.y);
 }
