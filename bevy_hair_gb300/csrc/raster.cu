@@ -18,34 +18,28 @@ namespace {
 
 // ------------------------------------------------------------------ clear
 
-// clear.wgsl:7-16.  Four pixels per thread with 16-byte stores.
-__global__ void clear_kernel(unsigned long long* __restrict__ center, unsigned long long* __restrict__ cons,
-                             uint32_t* __restrict__ beta, size_t pixels) {
-    size_t quads = pixels / 4;
-    size_t stride = (size_t)gridDim.x * blockDim.x;
-    const ulonglong2 e2 = make_ulonglong2(kEmptyU64, kEmptyU64);
-    const uint4 e4 = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
-    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < quads; q += stride) {
-        reinterpret_cast<ulonglong2*>(center)[2 * q] = e2;
-        reinterpret_cast<ulonglong2*>(center)[2 * q + 1] = e2;
-        reinterpret_cast<ulonglong2*>(cons)[2 * q] = e2;
-        reinterpret_cast<ulonglong2*>(cons)[2 * q + 1] = e2;
-        reinterpret_cast<uint4*>(beta)[q] = e4;
-    }
-    size_t tail = quads * 4 + (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (tail < pixels) {
-        center[tail] = kEmptyU64;
-        cons[tail] = kEmptyU64;
-        beta[tail] = 0xffffffffu;
-    }
+// p[0 .. n): the value v, by the whole grid; whole 16-byte units with
+// consecutive lanes on consecutive units, so that every store of a warp fills
+// its sectors.  p on a 16-byte boundary.
+template <class T>
+__device__ __forceinline__ void fill(T* __restrict__ p, size_t n, T v) {
+    constexpr size_t kPer = 16 / sizeof(T);
+    const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+    union {
+        T t[kPer];
+        uint4 u;
+    } unit;
+#pragma unroll
+    for (size_t k = 0; k < kPer; ++k) unit.t[k] = v;
+    for (size_t q = first; q < n / kPer; q += stride) reinterpret_cast<uint4*>(p)[q] = unit.u;
+    if (first < n % kPer) p[n / kPer * kPer + first] = v;
 }
 
 // clear_dom.wgsl:8-21: words below `texels` are front depths, the rest counters.
-__global__ void clear_dom_kernel(uint32_t* __restrict__ dom, size_t texels, size_t words) {
-    size_t quads = words / 4;
-    size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < quads; q += stride) {
-        size_t w = q * 4;
+__device__ __forceinline__ void fill_dom(uint32_t* __restrict__ dom, size_t texels, size_t words) {
+    const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t q = first; q < words / 4; q += stride) {
+        const size_t w = q * 4;
         uint4 v;
         v.x = w + 0 < texels ? kDomEmpty : 0u;
         v.y = w + 1 < texels ? kDomEmpty : 0u;
@@ -53,43 +47,32 @@ __global__ void clear_dom_kernel(uint32_t* __restrict__ dom, size_t texels, size
         v.w = w + 3 < texels ? kDomEmpty : 0u;
         reinterpret_cast<uint4*>(dom)[q] = v;
     }
-    size_t tail = quads * 4 + (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t tail = words / 4 * 4 + first;
     if (tail < words) dom[tail] = tail < texels ? kDomEmpty : 0u;
 }
 
-// Both of the above in one launch, for a whole frame: the G-buffer's quads,
-// then the map's.
+// clear.wgsl:7-16.  Bound by the memory's writes: the 183 MB of 24 batched
+// grooms' views 26 us; with four pixels a thread, whose two 16-byte stores per
+// array each half filled their sectors, 38.
+__global__ void clear_kernel(unsigned long long* __restrict__ center, unsigned long long* __restrict__ cons,
+                             uint32_t* __restrict__ beta, size_t pixels) {
+    fill(center, pixels, kEmptyU64);
+    fill(cons, pixels, kEmptyU64);
+    fill(beta, pixels, 0xffffffffu);
+}
+
+__global__ void clear_dom_kernel(uint32_t* __restrict__ dom, size_t texels, size_t words) {
+    fill_dom(dom, texels, words);
+}
+
+// Both of the above in one launch, for a whole frame.
 __global__ void frame_clear_kernel(unsigned long long* __restrict__ center, unsigned long long* __restrict__ cons,
                                    uint32_t* __restrict__ beta, size_t pixels, uint32_t* __restrict__ dom,
                                    size_t texels, size_t words) {
-    const size_t px_quads = pixels / 4, quads = px_quads + words / 4;
-    const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
-    const ulonglong2 e2 = make_ulonglong2(kEmptyU64, kEmptyU64);
-    const uint4 e4 = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
-    for (size_t q = first; q < quads; q += stride) {
-        if (q < px_quads) {
-            reinterpret_cast<ulonglong2*>(center)[2 * q] = e2;
-            reinterpret_cast<ulonglong2*>(center)[2 * q + 1] = e2;
-            reinterpret_cast<ulonglong2*>(cons)[2 * q] = e2;
-            reinterpret_cast<ulonglong2*>(cons)[2 * q + 1] = e2;
-            reinterpret_cast<uint4*>(beta)[q] = e4;
-        } else {
-            const size_t w = (q - px_quads) * 4;
-            uint4 v;
-            v.x = w + 0 < texels ? kDomEmpty : 0u;
-            v.y = w + 1 < texels ? kDomEmpty : 0u;
-            v.z = w + 2 < texels ? kDomEmpty : 0u;
-            v.w = w + 3 < texels ? kDomEmpty : 0u;
-            reinterpret_cast<uint4*>(dom)[q - px_quads] = v;
-        }
-    }
-    const size_t px_tail = px_quads * 4 + first, dom_tail = words / 4 * 4 + first;
-    if (px_tail < pixels) {
-        center[px_tail] = kEmptyU64;
-        cons[px_tail] = kEmptyU64;
-        beta[px_tail] = 0xffffffffu;
-    }
-    if (dom_tail < words) dom[dom_tail] = dom_tail < texels ? kDomEmpty : 0u;
+    fill(center, pixels, kEmptyU64);
+    fill(cons, pixels, kEmptyU64);
+    fill(beta, pixels, 0xffffffffu);
+    fill_dom(dom, texels, words);
 }
 
 // ------------------------------------------------------------------ lod
@@ -115,39 +98,58 @@ __device__ __forceinline__ uint32_t control_points_for_lod(float l) {
 
 constexpr uint32_t kDepthBuckets = 1024;
 
-// lod.wgsl:6-59, one warp per bundle (two of the 64 cage corners per lane).
+// lod.wgsl:6-59 of one bundle (its 64 cage corners).
 // Also writes the bundle's nearest view distance as one of kDepthBuckets
 // buckets between near and far, for the front-to-back draw order.
+// L lanes (32 or 8) take one bundle, lane `lane` of them; every lane of the
+// warp calls it, those without a bundle with valid false.  A warp per bundle
+// spends most of its time on latency (bundle, cage, 25 shuffles) and on one
+// lane's end; four bundles a warp overlap theirs, which pays once a warp per
+// bundle no longer fits on the chip at a time (lod_lanes).  A warp against 8
+// lanes, us: 24 batched grooms 57 against 42, both views of 3840 x 2160 18
+// against 14, of 1920 x 1080 (14,000 bundles) 9.9 against 8.9, of 512 x 512
+// (5,800) 6.2 against 6.2, of 96 x 64 4.0 against 4.9.
+template <int L>
 __device__ __forceinline__ void lod_bundle(const hg_hair_params& p, const hg_gpu_bundle* __restrict__ bundles,
                                            const float4* __restrict__ layers, hg_lod_record* __restrict__ out,
-                                           uint32_t* __restrict__ depth_key, uint32_t b, uint32_t lane) {
-    hg_gpu_bundle bundle = bundles[b];
+                                           uint32_t* __restrict__ depth_key, uint32_t b, uint32_t lane, bool valid) {
+    hg_gpu_bundle bundle = {};
     float mnx = 1e20f, mny = 1e20f, mxx = -1e20f, mxy = -1e20f, mnd = 3.0e38f;
     bool front = false;
-    for (uint32_t c = lane; c < 64u; c += 32u) {
-        float4 pa = __ldg(&layers[2u * (bundle.layer_offset + c)]);
-        f3 world = to_world(p, xyz(pa));
-        float4 clip = mat_mul(p.clip_from_world, world.x, world.y, world.z, 1.0f);
-        float dist = dot3(sub3(world, mk3(p.camera_pos[0], p.camera_pos[1], p.camera_pos[2])),
-                          mk3(p.camera_forward[0], p.camera_forward[1], p.camera_forward[2]));
-        if (clip.w > 0.0f && dist > 0.0f) front = true;
-        mnd = fminf(mnd, dist);
-        Projected pr = project_world(p, world);
-        mnx = fminf(mnx, pr.screen.x);
-        mny = fminf(mny, pr.screen.y);
-        mxx = fmaxf(mxx, pr.screen.x);
-        mxy = fmaxf(mxy, pr.screen.y);
+    if (valid) {
+        bundle = bundles[b];
+        constexpr int kPoints = 64 / L;
+        float4 cage[kPoints];
+#pragma unroll
+        for (int k = 0; k < kPoints; ++k)
+            cage[k] = __ldg(&layers[2u * (bundle.layer_offset + lane + (uint32_t)(L * k))]);
+#pragma unroll
+        for (int k = 0; k < kPoints; ++k) {
+            f3 world = to_world(p, xyz(cage[k]));
+            float4 clip = mat_mul(p.clip_from_world, world.x, world.y, world.z, 1.0f);
+            float dist = dot3(sub3(world, mk3(p.camera_pos[0], p.camera_pos[1], p.camera_pos[2])),
+                              mk3(p.camera_forward[0], p.camera_forward[1], p.camera_forward[2]));
+            if (clip.w > 0.0f && dist > 0.0f) front = true;
+            mnd = fminf(mnd, dist);
+            Projected pr = project_world(p, world);
+            mnx = fminf(mnx, pr.screen.x);
+            mny = fminf(mny, pr.screen.y);
+            mxx = fmaxf(mxx, pr.screen.x);
+            mxy = fmaxf(mxy, pr.screen.y);
+        }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = L / 2; o > 0; o >>= 1) {
         mnx = fminf(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
         mny = fminf(mny, __shfl_xor_sync(0xffffffffu, mny, o));
         mxx = fmaxf(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
         mxy = fmaxf(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
         mnd = fminf(mnd, __shfl_xor_sync(0xffffffffu, mnd, o));
     }
-    bool any_front = __any_sync(0xffffffffu, front);
-    if (lane != 0) return;
+    const uint32_t fronts = __ballot_sync(0xffffffffu, front);
+    const uint32_t group = (threadIdx.x & 31u) / L;
+    const bool any_front = (fronts >> (group * L) & (0xffffffffu >> (32 - L))) != 0u;
+    if (lane != 0 || !valid) return;
     const float rel = (mnd - p.screen[2]) / fmaxf(p.screen[3] - p.screen[2], 1e-3f);
     depth_key[b] = min(f2u(clampf(rel, 0.0f, 1.0f) * (float)kDepthBuckets), kDepthBuckets - 1u);
     bool culled = !any_front || mxx < 0.0f || mxy < 0.0f || mnx > p.screen[0] || mny > p.screen[1];
@@ -173,14 +175,17 @@ __device__ __forceinline__ void lod_bundle(const hg_hair_params& p, const hg_gpu
     out[b] = hg_lod_record{n_lod, cps, bundle.strand_count, 0u};
 }
 
-__global__ void lod_kernel(const hg_hair_params p, const hg_gpu_bundle* __restrict__ bundles,
-                           const float4* __restrict__ layers, hg_lod_record* __restrict__ out,
-                           uint32_t* __restrict__ depth_key, uint32_t count) {
-    uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint32_t lane = threadIdx.x & 31u;
-    if (b >= count) return;
-    lod_bundle(p, bundles, layers, out, depth_key, b, lane);
+template <int L>
+__global__ void __launch_bounds__(256) lod_kernel(const hg_hair_params p, const hg_gpu_bundle* __restrict__ bundles,
+                                                  const float4* __restrict__ layers, hg_lod_record* __restrict__ out,
+                                                  uint32_t* __restrict__ depth_key, uint32_t count) {
+    const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) / L;
+    lod_bundle<L>(p, bundles, layers, out, depth_key, b, threadIdx.x % L, b < count);
 }
+
+// Lanes per bundle, and blocks of 256 threads, for `bundles` of them.
+int lod_lanes(const hg_ctx* ctx, uint32_t bundles) { return bundles <= (uint32_t)ctx->sm_count * 64u ? 32 : 8; }
+uint32_t lod_blocks(uint32_t bundles, int lanes) { return (bundles + 256u / lanes - 1u) / (256u / lanes); }
 
 // ------------------------------------------------------------------ scan
 
@@ -407,11 +412,11 @@ struct SetupArgs {
     uint32_t capacity;
 };
 
+template <int L>
 __global__ void __launch_bounds__(256) frame_lod_kernel(const SetupArgs a) {
-    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) / L;
     const uint32_t k = w < a.v[0].count ? 0u : 1u, b = w - (k ? a.v[0].count : 0u);
-    if (b >= a.v[k].count) return;
-    lod_bundle(a.p[k], a.bundles, a.layers, a.v[k].lod, a.v[k].depth_key, b, lane);
+    lod_bundle<L>(a.p[k], a.bundles, a.layers, a.v[k].lod, a.v[k].depth_key, b, threadIdx.x % L, b < a.v[k].count);
 }
 
 __global__ void __launch_bounds__(kScanThreads) frame_scan_offsets_kernel(const SetupArgs a) {
@@ -1772,9 +1777,7 @@ __global__ void batch_clear_dom_kernel(const BatchView* __restrict__ views, cons
                                        uint32_t* __restrict__ dom) {
     const BatchView& v = views[blockIdx.y];
     const size_t texels = (size_t)v.dom_w * v.dom_h, words = texels * (1 + kDomLayers);
-    uint32_t* map = dom + dom_prefix[blockIdx.y];
-    for (size_t w = (size_t)blockIdx.x * blockDim.x + threadIdx.x; w < words; w += (size_t)gridDim.x * blockDim.x)
-        map[w] = w < texels ? kDomEmpty : 0u;
+    fill_dom(dom + dom_prefix[blockIdx.y], texels, words);
 }
 
 // grid (X, DOM views): dom_front_kernel of every deep-opacity view.
@@ -1785,13 +1788,14 @@ __global__ void __launch_bounds__(256) batch_dom_front_kernel(const BatchView* _
         front_quad(v.p, v.dom, v.front, v.dom_w, v.dom_h, lines_x, q);
 }
 
-__global__ void batch_lod_kernel(const BatchView* __restrict__ views, const uint32_t* __restrict__ prefix,
-                                 uint32_t n_views, uint32_t total) {
-    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
-    if (w >= total) return;
-    const uint32_t v = find_view(prefix, n_views, w);
+template <int L>
+__global__ void __launch_bounds__(256) batch_lod_kernel(const BatchView* __restrict__ views,
+                                                        const uint32_t* __restrict__ prefix, uint32_t n_views,
+                                                        uint32_t total) {
+    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) / L;
+    const uint32_t v = find_view(prefix, n_views, min(w, total - 1u));
     const BatchView& a = views[v];
-    lod_bundle(a.p, a.bundles, a.layers, a.lod, a.depth_key, w - prefix[v], lane);
+    lod_bundle<L>(a.p, a.bundles, a.layers, a.lod, a.depth_key, w - prefix[v], threadIdx.x % L, w < total);
 }
 
 // Camera views also get the front-to-back draw order of the single-view scan.
@@ -2539,10 +2543,9 @@ cudaError_t launch_clear_dom(hg_ctx* ctx) {
 cudaError_t launch_lod(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p, int slot) {
     uint32_t count = std::min(p.pass_mode[1], g->bundle_count);
     if (count == 0) return cudaSuccess;
-    int threads = 256;
-    int blocks = (int)((count * 32u + threads - 1) / threads);
-    lod_kernel<<<blocks, threads, 0, ctx->stream>>>(p, g->bundles, g->layers, g->lod[slot], g->depth_key[slot],
-                                                    count);
+    const int lanes = lod_lanes(ctx, count);
+    (lanes == 8 ? lod_kernel<8> : lod_kernel<32>)<<<lod_blocks(count, lanes), 256, 0, ctx->stream>>>(
+        p, g->bundles, g->layers, g->lod[slot], g->depth_key[slot], count);
     return cudaGetLastError();
 }
 
@@ -2607,7 +2610,8 @@ cudaError_t launch_frame_setup(hg_ctx* ctx, hg_groom* g, const hg_hair_params& c
     const int threads = 256;
     cudaError_t e = cudaSuccess;
     if (total) {
-        frame_lod_kernel<<<(total * 32u + threads - 1) / threads, threads, 0, ctx->stream>>>(a);
+        const int lanes = lod_lanes(ctx, total);
+        (lanes == 8 ? frame_lod_kernel<8> : frame_lod_kernel<32>)<<<lod_blocks(total, lanes), 256, 0, ctx->stream>>>(a);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     frame_scan_offsets_kernel<<<dom ? 2 : 1, kScanThreads, 0, ctx->stream>>>(a);
@@ -2721,8 +2725,10 @@ cudaError_t launch_batch_setup(hg_ctx* ctx, const BatchDev& b) {
     if (e != cudaSuccess) return e;
     const int threads = 256;
     if (b.total_bundles) {
-        const uint32_t blocks = (b.total_bundles * 32u + threads - 1) / threads;
-        batch_lod_kernel<<<blocks, threads, 0, ctx->stream>>>(b.views, b.bundle_prefix, b.n_views, b.total_bundles);
+        const int lanes = lod_lanes(ctx, b.total_bundles);
+        (lanes == 8 ? batch_lod_kernel<8> : batch_lod_kernel<32>)<<<lod_blocks(b.total_bundles, lanes), 256, 0,
+                                                                  ctx->stream>>>(b.views, b.bundle_prefix, b.n_views,
+                                                                                 b.total_bundles);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     batch_scan_offsets_kernel<<<b.n_views, kScanThreads, 0, ctx->stream>>>(b.views);

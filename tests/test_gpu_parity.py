@@ -14,7 +14,7 @@ import numpy as np
 import pytest
 
 import oracle
-from bevy_hair_gb300 import abi, configs, host
+from bevy_hair_gb300 import abi, configs, groom, host
 from bevy_hair_gb300.pipeline import HairRenderer, Light, pack_lights
 
 pytestmark = pytest.mark.gpu
@@ -193,6 +193,24 @@ def test_strand_cache_equals_strands_generated_in_the_raster(renderer, n):
     for name, want, have in zip(("center", "conservative", "beta", "dom"), *got):
         _assert_equal(name, have, want)
     assert (got[0][1] != EMPTY).any()
+
+
+@pytest.mark.parametrize("n", [1, 3, 32, 9728, 9729, 9731, 20_000])
+def test_lod_of_many_bundles_matches_the_oracle(renderer, n):
+    """Four bundles share a warp from sm_count x 64 bundles up (9,728 on 152
+    SMs), a bundle has its own below; last warps in part."""
+    sc = configs.config2(scale=0.001)
+    mesh = sc.mesh
+    sc.mesh = groom.HairMesh(np.resize(mesh.bundles, n), mesh.layers, mesh.style, mesh.bounds_min, mesh.bounds_max)
+    cam, dom = sc.params()
+    renderer.ensure_targets(sc.view.width, sc.view.height, *sc.dom_size)
+    g = renderer.upload(sc.mesh)
+    for p, slot in ((cam, abi.SLOT_CAMERA), (dom, abi.SLOT_DOM)):
+        renderer.lod(g, p, slot)
+        assert renderer.synchronize() == 0
+        want = oracle.lod(p, sc.mesh)
+        _assert_equal("lod", g.read(slot, abi.GBUF_LOD)[:n].view(np.uint32), want[:n].view(np.uint32))
+    g.close()
 
 
 def test_dense_groom_with_tile_depth_rejection(renderer):
