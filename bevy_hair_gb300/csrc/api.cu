@@ -733,8 +733,10 @@ hg_status hg_hair_visibility(hg_ctx* ctx, const hg_shadow_light* light, const fl
 // Work before and after the frame stays ordered on the main stream.
 // Frame, us, with the setup on one stream per view and a launch per pass and
 // target (18 launches) -> so (11): 96 x 64 thumbnail 92 -> 76, 512 x 512
-// 210 -> 192, 1920 x 1080 1134 -> 1089, 3840 x 2160 2426 -> 2251.  The clears
-// on the side stream behind the scan: 2 to 5 us slower at every size.
+// 210 -> 192, 1920 x 1080 1134 -> 1089, 3840 x 2160 2426 -> 2251.  (A small
+// groom's single camera stage takes two launches fewer, 76 -> 69 us; a large
+// groom's front plane one more.)  The clears on the side stream behind the
+// scan: 2 to 5 us slower at every size.
 hg_status hg_groom_frame(hg_ctx* ctx, hg_groom* g, const hg_frame_desc* d) {
     if (!ctx || !g || !d || !d->camera) return HG_INVALID_ARG;
     const hg_hair_params& cam = *d->camera;
@@ -790,7 +792,7 @@ hg_status hg_groom_frame(hg_ctx* ctx, hg_groom* g, const hg_frame_desc* d) {
     HG_CUDA(ctx, cudaEventRecord(ctx->ev_join, ctx->side));
     on(main_stream);
     HG_CUDA(ctx, cudaStreamWaitEvent(main_stream, ctx->ev_setup, 0));
-    HG_CUDA(ctx, hg::launch_raster(ctx, g, cam, HG_SLOT_CAMERA, d->scene_depth));
+    HG_CUDA(ctx, hg::launch_raster(ctx, g, cam, HG_SLOT_CAMERA, d->scene_depth, true));
     HG_CUDA(ctx, cudaStreamWaitEvent(main_stream, ctx->ev_join, 0));
     HG_CUDA(ctx, guard_writes(ctx, 1u << HG_BUF_SHADED | 1u << HG_BUF_SHADED_DEPTH));
     HG_CUDA(ctx, hg::launch_shade(ctx, cam, d->shade.light_count, d->shade.ortho, d->shade.exposure,

@@ -246,7 +246,9 @@ cudaError_t launch_scan(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p, int s
 // A whole frame's setup: both targets' clears; lod and scan of both views (dom may be null).
 cudaError_t launch_frame_clear(hg_ctx* ctx, bool with_dom);
 cudaError_t launch_frame_setup(hg_ctx* ctx, hg_groom* g, const hg_hair_params& cam, const hg_hair_params* dom);
-cudaError_t launch_raster(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p, int slot, const float* scene);
+// in_frame: the camera pass of a whole frame, which may take one stage.
+cudaError_t launch_raster(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p, int slot, const float* scene,
+                          bool in_frame = false);
 cudaError_t launch_generate(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p);
 void release_bins(hg_groom* g);  // frees the binned camera raster's scratch
 constexpr uint32_t kStrandCacheCps = 65;

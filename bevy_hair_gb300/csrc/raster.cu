@@ -908,6 +908,13 @@ __device__ __forceinline__ int32_t run_of_lane(const StrandSmem& sm, int32_t run
 constexpr uint32_t kCameraFirstStage = 112;
 constexpr uint32_t kCameraStages[] = {0, kCameraFirstStage, 256};
 constexpr int kCameraStageCount = sizeof(kCameraStages) / sizeof(kCameraStages[0]);
+// A frame's camera pass takes one stage while its warps draw at most this many
+// refs each: a stage then lasts as long as one or two strands' chains, and the
+// tile depths and the second stage only add theirs.  Two stages against one,
+// frame in us: 500 strands 76.9 against 69.8, 3,600 (512 x 288) 109 against 98,
+// 3,600 (1280 x 720) 214 against 189, 7,000 118 against 116; 14,000 and more the
+// same within the noise.
+constexpr size_t kOneStageRounds = 2;
 
 // True when no sample of segment (pa, pb) (world, in sm.cp) / (A, B) (screen)
 // can change a G-buffer word: every pixel it can reach is off screen, or
@@ -2637,7 +2644,8 @@ cudaError_t launch_generate(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_raster(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p, int slot, const float* scene) {
+cudaError_t launch_raster(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p, int slot, const float* scene,
+                          bool in_frame) {
     if (g->bundle_count == 0) return cudaSuccess;
     RasterArgs a;
     a.p = p;
@@ -2682,9 +2690,11 @@ cudaError_t launch_raster(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p, int
         // the earlier stages left, and segments behind them are skipped.
         const uint32_t tiles_x = tiles_along(ctx->width);
         const uint32_t tiles = tiles_x * tiles_along(ctx->height);
-        for (int k = 0; k + 1 < kCameraStageCount; ++k) {
+        const size_t resident = (size_t)ctx->sm_count * raster_min_blocks<0>() * kRasterWarps;
+        const bool one_stage = in_frame && g->ref_capacity <= kOneStageRounds * resident;
+        for (int k = 0; k + 1 < (one_stage ? 2 : kCameraStageCount); ++k) {
             a.part_lo = kCameraStages[k];
-            a.part_hi = kCameraStages[k + 1];
+            a.part_hi = one_stage ? kCameraStages[kCameraStageCount - 1] : kCameraStages[k + 1];
             if (k > 0 && tiles && ctx->tile_depth) {
                 tile_depth_kernel<<<(tiles + 7) / 8, 256, 0, ctx->stream>>>(ctx->center, ctx->cons, ctx->beta,
                                                                            ctx->width, ctx->height, tiles_x, tiles,

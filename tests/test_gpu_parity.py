@@ -213,6 +213,25 @@ def test_lod_of_many_bundles_matches_the_oracle(renderer, n):
     g.close()
 
 
+@pytest.mark.parametrize("n", [1, 3648, 3649, 7296, 7297])
+def test_one_camera_stage_equals_two(renderer, n):
+    """A frame draws the camera's refs in one stage while its warps take at most
+    two each (2 x 3,648 on 152 SMs); the pass by itself always takes two."""
+    sc = configs.config1(scale=n / 10_000) if n > 16 else configs.config1(scale=0.0016)
+    if n == 1:
+        sc.mesh = configs._mesh(1, 32, "straight", 3)
+    assert sc.mesh.strand_count() == n
+    cam, dom = sc.params()
+    want = _visibility(renderer, sc, cam, dom)
+    g = renderer.upload(sc.mesh)
+    renderer.render_groom(g, cam, dom, sc.light_array())
+    assert renderer.synchronize() == 0
+    for name, which in (("center", abi.BUF_CENTER), ("cons", abi.BUF_CONSERVATIVE), ("beta", abi.BUF_BETA),
+                        ("dom", abi.BUF_DOM)):
+        _assert_equal(name, renderer.read(which), want[name])
+    g.close()
+
+
 def test_dense_groom_with_tile_depth_rejection(renderer):
     """A dense groom at low resolution (deep overdraw) with a small deep
     opacity map: the later stages of the camera and DOM depth passes skip most
