@@ -734,7 +734,8 @@ hg_status hg_hair_visibility(hg_ctx* ctx, const hg_shadow_light* light, const fl
 // Frame, us, with the setup on one stream per view and a launch per pass and
 // target (18 launches) -> so (11): 96 x 64 thumbnail 92 -> 76, 512 x 512
 // 210 -> 192, 1920 x 1080 1134 -> 1089, 3840 x 2160 2426 -> 2251.  (A small
-// groom's single camera stage takes two launches fewer, 76 -> 69 us; a large
+// groom's single camera stage takes two launches fewer, 76 -> 69 us, and its
+// scan makes no draw order, 69 -> 62; a large
 // groom's front plane one more.)  The clears on the side stream behind the
 // scan: 2 to 5 us slower at every size.
 hg_status hg_groom_frame(hg_ctx* ctx, hg_groom* g, const hg_frame_desc* d) {

@@ -285,7 +285,10 @@ __device__ __forceinline__ void scan_offsets_block(const hg_lod_record* __restri
         indirect[2] = 1u;
         indirect[3] = 0u;
     }
-    if (!sorted) return;
+    if (!sorted) {
+        if (order_meta && threadIdx.x == 0) order_meta[1] = 0u;  // an earlier scan's order is void
+        return;
+    }
     // Draw order: live bundles (n_lod > 0) counting-sorted by depth bucket,
     // then their n_lod scanned in that order.  The raster visits strands in
     // this order (near bundles first) so most later samples fail the depth
@@ -914,7 +917,13 @@ constexpr int kCameraStageCount = sizeof(kCameraStages) / sizeof(kCameraStages[0
 // frame in us: 500 strands 76.9 against 69.8, 3,600 (512 x 288) 109 against 98,
 // 3,600 (1280 x 720) 214 against 189, 7,000 118 against 116; 14,000 and more the
 // same within the noise.
+// Without a second stage the front-to-back order serves nothing, and the
+// frame's scan leaves it out (11 -> 5 us at 300 strands, in the chain of setup
+// launches).
 constexpr size_t kOneStageRounds = 2;
+bool one_camera_stage(const hg_ctx* ctx, const hg_groom* g) {
+    return g->ref_capacity <= kOneStageRounds * ctx->sm_count * raster_min_blocks<0>() * kRasterWarps;
+}
 
 // True when no sample of segment (pa, pb) (world, in sm.cp) / (A, B) (screen)
 // can change a G-buffer word: every pixel it can reach is off screen, or
@@ -2607,7 +2616,8 @@ cudaError_t launch_frame_setup(hg_ctx* ctx, hg_groom* g, const hg_hair_params& c
         v.offsets = g->offsets[s];
         v.indirect = g->indirect[s];
         v.refs = g->refs[s];
-        v.sorted = s == 0 ? g->sorted[s] : nullptr;  // as launch_scan: the camera view's draw order only
+        // as launch_scan: the camera view's draw order only
+        v.sorted = s == 0 && !one_camera_stage(ctx, g) ? g->sorted[s] : nullptr;
         v.sorted_off = g->sorted_off[s];
         v.draw_order = g->draw_order[s];
         v.order_meta = g->order_meta[s];
@@ -2690,8 +2700,8 @@ cudaError_t launch_raster(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p, int
         // the earlier stages left, and segments behind them are skipped.
         const uint32_t tiles_x = tiles_along(ctx->width);
         const uint32_t tiles = tiles_x * tiles_along(ctx->height);
-        const size_t resident = (size_t)ctx->sm_count * raster_min_blocks<0>() * kRasterWarps;
-        const bool one_stage = in_frame && g->ref_capacity <= kOneStageRounds * resident;
+        const bool one_stage = in_frame && one_camera_stage(ctx, g);
+        if (one_stage) a.draw_order = nullptr;  // launch_frame_setup made none
         for (int k = 0; k + 1 < (one_stage ? 2 : kCameraStageCount); ++k) {
             a.part_lo = kCameraStages[k];
             a.part_hi = one_stage ? kCameraStages[kCameraStageCount - 1] : kCameraStages[k + 1];

@@ -229,6 +229,14 @@ def test_one_camera_stage_equals_two(renderer, n):
     for name, which in (("center", abi.BUF_CENTER), ("cons", abi.BUF_CONSERVATIVE), ("beta", abi.BUF_BETA),
                         ("dom", abi.BUF_DOM)):
         _assert_equal(name, renderer.read(which), want[name])
+    # the frame's refs drawn once more by the pass: no draw order of an earlier scan is taken for theirs
+    renderer.lod(g, dom, abi.SLOT_CAMERA)
+    renderer.scan(g, cam, abi.SLOT_CAMERA)
+    renderer.render_groom(g, cam, dom, sc.light_array())
+    renderer.clear()
+    renderer.raster(g, cam, abi.SLOT_CAMERA)
+    assert renderer.synchronize() == 0
+    _assert_equal("center", renderer.read(abi.BUF_CENTER), want["center"])
     g.close()
 
 
