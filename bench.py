@@ -744,8 +744,9 @@ def run_ours(args, rank, world, local):
     e2e_value, e2e_ms, _ = aggregate(dist, e2e_total * 1e3, float(seg_c) * args.steps)
     # per frame: generate, lod, scan offsets and expand of both views, clear of both
     # targets, camera raster (direct, the default: 2 stages + tile depths between
-    # them), 2 x DOM raster, shade, filter with colour clear and composite
-    launches = 11 * args.steps
+    # them), 2 x DOM raster (and, from 32,768 strands up, the front plane of the
+    # layers pass), shade, filter with colour clear and composite
+    launches = (11 + (sc.mesh.strand_count() >= 32_768)) * args.steps
 
     cpu = None
     if rank == 0 and not args.no_cpu_baseline:

@@ -245,7 +245,7 @@ __device__ __forceinline__ Lobes azimuthal_at(const AzimuthPixel& q, const Scatt
     return r;
 }
 
-__device__ Dual dual_scatter_by_angle(float cos_theta_d, f3 sigma_a, const Shape& shape) {
+__device__ __forceinline__ Dual dual_scatter_by_angle(float cos_theta_d, f3 sigma_a, const Shape& shape) {
     Lobes fwd = {spl(0.0f), spl(0.0f), spl(0.0f)}, back = fwd;
     const AzimuthPixel q = azimuth_pixel(cos_theta_d, sigma_a);
 #pragma unroll 2

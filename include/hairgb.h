@@ -265,8 +265,9 @@ hg_status hg_raster(hg_ctx* ctx, hg_groom* groom, const hg_hair_params* params,
  * same words (every write is a commutative min).
  *  HG_CAMERA_RASTER_DIRECT (the default): every sample's atomicMin goes to
  *    global memory, after a read of the current word's high half, in two
- *    launches (the nearest quarter of the refs, then the rest, whose segments
- *    hidden behind per-8x8-tile depths are skipped).
+ *    launches (the nearest 7/16 of the refs, then the rest, whose segments
+ *    hidden behind per-8x8-tile depths are skipped); hg_groom_frame draws a
+ *    small groom (at most two strands per resident warp) in one.
  *  HG_CAMERA_RASTER_BINNED: every segment is listed under the 32x32 screen
  *    tiles its pixels can touch; a block per tile (and chunk of its list)
  *    resolves the tile's centre, conservative and beta words in shared memory,
