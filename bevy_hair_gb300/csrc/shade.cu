@@ -326,7 +326,7 @@ __device__ __forceinline__ f3 reject_fixed(f3 v, f3 t, float s) {
 // 0.02), so exponent scale and norm of the first serve all, times powers of
 // two; the back lobe's a_back 2 / pi kDensityBack is in its norm.
 struct Fibre {
-    f3 t, v, t_o, sigma_a;
+    f3 t, t_o, sigma_a;
     float theta_o, to2, tilt;
     float g_k, g_k_low, g_n;  // -1 / (2 b^2) and what its rounding left, 1 / (b sqrt(2 pi))
     f3 back_k, back_n, delta_b;
@@ -336,7 +336,6 @@ __device__ __forceinline__ Fibre make_fibre(f3 t_n, f3 v_n, f3 sigma_a, const Sh
     const float norm = 0.398942280f;  // 1 / sqrt(2 pi)
     Fibre f;
     f.t = t_n;
-    f.v = v_n;
     f.sigma_a = sigma_a;
     const float sin_o = clampf(dot_fixed(t_n, v_n), -1.0f, 1.0f);
     f.theta_o = asinf(sin_o);
