@@ -140,6 +140,14 @@ struct FilterPixel {
     bool use_color;
 };
 
+// The sums of one group of rows.
+struct FilterSums {
+    float x, y, z, weight;
+};
+__device__ __forceinline__ FilterSums operator+(FilterSums a, FilterSums b) {
+    return {a.x + b.x, a.y + b.y, a.z + b.z, a.weight + b.weight};
+}
+
 // P's sums over tap's colour with weight w, where `keep`.
 __device__ __forceinline__ void accumulate(bool keep, float4 tap, float w, FilterPixel& P) {
     asm("{\n.reg .pred p;\nsetp.ne.u32 p, %8, 0;\n"
@@ -164,8 +172,11 @@ __device__ __forceinline__ void accumulate(bool keep, float4 tap, float w, Filte
 // bit masks (strip_row), row by row, instead of a distance and two tests per
 // tap; the spatial exponent is a quadratic form in (dx, dy) with one add and
 // one FMA per tap; and the depth test alone also rejects the texels without a
-// centre hit.  S threads (1, 2 or 4) share a pair, 12 / S rows each, and add
-// up by shuffles: small images leave the chip idle otherwise.  Coverage
+// centre hit.  S threads (1, 2 or 4) share a pair, 12 / S rows each: small
+// images leave the chip idle otherwise.  However many share it, each group of
+// three rows is summed by itself and the four sums are added in the order of
+// the groups, so that an image's colours do not depend on S (a batch takes
+// one thread a pair for views of any size).  Coverage
 // decisions use exact arithmetic; the colour weights only scale colour, so
 // they use fused operations and the fast exponential.  Against a thread per pixel with 121 tests and a
 // distance each (us): 1920 x 1080 113 -> 79, 3840 x 2160 200 -> 141, 512 x 512
@@ -175,7 +186,8 @@ __device__ __forceinline__ void filter_tile(const V& a, int32_t bx, int32_t by, 
     constexpr int kHaloX = TX + 2 * kFilterRadius, kHaloY = TY + 2 * kFilterRadius;
     constexpr int kPairs = TX * TY / 2, kThreads = kPairs * S, kWarps = kThreads / 32, kPairWarps = kPairs / 32;
     constexpr int kRows = 2 * kFilterRadius + 2;  // rows a pair's two windows cover
-    static_assert(kPairs % 32 == 0 && kRows % S == 0 && kHaloX <= 64 && TX <= 32, "tile shape");
+    constexpr int kGroups = 4, kGroupRows = kRows / kGroups;
+    static_assert(kPairs % 32 == 0 && kRows % kGroups == 0 && kGroups % S == 0 && kHaloX <= 64 && TX <= 32, "tile shape");
     __shared__ float4 s_tap[kHaloY][kHaloX];  // colour, normalised depth or mark
     __shared__ uint4 s_hits[kHaloY];          // bit per texel: centre hit (x, y), conservative hit only (z, w)
     __shared__ uint16_t s_list[kPairs];       // pair | hair in its upper / lower pixel << 14, 15
@@ -328,6 +340,9 @@ __device__ __forceinline__ void filter_tile(const V& a, int32_t bx, int32_t by, 
         P_.c = __fmaf_rn(yy, k_par, xx * k_perp);
     }
 
+    // `done`: one thread, the sum of the groups behind it; two, their first group
+    FilterSums done[2] = {};
+    int left = kGroupRows;
 #pragma unroll 1
     for (int r = sub * (kRows / S); r < (sub + 1) * (kRows / S); ++r) {
         const uint4 hits = s_hits[sy + r];
@@ -364,21 +379,41 @@ __device__ __forceinline__ void filter_tile(const V& a, int32_t bx, int32_t by, 
                 accumulate(fabsf(tap.w - P_.p_norm) <= reject[q], tap, ex2(-e), P_);
             }
         }
-    }
-    if (S > 1) {
+        if (S < kGroups && --left == 0) {  // a group's end
+            left = kGroupRows;
+            if (S == 1 || r == sub * (kRows / S) + kGroupRows - 1) {
 #pragma unroll
-        for (int q = 0; q < 2; ++q)
+                for (int q = 0; q < 2; ++q) {
+                    const FilterSums own = {P[q].ax, P[q].ay, P[q].az, P[q].weight};
+                    done[q] = S == 1 && r >= kGroupRows ? done[q] + own : own;
+                    P[q].ax = P[q].ay = P[q].az = P[q].weight = 0.0f;
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        FilterSums sum = done[q];
+        if (S > 1) {
+            const FilterSums own = {P[q].ax, P[q].ay, P[q].az, P[q].weight};
+            auto from = [&](const FilterSums& v, int k) {  // thread k of the pair's
+                return FilterSums{__shfl_sync(0xffffffffu, v.x, k, S), __shfl_sync(0xffffffffu, v.y, k, S),
+                                  __shfl_sync(0xffffffffu, v.z, k, S), __shfl_sync(0xffffffffu, v.weight, k, S)};
+            };
+            if (S == 2) sum = ((from(done[q], 0) + from(own, 0)) + from(done[q], 1)) + from(own, 1);
+            else sum = ((from(own, 0) + from(own, 1)) + from(own, 2)) + from(own, 3);
 #pragma unroll
             for (int o = 1; o < S; o <<= 1) {
-                P[q].ax += __shfl_xor_sync(0xffffffffu, P[q].ax, o);
-                P[q].ay += __shfl_xor_sync(0xffffffffu, P[q].ay, o);
-                P[q].az += __shfl_xor_sync(0xffffffffu, P[q].az, o);
-                P[q].weight += __shfl_xor_sync(0xffffffffu, P[q].weight, o);
                 P[q].h_center += __shfl_xor_sync(0xffffffffu, P[q].h_center, o);
                 P[q].h_cons += __shfl_xor_sync(0xffffffffu, P[q].h_cons, o);
             }
-        if (slot >= total) return;
+        }
+        P[q].ax = sum.x;
+        P[q].ay = sum.y;
+        P[q].az = sum.z;
+        P[q].weight = sum.weight;
     }
+    if (S > 1 && slot >= total) return;
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
         // with several threads a pair, the first writes the upper pixel, the second the lower

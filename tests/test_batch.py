@@ -369,3 +369,24 @@ def test_large_groom_layers_walk_equals_the_batched_one(renderer):
     _compare(graph, _read_all(b, 2))
     assert b.launches(abi.BATCH_SEPARATE) == 18 + 19
     _close(b, grooms)
+
+
+@pytest.mark.parametrize("size, scale", [((96, 64), 0.003), ((701, 399), 0.03), ((1023, 577), 0.05)])
+def test_batched_colour_equals_the_frame_at_every_filter_split(renderer, size, scale):
+    """hg_groom_frame's filter gives a pixel pair four, two or one threads by
+    the image's size, the batch's always one: the colours are the same bits."""
+    bs = configs.config4(scale=scale, items=2)
+    for s in bs.scenes:
+        s.view = configs._camera(*size, 900.0)
+    b, grooms, params = _make(renderer, bs)
+    lights = bs.light_array()
+    b.frame(lights)
+    assert renderer.synchronize() == 0
+    batched = _read_all(b, 2)
+    for k, (cam, dom) in enumerate(params):
+        renderer.ensure_targets(*size, *bs.scenes[k].dom_size)
+        renderer.render_groom(grooms[k], cam, dom, lights)
+        assert renderer.synchronize() == 0
+        for which in VIS + COLOUR:
+            np.testing.assert_array_equal(batched[k][which], renderer.read(which), err_msg=f"item {k} buffer {which}")
+    _close(b, grooms)
