@@ -122,10 +122,66 @@ __device__ __forceinline__ uint32_t strip_row(float2 ts, float inv_ty, int dy, f
     return m;
 }
 
+// 2^x, results below 2^-126 flushed to zero: a pixel's weights count only from
+// a sum of 1e-5 up, where 121 such weights are below half a unit in the last
+// place of it.  exp2f, which scales to keep them, gives the same outputs and
+// takes 1 to 2.5 % of a frame (1920 x 1080 1,017 -> 1,026 us, 24 grooms
+// 2,489 -> 2,551).
 __device__ __forceinline__ float ex2(float x) {
     float r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
+}
+
+// The spatial exponent of a tap (dx, dy), k_par d_par^2 + k_perp d_perp^2 with
+// d_par and d_perp its coordinates along the strand's direction ts and across
+// it, with the square in dx completed: a (dx - r dy)^2 + c dy^2.  Three
+// operations a tap, and nothing cancels in them; expanded to dx^2, dx dy and
+// dy^2 terms it would take one, but along the strand of a narrow filter terms
+// of thousands leave a few units.  a and c are correctly rounded but for a few
+// in a thousand, r is a sum rh + rl (error-free products and sums), and the
+// rounded ts' distance from length 1, which leaves d_perp as it is, is taken
+// out.  RMS error of a weight above 1e-5, relative, emulated over 1e5
+// directions: filter_params 1, 0.2 (the default) 3.1e-7, with d_par, the vector
+// across and its length formed anew for every tap 3.6e-7, expanded 5.6e-7;
+// 1, 0.02: 1.3e-6, 1.8e-6 and 3.3e-5; 0.05, 1: 5.8e-7, 6.1e-7 and 6.8e-6.
+struct SpatialForm {
+    float a, rh, rl, c;
+};
+__device__ __forceinline__ SpatialForm spatial_form(float2 ts, float k_par, float k_perp) {
+    const float xx = ts.x * ts.x, yy = ts.y * ts.y, xy = ts.x * ts.y;
+    const float xx_low = __fmaf_rn(ts.x, ts.x, -xx), yy_low = __fmaf_rn(ts.y, ts.y, -yy);
+    const float xy_low = __fmaf_rn(ts.x, ts.y, -xy);
+    const bool flat = fabsf(ts.x) >= fabsf(ts.y);
+    const float major = flat ? ts.x : ts.y, minor = flat ? ts.y : ts.x;
+    const float excess = __fmaf_rn(minor, minor, __fmaf_rn(major, major, -1.0f));  // |ts|^2 - 1
+    // a = k_par xx + k_perp yy / |ts|^2
+    const float a1 = k_par * xx, a2 = k_perp * yy, a = a1 + a2, a2_in = a - a1;
+    const float a_low = ((a1 - (a - a2_in)) + (a2 - a2_in)) + (__fmaf_rn(k_par, xx, -a1) + k_par * xx_low) +
+                        (__fmaf_rn(k_perp, yy, -a2) + k_perp * (yy_low - yy * excess));
+    // r = xy (k_perp / |ts|^2 - k_par) / a
+    const float diff = k_perp - k_par, diff_in = diff - k_perp;
+    const float diff_low = ((k_perp - (diff - diff_in)) - (k_par + diff_in)) - k_perp * excess;
+    const float b = xy * diff, b_low = __fmaf_rn(xy, diff, -b) + __fmaf_rn(xy, diff_low, xy_low * diff);
+    const float inv = 1.0f / a;
+    SpatialForm f;
+    f.a = a + a_low;
+    f.rh = b * inv;
+    f.rl = (__fmaf_rn(-f.rh, a, b) + (b_low - f.rh * a_low)) * inv;
+    // c = k_par k_perp |ts|^2 / a
+    const float kk = k_par * k_perp, kk_low = __fmaf_rn(k_par, k_perp, -kk) + kk * excess;
+    const float c = kk * inv;
+    f.c = c + (__fmaf_rn(-c, a, kk) + (kk_low - c * a_low)) * inv;
+    // a vanishes where the filter has no bound along the rows: the exponent
+    // is then the same for every dx.  (0, 0), the direction of a strand whose
+    // screen length overflows, has all taps across it.
+    if (!(a >= 1e-30f)) {
+        const bool none = xx + yy == 0.0f;
+        f.a = none ? k_perp : a;
+        f.rh = f.rl = 0.0f;
+        f.c = none ? k_perp : yy * k_par + xx * k_perp;
+    }
+    return f;
 }
 
 // One pixel of a thread's pair: what its taps are weighed against, and its
@@ -134,7 +190,7 @@ struct FilterPixel {
     float2 ts;
     float inv_ty;
     float cx, cy, cz, p_norm;          // centre colour, normalised depth
-    float a, b, c;                     // dx^2, dx dy and dy^2 factors of a tap's exponent
+    SpatialForm form;
     float ax, ay, az, weight;          // weighted colour and weight
     int h_center, h_cons;              // strip taps with a centre hit, with a conservative hit only
     bool use_color;
@@ -170,8 +226,7 @@ __device__ __forceinline__ void accumulate(bool keep, float4 tap, float w, Filte
 // The tap loop is bound by instruction issue and shared-memory bandwidth.  A
 // pair shares its taps' loads (12 rows for 2 x 11); the strip counts come from
 // bit masks (strip_row), row by row, instead of a distance and two tests per
-// tap; the spatial exponent is a quadratic form in (dx, dy) with one add and
-// one FMA per tap; and the depth test alone also rejects the texels without a
+// tap; the spatial exponent takes three operations a tap (spatial_form); and the depth test alone also rejects the texels without a
 // centre hit.  S threads (1, 2 or 4) share a pair, 12 / S rows each: small
 // images leave the chip idle otherwise.  However many share it, each group of
 // three rows is summed by itself and the four sums are added in the order of
@@ -334,10 +389,7 @@ __device__ __forceinline__ void filter_tile(const V& a, int32_t bx, int32_t by, 
             P_.use_color = center_hit && cc.w > 0.0f;
         }
         P_.inv_ty = 1.0f / P_.ts.y;
-        const float xx = P_.ts.x * P_.ts.x, yy = P_.ts.y * P_.ts.y;
-        P_.a = __fmaf_rn(xx, k_par, yy * k_perp);
-        P_.b = 2.0f * P_.ts.x * P_.ts.y * (k_par - k_perp);
-        P_.c = __fmaf_rn(yy, k_par, xx * k_perp);
+        P_.form = spatial_form(P_.ts, k_par, k_perp);
     }
 
     // `done`: one thread, the sum of the groups behind it; two, their first group
@@ -348,16 +400,15 @@ __device__ __forceinline__ void filter_tile(const V& a, int32_t bx, int32_t by, 
         const uint4 hits = s_hits[sy + r];
         const float4* row = &s_tap[sy + r][sx + kFilterRadius];
         // window rows: dy = r - 5 of the upper pixel, r - 6 of the lower
-        float base[2][kFilterRadius + 1], slope[2], reject[2];
+        float vertex[2], across[2], reject[2];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const int dy = r - kFilterRadius - q;
             const bool in = dy >= -kFilterRadius && dy <= kFilterRadius;
             reject[q] = in ? depth_reject : -1.0f;
-            slope[q] = P[q].b * (float)dy;
-            const float c = P[q].c * (float)(dy * dy);
-#pragma unroll
-            for (int k = 0; k <= kFilterRadius; ++k) base[q][k] = __fmaf_rn(P[q].a, (float)(k * k), c);
+            const float fdy = (float)dy;
+            vertex[q] = __fmaf_rn(P[q].form.rh, fdy, P[q].form.rl * fdy);
+            across[q] = P[q].form.c * (fdy * fdy);
             if (in) {
                 const uint32_t strip = strip_row(P[q].ts, P[q].inv_ty, dy, strip2);
                 P[q].h_center += __popc(__funnelshift_r(hits.x, hits.y, sx) & strip);
@@ -372,7 +423,8 @@ __device__ __forceinline__ void filter_tile(const V& a, int32_t bx, int32_t by, 
                 FilterPixel& P_ = P[q];
                 // evaluated for every tap, kept for those near in depth: predicated
                 // sums cost less than the branches around them
-                float e = __fmaf_rn(slope[q], (float)dx, base[q][dx < 0 ? -dx : dx]);
+                const float u = (float)dx - vertex[q];
+                float e = __fmaf_rn(u * u, P_.form.a, across[q]);
                 const float cx = P_.cx - tap.x, cy = P_.cy - tap.y, cz = P_.cz - tap.z;
                 const float ec = __fmaf_rn(__fmaf_rn(cz, cz, __fmaf_rn(cy, cy, cx * cx)), k_col, e);
                 e = P_.use_color ? ec : e;

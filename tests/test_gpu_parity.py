@@ -459,6 +459,48 @@ def test_filter_at_the_edges_of_its_thread_split(renderer, size):
     np.testing.assert_allclose(filt[:, :3], want[:, :3], rtol=FILTER_RTOL, atol=FILTER_ATOL)
 
 
+@pytest.mark.parametrize("s_par, s_perp", [(1.0, 0.2), (1.0, 0.02), (100.0, 0.02), (0.05, 0.02), (0.05, 1.0), (0.3, 0.3)])
+@pytest.mark.parametrize("size", [(97, 61), (800, 500), (1021, 531)])
+def test_filter_widths_at_the_ends_of_their_ranges(renderer, size, s_par, s_perp):
+    """Narrow and wide filters (the widths are clamped to 0.05 along the strand
+    and 0.02 across it) in every direction, four, two and one threads a pair.
+
+    A weight's relative error is at most 1.3e-5 here and 2.3e-5 in the oracle,
+    whose float distance across the strand it comes from, both at width 0.02;
+    a colour, the weighted mean of values in [0, 1], moves by no more than their
+    sum, and by 3e-6 for the 121 terms of its sums."""
+    w, h = size
+    sc = configs.config1(scale=0.02)
+    cam, _ = host.groom_params(configs._camera(w, h, 1000.0), sc.groom, sc.mesh.bounds_min, sc.mesh.bounds_max,
+                               sc.mesh.bundle_count, sc.directionals, sc.dom_size)
+    cam = cam.copy()
+    cam["filter_params"][:2] = s_par, s_perp
+    rng = np.random.default_rng(w + h)
+    n = w * h
+    depth = ((0.4 + rng.normal(0.0, 2e-4, n)) * 16777214.0).astype(np.uint64)
+    oct_x, oct_y = rng.integers(0, 256, n, dtype=np.uint64), rng.integers(0, 256, n, dtype=np.uint64)
+    words = (depth << np.uint64(40)) | (oct_x << np.uint64(32)) | (oct_y << np.uint64(24)) | np.uint64(0xFFF)
+    center = np.where(rng.random(n) < 0.9, words, EMPTY)
+    shaded = rng.random((n, 4)).astype(np.float32)
+    shaded[:, 3] = (rng.random(n) < 0.5).astype(np.float32)
+    renderer.ensure_targets(w, h, 0, 0)
+    renderer.write(abi.BUF_CENTER, center)
+    renderer.write(abi.BUF_CONSERVATIVE, words)
+    renderer.write(abi.BUF_SHADED, shaded)
+    renderer.filter(cam)
+    assert renderer.synchronize() == 0
+    filt = renderer.read(abi.BUF_FILTERED).reshape(-1, 4)
+    want, want_depth = oracle.filter_(cam, center, words, shaded, np.zeros(n, dtype=np.float32))
+    want = np.asarray(want).reshape(-1, 4)
+    _assert_equal("filter depth", renderer.read(abi.BUF_FILTERED_DEPTH), np.asarray(want_depth))
+    # without a centre hit a pixel counts only from a total weight of 1e-5 up,
+    # which the two sides may see on either side of it
+    sure = (center != EMPTY) | ((filt[:, 3] > 0) == (want[:, 3] > 0))
+    assert sure.mean() > 0.999
+    _assert_equal("filter alpha", filt[sure, 3], want[sure, 3])
+    np.testing.assert_allclose(filt[sure, :3], want[sure, :3], rtol=0.0, atol=1.3e-5 + 2.3e-5 + 3e-6)
+
+
 @pytest.mark.parametrize("scale", [0.02, 1.0])
 def test_full_frame_against_the_oracle_frame(renderer, scale):
     """hg_groom_frame against the oracle's whole hair_pass sequence; at scale 1
