@@ -18,6 +18,7 @@
 #include "hg_mlp.cuh"
 #include "hg_mlp_small.cuh"
 #include "hg_mlp_tc.cuh"
+#include "hg_ring.h"
 
 namespace hg {
 namespace {
@@ -802,7 +803,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1) train_kernel(const TrainArgs
 // 16 us a step instead of 22, but round differently: 4e-6 of the gradient,
 // which a few steps at a high learning rate amplify.)
 constexpr uint32_t kChunkTiles = 16;
-constexpr int kWgradUnits = 8, kWgradStages = 6, kWgradWarps = 4, kWgradThreads = 32 * (kWgradWarps + 1);
+constexpr uint32_t kWgradStages = 6;
+constexpr int kWgradUnits = 8, kWgradWarps = 4, kWgradThreads = 32 * (kWgradWarps + 1);
 struct WgradStage {
     __half rows[96][kTilePad];  // dZ rows, then H rows
 };
@@ -836,9 +838,7 @@ __device__ __forceinline__ float h2sum(uint32_t v) {
 // stage each, as stages become free.  False when one did not in time.
 __device__ __forceinline__ bool wgrad_copy(WgradSmem& S, const TileActs* acts, uint32_t tiles, WgradRows u) {
     const uint32_t full = (uint32_t)__cvta_generic_to_shared(S.full), empty = (uint32_t)__cvta_generic_to_shared(S.empty);
-    for (uint32_t k = 0; k < tiles; ++k) {
-        const uint32_t s = k % kWgradStages, round = k / kWgradStages;
-        if (round > 0 && !tc::mbar_wait(empty + 8u * s, (round - 1u) & 1u)) return false;
+    auto start = [&](uint32_t s, uint32_t k) {
         const char* tile = reinterpret_cast<const char*>(acts + k);
         const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&S.st[s]), mbar = full + 8u * s;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(mbar),
@@ -852,14 +852,10 @@ __device__ __forceinline__ bool wgrad_copy(WgradSmem& S, const TileActs* acts, u
         };
         copy(dst, u.a, u.rows_a);
         copy(dst + u.rows_a * kActRowBytes, u.b, u.rows_b);
-    }
-    // every copy has landed before the block may end, whatever the other warps did
-    bool ok = true;
-    for (uint32_t s = 0; s < kWgradStages && s < tiles; ++s) {
-        const uint32_t last = (tiles - 1u - s) / kWgradStages;
-        ok = tc::mbar_wait(full + 8u * s, last & 1u) && ok;
-    }
-    return ok;
+    };
+    return feed_ring<kWgradStages>(
+        tiles, [&](uint32_t s, uint32_t parity) { return tc::mbar_wait(empty + 8u * s, parity); }, start,
+        [&](uint32_t s, uint32_t parity) { return tc::mbar_wait(full + 8u * s, parity); });
 }
 
 // One warp's 16 x (8 NT) products over the chunk's tiles; a_row, b_row: its
@@ -909,7 +905,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) wgrad_kernel(const WgradArgs
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const uint32_t chunk = blockIdx.x, unit = blockIdx.y;
     if (threadIdx.x == 0) {
-        for (int k = 0; k < kWgradStages; ++k) {
+        for (uint32_t k = 0; k < kWgradStages; ++k) {
             tc::mbar_init((uint32_t)__cvta_generic_to_shared(&S.full[k]), 1);
             tc::mbar_init((uint32_t)__cvta_generic_to_shared(&S.empty[k]), kWgradWarps);
         }
