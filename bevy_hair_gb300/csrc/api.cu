@@ -231,7 +231,9 @@ hg_status hg_create(int device, void* stream, hg_ctx** out) {
         if (!ctx->dual_table) e = cudaErrorMemoryAllocation;
     }
     if (e == cudaSuccess) e = cudaMalloc(&ctx->dual_table->table, sizeof(float4) * hg::kDualTableFloat4);
-    if (e == cudaSuccess) e = cudaMallocHost(&ctx->lights_host, sizeof(hg_light) * HG_MAX_LIGHTS * hg_ctx::kLightSlots);
+    constexpr size_t kStagedLights = (size_t)HG_MAX_LIGHTS * hg_ctx::kLightSlots;
+    if (e == cudaSuccess) e = cudaMallocHost(&ctx->lights_host, sizeof(hg_light) * kStagedLights + sizeof(uint32_t));
+    if (e == cudaSuccess) ctx->err_host = reinterpret_cast<uint32_t*>(ctx->lights_host + kStagedLights);
     for (int i = 0; i < hg_ctx::kLightSlots && e == cudaSuccess; ++i)
         e = cudaEventCreateWithFlags(&ctx->light_events[i], cudaEventDisableTiming);
     if (e != cudaSuccess) {

@@ -1149,6 +1149,7 @@ struct AdamArgs {
     const float* loss_part;  // [blocks]
     uint32_t parts, blocks;
     float* loss;             // the batch's sum of squared errors, nullable
+    const uint32_t* err;     // the context's error word
     float lr_t, beta1, beta2, eps_t, gscale;
     int update;              // 1: Adam step; 0: the summed gradient into grad, parameters as they are
 };
@@ -1159,7 +1160,9 @@ constexpr int kAdamParams = 32, kAdamSplit = 16;  // parameters per block, threa
 // with the bias corrections folded into lr_t and eps_t, then the FP16 forward
 // (and, for the 4 x 64 network, transposed) copies.  Sixteen threads share a
 // parameter's partials, so that each has its loads in flight at once, and add
-// up in a fixed order.
+// up in a fixed order.  While the context has a timeout to report, a partial
+// gradient may be missing: nothing is summed into the parameters then, their
+// moments or grad.
 template <int N, bool TRANSPOSED>
 __global__ void __launch_bounds__(kAdamParams* kAdamSplit) adam_kernel(const AdamArgs a) {
     __shared__ float s_sum[kAdamSplit][kAdamParams];
@@ -1180,6 +1183,7 @@ __global__ void __launch_bounds__(kAdamParams* kAdamSplit) adam_kernel(const Ada
         for (uint32_t b = split; b < a.parts; b += kAdamSplit) gr += __ldcg(&a.part[(size_t)b * N + i]);
     }
     s_sum[split][q] = gr;
+    const bool missing = threadIdx.x == 0 && a.part && (__ldcg(a.err) & tc::kErrTimeout) != 0u;
     if (a.loss && blockIdx.x == 0 && split == 1) {
         float l = 0.0f;
         for (uint32_t b = q; b < a.blocks; b += kAdamParams) l += __ldcg(&a.loss_part[b]);
@@ -1187,8 +1191,7 @@ __global__ void __launch_bounds__(kAdamParams* kAdamSplit) adam_kernel(const Ada
         for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
         if (q == 0) *a.loss = l;
     }
-    __syncthreads();
-    if (!own) return;
+    if (__syncthreads_or(missing) || !own) return;
     gr = 0.0f;
 #pragma unroll
     for (int s = 0; s < kAdamSplit; ++s) gr += s_sum[s][q];
@@ -1312,6 +1315,16 @@ hg_status cuda_fail(hg_ctx* ctx, cudaError_t e, const char* where) {
         if (e_ != cudaSuccess) return cuda_fail(ctx, e_, #expr); \
     } while (0)
 
+// The error word's copy to the host, behind the stream's work; after the
+// stream was waited for, what a timeout in that work makes of `done`.
+cudaError_t copy_error_word(hg_ctx* ctx) {
+    return cudaMemcpyAsync(ctx->err_host, ctx->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream);
+}
+hg_status unless_timed_out(hg_ctx* ctx, hg_status done) {
+    if (!(*ctx->err_host & tc::kErrTimeout)) return done;
+    return fail(ctx, HG_DEVICE_TIMEOUT, "a tensor-core wait timed out; no training step since has been taken");
+}
+
 // Most blocks a training launch uses: one (the 4 x 64 network, whose tile
 // fills an SM's shared memory) or two per SM.
 uint32_t max_train_blocks(const hg_mlp* m) {
@@ -1380,6 +1393,7 @@ cudaError_t convert(hg_mlp* m, uint32_t n, int update, float lr_t, float eps_t, 
     a.parts = n ? train_parts(m, n) : 0u;
     a.blocks = n ? train_blocks(m, n) : 0u;
     a.loss = n ? loss : nullptr;
+    a.err = m->ctx->err;
     a.lr_t = lr_t;
     a.beta1 = 0.9f;
     a.beta2 = 0.999f;
@@ -1561,9 +1575,10 @@ hg_status hg_mlp_get_params(hg_mlp* m, float* params, uint32_t count) {
     if (!m || !params) return HG_INVALID_ARG;
     hg_ctx* ctx = m->ctx;
     if (count != m->n_params) return fail(ctx, HG_INVALID_ARG, "parameter count must be hg_mlp_param_count");
+    MLP_CUDA(ctx, hg::copy_error_word(ctx));
     MLP_CUDA(ctx, cudaMemcpyAsync(params, m->params, sizeof(float) * count, cudaMemcpyDeviceToHost, ctx->stream));
     MLP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return HG_OK;
+    return hg::unless_timed_out(ctx, HG_OK);
 }
 
 hg_status hg_mlp_samples(hg_ctx* ctx, uint64_t seed, uint64_t first, uint32_t count, float tilt, float* inputs,
@@ -1630,12 +1645,13 @@ hg_status hg_mlp_gradients(hg_mlp* m, const float* inputs, const float* targets,
     MLP_CUDA(ctx, hg::ensure_scratch(m, count));
     MLP_CUDA(ctx, hg::run_gradients(m, inputs, targets, count));
     MLP_CUDA(ctx, hg::convert(m, count, 0, 0.0f, 0.0f, 0.0f, m->loss));
+    MLP_CUDA(ctx, hg::copy_error_word(ctx));
     MLP_CUDA(ctx, cudaMemcpyAsync(grad, m->grad, pf, cudaMemcpyDeviceToHost, ctx->stream));
     float l = 0.0f;
     MLP_CUDA(ctx, cudaMemcpyAsync(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     MLP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     if (loss) *loss = l;
-    return HG_OK;
+    return hg::unless_timed_out(ctx, HG_OK);
 }
 
 hg_status hg_mlp_train_step(hg_mlp* m, const float* inputs, const float* targets, uint32_t count, float lr,

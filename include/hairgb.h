@@ -556,6 +556,9 @@ uint32_t hg_mlp_param_count(const hg_mlp* mlp);
 uint32_t hg_mlp_output_count(const hg_mlp* mlp);
 /* Host float[count], count == hg_mlp_param_count; resets the optimiser state. */
 hg_status hg_mlp_set_params(hg_mlp* mlp, const float* params, uint32_t count);
+/* Like hg_mlp_gradients, HG_DEVICE_TIMEOUT while the context has a timeout
+ * that hg_synchronize has not reported: training steps since then were not
+ * taken, and the parameters are those before them. */
 hg_status hg_mlp_get_params(hg_mlp* mlp, float* params, uint32_t count);
 /* Training samples with FP64 lobes (Gauss-Legendre integration of the
  * Marschner/d'Eon azimuthal scattering, Zinke back-scattering) at the
@@ -582,7 +585,9 @@ hg_status hg_mlp_gradients(hg_mlp* mlp, const float* inputs, const float* target
                            float* loss);
 /* One Adam step (beta1 0.9, beta2 0.999, eps 1e-8) on the mean squared error
  * of one batch (device inputs/targets).  loss_sum: nullable device float that
- * receives the batch's sum of squared errors.  Asynchronous on the stream. */
+ * receives the batch's sum of squared errors.  Asynchronous on the stream.
+ * While the context has a timeout that hg_synchronize has not reported, the
+ * parameters and moments stay as they are. */
 hg_status hg_mlp_train_step(hg_mlp* mlp, const float* inputs, const float* targets, uint32_t count, float lr,
                             float* loss_sum);
 /* The same 12 lobes from the Karis fits of shade.wesl:94-190 in FP32, as

@@ -524,6 +524,41 @@ def test_gradients_at_the_edges_of_the_training_tiles(renderer, arch, n):
 
 
 @gpu
+@pytest.mark.parametrize("arch", [0, COMPACT])
+def test_no_training_step_after_a_timeout(renderer, arch):
+    """A training kernel whose wait ran out sets the timeout bit and leaves its
+    partial gradient unwritten.  With the bit set (here by the host): no step is
+    taken, the calls that wait for the stream say so, and training goes on from
+    the same parameters and moments once hg_synchronize has reported it."""
+    import internals
+
+    torch, dev = _torch()
+    x = torch.empty((300, 10), dtype=torch.float32, device=dev)
+    t = torch.empty((300, 12), dtype=torch.float32, device=dev)
+    S.samples(renderer, 11, 0, 300, x, t)
+    s = S.Surrogate(renderer, S.init_params(5, arch), arch)
+    s.train_step(x, t, 300, 1e-3)
+    before, (gradient, _) = s.get_params(), s.gradients(x, t, 300)
+    lib = internals.load()
+    word = internals.device_words(lib.error_word(renderer.ctx), 1)
+    moments = [internals.device_words(lib.moments(s.handle, k), s.n_params) for k in (0, 1)]
+    held = [m.clone() for m in moments]
+    word |= 2  # the bit of a timeout
+    torch.cuda.synchronize()
+    s.train_step(x[1:], t[1:], 299, 1e-2)
+    for call in (s.get_params, lambda: s.gradients(x, t, 300), renderer.synchronize):
+        with pytest.raises(abi.HairGbError) as e:
+            call()
+        assert e.value.status == abi.HG_DEVICE_TIMEOUT
+    np.testing.assert_array_equal(s.get_params(), before)
+    assert all(torch.equal(a, b) for a, b in zip(moments, held))
+    np.testing.assert_array_equal(s.gradients(x, t, 300)[0], gradient)
+    s.train_step(x, t, 300, 1e-3)
+    assert not np.array_equal(s.get_params(), before)
+    s.close()
+
+
+@gpu
 def test_compact_gradients_match_the_fp64_reference(renderer):
     torch, dev = _torch()
     n = 3000  # not a multiple of 32: the ragged last block must contribute nothing extra
