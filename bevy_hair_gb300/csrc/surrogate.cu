@@ -1667,8 +1667,12 @@ hg_status hg_mlp_train_step(hg_mlp* m, const float* inputs, const float* targets
     const double b1t = 1.0 - std::pow(0.9, (double)m->step), b2t = 1.0 - std::pow(0.999, (double)m->step);
     const float lr_t = (float)(lr * std::sqrt(b2t) / b1t);
     const float eps_t = (float)(1e-8 * std::sqrt(b2t));
+    // the kernel stores a float; any other address takes a copy
+    const bool aligned = reinterpret_cast<uintptr_t>(loss_sum) % sizeof(float) == 0;
     MLP_CUDA(ctx, hg::convert(m, count, 1, lr_t, eps_t,
-                              1.0f / ((float)count * (float)hg_mlp_output_count(m)), loss_sum));
+                              1.0f / ((float)count * (float)hg_mlp_output_count(m)), aligned ? loss_sum : m->loss));
+    if (!aligned)
+        MLP_CUDA(ctx, cudaMemcpyAsync(loss_sum, m->loss, sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
     return HG_OK;
 }
 

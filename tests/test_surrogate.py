@@ -559,6 +559,26 @@ def test_no_training_step_after_a_timeout(renderer, arch):
 
 
 @gpu
+@pytest.mark.parametrize("arch", [0, COMPACT])
+def test_loss_at_any_address(renderer, arch):
+    """loss_sum off a 4-byte boundary (a record packed by the caller)."""
+    torch, dev = _torch()
+    x = torch.empty((300, 10), dtype=torch.float32, device=dev)
+    t = torch.empty((300, 12), dtype=torch.float32, device=dev)
+    S.samples(renderer, 12, 0, 300, x, t)
+    s = S.Surrogate(renderer, S.init_params(5, arch), arch)
+    record = torch.full((12,), 0x5A, dtype=torch.uint8, device=dev)
+    want = torch.zeros(1, dtype=torch.float32, device=dev)
+    s.train_step(x, t, 300, 0.0, want)
+    s.train_step(x, t, 300, 0.0, record.data_ptr() + 5)
+    renderer.synchronize()
+    got = record.cpu().numpy()
+    np.testing.assert_array_equal(got[5:9].copy().view(np.float32), want.cpu().numpy())
+    assert (got[:5] == 0x5A).all() and (got[9:] == 0x5A).all()
+    s.close()
+
+
+@gpu
 def test_compact_gradients_match_the_fp64_reference(renderer):
     torch, dev = _torch()
     n = 3000  # not a multiple of 32: the ragged last block must contribute nothing extra
