@@ -341,7 +341,8 @@ __device__ __forceinline__ Fibre make_fibre(f3 t_n, f3 v_n, f3 sigma_a, const Sh
     f.theta_o = asinf(sin_o);
     f.t_o = reject_fixed(v_n, t_n, sin_o);
     f.to2 = dot_fixed(f.t_o, f.t_o);
-    f.tilt = shape.alpha.x;
+    // beyond 1e18 every tilted lobe is zero; its angle's square must not overflow
+    f.tilt = fabsf(shape.alpha.x) > 1e18f ? copysignf(1e18f, shape.alpha.x) : shape.alpha.x;
     const float b = shape.beta.x;
     const float b2 = b * b, b2_low = __fmaf_rn(b, b, -b2);
     f.g_k = -0.5f / b2;

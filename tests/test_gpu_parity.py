@@ -643,6 +643,26 @@ def test_shade_lists_hair_pixels_of_partial_blocks(renderer, size, keep):
     g.close()
 
 
+@pytest.mark.parametrize("tilt", [0.0, -0.3, 1e4, 1e20, -3e38])
+def test_shade_at_any_tilt(renderer, tilt):
+    """The cuticle tilt is any float: lobes tilted out of reach vanish."""
+    sc = configs.config1(scale=0.02)
+    cam, dom = sc.params()
+    cam = cam.copy()
+    cam["appearance"][1] = tilt
+    lights = sc.light_array()
+    renderer.ensure_targets(sc.view.width, sc.view.height, *sc.dom_size)
+    g = renderer.upload(sc.mesh)
+    renderer.render_groom(g, cam, dom, lights)
+    assert renderer.synchronize() == 0
+    want, want_depth = oracle.shade(cam, renderer.read(abi.BUF_CENTER), renderer.read(abi.BUF_BETA),
+                                    renderer.read(abi.BUF_DOM), lights)
+    np.testing.assert_array_equal(renderer.read(abi.BUF_SHADED_DEPTH), want_depth)
+    np.testing.assert_allclose(renderer.read(abi.BUF_SHADED), want, rtol=SHADE_RTOL, atol=SHADE_ATOL)
+    assert np.isfinite(want).all()
+    g.close()
+
+
 def test_invalid_arguments_are_rejected(renderer):
     import ctypes as C
 
