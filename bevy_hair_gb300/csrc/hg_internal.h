@@ -262,14 +262,32 @@ constexpr size_t front_words(uint32_t w, uint32_t h) {
 // Whether a single groom's layers pass forms the front plane and walks its
 // texels flattened (raster_dom_layers) or takes a segment per lane on the map.
 // Forming the plane is a launch (3 to 4 us) and reads and writes the map once.
-// Measured, segment per lane against plane + flattened: 10,000 strands on a
-// 256^2 map 20.5 against 3.2 + 20.4 us; 100,000 on 1024^2 212 against
-// 4.0 + 202; 200,000 on 2048^2 775 against 8.3 + 636.  The line is where the
-// smallest gain per strand (0.1 ns) pays for the launch; a map of more texels
-// than the strands draw would pay for texels that nothing reads.
-constexpr uint32_t kPlaneMinStrands = 32768, kPlaneTexelsPerStrand = 64;
+// What it saves are the lines of the front depths, which grow with the texels
+// that a segment crosses: the pass, segment per lane against plane and
+// flattened walk (us), and the frame around it (wavy strands, 640 x 360):
+//   33,000 strands on  256^2  43.9 against  50.5, frame 279.7 against 281.5
+//                      512^2  52.5 against  56.1,       293.2 against 291.9
+//                     1024^2  75.7 against  74.6,       330.6 against 329.7
+//                     2048^2 139.0 against 128.4,       449.3 against 434.4
+//   100,000 on         128^2 119.4 against 134.6,       592.6 against 604.2
+//                      256^2 128.3 against 138.8,       590.6 against 599.5
+//                      512^2 151.3 against 154.2,       625.2 against 624.6
+//                     1024^2 212.6 against 208.4,       719.6 against 714.5
+//                     2048^2 378.6 against 324.0,       994.1 against 936.7
+//   16,000 on         1024^2  42.2 against  42.3,       223.7 against 224.1
+//                     2048^2  73.1 against  75.6,       303.3 against 303.7
+// Hence from 32,768 strands up on maps of more than 512^2 texels, where the
+// frame gains although the pass by itself breaks even only near 1024^2; and
+// not on a map of many more texels than the strands draw, whose plane would be
+// formed for texels that nothing reads (between the 262 texels a strand of
+// 16,000 on 2048^2 and the 127 of 33,000).  The batch forms the planes of all
+// its maps in one launch and gains at every size (8 x 2,000 strands on 64^2
+// 491 against 499 us, 16 x 20,000 on 64^2 2,820 against 2,912, on 512^2 2,806
+// against 3,255).
+constexpr uint32_t kPlaneMinStrands = 32768, kPlaneMinTexels = 512 * 512 + 1, kPlaneTexelsPerStrand = 64;
 constexpr bool layers_use_plane(uint32_t strands, uint32_t w, uint32_t h) {
-    return strands >= kPlaneMinStrands && (uint64_t)strands * kPlaneTexelsPerStrand >= (uint64_t)w * h;
+    return strands >= kPlaneMinStrands && (uint64_t)w * h >= kPlaneMinTexels &&
+           (uint64_t)strands * kPlaneTexelsPerStrand >= (uint64_t)w * h;
 }
 
 // Pixels per side of a tile of the camera pass's tile-depth buffer, as a

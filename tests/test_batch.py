@@ -390,3 +390,22 @@ def test_batched_colour_equals_the_frame_at_every_filter_split(renderer, size, s
         for which in VIS + COLOUR:
             np.testing.assert_array_equal(batched[k][which], renderer.read(which), err_msg=f"item {k} buffer {which}")
     _close(b, grooms)
+
+
+@pytest.mark.parametrize("size, launches", [((256, 256), 18), ((512, 512), 18), ((513, 512), 19), ((1024, 1024), 19)])
+def test_small_maps_layers_walk_takes_a_segment_a_lane(renderer, size, launches):
+    """Many strands on a small map (up to 512^2 texels) gain nothing from a
+    front plane; either way the maps are those of the batch."""
+    bs = configs.BatchScene("layers", [configs.config2(scale=0.4)], configs.config2(scale=0.4).lights)
+    assert bs.scenes[0].mesh.strand_count() == 40_000
+    bs.scenes[0].dom_size = size
+    b, grooms, _ = _make(renderer, bs)
+    lights = bs.light_array()
+    b.frame(lights, abi.BATCH_GRAPH)
+    assert renderer.synchronize() == 0
+    graph = _read_all(b, 1)
+    b.frame(lights, abi.BATCH_SEPARATE)
+    assert renderer.synchronize() == 0
+    _compare(graph, _read_all(b, 1))
+    assert b.launches(abi.BATCH_SEPARATE) == launches
+    _close(b, grooms)
