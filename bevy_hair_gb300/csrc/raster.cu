@@ -919,7 +919,9 @@ constexpr int kCameraStageCount = sizeof(kCameraStages) / sizeof(kCameraStages[0
 // same within the noise.
 // Without a second stage the front-to-back order serves nothing, and the
 // frame's scan leaves it out (11 -> 5 us at 300 strands, in the chain of setup
-// launches).
+// launches).  The binned raster of such a groom does without it, too: frames of
+// 64, 300, 2,000 and 7,000 strands 120, 124, 168 and 254 us with the order, 114,
+// 119, 162 and 243 without.
 constexpr size_t kOneStageRounds = 2;
 bool one_camera_stage(const hg_ctx* ctx, const hg_groom* g) {
     return g->ref_capacity <= kOneStageRounds * ctx->sm_count * raster_min_blocks<0>() * kRasterWarps;
@@ -1462,6 +1464,7 @@ struct GenArgs {
     const uint32_t* strand_base;    // first strand of each bundle
     float4* cache;
     uint32_t strands;
+    uint32_t per;                   // strands a warp takes at a time
 };
 
 // Per-warp shared memory of the cache's generation.  `tails`: the last
@@ -1641,18 +1644,20 @@ __device__ __forceinline__ void finish_tail(const Args& a, const GenSmem& sm, ui
 
 // Strands 0 .. total - 1 over the grid's warps, a pair at a time.
 // locate(g): g's view and its index in that view; of(v): view v's arguments.
+// per: strands a warp takes at a time, 2 or 1 (its odd lanes then help with the
+// samples and have no strand of their own).
 template <class Locate, class Of>
-__device__ __forceinline__ void generate_strands(GenSmem& sm, uint32_t total, Locate locate, Of of) {
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t step = 2u * gridDim.x * kRasterWarps;
+__device__ __forceinline__ void generate_strands(GenSmem& sm, uint32_t total, uint32_t per, Locate locate, Of of) {
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, own = lane & (per - 1u);
+    const uint32_t step = per * gridDim.x * kRasterWarps;
     uint32_t n = 0;
-    for (uint32_t g0 = 2u * (blockIdx.x * kRasterWarps + warp); g0 < total; g0 += step) {
-        const uint32_t g = min(g0 + (lane & 1u), total - 1u);
-        const bool valid = g0 + (lane & 1u) < total;
+    for (uint32_t g0 = per * (blockIdx.x * kRasterWarps + warp); g0 < total; g0 += step) {
+        const uint32_t g = min(g0 + own, total - 1u);
+        const bool valid = (lane & 1u) < per && g0 + own < total;
         uint32_t v = 0, s = g;
         locate(g, v, s);
         generate_pair(of(v), of, s, valid, v, sm, n, lane);
-        n += g0 + 1u < total ? 2u : 1u;
+        n += per == 2u && g0 + 1u < total ? 2u : 1u;
         if (n == 32u || total - g0 <= step) {
             if (lane < n) finish_tail(of(sm.tails.view[lane]), sm, lane);
             __syncwarp();
@@ -1663,7 +1668,7 @@ __device__ __forceinline__ void generate_strands(GenSmem& sm, uint32_t total, Lo
 
 __global__ void __launch_bounds__(kRasterThreads, kGenBlocks) generate_kernel(const GenArgs a) {
     __shared__ GenSmem sm[kRasterWarps];
-    generate_strands(sm[threadIdx.x >> 5], a.strands, [](uint32_t, uint32_t&, uint32_t&) {},
+    generate_strands(sm[threadIdx.x >> 5], a.strands, a.per, [](uint32_t, uint32_t&, uint32_t&) {},
                      [&](uint32_t) -> const GenArgs& { return a; });
 }
 
@@ -1865,7 +1870,7 @@ __global__ void __launch_bounds__(kRasterThreads, kGenBlocks) batch_generate_ker
                                                                         uint32_t n_cam, uint32_t total) {
     __shared__ GenSmem sm[kRasterWarps];
     generate_strands(
-        sm[threadIdx.x >> 5], total,
+        sm[threadIdx.x >> 5], total, 2u,
         [&](uint32_t g, uint32_t& v, uint32_t& s) {
             v = find_view(prefix, n_cam, g);
             s = g - prefix[v];
@@ -2649,7 +2654,12 @@ cudaError_t launch_generate(hg_ctx* ctx, hg_groom* g, const hg_hair_params& p) {
     a.strand_base = g->strand_base;
     a.cache = g->cache;
     a.strands = g->strand_total;
-    int blocks = blocks_for(ctx, (const void*)generate_kernel, kRasterThreads, g->strand_total, 2 * kRasterWarps);
+    // Few strands: a warp each, as the second of a pair only lengthens the pass.
+    // hg_generate by itself, us, pairs against single strands: 64 strands 11.5
+    // against 10.0, 600 11.5 against 10.1, 1,200 11.5 against 11.1, 2,000 12.0
+    // against 12.2, 4,864 10.5 against 12.6 back to back.
+    a.per = g->strand_total <= (uint32_t)ctx->sm_count * 8u ? 1u : 2u;
+    int blocks = blocks_for(ctx, (const void*)generate_kernel, kRasterThreads, g->strand_total, a.per * kRasterWarps);
     generate_kernel<<<blocks, kRasterThreads, 0, ctx->stream>>>(a);
     return cudaGetLastError();
 }

@@ -195,6 +195,13 @@ def test_strand_cache_equals_strands_generated_in_the_raster(renderer, n):
     assert (got[0][1] != EMPTY).any()
 
 
+@pytest.mark.parametrize("n", [1216, 1217, 1219])
+def test_strand_cache_at_the_line_of_single_strands(renderer, n):
+    """Up to sm_count x 8 strands (1,216 on 152 SMs) a warp takes one strand,
+    above a pair, the last one cut short at an odd count."""
+    test_strand_cache_equals_strands_generated_in_the_raster(renderer, n)
+
+
 @pytest.mark.parametrize("n", [1, 3, 32, 9728, 9729, 9731, 20_000])
 def test_lod_of_many_bundles_matches_the_oracle(renderer, n):
     """Four bundles share a warp from sm_count x 64 bundles up (9,728 on 152
