@@ -14,9 +14,12 @@ namespace {
 constexpr int kFilterRadius = 5;
 
 // Images of at most this many pixels give a pair four threads, or two.
-// Measured (us): 96 x 64: 10.3 with four, 14.4 with two, 16.5 with one;
-// 640 x 360: 20.6, 26.2, 20.8; 512 x 512: 30.8, 28.7 (64 registers), 33.0;
-// 960 x 540: 33.4, 29.0, 32.7; 1280 x 720: 51.1, 45.1, 36.6.
+// Measured (us): 96 x 64: 11.0 with four, 14.8 with two, 16.9 with one;
+// 400 x 300: 17.1, 23.2, 23.6; 640 x 360: 23.7, 23.8, 23.7; 512 x 512: 33.3,
+// 30.5, 35.8; 800 x 600: 43.8, 35.7, 37.5; 960 x 540: 38.4, 35.5, 36.4;
+// 1280 x 720: 60.6, 50.2, 47.7.  Two threads take three blocks an SM (80
+// registers): at four, with spills, 700 x 400 29.8 us instead of 23.9, 800 x 600
+// 40.6 instead of 35.7, though 960 x 540 31.9 instead of 35.5.
 constexpr uint64_t kFilterSplit4 = 240u * 1024u, kFilterSplit2 = 512u * 1024u;
 
 struct FilterArgs {
@@ -587,7 +590,7 @@ cudaError_t launch_filter_kind(hg_ctx* ctx, const FilterArgs& a) {
     };
     const uint64_t px = (uint64_t)ctx->width * ctx->height;
     if (px <= kFilterSplit4) filter_kernel<16, 8, 4, 3, KIND><<<tiles(16, 8), 256, 0, ctx->stream>>>(a);
-    else if (px <= kFilterSplit2) filter_kernel<32, 8, 2, 4, KIND><<<tiles(32, 8), 256, 0, ctx->stream>>>(a);
+    else if (px <= kFilterSplit2) filter_kernel<32, 8, 2, 3, KIND><<<tiles(32, 8), 256, 0, ctx->stream>>>(a);
     else filter_kernel<16, 16, 1, 6, KIND><<<tiles(16, 16), 128, 0, ctx->stream>>>(a);
     return cudaGetLastError();
 }
