@@ -355,6 +355,21 @@ def pass_bytes(sc, seg_refs: dict) -> dict:
     }
 
 
+def frame_launches(strands: int, map_w: int, map_h: int, sm_count: int) -> int:
+    """Kernels that hg_groom_frame launches with a deep opacity map (0 x 0: without),
+    the Karis shading, the filter, and composite onto a cleared target."""
+    # lod, scan offsets and expansion (of both views), clears; shade; filter with colour clear and composite
+    n = 4 + 1 + 1
+    # camera raster: one stage while its warps take at most two strands each
+    # (24 an SM), else two with the tile depths between them
+    n += 1 if strands <= 48 * sm_count else 3
+    if map_w:
+        texels = map_w * map_h
+        plane = strands >= 32768 and 512 * 512 < texels <= 64 * strands
+        n += 1 + 2 + plane  # strand cache, DOM depth, layers and their front plane
+    return n
+
+
 BATCH_WORKLOAD = ("config4: 64 seeded grooms of uneven size (1k-50k strands, 16-128 segments, mixed straight/wavy/"
                   "curly), each with its own square camera view (side 256-1024) and 512^2 x16 deep opacity map, "
                   "one launch per pass over all items, replayed as one CUDA graph")
@@ -742,11 +757,8 @@ def run_ours(args, rank, world, local):
     r.copy_wait()
     e2e_total = time.perf_counter() - t_s
     e2e_value, e2e_ms, _ = aggregate(dist, e2e_total * 1e3, float(seg_c) * args.steps)
-    # per frame: generate, lod, scan offsets and expand of both views, clear of both
-    # targets, camera raster (direct, the default: 2 stages + tile depths between
-    # them), 2 x DOM raster (and, from 32,768 strands up, the front plane of the
-    # layers pass), shade, filter with colour clear and composite
-    launches = (11 + (sc.mesh.strand_count() >= 32_768)) * args.steps
+    launches = frame_launches(sc.mesh.strand_count(), *sc.dom_size,
+                              torch.cuda.get_device_properties(local).multi_processor_count) * args.steps
 
     cpu = None
     if rank == 0 and not args.no_cpu_baseline:

@@ -734,11 +734,11 @@ hg_status hg_hair_visibility(hg_ctx* ctx, const hg_shadow_light* light, const fl
 // the deep-opacity rasters on the side stream.  They join before shading.
 // Work before and after the frame stays ordered on the main stream.
 // Frame, us, with the setup on one stream per view and a launch per pass and
-// target (18 launches) -> so (11): 96 x 64 thumbnail 92 -> 76, 512 x 512
+// target (18 launches) -> so (12): 96 x 64 thumbnail 92 -> 76, 512 x 512
 // 210 -> 192, 1920 x 1080 1134 -> 1089, 3840 x 2160 2426 -> 2251.  (A small
 // groom's single camera stage takes two launches fewer, 76 -> 69 us, and its
-// scan makes no draw order, 69 -> 62; a large
-// groom's front plane one more.)  The clears on the side stream behind the
+// scan makes no draw order, 69 -> 62; the front plane of a large groom's large
+// map one more.)  The clears on the side stream behind the
 // scan: 2 to 5 us slower at every size.
 hg_status hg_groom_frame(hg_ctx* ctx, hg_groom* g, const hg_frame_desc* d) {
     if (!ctx || !g || !d || !d->camera) return HG_INVALID_ARG;
