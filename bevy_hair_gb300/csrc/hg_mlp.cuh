@@ -186,14 +186,14 @@ __device__ __forceinline__ uint32_t pack_relu(float lo, float hi) {
 }
 
 // One layer: acc[mt][nt] = bias + A[mt] * W^T for N = 8*NT outputs, K = 16*KT
-// inputs; bias may be null (zero).  Four B fragments per ldmatrix.
+// inputs.  Four B fragments per ldmatrix.
 template <int NT, int KT, int PAD>
 __device__ __forceinline__ void layer_ldsm(float acc[2][NT][4], const uint32_t a[2][KT][4], const __half (*w)[PAD],
                                            const float* bias, int lane) {
     const int t = lane & 3, mat = lane >> 3, r = lane & 7;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-        const float bl = bias ? bias[nt * 8 + 2 * t] : 0.0f, bh = bias ? bias[nt * 8 + 2 * t + 1] : 0.0f;
+        const float bl = bias[nt * 8 + 2 * t], bh = bias[nt * 8 + 2 * t + 1];
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt) {
             acc[mt][nt][0] = bl;
