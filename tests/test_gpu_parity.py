@@ -600,6 +600,54 @@ def test_frame_equals_its_passes(renderer, deep_opacity, use_filter, composite, 
     g.close()
 
 
+@pytest.mark.parametrize("deep_opacity", [True, False])
+def test_frame_behind_scene_depth_equals_its_passes(renderer, deep_opacity):
+    """hg_groom_frame with a scene depth that hides some of the hair, with and
+    without a map, against the single passes."""
+    import torch
+
+    sc = configs.config1(scale=0.02)
+    sc.groom.deep_opacity = deep_opacity
+    w, h = 197, 131
+    sc.view = configs._camera(w, h, 1000.0)
+    cam, dom = sc.params()
+    lights = sc.light_array()
+    r = renderer
+    r.ensure_targets(w, h, *sc.dom_size)
+    g = r.upload(sc.mesh)
+    names = ["CENTER", "CONSERVATIVE", "BETA", "SHADED", "FILTERED", "COLOR", "DEPTH"]
+    scene = torch.from_numpy(np.random.default_rng(8).random(w * h).astype(np.float32) * np.float32(2e-4)).cuda()
+    torch.cuda.synchronize()
+
+    def outputs():
+        assert r.synchronize() == 0
+        return {n: r.read(getattr(abi, "BUF_" + n)).copy() for n in names}
+
+    r.clear()
+    r.clear_color(0.0)
+    for p, slot in ((cam, abi.SLOT_CAMERA), (dom, abi.SLOT_DOM))[:1 + deep_opacity]:
+        r.lod(g, p, slot)
+        r.scan(g, p, slot)
+    if deep_opacity:
+        r.generate(g, cam)
+        r.clear_dom()
+        r.raster(g, dom, abi.SLOT_DOM)
+        r.raster(g, host.dom_layers_params(dom), abi.SLOT_DOM)
+    r.raster(g, cam, abi.SLOT_CAMERA, scene.data_ptr())
+    r.shade(cam, lights)
+    r.filter(cam)
+    r.composite(cam, True)
+    want = outputs()
+    r.render_groom(g, cam, dom if deep_opacity else None, lights)
+    open_view = outputs()
+    r.render_groom(g, cam, dom if deep_opacity else None, lights, scene_depth_ptr=scene.data_ptr())
+    got = outputs()
+    for n in names:
+        _assert_equal(n, got[n].view(np.uint32), want[n].view(np.uint32))
+    assert 0 < (got["CENTER"] != EMPTY).sum() < (open_view["CENTER"] != EMPTY).sum()
+    g.close()
+
+
 def test_light_kinds(renderer):
     """Point, spot, directional (DOM) and rect lights, given out of kind order."""
     sc = configs.config1(scale=0.05)
