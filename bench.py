@@ -377,11 +377,14 @@ BATCH_WORKLOAD = ("config4: 64 seeded grooms of uneven size (1k-50k strands, 16-
 
 def batch_measure(r, stream, flush, steps: int, warmup: int, scale: float) -> dict:
     """The config-4 batched frame: graph replay against direct batched
-    launches and against hg_groom_frame per groom, with the autotuner's table."""
+    launches, against hg_groom_frame per groom (what a program without the
+    batch calls: a context of its own for every groom's targets, one stream)
+    and against the single passes groom by groom (HG_BATCH_SEPARATE), with the
+    autotuner's table."""
     import torch
 
     from bevy_hair_gb300 import abi, configs
-    from bevy_hair_gb300.pipeline import HairBatch
+    from bevy_hair_gb300.pipeline import HairBatch, HairRenderer
 
     t_bake = time.perf_counter()
     bs = configs.config4(scale)
@@ -401,23 +404,34 @@ def batch_measure(r, stream, flush, steps: int, warmup: int, scale: float) -> di
         segs += configs.segments_of(g.read(abi.SLOT_CAMERA, abi.GBUF_REFS), total)
     tuning = b.tune(lights)
 
-    def timed(mode: int, n: int) -> float:
+    def timed(draw, n: int) -> float:
         for _ in range(warmup):
             flush.fill_(7)
-            b.frame(lights, mode)
+            draw()
         torch.cuda.synchronize()
         ev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(n)]
         for i in range(n):
             flush.fill_(i & 0xFF)
             ev[i][0].record(stream)
-            b.frame(lights, mode)
+            draw()
             ev[i][1].record(stream)
         torch.cuda.synchronize()
         return float(np.mean([a.elapsed_time(z) for a, z in ev]))
 
-    graph_ms = timed(abi.BATCH_GRAPH, steps)
-    direct_ms = timed(abi.BATCH_LAUNCHES, max(3, steps // 2))
-    separate_ms = timed(abi.BATCH_SEPARATE, max(3, steps // 4))
+    graph_ms = timed(lambda: b.frame(lights, abi.BATCH_GRAPH), steps)
+    direct_ms = timed(lambda: b.frame(lights, abi.BATCH_LAUNCHES), max(3, steps // 2))
+    separate_ms = timed(lambda: b.frame(lights, abi.BATCH_SEPARATE), max(3, steps // 4))
+    views = [HairRenderer(torch.cuda.current_device(), stream.cuda_stream) for _ in grooms]
+    for v, size in zip(views, bs.sizes()):
+        v.ensure_targets(*size)
+
+    def groom_frames():
+        for v, g, (c, d) in zip(views, grooms, params):
+            v.render_groom(g, c, d, lights)
+
+    groom_frames_ms = timed(groom_frames, max(3, steps // 4))
+    for v in views:
+        v.close()
     phases = [b.profile(lights) for _ in range(3)]
     phase_ms = {k: round(float(np.mean([p[k] for p in phases])), 4) for k in phases[0]}
     # end to end: every item's uniforms from the host, the graph frame, and every
@@ -455,7 +469,10 @@ def batch_measure(r, stream, flush, steps: int, warmup: int, scale: float) -> di
         "items": len(grooms), "strands": sum(sc.mesh.strand_count() for sc in bs.scenes),
         "camera_pixels": int(sum(px)), "camera_refs": refs, "camera_segments": segs,
         "graph_ms": round(graph_ms, 4), "batched_launches_ms": round(direct_ms, 4),
+        "groom_frames_ms": round(groom_frames_ms, 4),
+        "speedup_vs_groom_frames": round(groom_frames_ms / graph_ms, 3),
         "separate_ms": round(separate_ms, 4), "speedup_vs_separate": round(separate_ms / graph_ms, 3),
+        "separate_note": "the single passes groom by groom, a launch per pass and view",
         "gseg_per_s": round(segs / (graph_ms * 1e-3) / 1e9, 4),
         "launches": {"graph": b.launches(abi.BATCH_GRAPH), "separate": b.launches(abi.BATCH_SEPARATE)},
         "phase_ms": phase_ms,
