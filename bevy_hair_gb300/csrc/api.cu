@@ -233,7 +233,10 @@ hg_status hg_create(int device, void* stream, hg_ctx** out) {
     if (e == cudaSuccess) e = cudaMalloc(&ctx->dual_table->table, sizeof(float4) * hg::kDualTableFloat4);
     constexpr size_t kStagedLights = (size_t)HG_MAX_LIGHTS * hg_ctx::kLightSlots;
     if (e == cudaSuccess) e = cudaMallocHost(&ctx->lights_host, sizeof(hg_light) * kStagedLights + sizeof(uint32_t));
-    if (e == cudaSuccess) ctx->err_host = reinterpret_cast<uint32_t*>(ctx->lights_host + kStagedLights);
+    if (e == cudaSuccess) {
+        ctx->skipped = reinterpret_cast<volatile uint32_t*>(ctx->lights_host + kStagedLights);
+        *ctx->skipped = 0u;
+    }
     for (int i = 0; i < hg_ctx::kLightSlots && e == cudaSuccess; ++i)
         e = cudaEventCreateWithFlags(&ctx->light_events[i], cudaEventDisableTiming);
     if (e != cudaSuccess) {
@@ -339,6 +342,7 @@ hg_status hg_synchronize(hg_ctx* ctx, uint32_t* device_error) {
     HG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     if (device_error) *device_error = word;
     if (word != 0) {
+        *ctx->skipped = 0u;
         HG_CUDA(ctx, cudaMemsetAsync(ctx->err, 0, sizeof(uint32_t), ctx->stream));
         return fail(ctx, word & 2u ? HG_DEVICE_TIMEOUT : HG_DEVICE_ERROR,
                     word & 2u ? "a tensor-core wait timed out" : "a kernel reported an invalid strand reference");

@@ -128,8 +128,10 @@ struct hg_ctx {
     // Pinned staging ring for the light list; slot k is reused only after
     // the event recorded behind its last copy has completed.
     static constexpr int kLightSlots = 8;
-    hg_light* lights_host = nullptr;  // kLightSlots * HG_MAX_LIGHTS, then err_host
-    uint32_t* err_host = nullptr;     // pinned copy of the error word, for calls that wait for the stream
+    hg_light* lights_host = nullptr;  // kLightSlots * HG_MAX_LIGHTS, then `skipped`
+    // Pinned, set by an Adam kernel that left its step out over a timeout;
+    // cleared when hg_synchronize reports the timeout.
+    volatile uint32_t* skipped = nullptr;
     cudaEvent_t light_events[kLightSlots] = {};
     int light_slot = 0;
     // Side stream and events for the frame's independent DOM half.

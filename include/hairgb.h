@@ -556,9 +556,9 @@ uint32_t hg_mlp_param_count(const hg_mlp* mlp);
 uint32_t hg_mlp_output_count(const hg_mlp* mlp);
 /* Host float[count], count == hg_mlp_param_count; resets the optimiser state. */
 hg_status hg_mlp_set_params(hg_mlp* mlp, const float* params, uint32_t count);
-/* Like hg_mlp_gradients, HG_DEVICE_TIMEOUT while the context has a timeout
- * that hg_synchronize has not reported: training steps since then were not
- * taken, and the parameters are those before them. */
+/* Like hg_mlp_gradients, HG_DEVICE_TIMEOUT when a timeout in the context that
+ * hg_synchronize has not reported yet kept training steps from being taken:
+ * the parameters are those before them. */
 hg_status hg_mlp_get_params(hg_mlp* mlp, float* params, uint32_t count);
 /* Training samples with FP64 lobes (Gauss-Legendre integration of the
  * Marschner/d'Eon azimuthal scattering, Zinke back-scattering) at the
