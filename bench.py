@@ -715,9 +715,10 @@ def run_ours(args, rank, world, local):
     peak, peak_kind = peaks()
     achieved = nbytes[dominant] / (acc[dominant] * 1e-3) / 1e9
     traffic, traffic_src = None, None
-    try:  # DRAM bytes of the pass (its launches summed) from the committed ncu capture of this workload
+    try:  # DRAM bytes of the pass (its launches summed) from the committed ncu capture, if it is of this workload
         tj = json.loads((ROOT / "profiles" / "traffic.json").read_text())
-        traffic, traffic_src = tj["per_pass"][dominant]["dram_bytes"], tj["profile"]
+        if tj["config"] == args.config and args.scale == 1.0:
+            traffic, traffic_src = tj["per_pass"][dominant]["dram_bytes"], tj["profile"]
     except (OSError, KeyError, ValueError):
         pass
     per_pass_roofline = {
@@ -834,6 +835,8 @@ def run_ours(args, rank, world, local):
                    "lights": int(len(lights)), "l2": "flushed between timed steps (256 MB device write)",
                    "parallelism": f"replicas x{world}"},
         "per_pass_ms": per_pass,
+        "per_pass_note": "the single passes called one by one; the frame merges the clears, lod and scan of both views, "
+                         "and the filter with the colour clear and composite",
         "camera_raster_kinds": camera_kinds,
         "per_pass_roofline": per_pass_roofline,
         "roofline": roofline,
