@@ -236,9 +236,9 @@ __device__ __forceinline__ void accumulate(bool keep, float4 tap, float w, Filte
 // the groups, so that an image's colours do not depend on S (a batch takes
 // one thread a pair for views of any size).  Coverage
 // decisions use exact arithmetic; the colour weights only scale colour, so
-// they use fused operations and the fast exponential.  Against a thread per pixel with 121 tests and a
-// distance each (us): 1920 x 1080 113 -> 79, 3840 x 2160 200 -> 141, 512 x 512
-// 42 -> 29, 96 x 64 22 -> 10.
+// they use fused operations and the fast exponential.  Against a thread per
+// pixel with 121 tests and a distance each (us): 1920 x 1080 113 -> 94,
+// 3840 x 2160 200 -> 166, 512 x 512 42 -> 32, 96 x 64 22 -> 11.
 template <int TX, int TY, int S, CompositeKind KIND, class V>
 __device__ __forceinline__ void filter_tile(const V& a, int32_t bx, int32_t by, float depth_clear) {
     constexpr int kHaloX = TX + 2 * kFilterRadius, kHaloY = TY + 2 * kFilterRadius;
@@ -519,8 +519,8 @@ __device__ __forceinline__ uint32_t tile_view(const uint32_t* __restrict__ prefi
     return lo;
 }
 
-// Five blocks per SM (96 registers): 675 us on 24 grooms of the batch benchmark,
-// six (80) 690, eight (64, spilled) 688.
+// Five blocks per SM (96 registers): 744 us on 24 grooms of the batch benchmark;
+// six (80) 8 us more, eight (64, spilled) 47 more.
 template <int TX, int TY>
 __global__ void __launch_bounds__(TX* TY / 2, 5) batch_filter_kernel(const BatchView* __restrict__ views,
                                                              const uint32_t* __restrict__ prefix, uint32_t n_cam,

@@ -1,8 +1,9 @@
 // Learned shading surrogate: FP64 training samples of the hair lobes, the
-// FP16 tensor-core networks' inference and training kernels (4 x 64 and compact
-// 2 x 32: forward, backward and weight gradients of a 128-sample tile per
-// block on mma.sync, partial gradients summed by the Adam kernel), and their
-// C entry points.  The reference has no counterpart; the shading it replaces is the
+// FP16 tensor-core networks' inference and training kernels (forward and
+// backward of a 128-sample tile per block on mma.sync; weight gradients in the
+// same block for the compact 2 x 32 network, in a kernel of their own for the
+// 4 x 64 one; partial gradients summed by the Adam kernel), and their C entry
+// points.  The reference has no counterpart; the shading it replaces is the
 // Karis fit of shade.wesl:94-190.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
