@@ -229,14 +229,15 @@ __device__ __forceinline__ void accumulate(bool keep, float4 tap, float w, Filte
 // The tap loop is bound by instruction issue and shared-memory bandwidth.  A
 // pair shares its taps' loads (12 rows for 2 x 11); the strip counts come from
 // bit masks (strip_row), row by row, instead of a distance and two tests per
-// tap; the spatial exponent takes three operations a tap (spatial_form); and the depth test alone also rejects the texels without a
-// centre hit.  S threads (1, 2 or 4) share a pair, 12 / S rows each: small
-// images leave the chip idle otherwise.  However many share it, each group of
-// three rows is summed by itself and the four sums are added in the order of
-// the groups, so that an image's colours do not depend on S (a batch takes
-// one thread a pair for views of any size).  Coverage
-// decisions use exact arithmetic; the colour weights only scale colour, so
-// they use fused operations and the fast exponential.  Against a thread per
+// tap; the spatial exponent takes three operations a tap (spatial_form); and
+// the depth test alone also rejects the texels without a centre hit.  S threads
+// (1, 2 or 4) share a pair, 12 / S rows each: small images leave the chip idle
+// otherwise.  However many share it, each group of three rows is summed by
+// itself and the four sums are added in the order of the groups, so that an
+// image's colours do not depend on S (a batch takes one thread a pair for views
+// of any size).  Coverage decisions use exact arithmetic; the colour weights
+// only scale colour, so they use fused operations and the fast exponential
+// (ex2).  Against a thread per
 // pixel with 121 tests and a distance each (us): 1920 x 1080 113 -> 94,
 // 3840 x 2160 200 -> 166, 512 x 512 42 -> 32, 96 x 64 22 -> 11.
 template <int TX, int TY, int S, CompositeKind KIND, class V>
